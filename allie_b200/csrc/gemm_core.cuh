@@ -23,8 +23,9 @@ struct GemmArgs {
   int M, N, K;
   int k_splits;
   int pdl;            // launched as a programmatic dependent: B (weights) may be fetched before griddep_wait
-  int aux_tma;        // act == 2 in the CTA-pair kernel: the aux tile of an epilogue warp arrives by TMA in
-                      // the warp's staging tile (tmAux is a load map) instead of by row loads
+  int aux_tma;        // CTA-pair kernel: a second epilogue operand arrives by TMA in the warp's staging tile
+                      // (tmAux is a load map) instead of by row loads.  1: the aux tile of act == 2,
+                      // 64 bf16 columns; 2: the residual, 32 fp32 columns at a time
   AbGemmEpilogue ep;
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into ep.drop_seed when not null
   int* status;
@@ -36,7 +37,9 @@ struct GemmArgs {
 // `bias_off` shifts the bias vector (grouped GEMMs: one bias row per group).
 __device__ __forceinline__ void epilogue_math8(const GemmArgs& g, float* v, uint4& pre, int m, int n,
                                                bool ok, bool add_bias, int bias_off = 0,
-                                               const uint4* aux_staged = nullptr) {
+                                               const uint4* aux_staged = nullptr,
+                                               const float4* resid_staged0 = nullptr,
+                                               const float4* resid_staged1 = nullptr) {
   const AbGemmEpilogue& ep = g.ep;
   if (ep.alpha != 1.f) {
 #pragma unroll
@@ -87,8 +90,13 @@ __device__ __forceinline__ void epilogue_math8(const GemmArgs& g, float* v, uint
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = ((keep >> j) & 1u) ? v[j] * s : 0.f;
     }
-    const float4 r0 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n);
-    const float4 r1 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n + 4);
+    float4 r0, r1;       // from the staged tile in shared memory, or straight from global
+    if (resid_staged0) {
+      r0 = *resid_staged0; r1 = *resid_staged1;
+    } else {
+      r0 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n);
+      r1 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n + 4);
+    }
     v[0] += r0.x; v[1] += r0.y; v[2] += r0.z; v[3] += r0.w;
     v[4] += r1.x; v[5] += r1.y; v[6] += r1.z; v[7] += r1.w;
   }
@@ -143,6 +151,51 @@ __device__ __forceinline__ void epilogue_drain(const GemmArgs& g, const CUtensor
       tma_store_commit();
     }
   }
+}
+
+// Drain of a fp32 output with a residual whose tiles travel by TMA (CTA-pair kernel).  A lane owns a
+// row, so residual loads straight from global touch 32 rows per instruction and keep the load unit
+// busy for longer than the tensor core needs for K <= 1024; here the 32 x 32 residual tile of a
+// column group lies in the warp's staging tile, in the layout of the output tile, and each lane
+// replaces its values by the results before the tile leaves.  `wait_tile()` returns false when the
+// wait for the current group's tile ran out; `next_tile(g)` is called once that group has been
+// stored and the staging tile is free again.
+template <int COLS, typename Wait, typename Next>
+__device__ __forceinline__ bool epilogue_drain_resid(const GemmArgs& g, const CUtensorMap& tmOut, uint32_t taddr,
+                                                     int m, int m0w, int nbase, bool row_ok, uint8_t* stg, int lane,
+                                                     Wait wait_tile, Next next_tile) {
+  uint8_t* rowp = stg + lane * 128;        // 32 fp32 columns = 128-byte rows, 128B swizzle
+  const int sw = lane & 7;
+#pragma unroll 1
+  for (int grp = 0; grp < COLS / 32; ++grp) {
+    const int gn0 = nbase + grp * 32;
+    if (gn0 >= g.N) break;                 // warp-uniform
+    uint32_t r[32];
+    tmem_ld32(taddr + grp * 32, r);
+    if (!wait_tile()) return false;
+    tmem_ld_wait();
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[c * 4 + j]);
+      float4* s0 = reinterpret_cast<float4*>(rowp + ((c ^ sw) << 4));
+      float4* s1 = reinterpret_cast<float4*>(rowp + (((c + 1) ^ sw) << 4));
+      uint4 pre;
+      epilogue_math8(g, v, pre, m, gn0 + c * 4, row_ok && gn0 + c * 4 < g.N, true, 0, nullptr, s0, s1);
+      *s0 = make_float4(v[0], v[1], v[2], v[3]);
+      *s1 = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(&tmOut, stg, gn0, m0w);
+      tma_store_commit();
+      tma_store_wait_read<0>();            // the store has read the staging tile
+      next_tile(grp);
+    }
+  }
+  return true;
 }
 
 // Drain used by the CTA-pair kernel: the same per-round math, but several 16-column rounds are

@@ -478,23 +478,25 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     constexpr int COLS_PER_WARP = BN / 4;
     uint8_t* my_stage = stage_out + e * PAIR_WARP_STAGING;
     uint32_t acc_phase[2] = {0, 0};
-    // GELU backward (act == 2): the warp's 32 x 64 tile of aux values is fetched by TMA into its
+    // GELU backward (aux_tma == 1): the warp's 32 x 64 tile of aux values is fetched by TMA into its
     // staging tile one unit ahead (right after the store of the unit before has read the tile), so
     // the loads that the epilogue math depends on are in flight while the accumulator is still
-    // being computed instead of being issued, row by row, once it is ready.
+    // being computed instead of being issued, row by row, once it is ready.  Residual outputs
+    // (aux_tma == 2) do the same with 32 x 32 fp32 tiles: the second of a unit's two tiles follows
+    // when the first has left, the next unit's first one unit ahead.
     static_assert(COLS_PER_WARP == 64, "the staged aux tile is one 64-column store group");
     const bool stage_aux = g.aux_tma != 0;
     uint32_t aux_phase = 0;
-    auto fetch_aux = [&](int u) {          // lane 0; the staging tile must be free
+    auto fetch_aux = [&](int u, int grp) {          // lane 0; the staging tile must be free
       if (u >= num_units) return;
       const int tile = u % num_tiles;
       const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
-      const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
-      if (m0w >= g.M || nbase >= g.N) return;       // the same test skips the drain below
+      const int n = (tile % n_tiles) * BN + part * COLS_PER_WARP + grp * 32;
+      if (m0w >= g.M || n >= g.N) return;           // the same test skips the drain below
       mbar_expect_tx(&aux_bar[e], 32 * 128);
-      tma_load_2d(my_stage, &tmAux, &aux_bar[e], nbase, m0w);
+      tma_load_2d(my_stage, &tmAux, &aux_bar[e], n, m0w);
     };
-    if (stage_aux && lane == 0) fetch_aux(pair_id);
+    if (stage_aux && lane == 0) fetch_aux(pair_id, 0);
     int it = 0;
     for (int u = pair_id; u < num_units; u += num_pairs, ++it) {
       const int ks = u / num_tiles;
@@ -516,25 +518,39 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
       const bool staged = stage_aux && m0w < g.M && nbase < g.N;
-      if (staged) {
+      auto wait_aux = [&]() {
         if (!mbar_wait(&aux_bar[e], aux_phase, abort_flag)) {
           *abort_flag = ST_TIMEOUT_FULL;
           atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
-          break;
+          return false;
         }
         aux_phase ^= 1;
+        return true;
+      };
+      if (g.aux_tma == 2) {
+        // past the last column group of this unit: the first tile of the next one
+        auto next_tile = [&](int grp) {
+          if (grp + 1 < COLS_PER_WARP / 32 && nbase + (grp + 1) * 32 < g.N) fetch_aux(u, grp + 1);
+          else fetch_aux(u + num_pairs, 0);
+        };
+        if (staged && !epilogue_drain_resid<COLS_PER_WARP>(g, tmOut, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
+                                                           wait_aux, next_tile))
+          break;
+        if (!staged && lane == 0) fetch_aux(u + num_pairs, 0);
+      } else {
+        if (staged && !wait_aux()) break;
+        // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
+        // from zero-filled loads); it still hands the buffer back
+        if (m0w < g.M)
+          epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
+                                             ks == 0, 0, staged);
       }
-      // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
-      // from zero-filled loads); it still hands the buffer back
-      if (m0w < g.M)
-        epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
-                                           ks == 0, 0, staged);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
-      if (stage_aux && lane == 0) {
+      if (g.aux_tma == 1 && lane == 0) {
         tma_store_wait_read<0>();           // the store just issued has read the staging tile
-        fetch_aux(u + num_pairs);
+        fetch_aux(u + num_pairs, 0);
       }
     }
     if (lane == 0) tma_store_wait<0>();
@@ -579,6 +595,12 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
     rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 64, 2, 128);
     if (rc) return rc;
     ga.aux_tma = 1;
+  } else if (ep.resid && ep.out_fp32 && !ep.accumulate && ep.act == 0 && g.k_splits == 1 &&
+             (reinterpret_cast<uintptr_t>(ep.resid) & 15) == 0 && (ep.ldr & 3) == 0) {
+    // residual tiles likewise, in the geometry of the fp32 output tiles
+    rc = make_tmap_2d_sw(&tmAux, ep.resid, g.M, g.N, ep.ldr, 32, 32, 4, 128);
+    if (rc) return rc;
+    ga.aux_tma = 2;
   } else {
     tmAux = tmOut;
   }

@@ -182,3 +182,34 @@ def test_gemm_gelu_derivative_kept_in_aux():
     assert torch.allclose(dact.float(), want_d, rtol=1e-2, atol=1e-2), (dact.float() - want_d).abs().max().item()
     want = (dy.float() @ w2.float().t()) * want_d
     assert torch.allclose(dpre.float(), want, rtol=3e-2, atol=3e-2), (dpre.float() - want).abs().max().item()
+
+
+@pytest.mark.parametrize("drop_p", [0.0, 0.1])
+@pytest.mark.parametrize("M,N,K", [(512, 256, 64),      # one tile per pair, both column groups of every warp
+                                   (520, 264, 72),      # rows past a tile, eight columns in the last tile
+                                   (1100, 800, 256),    # last column tile ends inside a warp's first group
+                                   (20000, 512, 128)])  # several units per pair: tiles fetched one unit ahead
+def test_gemm_pair_residual_tiles(M, N, K, drop_p):
+    """CTA-pair kernel with a fp32 residual: its tiles travel by TMA through the output staging tile."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(4)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(K, N, device="cuda") * 0.05).bfloat16()
+    bias, resid = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda")
+    kw = dict(b_mn=True, bias=bias, drop_p=drop_p, drop_seed=11, drop_stream=3)
+    out = torch.full((M, N), float("nan"), device="cuda")
+    gemm(a, w, out=out, resid=resid, **kw)
+    masked = gemm(a, w, out=torch.empty_like(out), resid=torch.zeros_like(resid), **kw)
+    inplace = resid.clone()
+    gemm(a, w, out=inplace, resid=inplace, **kw)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    # the same accumulators and mask: only the last addition of the residual rounds differently (half
+    # an ulp of values below 16)
+    assert torch.equal(out, inplace)
+    assert torch.allclose(out, masked + resid, rtol=0, atol=2e-6)
+    if drop_p == 0:
+        ref = a.float() @ w.float() + bias + resid
+        assert torch.allclose(out, ref, rtol=1e-4, atol=1e-4 * K ** 0.5)
