@@ -37,9 +37,7 @@ struct GemmArgs {
 // `bias_off` shifts the bias vector (grouped GEMMs: one bias row per group).
 __device__ __forceinline__ void epilogue_math8(const GemmArgs& g, float* v, uint4& pre, int m, int n,
                                                bool ok, bool add_bias, int bias_off = 0,
-                                               const uint4* aux_staged = nullptr,
-                                               const float4* resid_staged0 = nullptr,
-                                               const float4* resid_staged1 = nullptr) {
+                                               const uint4* aux_staged = nullptr) {
   const AbGemmEpilogue& ep = g.ep;
   if (ep.alpha != 1.f) {
 #pragma unroll
@@ -90,13 +88,8 @@ __device__ __forceinline__ void epilogue_math8(const GemmArgs& g, float* v, uint
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = ((keep >> j) & 1u) ? v[j] * s : 0.f;
     }
-    float4 r0, r1;       // from the staged tile in shared memory, or straight from global
-    if (resid_staged0) {
-      r0 = *resid_staged0; r1 = *resid_staged1;
-    } else {
-      r0 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n);
-      r1 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n + 4);
-    }
+    const float4 r0 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n);
+    const float4 r1 = *reinterpret_cast<const float4*>(ep.resid + (long long)m * ep.ldr + n + 4);
     v[0] += r0.x; v[1] += r0.y; v[2] += r0.z; v[3] += r0.w;
     v[4] += r1.x; v[5] += r1.y; v[6] += r1.z; v[7] += r1.w;
   }
@@ -153,52 +146,230 @@ __device__ __forceinline__ void epilogue_drain(const GemmArgs& g, const CUtensor
   }
 }
 
-// Drain of a fp32 output with a residual whose tiles travel by TMA (CTA-pair kernel).  A lane owns a
-// row, so residual loads straight from global touch 32 rows per instruction and keep the load unit
-// busy for longer than the tensor core needs for K <= 1024; here the 32 x 32 residual tile of a
-// column group lies in the warp's staging tile, in the layout of the output tile, and each lane
-// replaces its values by the results before the tile leaves.  `wait_tile()` returns false when the
-// wait for the current group's tile ran out; `next_tile(g)` is called once that group has been
-// stored and the staging tile is free again.
-template <int COLS, typename Wait, typename Next>
-__device__ __forceinline__ bool epilogue_drain_resid(const GemmArgs& g, const CUtensorMap& tmOut, uint32_t taddr,
-                                                     int m, int m0w, int nbase, bool row_ok, uint8_t* stg, int lane,
-                                                     Wait wait_tile, Next next_tile) {
-  uint8_t* rowp = stg + lane * 128;        // 32 fp32 columns = 128-byte rows, 128B swizzle
-  const int sw = lane & 7;
-#pragma unroll 1
-  for (int grp = 0; grp < COLS / 32; ++grp) {
-    const int gn0 = nbase + grp * 32;
-    if (gn0 >= g.N) break;                 // warp-uniform
-    uint32_t r[32];
-    tmem_ld32(taddr + grp * 32, r);
-    if (!wait_tile()) return false;
-    tmem_ld_wait();
+// ------------------------------------------------------------------------------------------
+// Specialised drains of the CTA-pair kernels.  The general routine below decides per eight columns
+// what an output needs; at 256 x 256 tiles and K = 1024 its branches cost as many issue slots as
+// the tensor core leaves (32768 x 4096 x 1024, bf16 output: 227 us against 191 us with the stores
+// and the math taken out).  The kernels of the training and inference schedule therefore know at
+// compile time which of these they are; everything else takes EPI_ANY.
+enum EpiKind : int {
+  EPI_ANY = 0,
+  EPI_BF16,        // bf16 out (+ bias)
+  EPI_GELU,        // bf16 out = gelu(. + bias), nothing kept
+  EPI_GELU_GRAD,   // bf16 out = gelu(. + bias), second bf16 output = gelu'
+  EPI_MUL,         // bf16 out = . * aux tile (aux_grad), aux staged by TMA
+  EPI_RESID,       // fp32 out = dropout(. + bias) + residual, residual staged by TMA
+  EPI_ACCUM,       // fp32 out += .
+};
+
+// which specialised drain an epilogue description fits (aux_tma as chosen by the launcher)
+inline EpiKind epi_kind(const GemmArgs& g) {
+  const AbGemmEpilogue& ep = g.ep;
+  if (ep.alpha != 1.f) return EPI_ANY;
+  if (ep.accumulate) return (!ep.bias && !ep.act && !ep.resid) ? EPI_ACCUM : EPI_ANY;
+  if (ep.resid) return g.aux_tma == 2 ? EPI_RESID : EPI_ANY;
+  if (ep.out_fp32) return EPI_ANY;
+  if (ep.act == 0) return EPI_BF16;
+  if (ep.act == 3) return EPI_GELU;
+  if (ep.act == 1 && ep.aux_grad) return EPI_GELU_GRAD;
+  if (ep.act == 2 && ep.aux_grad && g.aux_tma == 1 && !ep.bias) return EPI_MUL;
+  return EPI_ANY;
+}
+
+// eight accumulators (+ bias) as four packed pairs; `n` and `has` are warp-uniform
+__device__ __forceinline__ void epi_load8(const uint32_t* r, uint64_t* v, const float* bias, int n, bool has) {
 #pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-      float v[8];
+  for (int j = 0; j < 4; ++j) v[j] = f2_pack(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+  if (has) {
+    const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias + n));
+    const float4 b1 = __ldg(reinterpret_cast<const float4*>(bias + n + 4));
+    v[0] = f2_add(v[0], f2_pack(b0.x, b0.y)); v[1] = f2_add(v[1], f2_pack(b0.z, b0.w));
+    v[2] = f2_add(v[2], f2_pack(b1.x, b1.y)); v[3] = f2_add(v[3], f2_pack(b1.z, b1.w));
+  }
+}
+__device__ __forceinline__ uint4 epi_pack8(const uint64_t* v) {
+  return make_uint4(f2_to_bf16x2(v[0]), f2_to_bf16x2(v[1]), f2_to_bf16x2(v[2]), f2_to_bf16x2(v[3]));
+}
+
+// One epilogue warp drains its 32 rows x 64 columns.  Rows past the end of the output are clipped by
+// the TMA store; with MASK_ROWS (grouped kernels, whose regions are padded) rows with !row_ok are
+// written as zeros.  `wait_tile` / `next_tile`: see EPI_RESID.  Returns false when a wait ran out.
+template <int EPI, bool MASK_ROWS, typename Wait, typename Next>
+__device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUtensorMap& tmOut,
+                                                    const CUtensorMap& tmAux, uint32_t taddr, int m, int m0w,
+                                                    int nbase, bool row_ok, uint8_t* stg, int lane, int bias_off,
+                                                    Wait wait_tile, Next next_tile) {
+  const bool has_bias = g.ep.bias != nullptr;
+  const float* bias = g.ep.bias + bias_off;
+  if constexpr (EPI == EPI_BF16 || EPI == EPI_GELU || EPI == EPI_MUL) {
+    // one store group: 64 bf16 columns = 128-byte rows, 128B swizzle.  The aux tile of EPI_MUL
+    // lies in the staging tile already, in the same layout.
+    uint8_t* rowp = stg + lane * 128;
+    const int sw = lane & 7;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[c * 4 + j]);
-      float4* s0 = reinterpret_cast<float4*>(rowp + ((c ^ sw) << 4));
-      float4* s1 = reinterpret_cast<float4*>(rowp + (((c + 1) ^ sw) << 4));
-      uint4 pre;
-      epilogue_math8(g, v, pre, m, gn0 + c * 4, row_ok && gn0 + c * 4 < g.N, true, 0, nullptr, s0, s1);
-      *s0 = make_float4(v[0], v[1], v[2], v[3]);
-      *s1 = make_float4(v[4], v[5], v[6], v[7]);
+    for (int half = 0; half < 2; ++half) {
+      uint32_t r[32];
+      tmem_ld32(taddr + half * 32, r);
+      if (half == 0) {
+        if constexpr (EPI == EPI_MUL) {
+          if (!wait_tile()) return false;
+        } else {
+          if (lane == 0) tma_store_wait_read<0>();        // staging tile free again
+          __syncwarp();
+        }
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int n = nbase + half * 32 + c * 8;
+        uint64_t v[4];
+        epi_load8(r + c * 8, v, bias, n, EPI != EPI_MUL && has_bias && n < g.N);
+        uint4* chunk = reinterpret_cast<uint4*>(rowp + (((half * 4 + c) ^ sw) << 4));
+        if constexpr (EPI == EPI_GELU) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = f2_gelu_tanh(v[j]);
+        }
+        if constexpr (EPI == EPI_MUL) {
+          const uint4 q = *chunk;
+          v[0] = f2_mul(v[0], f2_pack(bf16_lo(q.x), bf16_hi(q.x)));
+          v[1] = f2_mul(v[1], f2_pack(bf16_lo(q.y), bf16_hi(q.y)));
+          v[2] = f2_mul(v[2], f2_pack(bf16_lo(q.z), bf16_hi(q.z)));
+          v[3] = f2_mul(v[3], f2_pack(bf16_lo(q.w), bf16_hi(q.w)));
+        }
+        uint4 o = epi_pack8(v);
+        if (MASK_ROWS && !row_ok) o = make_uint4(0, 0, 0, 0);
+        *chunk = o;
+      }
     }
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      tma_store_2d(&tmOut, stg, gn0, m0w);
+      tma_store_2d(&tmOut, stg, nbase, m0w);
       tma_store_commit();
-      tma_store_wait_read<0>();            // the store has read the staging tile
-      next_tile(grp);
+      if constexpr (EPI == EPI_MUL) {
+        tma_store_wait_read<0>();          // the store has read the staging tile
+        next_tile(0);
+      }
+    }
+  } else if constexpr (EPI == EPI_GELU_GRAD) {
+    // two bf16 outputs share the staging tile: 32 columns each = 64-byte rows, 64B swizzle
+    const int sw = (lane >> 1) & 3;
+#pragma unroll
+    for (int grp = 0; grp < 2; ++grp) {
+      const int gn0 = nbase + grp * 32;
+      if (gn0 >= g.N) break;               // warp-uniform
+      uint32_t r[32];
+      tmem_ld32(taddr + grp * 32, r);
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int n = gn0 + c * 8;
+        uint64_t v[4], d[4];
+        epi_load8(r + c * 8, v, bias, n, has_bias && n < g.N);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = f2_gelu_tanh_with_grad(v[j], d[j]);
+        uint4 o = epi_pack8(v), p = epi_pack8(d);
+        if (MASK_ROWS && !row_ok) { o = make_uint4(0, 0, 0, 0); p = o; }
+        uint8_t* dst = stg + lane * 64 + ((c ^ sw) << 4);
+        *reinterpret_cast<uint4*>(dst) = o;
+        *reinterpret_cast<uint4*>(dst + 2048) = p;
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmOut, stg, gn0, m0w);
+        tma_store_2d(&tmAux, stg + 2048, gn0, m0w);
+        tma_store_commit();
+      }
+    }
+  } else if constexpr (EPI == EPI_ACCUM) {
+    // 32 fp32 columns = 128-byte rows, 128B swizzle, added to the output by the TMA unit
+    uint8_t* rowp = stg + lane * 128;
+    const int sw = lane & 7;
+#pragma unroll
+    for (int grp = 0; grp < 2; ++grp) {
+      const int gn0 = nbase + grp * 32;
+      if (gn0 >= g.N) break;               // warp-uniform
+      uint32_t r[32];
+      tmem_ld32(taddr + grp * 32, r);
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = make_uint4(r[c * 4], r[c * 4 + 1], r[c * 4 + 2], r[c * 4 + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_reduce_add_2d(&tmOut, stg, gn0, m0w);
+        tma_store_commit();
+      }
+    }
+  } else {
+    static_assert(EPI == EPI_RESID, "no drain for this epilogue kind");
+    // fp32 output with a residual.  A lane owns a row, so residual loads straight from global would
+    // touch 32 rows per instruction and keep the load unit busy for longer than the tensor core
+    // needs at K <= 1024 (12136 x 768 x 768: 35.5 us; 27.9 us with the tiles by TMA).  The 32 x 32
+    // residual tile of a column group lies in the staging tile, in the layout of the output tile,
+    // and each lane replaces its values by the results before the tile leaves.  `wait_tile()` waits
+    // for the current group's tile; `next_tile(grp)` is called by lane 0 once group grp has been
+    // stored and the staging tile is free again.
+    uint8_t* rowp = stg + lane * 128;
+    const int sw = lane & 7;
+    const uint32_t thr16 = g.ep.drop_thr16;
+    const float s = dropout_scale(thr16);
+#pragma unroll 1
+    for (int grp = 0; grp < 2; ++grp) {
+      const int gn0 = nbase + grp * 32;
+      if (gn0 >= g.N) break;               // warp-uniform
+      uint32_t r[32];
+      tmem_ld32(taddr + grp * 32, r);
+      uint32_t keep = 0xffffffffu;         // does not depend on the accumulator: drawn under the load
+      if (thr16) {
+        const uint64_t seed = salted(g.ep.drop_seed, g.salt);
+        const uint64_t group0 = (static_cast<uint64_t>(m) * g.N + gn0) >> 3;
+        keep = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) keep |= dropout_keep8(seed, g.ep.drop_stream, group0 + c, thr16) << (8 * c);
+      }
+      if (!wait_tile()) return false;
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int n = gn0 + c * 8;
+        uint64_t v[4];
+        epi_load8(r + c * 8, v, bias, n, has_bias && n < g.N);
+        float4* s0 = reinterpret_cast<float4*>(rowp + (((2 * c) ^ sw) << 4));
+        float4* s1 = reinterpret_cast<float4*>(rowp + (((2 * c + 1) ^ sw) << 4));
+        const float4 r0 = *s0, r1 = *s1;
+        const uint64_t res[4] = {f2_pack(r0.x, r0.y), f2_pack(r0.z, r0.w), f2_pack(r1.x, r1.y), f2_pack(r1.z, r1.w)};
+        float o[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (thr16)
+            v[j] = f2_mul(v[j], f2_pack(((keep >> (c * 8 + 2 * j)) & 1u) ? s : 0.f,
+                                        ((keep >> (c * 8 + 2 * j + 1)) & 1u) ? s : 0.f));
+          f2_unpack(f2_add(v[j], res[j]), o[2 * j], o[2 * j + 1]);
+        }
+        *s0 = make_float4(o[0], o[1], o[2], o[3]);
+        *s1 = make_float4(o[4], o[5], o[6], o[7]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmOut, stg, gn0, m0w);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        next_tile(grp);
+      }
     }
   }
   return true;
 }
 
-// Drain used by the CTA-pair kernel: the same per-round math, but several 16-column rounds are
+// General drain of the CTA-pair kernels (EPI_ANY): the same per-round math as epilogue_drain, but several 16-column rounds are
 // staged side by side in one 4 KB tile per warp and leave in one TMA store with 128-byte rows
 // (64 bf16 or 32 fp32 columns; 64-byte rows when a second bf16 output shares the tile).  Wide
 // rows matter: the store path costs per row segment, not per byte.

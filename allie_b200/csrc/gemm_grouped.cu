@@ -279,7 +279,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase[2] = {0, 0};
+      uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
       int it = 0;
       bool ok = true;
       for (int u = pair_id; u < num_units && ok; u += num_pairs) {
@@ -288,7 +288,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         if (kb_total == 0) continue;
         const int ab = it & 1;
         ++it;
-        if (!mbar_wait(&tempty_bar[ab], acc_phase[ab] ^ 1, abort_flag)) {
+        if (!mbar_wait(&tempty_bar[ab], ((acc_phase >> ab) & 1) ^ 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_EMPTY;
           atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_EMPTY);
           break;
@@ -320,7 +320,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const uint32_t tb = smem_u32(&tfull_bar[ab]);
         umma_commit_pair(mapa_shared(tb, 0));
         umma_commit_pair(mapa_shared(tb, 1));
-        acc_phase[ab] ^= 1;
+        acc_phase ^= 1u << ab;
       }
     }
   } else {
@@ -330,7 +330,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     const int part = e >> 2;
     constexpr int COLS_PER_WARP = BN / 4;
     uint8_t* my_stage = stage_out + e * PAIR_WARP_STAGING;
-    uint32_t acc_phase[2] = {0, 0};
+    uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
     int it = 0;
     for (int u = pair_id; u < num_units; u += num_pairs) {
       int grp, mrow0, ncol0, kb_total;
@@ -341,12 +341,12 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const int mrow_w = mrow0 + rank * BM + quad * 32;        // first row of this warp, inside the group
       const int mrow = mrow_w + lane;
       const int nbase = ncol0 + part * COLS_PER_WARP;
-      if (!mbar_wait(&tfull_bar[ab], acc_phase[ab], abort_flag)) {
+      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         break;
       }
-      acc_phase[ab] ^= 1;
+      acc_phase ^= 1u << ab;
       tc_fence_after();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;

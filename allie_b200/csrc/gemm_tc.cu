@@ -202,7 +202,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase[2] = {0, 0};
+      uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
       int it = 0;
       bool ok = true;
       for (int u = blockIdx.x; u < num_units && ok; u += gridDim.x, ++it) {
@@ -211,7 +211,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         const int kb1 = min(kb_total, kb0 + kb_per);
         if (kb0 >= kb1) continue;
         const int ab = it & 1;
-        if (!mbar_wait(&tempty_bar[ab], acc_phase[ab] ^ 1, abort_flag)) {
+        if (!mbar_wait(&tempty_bar[ab], ((acc_phase >> ab) & 1) ^ 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_EMPTY;
           atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_EMPTY);
           break;
@@ -239,7 +239,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         }
         if (!ok) break;
         umma_commit(&tfull_bar[ab]);  // accumulator complete -> epilogue
-        acc_phase[ab] ^= 1;
+        acc_phase ^= 1u << ab;
       }
     }
   } else {
@@ -249,7 +249,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     const int part = e >> 2;             // which quarter of the BN columns
     constexpr int COLS_PER_WARP = BN / 4;
     uint8_t* my_stage = stage_out + e * 2048;
-    uint32_t acc_phase[2] = {0, 0};
+    uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
     int it = 0;
     for (int u = blockIdx.x; u < num_units; u += gridDim.x, ++it) {
       const int ks = u / num_tiles;
@@ -260,12 +260,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       const int ab = it & 1;
       const int m = (tile / n_tiles) * BM + quad * 32 + lane;
       const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
-      if (!mbar_wait(&tfull_bar[ab], acc_phase[ab], abort_flag)) {
+      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         break;
       }
-      acc_phase[ab] ^= 1;
+      acc_phase ^= 1u << ab;
       tc_fence_after();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
@@ -300,7 +300,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 //   tempty[b]  leader only, 2 x NUM_EPI_WARPS arrivals: the epilogue warps of both CTAs
 // Loads are plain unicast TMA loads whose completion is counted on the leader's barrier.
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
                               const __grid_constant__ CUtensorMap tmB,
@@ -426,7 +426,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase[2] = {0, 0};
+      uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
       int it = 0;
       bool ok = true;
       for (int u = pair_id; u < num_units && ok; u += num_pairs, ++it) {
@@ -435,7 +435,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const int kb1 = min(kb_total, kb0 + kb_per);
         if (kb0 >= kb1) continue;
         const int ab = it & 1;
-        if (!mbar_wait(&tempty_bar[ab], acc_phase[ab] ^ 1, abort_flag)) {
+        if (!mbar_wait(&tempty_bar[ab], ((acc_phase >> ab) & 1) ^ 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_EMPTY;
           atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_EMPTY);
           break;
@@ -467,7 +467,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const uint32_t tb = smem_u32(&tfull_bar[ab]);
         umma_commit_pair(mapa_shared(tb, 0));     // accumulator complete -> both epilogues
         umma_commit_pair(mapa_shared(tb, 1));
-        acc_phase[ab] ^= 1;
+        acc_phase ^= 1u << ab;
       }
     }
   } else {
@@ -477,7 +477,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     const int part = e >> 2;
     constexpr int COLS_PER_WARP = BN / 4;
     uint8_t* my_stage = stage_out + e * PAIR_WARP_STAGING;
-    uint32_t acc_phase[2] = {0, 0};
+    uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
     // GELU backward (aux_tma == 1): the warp's 32 x 64 tile of aux values is fetched by TMA into its
     // staging tile one unit ahead (right after the store of the unit before has read the tile), so
     // the loads that the epilogue math depends on are in flight while the accumulator is still
@@ -485,7 +485,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     // (aux_tma == 2) do the same with 32 x 32 fp32 tiles: the second of a unit's two tiles follows
     // when the first has left, the next unit's first one unit ahead.
     static_assert(COLS_PER_WARP == 64, "the staged aux tile is one 64-column store group");
-    const bool stage_aux = g.aux_tma != 0;
+    const bool stage_aux = EPI == EPI_RESID || EPI == EPI_MUL || (EPI == EPI_ANY && g.aux_tma != 0);
     uint32_t aux_phase = 0;
     auto fetch_aux = [&](int u, int grp) {          // lane 0; the staging tile must be free
       if (u >= num_units) return;
@@ -508,12 +508,12 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
       const int m = m0w + lane;
       const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
-      if (!mbar_wait(&tfull_bar[ab], acc_phase[ab], abort_flag)) {
+      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         break;
       }
-      acc_phase[ab] ^= 1;
+      acc_phase ^= 1u << ab;
       tc_fence_after();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
@@ -527,28 +527,31 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         aux_phase ^= 1;
         return true;
       };
-      if (g.aux_tma == 2) {
-        // past the last column group of this unit: the first tile of the next one
-        auto next_tile = [&](int grp) {
-          if (grp + 1 < COLS_PER_WARP / 32 && nbase + (grp + 1) * 32 < g.N) fetch_aux(u, grp + 1);
-          else fetch_aux(u + num_pairs, 0);
-        };
-        if (staged && !epilogue_drain_resid<COLS_PER_WARP>(g, tmOut, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
-                                                           wait_aux, next_tile))
-          break;
-        if (!staged && lane == 0) fetch_aux(u + num_pairs, 0);
-      } else {
+      // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
+      // from zero-filled loads); it still hands the buffer back
+      if constexpr (EPI == EPI_ANY) {
         if (staged && !wait_aux()) break;
-        // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
-        // from zero-filled loads); it still hands the buffer back
         if (m0w < g.M)
           epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
                                              ks == 0, 0, staged);
+      } else {
+        // past the last staged tile of this unit: the first one of the next
+        auto next_tile = [&](int grp) {
+          if (EPI == EPI_RESID && grp == 0 && nbase + 32 < g.N) fetch_aux(u, 1);
+          else fetch_aux(u + num_pairs, 0);
+        };
+        if (m0w < g.M && nbase < g.N) {
+          if (!epilogue_drain_kind<EPI, false>(g, tmOut, tmAux, taddr, m, m0w, nbase, true, my_stage, lane, 0,
+                                               wait_aux, next_tile))
+            break;
+        } else if ((EPI == EPI_RESID || EPI == EPI_MUL) && lane == 0) {
+          fetch_aux(u + num_pairs, 0);
+        }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
-      if (g.aux_tma == 1 && lane == 0) {
+      if (EPI == EPI_ANY && stage_aux && lane == 0) {
         tma_store_wait_read<0>();           // the store just issued has read the staging tile
         fetch_aux(u + num_pairs, 0);
       }
@@ -606,20 +609,40 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   }
   constexpr int SMEM = 1024 + PAIR_STAGES * (BM * BK * 2 + HALF_N * BK * 2) +
                        NUM_EPI_WARPS * PAIR_WARP_STAGING + 256;
-  auto kern = gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN>;
-  static PerDeviceOnce attr_set;
-  if (attr_set.first_use_on_device()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    attr_set.mark_device();
-  }
   const int m_tiles = (g.M + 2 * BM - 1) / (2 * BM), n_tiles = (g.N + PAIR_BN - 1) / PAIR_BN;
   const int units = m_tiles * n_tiles * g.k_splits;
   int pairs = max_ctas / 2;
   if (pairs > units) pairs = units;
   if (pairs < 1) pairs = 1;
-  launch_chained(kern, dim3(2 * pairs), dim3(NUM_THREADS), SMEM, stream, tmA, tmB, tmOut, tmAux, ga);
-  return static_cast<int>(cudaGetLastError());
+  auto go = [&](auto kern, PerDeviceOnce& attr_set) {
+    if (attr_set.first_use_on_device()) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      attr_set.mark_device();
+    }
+    launch_chained(kern, dim3(2 * pairs), dim3(NUM_THREADS), SMEM, stream, tmA, tmB, tmOut, tmAux, ga);
+    return static_cast<int>(cudaGetLastError());
+  };
+  static PerDeviceOnce attr[EPI_ACCUM + 1];      // one per kernel of this operand layout
+  const EpiKind kind = epi_kind(ga);
+  // forward layers: [in][out] weights; input gradients: the same weights read K-major; weight
+  // gradients: both operands MN-major
+  if constexpr (!A_MN) {
+    if (kind == EPI_BF16) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_BF16>, attr[EPI_BF16]);
+  }
+  if constexpr (!A_MN && B_MN) {
+    if (kind == EPI_GELU) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_GELU>, attr[EPI_GELU]);
+    if (kind == EPI_GELU_GRAD) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_GELU_GRAD>, attr[EPI_GELU_GRAD]);
+    if (kind == EPI_RESID) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_RESID>, attr[EPI_RESID]);
+  }
+  if constexpr (!A_MN && !B_MN) {
+    if (kind == EPI_MUL) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_MUL>, attr[EPI_MUL]);
+  }
+  if constexpr (A_MN && B_MN) {
+    if (kind == EPI_ACCUM) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_ACCUM>, attr[EPI_ACCUM]);
+  }
+  if (ga.aux_tma == 2) ga.aux_tma = 0;           // EPI_ANY reads the residual row by row
+  return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_ANY>, attr[EPI_ANY]);
 }
 
 template <int BN, int STAGES, bool A_MN, bool B_MN>

@@ -427,6 +427,59 @@ __device__ __forceinline__ float gelu_tanh_with_grad(float x, float& grad) {
   return fmaf(h, t, h);
 }
 
+// ------------------------------------------------------------ packed fp32 ---
+// Two fp32 values in one 64-bit register pair; one instruction does both (sm_100a).
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_bcast(float v) { return f2_pack(v, v); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t f2_to_bf16x2(uint64_t v) {
+  float lo, hi;
+  f2_unpack(v, lo, hi);
+  return pack_bf16x2(lo, hi);
+}
+// gelu_tanh / gelu_tanh_with_grad of two values (same formulas as above)
+__device__ __forceinline__ uint64_t f2_gelu_tanh(uint64_t x) {
+  const uint64_t u = f2_mul(x, f2_fma(f2_bcast(GELU_K01), f2_mul(x, x), f2_bcast(GELU_K0)));
+  float u0, u1;
+  f2_unpack(u, u0, u1);
+  const uint64_t t = f2_pack(tanh_fast(u0), tanh_fast(u1));
+  const uint64_t h = f2_mul(x, f2_bcast(0.5f));
+  return f2_fma(h, t, h);
+}
+__device__ __forceinline__ uint64_t f2_gelu_tanh_with_grad(uint64_t x, uint64_t& grad) {
+  const uint64_t x2 = f2_mul(x, x);
+  const uint64_t u = f2_mul(x, f2_fma(f2_bcast(GELU_K01), x2, f2_bcast(GELU_K0)));
+  float u0, u1;
+  f2_unpack(u, u0, u1);
+  const uint64_t t = f2_pack(tanh_fast(u0), tanh_fast(u1));
+  const uint64_t h = f2_mul(x, f2_bcast(0.5f));
+  const uint64_t sech2 = f2_fma(f2_mul(t, f2_bcast(-1.f)), t, f2_bcast(1.f));
+  const uint64_t du = f2_fma(f2_bcast(3.f * GELU_K01), x2, f2_bcast(GELU_K0));
+  grad = f2_fma(h, f2_mul(sech2, du), f2_fma(f2_bcast(0.5f), t, f2_bcast(0.5f)));
+  return f2_fma(h, t, h);
+}
+
 // ---------------------------------------------------------------- philox ---
 // Counter-based generator (Philox4x32, 7 rounds) used for every dropout mask:
 // the mask of element i of stream `stream` under `seed` is a pure function of

@@ -213,3 +213,39 @@ def test_gemm_pair_residual_tiles(M, N, K, drop_p):
     if drop_p == 0:
         ref = a.float() @ w.float() + bias + resid
         assert torch.allclose(out, ref, rtol=1e-4, atol=1e-4 * K ** 0.5)
+
+
+@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (520, 264, 72), (1100, 800, 256), (20000, 512, 128)])
+def test_gemm_pair_specialised_epilogues(M, N, K):
+    """Every specialised drain of the CTA-pair kernel at tile edges: rows and columns past a tile, a last
+    column tile that ends inside a warp's columns, several units per pair."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(5)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(K, N, device="cuda") * K ** -0.5).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    ref = a.float() @ w.float() + bias
+    # one bf16 rounding of a value of known size (2^-9 of it), plus the rounding of the fp32 sums and
+    # of tanh.approx (2^-11)
+    close = lambda x, y: torch.allclose(x.float(), y, rtol=2 ** -8, atol=2 ** -9)
+    assert close(gemm(a, w, b_mn=True, bias=bias), ref)
+    assert close(gemm(a, w, b_mn=True), ref - bias)
+    gelu = torch.nn.functional.gelu(ref, approximate="tanh")
+    assert close(gemm(a, w, b_mn=True, bias=bias, act=3), gelu)
+    aux = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert close(gemm(a, w, b_mn=True, bias=bias, act=1, aux=aux, aux_grad=True), gelu)
+    x = ref.clone().requires_grad_(True)
+    torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
+    assert close(aux, x.grad)
+    wt = w.t().contiguous()
+    assert close(gemm(a, wt, act=2, aux=aux, aux_grad=True), (ref - bias) * aux.float())
+    dy = torch.randn(M, N, device="cuda").bfloat16()
+    dw = torch.full((K, N), 3.0, device="cuda")
+    for splits in (1, 3):
+        gemm(a, dy, a_mn=True, b_mn=True, out=dw, accumulate=True, k_splits=splits)
+    # fp32 sums of M products in two orders: errors grow as sqrt(M) ulps of a sum of size sqrt(M)
+    assert torch.allclose(dw, 3.0 + 2 * (a.float().t() @ dy.float()), rtol=1e-4, atol=2 ** -22 * M)
+    torch.cuda.synchronize()
+    _lib.check_status()
