@@ -85,154 +85,185 @@ struct LnBwdArgs {
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into drop_seed when not null
 };
 
-// dy (+ rank-2 term) of lane-owned float4 column c4 of one row
-__device__ __forceinline__ float4 ln_dy_eff(const LnBwdArgs& a, uint2 p, bool has_dy, int c4,
-                                            float sc0, float sc1) {
-  float4 dyv = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (has_dy) dyv = make_float4(bf16_lo(p.x), bf16_hi(p.x), bf16_lo(p.y), bf16_hi(p.y));
-  if (a.s0) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(a.w0) + c4);
-    dyv.x += sc0 * w.x; dyv.y += sc0 * w.y; dyv.z += sc0 * w.z; dyv.w += sc0 * w.w;
-  }
-  if (a.s1) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(a.w1) + c4);
-    dyv.x += sc1 * w.x; dyv.y += sc1 * w.y; dyv.z += sc1 * w.z; dyv.w += sc1 * w.w;
-  }
-  return dyv;
+// Backward kernel.  A group of threads owns a row and every thread of it the same eight columns of
+// each row it meets (float4 columns t and t + d/8), so the column sums dgamma / dbeta / dbias stay in
+// 24 registers per thread from the first row to the last and no shared-memory accumulator limits how
+// many rows are in flight: bound by bytes (16 per element with a residual and a masked copy).  The
+// form before kept a warp per row and the sums of every warp in shared memory (96 bytes per column of
+// a block): 16 warps per SM at d <= 1024, 8 above.
+//   LNB_ROWS rows are loaded together (one memory round trip, one exchange of row sums through shared
+//   memory per LNB_ROWS rows); narrow rows put several groups in a block, folded at the end.
+// The eight columns of a thread belong to two dropout groups of eight; neighbouring lanes share both,
+// so each lane draws one and they swap.
+constexpr int LNB_ROWS = 2;
+constexpr int LNB_MAX_THREADS = 256;
+
+__device__ __forceinline__ float4 ln_unpack4(uint2 p) {
+  return make_float4(bf16_lo(p.x), bf16_hi(p.x), bf16_lo(p.y), bf16_hi(p.y));
+}
+__device__ __forceinline__ void ln_red4(float* dst, const float4& v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
 }
 
-// Row kernel: every global load of a row (x, dy, incoming residual gradient) is issued up front,
-// so a row costs one memory round trip; dy stays packed in registers and gamma*dy is recomputed.
-//
-// PARAMS: the warp also accumulates dgamma / dbeta of its rows in a private shared-memory row
-// (3 x d floats per warp: dgamma, dbeta and the column sums of the masked copy; plain
-// read-add-write, no atomics); the block folds its eight rows and
-// issues one vector atomic per four columns at the end.  This saves the second pass over x and dy
-// that a separate column kernel needs.
-template <int NV_MAX, bool PARAMS>
-__global__ void __launch_bounds__(LN_WARPS * 32, NV_MAX <= 8 ? 2 : 1)
+__global__ void __launch_bounds__(LNB_MAX_THREADS, 2)
 ln_bwd_kernel(const LnBwdArgs a) {
   griddep_enter();
-  extern __shared__ __align__(16) float ln_acc[];     // [LN_WARPS][3][d] when PARAMS
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int d = a.d, nv = d >> 7;
-  float4* acc_g = reinterpret_cast<float4*>(ln_acc + (warp * 3 + 0) * d);
-  float4* acc_b = reinterpret_cast<float4*>(ln_acc + (warp * 3 + 1) * d);
-  float4* acc_c = reinterpret_cast<float4*>(ln_acc + (warp * 3 + 2) * d);
-  const bool want_bias = PARAMS && a.dbias != nullptr && a.dbranch != nullptr;
-  if (PARAMS) {
-    for (int c4 = lane; c4 < (d >> 2); c4 += 32) {
-      acc_g[c4] = make_float4(0.f, 0.f, 0.f, 0.f);
-      acc_b[c4] = make_float4(0.f, 0.f, 0.f, 0.f);
-      acc_c[c4] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncwarp();
-  }
-  const float dscale = dropout_scale(a.drop_thr16);
+  constexpr int R = LNB_ROWS;
+  extern __shared__ __align__(16) float ln_fold[];          // [groups][3][d] when a block has several groups
+  __shared__ __align__(16) float red[2][LNB_MAX_THREADS / 32][2 * R];
+  const int gt = blockDim.x;                                // threads of a row group (multiple of 32)
+  const int t = threadIdx.x, grp = threadIdx.y, groups = blockDim.y;
+  const int lane = t & 31, gwarps = gt >> 5, warp = grp * gwarps + (t >> 5);
+  const int d = a.d, n = d >> 3;                            // n threads carry columns
+  const bool own = t < n;
+  const int c[2] = {own ? t : 0, own ? t + n : 0};          // float4 columns
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool has_dy = a.dy != nullptr, has_r = a.dres_in != nullptr;
-  for (int row = blockIdx.x * LN_WARPS + warp; row < a.M; row += gridDim.x * LN_WARPS) {
-    const float4* xr = reinterpret_cast<const float4*>(a.x + (long long)row * d);
-    const uint2* dyr = reinterpret_cast<const uint2*>(a.dy + (long long)row * d);
-    const float4* rr = reinterpret_cast<const float4*>(a.dres_in + (long long)row * d);
-    float4 xh[NV_MAX], rv[NV_MAX];
-    uint2 dyp[NV_MAX];
+  const bool want_bias = a.dgamma != nullptr && a.dbias != nullptr && a.dbranch != nullptr;
+  const float dscale = dropout_scale(a.drop_thr16);
+  const uint64_t seed = a.drop_thr16 ? salted(a.drop_seed, a.salt) : 0;
+  const float inv_d = 1.f / d;
+  float4 gam[2], sg[2] = {zero, zero}, sb[2] = {zero, zero}, sc[2] = {zero, zero};
 #pragma unroll
-    for (int i = 0; i < NV_MAX; ++i)
-      if (i < nv) {
-        const int c4 = lane + 32 * i;
-        xh[i] = xr[c4];
-        dyp[i] = has_dy ? dyr[c4] : make_uint2(0u, 0u);
-        rv[i] = has_r ? rr[c4] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    const float mean = a.rms ? 0.f : a.mean[row];
-    const float rstd = a.rstd[row];
-    const float sc0 = a.s0 ? a.s0[row] : 0.f, sc1 = a.s1 ? a.s1[row] : 0.f;
-    float s1 = 0.f, s2 = 0.f;
+  for (int u = 0; u < 2; ++u) gam[u] = own ? __ldg(reinterpret_cast<const float4*>(a.gamma) + c[u]) : zero;
+
+  int par = 0;
+  const int step = gridDim.x * groups * R;
+  for (int row0 = (blockIdx.x * groups + grp) * R; row0 < a.M; row0 += step, par ^= 1) {
+    float4 xh[R][2], rv[R][2], dy[R][2];
+    uint2 dyp[R][2];
+    float mean[R], rstd[R];
 #pragma unroll
-    for (int i = 0; i < NV_MAX; ++i)
-      if (i < nv) {
-        const int c4 = lane + 32 * i;
-        const float4 dyv = ln_dy_eff(a, dyp[i], has_dy, c4, sc0, sc1);
-        const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + c4);
-        xh[i] = make_float4((xh[i].x - mean) * rstd, (xh[i].y - mean) * rstd,
-                            (xh[i].z - mean) * rstd, (xh[i].w - mean) * rstd);
-        const float4 gy = make_float4(dyv.x * g.x, dyv.y * g.y, dyv.z * g.z, dyv.w * g.w);
-        s1 += gy.x + gy.y + gy.z + gy.w;
-        s2 += gy.x * xh[i].x + gy.y * xh[i].y + gy.z * xh[i].z + gy.w * xh[i].w;
+    for (int i = 0; i < R; ++i) {
+      const int row = row0 + i;
+      const bool live = own && row < a.M;
+      mean[i] = 0.f;
+      rstd[i] = 0.f;
+      if (row < a.M) {
+        rstd[i] = a.rstd[row];
+        if (!a.rms) mean[i] = a.mean[row];
       }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      for (int u = 0; u < 2; ++u) {
+        xh[i][u] = zero; rv[i][u] = zero; dyp[i][u] = make_uint2(0u, 0u);
+        if (live) {
+          xh[i][u] = reinterpret_cast<const float4*>(a.x + (long long)row * d)[c[u]];
+          if (has_dy) dyp[i][u] = reinterpret_cast<const uint2*>(a.dy + (long long)row * d)[c[u]];
+          if (has_r) rv[i][u] = reinterpret_cast<const float4*>(a.dres_in + (long long)row * d)[c[u]];
+        }
+      }
     }
-    const float m1 = a.rms ? 0.f : s1 / d, m2 = s2 / d;
-    float4* dxr = reinterpret_cast<float4*>(a.dx + (long long)row * d);
-    uint2* dbr = a.dbranch ? reinterpret_cast<uint2*>(a.dbranch + (long long)row * d) : nullptr;
+    float part[2 * R];
 #pragma unroll
-    for (int i = 0; i < NV_MAX; ++i)
-      if (i < nv) {
-        const int c4 = lane + 32 * i;
-        const float4 dyv = ln_dy_eff(a, dyp[i], has_dy, c4, sc0, sc1);
-        const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + c4);
-        if (PARAMS) {
-          float4 t = acc_g[c4];
-          t.x += dyv.x * xh[i].x; t.y += dyv.y * xh[i].y; t.z += dyv.z * xh[i].z; t.w += dyv.w * xh[i].w;
-          acc_g[c4] = t;
-          float4 u = acc_b[c4];
-          u.x += dyv.x; u.y += dyv.y; u.z += dyv.z; u.w += dyv.w;
-          acc_b[c4] = u;
+    for (int i = 0; i < R; ++i) {
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float4 g = ln_unpack4(dyp[i][u]);
+        if (a.s0 && own && row0 + i < a.M) {                // rank-2 term of the scalar heads
+          const float k = a.s0[row0 + i];
+          const float4 w = __ldg(reinterpret_cast<const float4*>(a.w0) + c[u]);
+          g.x += k * w.x; g.y += k * w.y; g.z += k * w.z; g.w += k * w.w;
         }
+        if (a.s1 && own && row0 + i < a.M) {
+          const float k = a.s1[row0 + i];
+          const float4 w = __ldg(reinterpret_cast<const float4*>(a.w1) + c[u]);
+          g.x += k * w.x; g.y += k * w.y; g.z += k * w.z; g.w += k * w.w;
+        }
+        const float4 x = xh[i][u];
+        const float4 h = make_float4((x.x - mean[i]) * rstd[i], (x.y - mean[i]) * rstd[i],
+                                     (x.z - mean[i]) * rstd[i], (x.w - mean[i]) * rstd[i]);
+        xh[i][u] = h;
+        dy[i][u] = g;
+        s1 += g.x * gam[u].x + g.y * gam[u].y + g.z * gam[u].z + g.w * gam[u].w;
+        s2 += g.x * gam[u].x * h.x + g.y * gam[u].y * h.y + g.z * gam[u].z * h.z + g.w * gam[u].w * h.w;
+        sg[u].x += g.x * h.x; sg[u].y += g.y * h.y; sg[u].z += g.z * h.z; sg[u].w += g.w * h.w;
+        sb[u].x += g.x; sb[u].y += g.y; sb[u].z += g.z; sb[u].w += g.w;
+      }
+      part[2 * i] = s1;
+      part[2 * i + 1] = s2;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 2 * R; ++k) part[k] += __shfl_xor_sync(0xffffffffu, part[k], o);
+    if (gwarps > 1) {
+      // the slot written two rounds ago is free: its readers passed the barrier of the round between
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 2 * R; ++k) red[par][warp][k] = part[k];
+      asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(gt) : "memory");
+#pragma unroll
+      for (int k = 0; k < 2 * R; ++k) part[k] = 0.f;
+      for (int w = 0; w < gwarps; ++w)
+#pragma unroll
+        for (int k = 0; k < 2 * R; ++k) part[k] += red[par][grp * gwarps + w][k];
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = row0 + i;
+      const float m1 = a.rms ? 0.f : part[2 * i] * inv_d, m2 = part[2 * i + 1] * inv_d;
+      uint32_t keep = 0xffu;                                // low 4 bits: column c[0], high 4: c[1]
+      if (a.drop_thr16 && a.dbranch) {
+        const uint64_t f4 = static_cast<uint64_t>(row) * (d >> 2) + ((lane & 1) ? t - 1 + n : t);
+        const uint32_t mine = dropout_keep8(seed, a.drop_stream, f4 >> 1, a.drop_thr16);
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
+        keep = (lane & 1) ? ((other >> 4) & 0xfu) | (mine & 0xf0u) : (mine & 0xfu) | ((other & 0xfu) << 4);
+      }
+      if (!own || row >= a.M) continue;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float4 g = dy[i][u], h = xh[i][u];
         float4 o;
-        o.x = (dyv.x * g.x - m1 - xh[i].x * m2) * rstd + rv[i].x;
-        o.y = (dyv.y * g.y - m1 - xh[i].y * m2) * rstd + rv[i].y;
-        o.z = (dyv.z * g.z - m1 - xh[i].z * m2) * rstd + rv[i].z;
-        o.w = (dyv.w * g.w - m1 - xh[i].w * m2) * rstd + rv[i].w;
-        dxr[c4] = o;
-        if (dbr) {
-          float4 m = o;
+        o.x = (g.x * gam[u].x - m1 - h.x * m2) * rstd[i] + rv[i][u].x;
+        o.y = (g.y * gam[u].y - m1 - h.y * m2) * rstd[i] + rv[i][u].y;
+        o.z = (g.z * gam[u].z - m1 - h.z * m2) * rstd[i] + rv[i][u].z;
+        o.w = (g.w * gam[u].w - m1 - h.w * m2) * rstd[i] + rv[i][u].w;
+        reinterpret_cast<float4*>(a.dx + (long long)row * d)[c[u]] = o;
+        if (a.dbranch) {
           if (a.drop_thr16) {
-            const uint64_t e0 = static_cast<uint64_t>(row) * d + c4 * 4;
-            const uint32_t keep =
-                dropout_keep8(salted(a.drop_seed, a.salt), a.drop_stream, e0 >> 3, a.drop_thr16) >> (e0 & 7);
-            m.x = (keep & 1u) ? m.x * dscale : 0.f;
-            m.y = (keep & 2u) ? m.y * dscale : 0.f;
-            m.z = (keep & 4u) ? m.z * dscale : 0.f;
-            m.w = (keep & 8u) ? m.w * dscale : 0.f;
+            const uint32_t k4 = keep >> (4 * u);
+            o.x = (k4 & 1u) ? o.x * dscale : 0.f;
+            o.y = (k4 & 2u) ? o.y * dscale : 0.f;
+            o.z = (k4 & 4u) ? o.z * dscale : 0.f;
+            o.w = (k4 & 8u) ? o.w * dscale : 0.f;
           }
-          uint2 p;
-          p.x = pack_bf16x2(m.x, m.y);
-          p.y = pack_bf16x2(m.z, m.w);
-          dbr[c4] = p;
-          if (want_bias) {
-            float4 t = acc_c[c4];
-            t.x += m.x; t.y += m.y; t.z += m.z; t.w += m.w;
-            acc_c[c4] = t;
-          }
+          reinterpret_cast<uint2*>(a.dbranch + (long long)row * d)[c[u]] =
+              make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+          sc[u].x += o.x; sc[u].y += o.y; sc[u].z += o.z; sc[u].w += o.w;
         }
+      }
+    }
+  }
+  if (!a.dgamma) return;
+  if (groups > 1) {                                         // block-uniform
+    float4* f = reinterpret_cast<float4*>(ln_fold);
+    const int d4 = d >> 2;
+    if (own && grp > 0)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        f[(grp * 3 + 0) * d4 + c[u]] = sg[u];
+        f[(grp * 3 + 1) * d4 + c[u]] = sb[u];
+        f[(grp * 3 + 2) * d4 + c[u]] = sc[u];
+      }
+    __syncthreads();
+    if (grp > 0) return;
+    for (int g = 1; g < groups; ++g)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float4 x = f[(g * 3 + 0) * d4 + c[u]], y = f[(g * 3 + 1) * d4 + c[u]], z = f[(g * 3 + 2) * d4 + c[u]];
+        sg[u].x += x.x; sg[u].y += x.y; sg[u].z += x.z; sg[u].w += x.w;
+        sb[u].x += y.x; sb[u].y += y.y; sb[u].z += y.z; sb[u].w += y.w;
+        sc[u].x += z.x; sc[u].y += z.y; sc[u].z += z.z; sc[u].w += z.w;
       }
   }
-  if (PARAMS) {
-    __syncthreads();
-    for (int c4 = threadIdx.x; c4 < (d >> 2); c4 += LN_WARPS * 32) {
-      float4 sg = make_float4(0.f, 0.f, 0.f, 0.f), sb = sg, sc = sg;
+  if (!own) return;
 #pragma unroll
-      for (int w = 0; w < LN_WARPS; ++w) {
-        const float4 tg = reinterpret_cast<const float4*>(ln_acc + (w * 3 + 0) * d)[c4];
-        const float4 tb = reinterpret_cast<const float4*>(ln_acc + (w * 3 + 1) * d)[c4];
-        const float4 tc = reinterpret_cast<const float4*>(ln_acc + (w * 3 + 2) * d)[c4];
-        sg.x += tg.x; sg.y += tg.y; sg.z += tg.z; sg.w += tg.w;
-        sb.x += tb.x; sb.y += tb.y; sb.z += tb.z; sb.w += tb.w;
-        sc.x += tc.x; sc.y += tc.y; sc.z += tc.z; sc.w += tc.w;
-      }
-      if (want_bias)
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a.dbias + c4 * 4),
-                     "f"(sc.x), "f"(sc.y), "f"(sc.z), "f"(sc.w) : "memory");
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a.dgamma + c4 * 4),
-                   "f"(sg.x), "f"(sg.y), "f"(sg.z), "f"(sg.w) : "memory");
-      if (a.dbeta)
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a.dbeta + c4 * 4),
-                     "f"(sb.x), "f"(sb.y), "f"(sb.z), "f"(sb.w) : "memory");
-    }
+  for (int u = 0; u < 2; ++u) {
+    ln_red4(a.dgamma + c[u] * 4, sg[u]);
+    if (a.dbeta) ln_red4(a.dbeta + c[u] * 4, sb[u]);
+    if (want_bias) ln_red4(a.dbias + c[u] * 4, sc[u]);
   }
 }
 
@@ -267,6 +298,7 @@ int ab_layernorm_fwd_dependent(const float* x, const float* gamma, const float* 
   int grid = (M + LN_WARPS - 1) / LN_WARPS;
   if (grid > 148 * 8) grid = 148 * 8;
   if (d <= 1024) return launch_ln_dependent<8>(grid, x, gamma, beta, y, mean, rstd, M, d, eps, rms, stream);
+  if (d <= 1280) return launch_ln_dependent<10>(grid, x, gamma, beta, y, mean, rstd, M, d, eps, rms, stream);
   return launch_ln_dependent<16>(grid, x, gamma, beta, y, mean, rstd, M, d, eps, rms, stream);
 }
 
@@ -298,29 +330,14 @@ int ab_layernorm_bwd(const void* dy, const float* x, const float* mean, const fl
   a.dres_in = dres_in; a.dx = dx; a.dbranch = (__nv_bfloat16*)dbranch; a.dgamma = dgamma;
   a.dbeta = dbeta; a.dbias = dbias; a.s0 = s0; a.w0 = w0; a.s1 = s1; a.w1 = w1; a.M = M; a.d = d; a.rms = rms;
   a.drop_seed = drop_seed; a.drop_stream = drop_stream; a.drop_thr16 = drop_thr16; a.salt = seed_salt_ptr();
-  int grid = (M + LN_WARPS - 1) / LN_WARPS;
-  if (!dgamma) {
-    if (grid > 148 * 16) grid = 148 * 16;
-    if (d <= 1024) launch_chained(ln_bwd_kernel<8, false>, dim3(grid), dim3(LN_WARPS * 32), 0, stream, a);
-    else           launch_chained(ln_bwd_kernel<16, false>, dim3(grid), dim3(LN_WARPS * 32), 0, stream, a);
-    return (int)cudaGetLastError();
-  }
-  // with parameter gradients: exactly the resident blocks, each warp keeps its column sums
-  const int smem = LN_WARPS * 3 * d * (int)sizeof(float);
-  static PerDeviceOnce attr_set;
-  if (attr_set.first_use_on_device()) {
-    cudaError_t e = cudaFuncSetAttribute(ln_bwd_kernel<8, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, LN_WARPS * 3 * 1024 * 4);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ln_bwd_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               LN_WARPS * 3 * 2048 * 4);
-    if (e != cudaSuccess) return (int)e;
-    attr_set.mark_device();
-  }
-  const int resident = d <= 1024 ? 148 * 2 : 148;
+  const int gt = ((d >> 3) + 31) / 32 * 32;                 // threads of a row group
+  const int groups = gt < 128 ? (gt < 64 ? 4 : 128 / gt) : 1;
+  const int rows = groups * LNB_ROWS;
+  int grid = (M + rows - 1) / rows;
+  const int resident = 148 * (512 / (gt * groups));         // 128 registers a thread
   if (grid > resident) grid = resident;
-  if (d <= 1024) launch_chained(ln_bwd_kernel<8, true>, dim3(grid), dim3(LN_WARPS * 32), smem, stream, a);
-  else           launch_chained(ln_bwd_kernel<16, true>, dim3(grid), dim3(LN_WARPS * 32), smem, stream, a);
+  const size_t smem = groups > 1 ? sizeof(float) * groups * 3 * d : 0;
+  launch_chained(ln_bwd_kernel, dim3(grid), dim3(gt, groups), smem, stream, a);
   return (int)cudaGetLastError();
 }
 }

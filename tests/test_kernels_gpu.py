@@ -138,6 +138,43 @@ def test_layernorm_backward_dropout_mask_is_the_element_indexed_one(M, d, params
     assert torch.equal((dbranch != 0).cpu(), want)
 
 
+@pytest.mark.parametrize("M,d", [(1, 128), (9, 256), (1001, 256), (13, 384), (6, 640), (2999, 768), (1201, 2048)])
+def test_layernorm_backward_column_sums_and_mask_at_row_group_edges(M, d):
+    """Widths that put several row groups into a block (d < 1024), leave lanes without columns
+    (d = 128, 640) or use the widest group, with row counts that end inside a group's pair of rows.
+    Sums of M fp32 terms: |error| <= M * 2^-24 * sum|terms| bounds any order; sqrt(M) of it is seen."""
+    from allie_b200.ops import kernels as K
+
+    torch.manual_seed(8)
+    x = torch.randn(M, d, device=DEV)
+    g = torch.randn(d, device=DEV)
+    mean, rstd = x.mean(-1), (x.var(-1, unbiased=False) + 1e-5).rsqrt()
+    dy = torch.randn(M, d, device=DEV).bfloat16()
+    dres = torch.randn(M, d, device=DEV) + 4.0
+    dx = torch.empty(M, d, device=DEV)
+    dbranch = torch.empty(M, d, device=DEV, dtype=torch.bfloat16)
+    sums = torch.zeros(3, d, device=DEV)
+    K.layernorm_bwd(dy, x, mean, rstd, g, dres, dx, dbranch, sums[0], sums[1], dbias=sums[2], drop_seed=3,
+                    drop_stream=2, drop_p=0.2)
+    _done()
+    xh = (x.double() - mean.double()[:, None]) * rstd.double()[:, None]
+    gy = dy.double() * g.double()
+    ref = (gy - gy.mean(-1, keepdim=True) - xh * (gy * xh).mean(-1, keepdim=True)) * rstd.double()[:, None] + dres.double()
+    assert torch.allclose(dx.double(), ref, rtol=1e-5, atol=2e-5)
+    keep = dbranch != 0
+    scale = 65536.0 / (65536 - _thr16(0.2))
+    assert torch.allclose(dbranch.float()[keep], dx[keep] * scale, rtol=2 ** -8, atol=1e-6)
+    masked = torch.where(keep, dx.double() * scale, torch.zeros_like(ref))
+    for got, terms in ((sums[0], dy.double() * xh), (sums[1], dy.double()), (sums[2], masked)):
+        assert ((got.double() - terms.sum(0)).abs() <= 1e-6 + M * 2.0 ** -22 * terms.abs().sum(0)).all()
+
+
+def _thr16(p):
+    from allie_b200.ops import _lib
+
+    return _lib.dropout_thr16(p)
+
+
 def test_cross_entropy_loss_and_gradient():
     from allie_b200.ops import kernels as K
 
