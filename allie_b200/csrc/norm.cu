@@ -92,11 +92,13 @@ struct LnBwdArgs {
 // form before kept a warp per row and the sums of every warp in shared memory (96 bytes per column of
 // a block): 16 warps per SM at d <= 1024, 8 above.
 //   LNB_ROWS rows are loaded together (one memory round trip, one exchange of row sums through shared
-//   memory per LNB_ROWS rows); narrow rows put several groups in a block, folded at the end.
+//   memory per LNB_ROWS rows).  A block holds as many groups as fit 512 threads (the registers of an
+//   SM) and folds their sums before its atomics: with a block per group, 740 blocks adding to the same
+//   2304 addresses cost 12136 x 768 more than the register sums gain.
 // The eight columns of a thread belong to two dropout groups of eight; neighbouring lanes share both,
 // so each lane draws one and they swap.
 constexpr int LNB_ROWS = 2;
-constexpr int LNB_MAX_THREADS = 256;
+constexpr int LNB_THREADS = 512;
 
 __device__ __forceinline__ float4 ln_unpack4(uint2 p) {
   return make_float4(bf16_lo(p.x), bf16_hi(p.x), bf16_lo(p.y), bf16_hi(p.y));
@@ -106,12 +108,12 @@ __device__ __forceinline__ void ln_red4(float* dst, const float4& v) {
                : "memory");
 }
 
-__global__ void __launch_bounds__(LNB_MAX_THREADS, 2)
+__global__ void __launch_bounds__(LNB_THREADS, 1)
 ln_bwd_kernel(const LnBwdArgs a) {
   griddep_enter();
   constexpr int R = LNB_ROWS;
   extern __shared__ __align__(16) float ln_fold[];          // [groups][3][d] when a block has several groups
-  __shared__ __align__(16) float red[2][LNB_MAX_THREADS / 32][2 * R];
+  __shared__ __align__(16) float red[2][LNB_THREADS / 32][2 * R];
   const int gt = blockDim.x;                                // threads of a row group (multiple of 32)
   const int t = threadIdx.x, grp = threadIdx.y, groups = blockDim.y;
   const int lane = t & 31, gwarps = gt >> 5, warp = grp * gwarps + (t >> 5);
@@ -331,12 +333,21 @@ int ab_layernorm_bwd(const void* dy, const float* x, const float* mean, const fl
   a.dbeta = dbeta; a.dbias = dbias; a.s0 = s0; a.w0 = w0; a.s1 = s1; a.w1 = w1; a.M = M; a.d = d; a.rms = rms;
   a.drop_seed = drop_seed; a.drop_stream = drop_stream; a.drop_thr16 = drop_thr16; a.salt = seed_salt_ptr();
   const int gt = ((d >> 3) + 31) / 32 * 32;                 // threads of a row group
-  const int groups = gt < 128 ? (gt < 64 ? 4 : 128 / gt) : 1;
+  // groups per block: what 512 threads hold, but no more than leaves every SM a block
+  const int want = (M + 148 * LNB_ROWS - 1) / (148 * LNB_ROWS);
+  const int groups = want < LNB_THREADS / gt ? want : LNB_THREADS / gt;
   const int rows = groups * LNB_ROWS;
   int grid = (M + rows - 1) / rows;
-  const int resident = 148 * (512 / (gt * groups));         // 128 registers a thread
-  if (grid > resident) grid = resident;
+  if (grid > 148) grid = 148;
   const size_t smem = groups > 1 ? sizeof(float) * groups * 3 * d : 0;
+  static PerDeviceOnce attr_set;
+  if (attr_set.first_use_on_device()) {
+    // groups * d <= LNB_THREADS / gt * 8 * gt
+    cudaError_t e = cudaFuncSetAttribute(ln_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         LNB_THREADS * 8 * 3 * (int)sizeof(float));
+    if (e != cudaSuccess) return (int)e;
+    attr_set.mark_device();
+  }
   launch_chained(ln_bwd_kernel, dim3(grid), dim3(gt, groups), smem, stream, a);
   return (int)cudaGetLastError();
 }
