@@ -9,7 +9,8 @@ constexpr int AT_BN = 128;   // keys per inner tile
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct AttnArgs {
-  int B, T, H, hd;
+  int B, T, H, hd;          // T: length of every sequence, or of the longest one with row0
+  const int* row0;          // [B + 1] first activation row of every sequence (packed batch), or null
   float scale;              // 1/sqrt(hd)
   unsigned long long seed;
   unsigned int stream_id, thr16;
@@ -22,15 +23,6 @@ struct AttnArgs {
 
 // byte offset of the 16-byte chunk holding columns [8*c16, 8*c16+8) of row r inside a
 // 128-row x 64-column bf16 panel with 128-byte swizzle (what TMA SWIZZLE_128B writes)
-// order-preserving float <-> int coding (so integer atomicMax orders floats)
-__device__ __forceinline__ int ord_encode(float f) {
-  const int i = __float_as_int(f);
-  return i ^ ((i >> 31) & 0x7fffffff);
-}
-__device__ __forceinline__ float ord_decode(int i) {
-  return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
-}
-
 __device__ __forceinline__ uint32_t sw128_chunk(int r, int c16) {
   return static_cast<uint32_t>(r * 128 + ((c16 ^ (r & 7)) << 4));
 }

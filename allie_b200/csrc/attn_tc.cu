@@ -1,36 +1,78 @@
 // Causal flash attention on tcgen05 (forward; the backward kernels follow further down).
 //
-// One CTA owns one 128-row query tile of one (batch, head).  Per 128-row key/value tile:
+// One CTA owns one 128-row query tile of one (batch, head); two CTAs share an SM.  Per 128-row
+// key/value tile:
 //   warp 5 (one thread) : S = Q K^T          -> TMEM (128 lanes = query rows, 128 fp32 columns)
-//   warps 0-3           : tcgen05.ld S, online softmax (row = thread), dropout, P -> smem (bf16,
-//                         128B-swizzled panels = the UMMA K-major A layout)
-//   warp 5              : PV = P V           -> TMEM (fresh, not accumulated)
-//   warps 0-3           : O = O * alpha + PV in registers
-//   warp 4 (one thread) : TMA loads of Q once and K/V tiles through a 2-stage ring
+//   warps 0-3           : one thread per query row: the whole row of S in registers, maximum, exponentials,
+//                         dropout, P -> TMEM as packed bf16 (the A operand of the second product)
+//   warp 5              : O += P V           -> TMEM
+//   warp 4 (one thread) : TMA loads of Q once and K/V tiles through a ring
 // Q, K and V are read straight out of the packed [B*T, 3*d] QKV activation with 2-D TMA boxes
 // (64 columns x 128 rows), and O is written in the [B*T, d] layout the projection GEMM reads.
 // V is consumed MN-major (rows = keys), so no transposes exist anywhere.
+//
+// What bounds it: the exponential unit (16 per SM and clock: 1024 clocks per tile pair against 512 of
+// the tensor core) and, with dropout, instruction issue (the generator is 8 of about 13 instructions
+// per element).  So nothing else may cost instructions or waits per element: S is read once (a row
+// per thread needs no exchange of maxima between warps), P never passes through shared memory, and O
+// stays in TMEM, rescaled there when the maximum of one of a warp's rows has grown.  (Keeping the old
+// scale until the maximum has grown by 2^8 saves little at these lengths and gives up that the largest
+// probability of a row is exactly one: error against 64 bits 0.00195 instead of 0.00181.)  The
+// reciprocal of the keep probability is applied at the end, too.
 #include "attn_common.cuh"
 
 namespace ab {
 
-constexpr int FWD_MATH_WARPS = 8;
-constexpr int FWD_MATH_THREADS = FWD_MATH_WARPS * 32;
+constexpr int FWD_MATH_WARPS = 4;
 constexpr int FWD_TMA_WARP = FWD_MATH_WARPS;
 constexpr int FWD_MMA_WARP = FWD_MATH_WARPS + 1;
 constexpr int FWD_THREADS = (FWD_MATH_WARPS + 2) * 32;
 
 template <int HD>
-__global__ void __launch_bounds__(FWD_THREADS, HD <= 64 ? 2 : 1)
+struct FwdCfg {
+  static constexpr int PANELS = HD / 64;               // 64-column panels per Q/K/V tile
+  static constexpr int TILE_BYTES = 128 * HD * 2;      // one Q / K / V tile
+  // head_dim 64: S, P and O side by side in 256 TMEM columns, two K/V stages.  head_dim 128: P takes
+  // the place of S (already in registers by then) and one K/V stage, so that two CTAs still fit an SM;
+  // the partner's math covers what this CTA's tensor work waits for.
+  static constexpr bool P_IN_S = HD == 128;
+  static constexpr int STAGES = HD == 128 ? 1 : 2;
+  static constexpr int TM_P = P_IN_S ? 0 : 128;
+  static constexpr int TM_O = 256 - HD;
+  static constexpr int SMEM = (1 + 2 * STAGES) * TILE_BYTES + 256;
+};
+
+// 16 AND-masks (one per packed bf16 pair) of 32 keep bits: the bit of each element is shifted into
+// the sign of its byte and spread over a half-word by the byte permute's sign mode.
+__device__ __forceinline__ void keep_masks16(uint32_t word, uint32_t* m) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t x = word << (7 - 2 * q), y = word << (6 - 2 * q);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t sel = (8u | k) * 0x11u | (8u | (4 + k)) * 0x1100u;
+      asm("prmt.b32 %0, %1, %2, %3;" : "=r"(m[4 * k + q]) : "r"(x), "r"(y), "r"(sel));
+    }
+  }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmO,
                 const AttnArgs a) {
-  griddep_enter();
-  constexpr int PANELS = HD / 64;               // 64-column panels per Q/K/V tile
-  constexpr int TILE_BYTES = 128 * HD * 2;      // one Q / K / V tile
-  constexpr int P_BYTES = 128 * 128 * 2;
-  constexpr int TMEM_COLS = (128 + HD) <= 256 ? 256 : 512;
+  griddep_wait();
+  using C = FwdCfg<HD>;
+  constexpr int PANELS = C::PANELS, TILE_BYTES = C::TILE_BYTES, STAGES = C::STAGES;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
   constexpr uint32_t IDESC_PV = make_idesc_bf16(128, HD, 0, 1);
+
+  // packed batch: sequence b owns rows [row0[b], row0[b + 1]) of the activation
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int first = a.row0 ? a.row0[b] : b * a.T;
+  const int T = a.row0 ? a.row0[b + 1] - first : a.T;
+  const int qt = (a.T + AT_BM - 1) / AT_BM - 1 - blockIdx.x;      // heaviest tiles first
+  if (qt * AT_BM >= T) return;
+  const int nkv = qt + 1;                                          // causal: key tiles 0..qt
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
@@ -39,67 +81,56 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     return;
   }
   uint8_t* sQ = smem;
-  uint8_t* sK = sQ + TILE_BYTES;            // 2 stages
-  uint8_t* sV = sK + 2 * TILE_BYTES;        // 2 stages
-  uint8_t* sP = sV + 2 * TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + P_BYTES);
-  uint64_t* q_full = bars;                  // 1
-  uint64_t* k_full = bars + 1;              // 2
-  uint64_t* v_full = bars + 3;              // 2
-  uint64_t* k_empty = bars + 5;             // 2
-  uint64_t* v_empty = bars + 7;             // 2
+  uint8_t* sK = sQ + TILE_BYTES;
+  uint8_t* sV = sK + STAGES * TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + STAGES * TILE_BYTES);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;              // STAGES (two reserved)
+  uint64_t* v_full = bars + 3;
+  uint64_t* k_empty = bars + 5;
+  uint64_t* v_empty = bars + 7;
   uint64_t* s_full = bars + 9;
   uint64_t* s_empty = bars + 10;
   uint64_t* p_full = bars + 11;
   uint64_t* pv_full = bars + 12;
-  uint64_t* pv_empty = bars + 13;
-  // row statistics exchange between the two column halves: one barrier per TMEM lane quarter,
-  // shared by the two warps that own the same 32 query rows (the quarters do not wait for each other)
-  uint64_t* xchg = bars + 14 + (threadIdx.x >> 5 & 3);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_stat = reinterpret_cast<int*>(tmem_slot + 2);       // [128 rows] running row maximum (ordered-int coded)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqt = (a.T + AT_BM - 1) / AT_BM;
-  const int qt = nqt - 1 - blockIdx.x;      // heaviest tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int nkv = qt + 1;                   // causal: key tiles 0..qt
   const int d_model = a.H * HD;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < STAGES; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1);
       mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
     }
     mbar_init(s_full, 1); mbar_init(s_empty, FWD_MATH_WARPS);
-    mbar_init(p_full, FWD_MATH_WARPS); mbar_init(pv_full, 1); mbar_init(pv_empty, FWD_MATH_WARPS);
-    for (int i = 0; i < 4; ++i) mbar_init(bars + 14 + i, 2);
+    mbar_init(p_full, FWD_MATH_WARPS); mbar_init(pv_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQKV);
   }
-  if (threadIdx.x < 128) s_stat[threadIdx.x] = ord_encode(-INFINITY);
-  if (warp == FWD_MMA_WARP) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+  if (warp == FWD_MMA_WARP) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base, tPV = tmem_base + 128;
+  // only now: a dependent GEMM's CTA must not take the TMEM columns that this grid still has to allocate
+  if (threadIdx.x == 0) griddep_launch_dependents();
+  const uint32_t tS = tmem_base, tP = tmem_base + C::TM_P, tO = tmem_base + C::TM_O;
 
   if (warp == FWD_TMA_WARP) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      const int row_q = b * a.T + qt * AT_BM;
       mbar_expect_tx(q_full, TILE_BYTES);
 #pragma unroll
       for (int p = 0; p < PANELS; ++p)
-        tma_load_2d(sQ + p * 16384, &tmQKV, q_full, h * HD + p * 64, row_q);
+        tma_load_2d(sQ + p * 16384, &tmQKV, q_full, h * HD + p * 64, first + qt * AT_BM);
       for (int j = 0; j < nkv; ++j) {
-        const int st = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        const int row_k = b * a.T + j * AT_BN;
+        const int st = j % STAGES;
+        const uint32_t par = ((j / STAGES) & 1) ^ 1;
+        const int row_k = first + j * AT_BN;
         if (!mbar_wait(&k_empty[st], par, abort_flag)) { *abort_flag = ST_TIMEOUT_EMPTY; atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY); break; }
         mbar_expect_tx(&k_full[st], TILE_BYTES);
 #pragma unroll
@@ -118,10 +149,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     // -------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       bool ok = mbar_wait(q_full, 0, abort_flag);
+      // S of tile j.  With P in the place of S the product P V of tile j - 1 was issued before (MMAs of
+      // one thread execute in order); otherwise the math warps must have read S of tile j - 1.
       auto issue_qk = [&](int j) {
-        const int st = j & 1;
-        if (!mbar_wait(&k_full[st], (j >> 1) & 1, abort_flag)) return false;
-        if (j > 0 && !mbar_wait(s_empty, (j - 1) & 1, abort_flag)) return false;
+        const int st = j % STAGES;
+        if (!mbar_wait(&k_full[st], (j / STAGES) & 1, abort_flag)) return false;
+        if (!C::P_IN_S && j > 0 && !mbar_wait(s_empty, (j - 1) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t q0 = smem_u32(sQ), k0 = smem_u32(sK + st * TILE_BYTES);
 #pragma unroll
@@ -136,196 +169,186 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       };
       if (ok) ok = issue_qk(0);
       for (int j = 0; j < nkv && ok; ++j) {
-        const int st = j & 1;
-        if (j + 1 < nkv) { ok = issue_qk(j + 1); if (!ok) break; }
-        if (!mbar_wait(&v_full[st], (j >> 1) & 1, abort_flag)) { ok = false; break; }
+        const int st = j % STAGES;
+        if (!C::P_IN_S && j + 1 < nkv) { ok = issue_qk(j + 1); if (!ok) break; }
+        if (!mbar_wait(&v_full[st], (j / STAGES) & 1, abort_flag)) { ok = false; break; }
         if (!mbar_wait(p_full, j & 1, abort_flag)) { ok = false; break; }
-        if (j > 0 && !mbar_wait(pv_empty, (j - 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t p0 = smem_u32(sP), v0 = smem_u32(sV + st * TILE_BYTES);
+        const uint32_t v0 = smem_u32(sV + st * TILE_BYTES);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {  // 128 keys = 8 UMMA_K steps
-          const uint64_t adesc = make_sdesc_sw128(p0 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024);
-          const uint64_t bdesc = make_sdesc_sw128(v0 + k * 2048, 16384, 1024);
-          umma_bf16(tPV, adesc, bdesc, IDESC_PV, k > 0);
-        }
+        for (int k = 0; k < 8; ++k)    // 128 keys = 8 UMMA_K steps of 8 TMEM columns each
+          umma_bf16_ts(tO, tP + k * 8, make_sdesc_sw128(v0 + k * 2048, 16384, 1024), IDESC_PV, (j > 0 || k > 0));
         umma_commit(&v_empty[st]);
         umma_commit(pv_full);
+        if (C::P_IN_S && j + 1 < nkv) ok = issue_qk(j + 1);
       }
       if (!ok) { *abort_flag = ST_TIMEOUT_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_FULL); }
     }
   } else {
     // ---------------------------------------------------- softmax / output warps
-    // warp w: TMEM lane quarter w & 3 (query rows), column half w >> 2 (64 keys of each tile and
-    // HD/2 output columns).  The halves exchange their partial row maxima through shared memory.
-    const int r = (warp & 3) * 32 + lane;         // query row inside the tile = TMEM lane
-    const int hf = warp >> 2;
+    const int r = warp * 32 + lane;               // query row inside the tile = TMEM lane
     const int q_idx = qt * AT_BM + r;
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
     const float sl2 = a.scale * LOG2E;
-    constexpr int OC = HD / 2;                    // output columns owned by this thread
-    float m_run = -INFINITY, l_part = 0.f;
-    float o[OC];
-#pragma unroll
-    for (int i = 0; i < OC; ++i) o[i] = 0.f;
-    const float dscale = dropout_scale(a.thr16);
-    const uint64_t row_elem0 = (static_cast<uint64_t>(b * a.H + h) * a.T + q_idx) * a.T + hf * 64;
+    const uint64_t sl2_2 = f2_bcast(sl2);
+    float m_ref = 0.f;                            // running maximum, which P and O are scaled to
+    // row sums of the two column halves, each added up in column order
+    float l_half[2] = {0.f, 0.f};
+    const uint64_t row_elem0 = (static_cast<uint64_t>(b * a.H + h) * a.T + q_idx) * a.T;
+    const uint64_t seed = a.thr16 ? salted(a.seed, a.salt) : 0;
     bool ok = true;
-    // Dropout keep bits of this thread's 64 keys of one key tile (two words of 32).  They do not
-    // depend on the scores, so the generator runs for tile j + 1 while the tensor core computes
-    // P V of tile j (the math warps would only be waiting then); the words are also what the
-    // backward pass reads back, so it never re-runs the generator.
-    uint32_t keep_w0 = 0xffffffffu, keep_w1 = 0xffffffffu;
-    auto make_keep = [&](int j) {
+    for (int j = 0; j < nkv; ++j) {
+      // dropout keep bits of this row's 128 keys; they are also what the backward pass reads back
+      uint32_t keep[4];
+      if (a.thr16) {
+        const uint64_t e0 = row_elem0 + static_cast<uint64_t>(j) * AT_BN;
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const uint64_t e0 = row_elem0 + static_cast<uint64_t>(j) * AT_BN + c * 32;
-        uint32_t word = 0;
+        for (int c = 0; c < 4; ++c) {
+          uint32_t word = 0;
 #pragma unroll
-        for (int g = 0; g < 4; ++g)
-          word |= dropout_keep8(salted(a.seed, a.salt), a.stream_id, (e0 >> 3) + g, a.thr16) << (8 * g);
-        if (c == 0) keep_w0 = word; else keep_w1 = word;
-        if (a.drop_mask && q_idx < a.T) a.drop_mask[e0 >> 5] = word;
+          for (int g = 0; g < 4; ++g)
+            word |= dropout_keep8(seed, a.stream_id, (e0 >> 3) + c * 4 + g, a.thr16) << (8 * g);
+          keep[c] = word;
+        }
+        if (a.drop_mask && q_idx < T) {
+          uint32_t* dst = a.drop_mask + (e0 >> 5);
+          if ((T & 127) == 0) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(keep[0], keep[1], keep[2], keep[3]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (j * AT_BN + c * 32 < T) dst[c] = keep[c];
+          }
+        }
       }
-    };
-    if (a.thr16 && nkv > 0) make_keep(0);
-    for (int j = 0; j < nkv && ok; ++j) {
       if (!mbar_wait(s_full, j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      const bool diag = (j == qt);
-      // pass 1: partial row maximum over this half's 64 keys
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tS + lane_addr + hf * 64 + c * 32, v);
-        tmem_ld_wait();
+      uint32_t v[128];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float sc = __uint_as_float(v[i]);
-          if (!diag || (hf * 64 + c * 32 + i) <= r) mx = fmaxf(mx, sc);
+      for (int c = 0; c < 4; ++c) tmem_ld32(tS + lane_addr + c * 32, v + c * 32);
+      tmem_ld_wait();
+      if (!C::P_IN_S) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty);       // the next S may be computed
+      }
+      if (j == qt) {                               // diagonal tile: keys after the row's own position
+#pragma unroll
+        for (int i = 0; i < 128; ++i) v[i] = i <= r ? v[i] : 0xff800000u;
+      }
+      float mx4[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) mx4[k] = __uint_as_float(v[k]);
+#pragma unroll
+      for (int i = 4; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));   // finite: key 0 is never masked
+      float grow = 1.f;                            // what sums and O are multiplied by
+      if (j == 0) {
+        m_ref = mx;
+      } else if (__any_sync(0xffffffffu, mx > m_ref)) {
+        if (!mbar_wait(pv_full, (j - 1) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const float m_new = fmaxf(m_ref, mx);
+        grow = ex2_fast((m_ref - m_new) * sl2);
+        const uint64_t f = f2_bcast(grow);
+        m_ref = m_new;
+#pragma unroll 1
+        for (int c = 0; c < HD / 16; ++c) {
+          uint32_t o[16];
+          tmem_ld16(tO + lane_addr + c * 16, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float lo, hi;
+            f2_unpack(f2_mul(f2_pack(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), f), lo, hi);
+            o[2 * i] = __float_as_uint(lo);
+            o[2 * i + 1] = __float_as_uint(hi);
+          }
+          tmem_st16(tO + lane_addr + c * 16, o);
         }
       }
-      // running maximum of the row, shared by the two column halves (monotone, so one slot per
-      // row updated with atomicMax is enough; its last reader is ordered before its next writer by
-      // the s_empty -> next S chain)
-      atomicMax(&s_stat[r], ord_encode(mx));
-      __syncwarp();
-      if (lane == 0) mbar_arrive(xchg);     // one arrival per warp (see below)
-      if (!mbar_wait(xchg, j & 1, abort_flag)) { ok = false; break; }
-      const float m_new = ord_decode(s_stat[r]);   // finite: key 0 is never masked
-      const float alpha = ex2_fast((m_run - m_new) * sl2);
-      const float mb = m_new * sl2;
-      float rs = 0.f;
-      // pass 2: probabilities -> smem (bf16), partial row sum
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tS + lane_addr + hf * 64 + c * 32, v);
-        tmem_ld_wait();
-        float p[32];
+      const uint64_t mb = f2_bcast(-m_ref * sl2);
+      float rs[2] = {0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float e = ex2_fast(__uint_as_float(v[i]) * sl2 - mb);
-          p[i] = (!diag || (hf * 64 + c * 32 + i) <= r) ? e : 0.f;
-          rs += p[i];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float x0, x1;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(v[c * 32 + 2 * i]), __uint_as_float(v[c * 32 + 2 * i + 1])), sl2_2, mb),
+                    x0, x1);
+          x0 = ex2_fast(x0);
+          x1 = ex2_fast(x1);
+          rs[c >> 1] += x0;
+          rs[c >> 1] += x1;
+          w[i] = pack_bf16x2(x0, x1);
         }
         if (a.thr16) {
-          const uint32_t word = c ? keep_w1 : keep_w0;
+          uint32_t m[16];
+          keep_masks16(keep[c], m);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) p[i] = ((word >> i) & 1u) ? p[i] * dscale : 0.f;
+          for (int i = 0; i < 16; ++i) w[i] &= m[i];
         }
-        uint8_t* panel = sP + hf * 16384;
+        // P of the tile before is read by its product until that completes
+        if (c == 0 && j > 0 && !mbar_wait(pv_full, (j - 1) & 1, abort_flag)) { ok = false; break; }
+        if (c == 0) tc_fence_after();
+        tmem_st16(tP + lane_addr + c * 16, w);
+      }
+      if (!ok) break;
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);          // one arrival per warp
+      l_half[0] = l_half[0] * grow + rs[0];
+      l_half[1] = l_half[1] * grow + rs[1];
+    }
+    if (ok && !mbar_wait(pv_full, (nkv - 1) & 1, abort_flag)) ok = false;
+    if (!ok) {
+      *abort_flag = ST_TIMEOUT_TMEM_FULL;
+      atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL);
+    } else {
+      tc_fence_after();
+      const float l = l_half[0] + l_half[1];
+      const float inv = dropout_scale(a.thr16) / l;
+      // The warp's 32 rows leave through the (now idle) Q tile with one TMA store per 64 columns; a
+      // warp with rows past the end of the sequence stores row by row.
+      const bool whole = qt * AT_BM + warp * 32 + 32 <= T;
+      __nv_bfloat16* orow = a.out + (static_cast<long long>(first) + q_idx) * d_model + h * HD;
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld32(tO + lane_addr + c * 32, o);
+        tmem_ld_wait();
+        uint8_t* rowp = sQ + (c >> 1) * 16384 + warp * 4096 + lane * 128;
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           uint4 w;
-          w.x = pack_bf16x2(p[g * 8 + 0], p[g * 8 + 1]); w.y = pack_bf16x2(p[g * 8 + 2], p[g * 8 + 3]);
-          w.z = pack_bf16x2(p[g * 8 + 4], p[g * 8 + 5]); w.w = pack_bf16x2(p[g * 8 + 6], p[g * 8 + 7]);
-          *reinterpret_cast<uint4*>(panel + sw128_chunk(r, c * 4 + g)) = w;
+          w.x = pack_bf16x2(__uint_as_float(o[g * 8 + 0]) * inv, __uint_as_float(o[g * 8 + 1]) * inv);
+          w.y = pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv);
+          w.z = pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv);
+          w.w = pack_bf16x2(__uint_as_float(o[g * 8 + 6]) * inv, __uint_as_float(o[g * 8 + 7]) * inv);
+          if (whole) *reinterpret_cast<uint4*>(rowp + ((((c & 1) * 4 + g) ^ (lane & 7)) << 4)) = w;
+          else if (q_idx < T) *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = w;
         }
       }
-      // one arrival per warp: hundreds of threads arriving on one mbarrier serialise on it
-      tc_fence_before();
-      fence_proxy_async_smem();          // P visible to the tensor core's async proxy
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(s_empty); mbar_arrive(p_full); }   // S reusable, P ready
-      l_part = l_part * alpha + rs;
-      m_run = m_new;
-      if (a.thr16 && j + 1 < nkv) make_keep(j + 1);
-      // fold in this tile's PV (this thread's HD/2 output columns)
-      if (!mbar_wait(pv_full, j & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
+      if (a.lse && q_idx < T)
+        a.lse[(static_cast<long long>(b) * a.H + h) * a.T + q_idx] = m_ref * a.scale + logf(l);
+      if (whole) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
 #pragma unroll
-      for (int c = 0; c < OC / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tPV + lane_addr + hf * OC + c * 32, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c * 32 + i] = o[c * 32 + i] * alpha + __uint_as_float(v[i]);
+          for (int p = 0; p < PANELS; ++p)
+            tma_store_2d(&tmO, sQ + p * 16384 + warp * 4096, h * HD + p * 64, first + qt * AT_BM + warp * 32);
+          tma_store_commit();
+          tma_store_wait_read<0>();                // the staging tile outlives the read
+        }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(pv_empty);
-    }
-    // total row sum = sum of the two halves' partial sums: half 1 publishes its part, half 0 adds
-    // its own and publishes the total (two rounds through the same slot)
-    if (ok) {
-      float* fs = reinterpret_cast<float*>(s_stat);
-      if (hf == 1) fs[r] = l_part;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(xchg);
-      if (!mbar_wait(xchg, nkv & 1, abort_flag)) ok = false;
-      if (ok && hf == 0) { l_part += fs[r]; fs[r] = l_part; }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(xchg);
-      if (ok && !mbar_wait(xchg, (nkv + 1) & 1, abort_flag)) ok = false;
-      if (ok && hf == 1) l_part = fs[r];
-    }
-    if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
-    if (ok && (a.T & 127) == 0) {
-      // Whole tile in range: the warp stages its 32 rows x HD/2 columns in the (now idle) P tile
-      // and stores them with one TMA store.  Direct stores of 64-byte row pieces one row pitch
-      // apart keep the load/store unit busy far longer than the bytes justify.
-      const float inv = 1.f / l_part;
-      constexpr int ROW_BYTES = OC * 2;                 // 64 (64B swizzle) or 128 (128B swizzle)
-      uint8_t* stg = sP + warp * (32 * ROW_BYTES);
-      uint8_t* rowp = stg + lane * ROW_BYTES;
-      const int sw = ROW_BYTES == 64 ? ((lane >> 1) & 3) : (lane & 7);
-#pragma unroll
-      for (int g = 0; g < OC / 8; ++g) {
-        uint4 w;
-        w.x = pack_bf16x2(o[g * 8 + 0] * inv, o[g * 8 + 1] * inv);
-        w.y = pack_bf16x2(o[g * 8 + 2] * inv, o[g * 8 + 3] * inv);
-        w.z = pack_bf16x2(o[g * 8 + 4] * inv, o[g * 8 + 5] * inv);
-        w.w = pack_bf16x2(o[g * 8 + 6] * inv, o[g * 8 + 7] * inv);
-        *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) = w;
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_2d(&tmO, stg, h * HD + hf * OC, b * a.T + qt * AT_BM + (warp & 3) * 32);
-        tma_store_commit();
-      }
-      if (a.lse && hf == 0) a.lse[(static_cast<long long>(b) * a.H + h) * a.T + q_idx] = m_run * a.scale + logf(l_part);
-      if (lane == 0) tma_store_wait_read<0>();          // the staging tile outlives the read
-    } else if (ok && q_idx < a.T) {
-      const float inv = 1.f / l_part;
-      __nv_bfloat16* orow = a.out + (static_cast<long long>(b) * a.T + q_idx) * d_model + h * HD + hf * OC;
-#pragma unroll
-      for (int g = 0; g < OC / 8; ++g) {
-        uint4 w;
-        w.x = pack_bf16x2(o[g * 8 + 0] * inv, o[g * 8 + 1] * inv);
-        w.y = pack_bf16x2(o[g * 8 + 2] * inv, o[g * 8 + 3] * inv);
-        w.z = pack_bf16x2(o[g * 8 + 4] * inv, o[g * 8 + 5] * inv);
-        w.w = pack_bf16x2(o[g * 8 + 6] * inv, o[g * 8 + 7] * inv);
-        *reinterpret_cast<uint4*>(orow + g * 8) = w;
-      }
-      if (a.lse && hf == 0) a.lse[(static_cast<long long>(b) * a.H + h) * a.T + q_idx] = m_run * a.scale + logf(l_part);
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == FWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+  if (warp == FWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
 }  // namespace ab
@@ -668,13 +691,13 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
                             cudaStream_t stream);   // attn_bwd_fused.cu
 
 template <int HD>
-static int launch_attn_fwd(const CUtensorMap& tm, const AttnArgs& a, cudaStream_t stream) {
-  // output map: boxes of 32 rows x HD/2 columns (one math warp's share of a query tile)
+static int launch_attn_fwd(const CUtensorMap& tm, const AttnArgs& a, uint64_t rows, int dependent,
+                           cudaStream_t stream) {
+  // output map: boxes of 32 rows x 64 columns (half a math warp's rows at head_dim 128)
   CUtensorMap tmo;
-  const int rc_o = make_tmap_2d_sw(&tmo, a.out, (uint64_t)a.B * a.T, (uint64_t)a.H * HD, (uint64_t)a.H * HD,
-                                   32, HD / 2, 2, HD);   // HD/2 bf16 columns = HD bytes per row
+  const int rc_o = make_tmap_2d_sw(&tmo, a.out, rows, (uint64_t)a.H * HD, (uint64_t)a.H * HD, 32, 64, 2, 128);
   if (rc_o) return rc_o;
-  constexpr int SMEM = 5 * 128 * HD * 2 + 128 * 128 * 2 + 1024;
+  constexpr int SMEM = FwdCfg<HD>::SMEM;
   auto kern = attn_fwd_kernel<HD>;
   static PerDeviceOnce attr;
   if (attr.first_use_on_device()) {
@@ -687,6 +710,19 @@ static int launch_attn_fwd(const CUtensorMap& tm, const AttnArgs& a, cudaStream_
     attr.mark_device();
   }
   dim3 grid((a.T + 127) / 128, a.H, a.B);
+  if (dependent) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(FWD_THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, tm, tmo, a);
+  }
   launch_chained(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, a);
   return (int)cudaGetLastError();
 }
@@ -726,8 +762,25 @@ int ab_attn_fwd(const void* qkv, void* out, float* lse, unsigned int* drop_mask,
   AttnArgs a;
   a.B = B; a.T = T; a.H = H; a.hd = hd; a.scale = scale; a.seed = seed; a.stream_id = stream_id;
   a.thr16 = thr16; a.out = (__nv_bfloat16*)out; a.lse = lse; a.status = status; a.salt = seed_salt_ptr();
-  a.drop_mask = drop_mask;
-  return hd == 64 ? launch_attn_fwd<64>(tm, a, stream) : launch_attn_fwd<128>(tm, a, stream);
+  a.drop_mask = drop_mask; a.row0 = nullptr;
+  const uint64_t rows = (uint64_t)B * T;
+  return hd == 64 ? launch_attn_fwd<64>(tm, a, rows, 0, stream) : launch_attn_fwd<128>(tm, a, rows, 0, stream);
+}
+
+// The same over a packed batch without padding (inference: no dropout, no log-sum-exp): sequence b is
+// rows [row0[b], row0[b+1]) of qkv [rows, 3*H*hd]; T = longest sequence.  `dependent`: launched as a
+// programmatic dependent of the kernel before it.
+int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
+                       int dependent, int* status, cudaStream_t stream) {
+  using namespace ab;
+  if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || rows < B || !row0) return -1;
+  CUtensorMap tm;
+  int rc = make_tmap_2d(&tm, qkv, (uint64_t)rows, 3ull * H * hd, 3ull * H * hd, 128, 64, 2, true);
+  if (rc) return rc;
+  AttnArgs a = {};
+  a.B = B; a.T = T; a.row0 = row0; a.H = H; a.hd = hd; a.scale = scale; a.out = (__nv_bfloat16*)out; a.status = status;
+  return hd == 64 ? launch_attn_fwd<64>(tm, a, rows, dependent, stream)
+                  : launch_attn_fwd<128>(tm, a, rows, dependent, stream);
 }
 
 // delta: fp32 scratch [B,H,T] owned by the caller.  drop_mask (optional): the keep bits the forward
