@@ -22,6 +22,7 @@ import math
 import os
 import re
 
+import numpy as np
 import torch
 import torch.nn as nn
 
@@ -262,6 +263,10 @@ class B200Engine:
         if (l, key) not in self._moe_layers:
             self._moe_layers[(l, key)] = MoELayer(self._moe_ctx[key], self.layers[l], train)
         return self._moe_layers[(l, key)]
+
+    @property
+    def dense(self) -> bool:
+        return not any(L["moe"] for L in self.layers)
 
     def moe_stats(self) -> dict | None:
         """Routing statistics of the last training forward pass of this rank (None for a dense
@@ -677,6 +682,66 @@ class B200Engine:
             lo = self.loss_out.clone()
             out.update(loss=lo[0], lm_loss=lo[1], value_loss=lo[2], time_loss=lo[3])
         return out
+
+    @torch.no_grad()
+    def infer_last(self, rows: list, kv=None) -> tuple[torch.Tensor, torch.Tensor | None, torch.Tensor | None]:
+        """Inference over token sequences of different lengths (integer arrays of raw ids): logits [n, V]
+        bf16 and, with the scalar heads, value and time [n] fp32 of every sequence's LAST position, on
+        the device.  The sequences lie packed behind one another, so no row is computed for padding.
+        ``kv``: optional ``(k, v)`` caches [layer, sequence, head, slot, head_dim] that receive the keys
+        and values of all positions.  Dense models only."""
+        from ..ops.gemm import num_sms
+        from ..ops.infer import Infer, InferLayer, infer_last
+
+        cfg, dev = self.cfg, self.device
+        assert self.dense
+        n = len(rows)
+        row0 = np.zeros(n + 1, dtype=np.int32)
+        np.cumsum([len(r) for r in rows], out=row0[1:])
+        lens = np.diff(row0)
+        M, T = int(row0[-1]), int(lens.max())
+        assert lens.min() > 0
+        if T > cfg.n_positions:
+            raise ValueError(f"sequence length {T} exceeds the model's {cfg.n_positions} learned positions")
+        d, F, V = cfg.n_embd, cfg.ffn_dim, cfg.vocab_size
+        host = torch.empty(2 * M + 2 * n + 1, dtype=torch.int32, pin_memory=True)
+        block = host.numpy()
+        np.concatenate(rows, out=block[:M], casting="unsafe")
+        block[M:2 * M] = np.arange(M, dtype=np.int32) - np.repeat(row0[:-1], lens)
+        block[2 * M:2 * M + n + 1] = row0
+        block[2 * M + n + 1:] = row0[1:] - 1
+        batch = host.to(dev, non_blocking=True)
+        e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device=dev)
+        f32 = torch.float32
+        scratch = dict(x=e(M, d, dt=f32), ln=e(M, d), qkv=e(M, 3 * d), att=e(M, d), act=e(M, F), x_last=e(n, d, dt=f32),
+                       att_last=e(n, d), h=e(n, d), logits=e(n, V))
+        if self.reg is not None:
+            scratch.update(value=e(n, dt=f32), time=e(n, dt=f32))
+        a = Infer(n_layer=cfg.n_layer, d=d, H=cfg.n_head, hd=cfg.head_dim, F=F, V=V, rms=int(self.rms),
+                  eps=cfg.layer_norm_epsilon, n=n, M=M, T=T, max_ctas=num_sms(), status=_lib.status_word().data_ptr())
+        for name, t in scratch.items():
+            setattr(a, name, t.data_ptr())
+        for name, off in (("ids", 0), ("pos", M), ("row0", 2 * M), ("last", 2 * M + n + 1)):
+            setattr(a, name, batch.data_ptr() + 4 * off)
+        address = lambda t: 0 if t is None else t.data_ptr()
+        for name, t in (("wte", self.wte[0]), ("wpe", self.wpe[0]), ("ctrl", self.ctrl_w[0]), ("lnf_w", self.lnf_w[0]),
+                        ("lnf_b", self.lnf_b[0]), ("wte_bf16", self.wte[1])):
+            setattr(a, name, address(t))
+        if self.reg is not None:
+            for name, t in (("wv", self.wv[0]), ("bv", self.bv[0]), ("wt", self.wt[0]), ("bt", self.bt[0])):
+                setattr(a, name, t.data_ptr())
+        if kv is not None:
+            k, v = kv
+            a.kc, a.vc, a.kv_layer, a.S = k.data_ptr(), v.data_ptr(), k.stride(0), k.shape[3]
+        # GEMM weights are read as bf16, norms and biases as fp32
+        layers = (InferLayer * cfg.n_layer)()
+        for dst, L in zip(layers, self.layers):
+            for name in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_b", "o_b", "fc_b", "pr_b"):
+                setattr(dst, name, address(L[name][0]))
+            for name in ("qkv_w", "o_w", "fc_w", "pr_w"):
+                setattr(dst, name, L[name][1].data_ptr())
+        infer_last(a, layers)
+        return scratch["logits"], scratch.get("value"), scratch.get("time")
 
     def zero_grad(self) -> None:
         self.arena.grad.zero_()

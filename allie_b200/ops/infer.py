@@ -1,0 +1,32 @@
+"""Binding of the native inference schedule (``csrc/infer.cu``): one forward pass over a packed batch
+whose last positions are the only outputs."""
+from __future__ import annotations
+
+import ctypes
+from ctypes import c_float, c_int, c_longlong, c_void_p
+
+from . import _lib
+from ._lib import stream_ptr
+
+
+class InferLayer(ctypes.Structure):
+    """``AbInferLayer``."""
+    _fields_ = [(n, c_void_p) for n in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_w", "qkv_b", "o_w", "o_b",
+                                        "fc_w", "fc_b", "pr_w", "pr_b")]
+
+
+class Infer(ctypes.Structure):
+    """``AbInfer``."""
+    _fields_ = ([(n, c_int) for n in ("n_layer", "d", "H", "hd", "F", "V", "rms")] + [("eps", c_float)]
+                + [(n, c_void_p) for n in ("wte", "wpe", "ctrl", "lnf_w", "lnf_b", "wte_bf16", "wv", "bv", "wt", "bt")]
+                + [(n, c_int) for n in ("n", "M", "T")]
+                + [(n, c_void_p) for n in ("ids", "pos", "row0", "last", "x", "ln", "qkv", "att", "act", "x_last",
+                                           "att_last", "h", "logits", "value", "time", "kc", "vc")]
+                + [("kv_layer", c_longlong), ("S", c_int), ("max_ctas", c_int), ("status", c_void_p)])
+
+
+def infer_last(args: Infer, layers) -> None:
+    rc = _lib.cuda().ab_infer_last(ctypes.byref(args), layers, stream_ptr())
+    if rc < 0:
+        raise RuntimeError(f"ab_infer_last failed with code {rc} (n={args.n} M={args.M} T={args.T})")
+    _lib.count_launches(rc)

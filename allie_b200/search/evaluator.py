@@ -70,14 +70,31 @@ class KVLeafEvaluator:
         eng, n = self.eng, self.n
         assert len(token_rows) == n
         lens = [len(r) for r in token_rows]
-        Lp = max(lens)
-        assert Lp <= self.max_prefix
+        assert max(lens) <= self.max_prefix
+        if eng.dense and min(lens) > 0:
+            d = eng.cfg.head_dim
+            shape = (eng.cfg.n_layer, n, eng.cfg.n_head, self.S, d)
+            logits, value, time = eng.infer_last(token_rows, (self.kc.view(shape), self.vc.view(shape)))
+        else:
+            logits, value, time = self._prefill_padded(token_rows, lens)
+        # one device-to-host copy
+        V = logits.size(1)
+        out = torch.zeros(n, V + 2, dtype=torch.float32, device=eng.device)
+        out[:, :V] = logits
+        if eng.reg is not None:
+            out[:, V], out[:, V + 1] = value, time
+        out = out.cpu()
+        self.view(self.req_host, "prefix_len").copy_(torch.tensor(lens, dtype=torch.int32))
+        return out[:, :V], out[:, V], out[:, V + 1]
+
+    def _prefill_padded(self, token_rows, lens):
+        """The same for models with experts, whose buffers are laid out for a fixed number of rows."""
+        eng, n, Lp = self.eng, self.n, max(lens)
         pad = eng.cfg.pad_token_id if eng.cfg.pad_token_id is not None else 0
         ids = np.full((n, Lp), pad, dtype=np.int64)
         for i, r in enumerate(token_rows):
             ids[i, :len(r)] = r
-        batch = {"input_ids": torch.from_numpy(ids)}
-        B, T = eng.load_batch(batch, False)
+        B, T = eng.load_batch({"input_ids": torch.from_numpy(ids)}, False)
         len_dev = torch.tensor(lens, dtype=torch.int32, device=eng.device)
         d = eng.cfg.n_embd
 
@@ -89,13 +106,8 @@ class KVLeafEvaluator:
 
         buf = eng.forward(B, T, False, 0, False, False, kv_hook=hook)
         rows = torch.arange(n, device=eng.device) * Lp + (len_dev.long() - 1)
-        logits = buf["logits"][rows].float().cpu()
-        if eng.reg is not None:
-            value, time = buf["value"][rows].cpu(), buf["time"][rows].cpu()
-        else:
-            value = time = torch.zeros(n)
-        self.view(self.req_host, "prefix_len").copy_(torch.tensor(lens, dtype=torch.int32))
-        return logits, value, time
+        return (buf["logits"][rows], buf["value"][rows] if eng.reg is not None else None,
+                buf["time"][rows] if eng.reg is not None else None)
 
     # --------------------------------------------------------------------- step
     def _launch_step(self) -> None:

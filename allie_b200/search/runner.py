@@ -11,6 +11,7 @@ from __future__ import annotations
 import weakref
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from ..data import Game, UCITokenizer
@@ -86,16 +87,25 @@ class EngineRunner(ModelRunner):
     @torch.no_grad()
     def evaluate(self, games: list[Game]) -> Evaluation:
         self.calls += 1
-        batch = self.tokenizer.pad_and_collate(list(games), return_labels=False)
-        out = self.engine.evaluate_batch(batch, with_loss=False)
-        idx = _last_index(batch).to(self.engine.device)
-        rows = torch.arange(len(games), device=idx.device)
-        V = out["logits"].size(-1)
-        packed = torch.empty(len(games), V + 2, dtype=torch.float32, device=idx.device)
-        packed[:, :V] = out["logits"][rows, idx].float()
+        games, eng, n = list(games), self.engine, len(games)
+        if eng.dense and games and not isinstance(games[0], np.ndarray):
+            words = [self.tokenizer.tokenize(g)[: self.tokenizer.max_length] for g in games]
+            assert all(int(((w & 0xFFFF) >> 14).max()) < 3 for w in words)
+            logits, value, time = eng.infer_last([w & 0x3FFF for w in words])
+        else:      # experts are laid out for a fixed number of rows; arrays come as equal windows already
+            batch = self.tokenizer.pad_and_collate(games, return_labels=False)
+            out = eng.evaluate_batch(batch, with_loss=False)
+            idx = _last_index(batch).to(eng.device)
+            rows = torch.arange(n, device=eng.device)
+            logits = out["logits"][rows, idx]
+            value, time = ((out["value_logits"][rows, idx], out["time_logits"][rows, idx]) if self.has_value_head
+                           else (None, None))
+        V = logits.size(-1)
+        packed = torch.empty(n, V + 2, dtype=torch.float32, device=eng.device)
+        packed[:, :V] = logits
         if self.has_value_head:
-            packed[:, V] = out["value_logits"][rows, idx]
-            packed[:, V + 1] = out["time_logits"][rows, idx]
+            packed[:, V] = value
+            packed[:, V + 1] = time
         else:
             packed[:, V:] = 0
         host = packed.cpu()          # the one device-to-host copy of this evaluation
