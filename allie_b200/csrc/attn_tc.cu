@@ -2,28 +2,30 @@
 //
 // One CTA owns one 128-row query tile of one (batch, head); two CTAs share an SM.  Per 128-row
 // key/value tile:
-//   warp 5 (one thread) : S = Q K^T          -> TMEM (128 lanes = query rows, 128 fp32 columns)
-//   warps 0-3           : one thread per query row: the whole row of S in registers, maximum, exponentials,
-//                         dropout, P -> TMEM as packed bf16 (the A operand of the second product)
-//   warp 5              : O += P V           -> TMEM
-//   warp 4 (one thread) : TMA loads of Q once and K/V tiles through a ring
+//   warp 9 (one thread) : S = Q K^T          -> TMEM (128 lanes = query rows, 128 fp32 columns)
+//   warps 0-7           : two threads per query row, 64 keys each: S in registers, maximum (exchanged
+//                         through shared memory), exponentials, dropout, P -> TMEM as packed bf16 (the A
+//                         operand of the second product)
+//   warp 9              : O += P V           -> TMEM
+//   warp 8 (one thread) : TMA loads of Q once and K/V tiles through a ring
 // Q, K and V are read straight out of the packed [B*T, 3*d] QKV activation with 2-D TMA boxes
 // (64 columns x 128 rows), and O is written in the [B*T, d] layout the projection GEMM reads.
 // V is consumed MN-major (rows = keys), so no transposes exist anywhere.
 //
-// What bounds it: the exponential unit (16 per SM and clock: 1024 clocks per tile pair against 512 of
-// the tensor core) and, with dropout, instruction issue (the generator is 8 of about 13 instructions
-// per element).  So nothing else may cost instructions or waits per element: S is read once (a row
-// per thread needs no exchange of maxima between warps), P never passes through shared memory, and O
-// stays in TMEM, rescaled there when the maximum of one of a warp's rows has grown.  (Keeping the old
-// scale until the maximum has grown by 2^8 saves little at these lengths and gives up that the largest
-// probability of a row is exactly one: error against 64 bits 0.00195 instead of 0.00181.)  The
-// reciprocal of the keep probability is applied at the end, too.
+// What bounds it: with dropout, instruction issue (17 per element, half of them the generator) and how
+// much of it the warps of an SM can overlap; without, latencies and then the exponential unit (16 per SM
+// and clock).  So: sixteen math warps per SM (with one thread per row, eight, issue was 39 % busy), S
+// is read once, P never passes through shared memory, O stays in TMEM and is rescaled there when the
+// maximum of one of a warp's rows has grown, and unrolled code stays small (fetching instructions was
+// a fifth of the stalls with 128 keys per thread).  Keeping the old scale until the maximum has grown
+// by 2^8 saves little at these lengths and gives up that the largest probability of a row is exactly
+// one: error against 64 bits 0.00195 instead of 0.00181.  The reciprocal of the keep probability is
+// applied at the end.
 #include "attn_common.cuh"
 
 namespace ab {
 
-constexpr int FWD_MATH_WARPS = 4;
+constexpr int FWD_MATH_WARPS = 8;
 constexpr int FWD_TMA_WARP = FWD_MATH_WARPS;
 constexpr int FWD_MMA_WARP = FWD_MATH_WARPS + 1;
 constexpr int FWD_THREADS = (FWD_MATH_WARPS + 2) * 32;
@@ -39,7 +41,7 @@ struct FwdCfg {
   static constexpr int STAGES = HD == 128 ? 1 : 2;
   static constexpr int TM_P = P_IN_S ? 0 : 128;
   static constexpr int TM_O = 256 - HD;
-  static constexpr int SMEM = (1 + 2 * STAGES) * TILE_BYTES + 256;
+  static constexpr int SMEM = (1 + 2 * STAGES) * TILE_BYTES + 256 + 2048;
 };
 
 // 16 AND-masks (one per packed bf16 pair) of 32 keep bits: the bit of each element is shifted into
@@ -93,8 +95,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   uint64_t* s_empty = bars + 10;
   uint64_t* p_full = bars + 11;
   uint64_t* pv_full = bars + 12;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* xchg = bars + 13;               // 4: the two warps of a TMEM lane quarter
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* s_row = reinterpret_cast<float*>(sV + STAGES * TILE_BYTES + 256);    // [2][2 halves][128] row values
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d_model = a.H * HD;
@@ -107,6 +111,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     }
     mbar_init(s_full, 1); mbar_init(s_empty, FWD_MATH_WARPS);
     mbar_init(p_full, FWD_MATH_WARPS); mbar_init(pv_full, 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&xchg[i], 2);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQKV);
@@ -186,46 +191,51 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     }
   } else {
     // ---------------------------------------------------- softmax / output warps
-    const int r = warp * 32 + lane;               // query row inside the tile = TMEM lane
+    const int quad = warp & 3, hf = warp >> 2;    // TMEM lane quarter; half of the keys and of O's columns
+    const int r = quad * 32 + lane;               // query row inside the tile = TMEM lane
     const int q_idx = qt * AT_BM + r;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    constexpr int OC = HD / 2;
+    // k-th meeting of the two warps of a lane quarter (bounded, one arrival per warp)
+    auto pair_sync = [&](int k) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&xchg[quad]);
+      return mbar_wait(&xchg[quad], k & 1, abort_flag);
+    };
     const float sl2 = a.scale * LOG2E;
     const uint64_t sl2_2 = f2_bcast(sl2);
     float m_ref = 0.f;                            // running maximum, which P and O are scaled to
-    // row sums of the two column halves, each added up in column order
-    float l_half[2] = {0.f, 0.f};
-    const uint64_t row_elem0 = (static_cast<uint64_t>(b * a.H + h) * a.T + q_idx) * a.T;
+    float l_run = 0.f;                            // row sum of this half's keys
+    const uint64_t row_elem0 = (static_cast<uint64_t>(b * a.H + h) * a.T + q_idx) * a.T + hf * 64;
     const uint64_t seed = a.thr16 ? salted(a.seed, a.salt) : 0;
     bool ok = true;
     for (int j = 0; j < nkv; ++j) {
-      // dropout keep bits of this row's 128 keys; they are also what the backward pass reads back
-      uint32_t keep[4];
+      // dropout keep bits of this thread's 64 keys; they are also what the backward pass reads back
+      uint32_t keep[2] = {0u, 0u};
       if (a.thr16) {
         const uint64_t e0 = row_elem0 + static_cast<uint64_t>(j) * AT_BN;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t word = 0;
+        for (int c = 0; c < 2; ++c) {
 #pragma unroll
           for (int g = 0; g < 4; ++g)
-            word |= dropout_keep8(seed, a.stream_id, (e0 >> 3) + c * 4 + g, a.thr16) << (8 * g);
-          keep[c] = word;
+            keep[c] |= dropout_keep8(seed, a.stream_id, (e0 >> 3) + c * 4 + g, a.thr16) << (8 * g);
         }
         if (a.drop_mask && q_idx < T) {
           uint32_t* dst = a.drop_mask + (e0 >> 5);
-          if ((T & 127) == 0) {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(keep[0], keep[1], keep[2], keep[3]);
+          if ((T & 63) == 0) {
+            if (j * AT_BN + hf * 64 < T) *reinterpret_cast<uint2*>(dst) = make_uint2(keep[0], keep[1]);
           } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (j * AT_BN + c * 32 < T) dst[c] = keep[c];
+            for (int c = 0; c < 2; ++c)
+              if (j * AT_BN + hf * 64 + c * 32 < T) dst[c] = keep[c];
           }
         }
       }
       if (!mbar_wait(s_full, j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      uint32_t v[128];
+      uint32_t v[64];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tS + lane_addr + c * 32, v + c * 32);
+      for (int c = 0; c < 2; ++c) tmem_ld32(tS + lane_addr + hf * 64 + c * 32, v + c * 32);
       tmem_ld_wait();
       if (!C::P_IN_S) {
         tc_fence_before();
@@ -234,14 +244,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       }
       if (j == qt) {                               // diagonal tile: keys after the row's own position
 #pragma unroll
-        for (int i = 0; i < 128; ++i) v[i] = i <= r ? v[i] : 0xff800000u;
+        for (int i = 0; i < 64; ++i) v[i] = hf * 64 + i <= r ? v[i] : 0xff800000u;
       }
       float mx4[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) mx4[k] = __uint_as_float(v[k]);
 #pragma unroll
-      for (int i = 4; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));   // finite: key 0 is never masked
+      for (int i = 4; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
+      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      // the other half's maximum (slots alternate: one is rewritten only after the meeting of the tile
+      // between, which its reader has passed)
+      float* slot = s_row + (j & 1) * 256;
+      slot[hf * 128 + r] = mx;
+      if (!pair_sync(j)) { ok = false; break; }
+      mx = fmaxf(mx, slot[(hf ^ 1) * 128 + r]);    // finite: key 0 is never masked
       float grow = 1.f;                            // what sums and O are multiplied by
       if (j == 0) {
         m_ref = mx;
@@ -253,9 +269,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         const uint64_t f = f2_bcast(grow);
         m_ref = m_new;
 #pragma unroll 1
-        for (int c = 0; c < HD / 16; ++c) {
+        for (int c = 0; c < OC / 16; ++c) {
           uint32_t o[16];
-          tmem_ld16(tO + lane_addr + c * 16, o);
+          tmem_ld16(tO + lane_addr + hf * OC + c * 16, o);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -264,13 +280,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             o[2 * i] = __float_as_uint(lo);
             o[2 * i + 1] = __float_as_uint(hi);
           }
-          tmem_st16(tO + lane_addr + c * 16, o);
+          tmem_st16(tO + lane_addr + hf * OC + c * 16, o);
         }
       }
       const uint64_t mb = f2_bcast(-m_ref * sl2);
-      float rs[2] = {0.f, 0.f};
+      float rs = 0.f;                              // added up in column order
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -279,8 +295,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     x0, x1);
           x0 = ex2_fast(x0);
           x1 = ex2_fast(x1);
-          rs[c >> 1] += x0;
-          rs[c >> 1] += x1;
+          rs += x0;
+          rs += x1;
           w[i] = pack_bf16x2(x0, x1);
         }
         if (a.thr16) {
@@ -292,15 +308,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         // P of the tile before is read by its product until that completes
         if (c == 0 && j > 0 && !mbar_wait(pv_full, (j - 1) & 1, abort_flag)) { ok = false; break; }
         if (c == 0) tc_fence_after();
-        tmem_st16(tP + lane_addr + c * 16, w);
+        tmem_st16(tP + lane_addr + hf * 32 + c * 16, w);
       }
       if (!ok) break;
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);          // one arrival per warp
-      l_half[0] = l_half[0] * grow + rs[0];
-      l_half[1] = l_half[1] * grow + rs[1];
+      l_run = l_run * grow + rs;
     }
     if (ok && !mbar_wait(pv_full, (nkv - 1) & 1, abort_flag)) ok = false;
     if (!ok) {
@@ -308,18 +323,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL);
     } else {
       tc_fence_after();
-      const float l = l_half[0] + l_half[1];
+      // slot nkv & 1: last read before the meeting of tile nkv - 1
+      float* slot = s_row + (nkv & 1) * 256;
+      slot[hf * 128 + r] = l_run;
+      ok = pair_sync(nkv);
+      const float l = slot[r] + slot[128 + r];
       const float inv = dropout_scale(a.thr16) / l;
-      // The warp's 32 rows leave through the (now idle) Q tile with one TMA store per 64 columns; a
-      // warp with rows past the end of the sequence stores row by row.
-      const bool whole = qt * AT_BM + warp * 32 + 32 <= T;
-      __nv_bfloat16* orow = a.out + (static_cast<long long>(first) + q_idx) * d_model + h * HD;
+      // The warps' 32 rows leave through the (now idle) Q tile with one TMA store per 64 columns; warps
+      // with rows past the end of the sequence store row by row.
+      const bool whole = qt * AT_BM + quad * 32 + 32 <= T;
+      __nv_bfloat16* orow = a.out + (static_cast<long long>(first) + q_idx) * d_model + h * HD + hf * OC;
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
+      for (int c = 0; c < OC / 32; ++c) {
         uint32_t o[32];
-        tmem_ld32(tO + lane_addr + c * 32, o);
+        tmem_ld32(tO + lane_addr + hf * OC + c * 32, o);
         tmem_ld_wait();
-        uint8_t* rowp = sQ + (c >> 1) * 16384 + warp * 4096 + lane * 128;
+        const int col8 = (hf * OC + c * 32) / 8;                  // first 16-byte chunk of the row
+        uint8_t* rowp = sQ + (col8 >> 3) * 16384 + quad * 4096 + lane * 128;
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           uint4 w;
@@ -327,23 +347,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           w.y = pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv);
           w.z = pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv);
           w.w = pack_bf16x2(__uint_as_float(o[g * 8 + 6]) * inv, __uint_as_float(o[g * 8 + 7]) * inv);
-          if (whole) *reinterpret_cast<uint4*>(rowp + ((((c & 1) * 4 + g) ^ (lane & 7)) << 4)) = w;
+          if (whole) *reinterpret_cast<uint4*>(rowp + ((((col8 & 7) + g) ^ (lane & 7)) << 4)) = w;
           else if (q_idx < T) *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = w;
         }
       }
-      if (a.lse && q_idx < T)
+      if (a.lse && hf == 0 && q_idx < T)
         a.lse[(static_cast<long long>(b) * a.H + h) * a.T + q_idx] = m_ref * a.scale + logf(l);
       if (whole) {
         fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-#pragma unroll
-          for (int p = 0; p < PANELS; ++p)
-            tma_store_2d(&tmO, sQ + p * 16384 + warp * 4096, h * HD + p * 64, first + qt * AT_BM + warp * 32);
+        ok = pair_sync(nkv + 1) && ok;
+        // head_dim 64: one panel of both halves; 128: each half filled a panel of its own
+        if (ok && lane == 0 && hf < PANELS) {
+          tma_store_2d(&tmO, sQ + hf * 16384 + quad * 4096, h * HD + hf * 64, first + qt * AT_BM + quad * 32);
           tma_store_commit();
           tma_store_wait_read<0>();                // the staging tile outlives the read
         }
       }
+      if (!ok) { *abort_flag = ST_TIMEOUT_MISC; atomicCAS(a.status, 0, ST_TIMEOUT_MISC); }
     }
   }
   tc_fence_before();
