@@ -245,7 +245,6 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
         }
       }
       if (!mbar_wait(sdp_full, it & 1, abort_flag)) { ok = false; break; }
-      if (it > 0 && !mbar_wait(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
@@ -254,6 +253,13 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
         tmem_ld16(tS + lane_addr + col0, sv);
         tmem_ld16(tDP + lane_addr + col0, dv);
         tmem_ld_wait();
+        if (hf == 1) {
+          // S and dP are in registers: handed back before the math of the second half, so the tensor
+          // core computes the next pair's under it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sdp_empty);
+        }
         float p[16], ds[16];
         const uint32_t k16 = keep32 >> (hf * 16);
         if (a.thr16) {
@@ -263,6 +269,8 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
           if (diag) fb_math16<true, false>(sv, dv, p, ds, r, col0, sl2, lse_l2, dlt * a.scale, a.scale, dscale, k16);
           else      fb_math16<false, false>(sv, dv, p, ds, r, col0, sl2, lse_l2, dlt * a.scale, a.scale, dscale, k16);
         }
+        // the shared P / dS tiles feed the previous pair's products until pds_empty completes
+        if (hf == 0 && it > 0 && !mbar_wait(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
         const uint32_t poff = (col0 >> 6) * 16384;
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
@@ -276,11 +284,12 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
           *reinterpret_cast<uint4*>(sDS + off) = w;
         }
       }
+      if (!ok) break;
       // one arrival per warp: hundreds of threads arriving on one mbarrier serialise on it
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(sdp_empty); mbar_arrive(pds_full); }
+      if (lane == 0) mbar_arrive(pds_full);
       // the previous pair's dQ tile finished long ago: drain it while the tensor core works
       if (it > 0) ok = drain_dq(it - 1);
     }
@@ -656,6 +665,13 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
         tmem_ld16(tS + lane_addr + col0, sv);
         tmem_ld16(tDP + lane_addr + col0, dv);
         tmem_ld_wait();
+        if (hf == 1) {
+          // S and dP are in registers: handed back before the math of the second half, so the tensor
+          // core computes the next pair's under it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sdp_empty);
+        }
         float pp[16], ds[16];
         const uint32_t k16 = keep32 >> (hf * 16);
         if (a.thr16) {
@@ -687,7 +703,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(sdp_empty); mbar_arrive(pds_full); }
+      if (lane == 0) mbar_arrive(pds_full);
       // work left over from the previous pair, done while the tensor core runs this one
       if (p.g > 0) {
         ok = drain_dq(p.g - 1, prev_row0, prev_h);
