@@ -767,6 +767,16 @@ static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& td, const A
 
 extern "C" {
 
+// delta[b][h][t] = sum over the head's columns of dO * O (o, dout: bf16 [B*T, H*hd])
+int ab_attn_delta(const void* o, const void* dout, float* delta, int B, int T, int H, int hd, cudaStream_t stream) {
+  using namespace ab;
+  if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || H <= 0) return -1;
+  const long long n = (long long)B * T * H * (hd / 8);
+  launch_chained(attn_delta_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream,
+                 (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, T, H, hd);
+  return (int)cudaGetLastError();
+}
+
 // qkv: bf16 [B*T, 3*H*hd]; out: bf16 [B*T, H*hd]; lse: fp32 [B,H,T] (may be null).
 // hd must be 64 or 128.  With dropout (thr16 > 0) T must be a multiple of 8.
 // drop_mask (optional): uint32 [B,H,T,T/32], receives the dropout keep bits (needs T % 32 == 0).
@@ -806,10 +816,11 @@ int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T
 // delta: fp32 scratch [B,H,T] owned by the caller.  drop_mask (optional): the keep bits the forward
 // pass wrote.  dq_acc (optional, hd == 64): fp32 [B*T, H*hd] accumulator that must be all zero on
 // entry and is all zero again on return; when given, the single-kernel backward runs.
+// delta_ready: delta already holds the row sums of dO * O.
 int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* dout, void* dqkv,
                 float* delta, const unsigned int* drop_mask, float* dq_acc, int B, int T, int H, int hd,
                 float scale, unsigned long long seed, unsigned int stream_id, unsigned int thr16,
-                int* status, cudaStream_t stream) {
+                int delta_ready, int* status, cudaStream_t stream) {
   using namespace ab;
   if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || (thr16 && (T & 7))) return -1;
   if (drop_mask && (T & 31)) return -1;
@@ -818,9 +829,7 @@ int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* 
   if (rc) return rc;
   rc = make_tmap_2d(&td, dout, (uint64_t)B * T, (uint64_t)H * hd, (uint64_t)H * hd, 128, 64, 2, true);
   if (rc) return rc;
-  const long long n = (long long)B * T * H * (hd / 8);
-  launch_chained(attn_delta_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream,
-                 (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, T, H, hd);
+  if (!delta_ready && (rc = ab_attn_delta(out, dout, delta, B, T, H, hd, stream)) != 0) return rc;
   AttnBwdArgs a;
   a.B = B; a.T = T; a.H = H; a.hd = hd; a.scale = scale; a.seed = seed; a.stream_id = stream_id;
   a.thr16 = thr16; a.lse = lse; a.delta = delta; a.dqkv = (__nv_bfloat16*)dqkv; a.status = status;
@@ -875,5 +884,5 @@ extern "C" int ab_attn_bwd_static(const void* qkv, const void* out, const float*
     g_attn_static_ptr[dev].store(scratch, std::memory_order_release);
   }
   return ab_attn_bwd(qkv, out, lse, dout, dqkv, scratch, drop_mask, nullptr, B, T, H, hd,
-                     scale, seed, stream_id, thr16, status, stream);
+                     scale, seed, stream_id, thr16, 0, status, stream);
 }

@@ -160,6 +160,7 @@ enum EpiKind : int {
   EPI_MUL,         // bf16 out = . * aux tile (aux_grad), aux staged by TMA
   EPI_RESID,       // fp32 out = dropout(. + bias) + residual, residual staged by TMA
   EPI_ACCUM,       // fp32 out += .
+  EPI_DOT,         // bf16 out, and per row and 64 columns its product with the aux tile (staged by TMA)
 };
 
 // which specialised drain an epilogue description fits (aux_tma as chosen by the launcher)
@@ -171,6 +172,7 @@ inline EpiKind epi_kind(const GemmArgs& g) {
   if (ep.out_fp32) return EPI_ANY;
   if (ep.act == 0) return EPI_BF16;
   if (ep.act == 3) return EPI_GELU;
+  if (ep.act == 4) return EPI_DOT;       // the entry point has checked the rest
   if (ep.act == 1 && ep.aux_grad) return EPI_GELU_GRAD;
   if (ep.act == 2 && ep.aux_grad && g.aux_tma == 1 && !ep.bias) return EPI_MUL;
   return EPI_ANY;
@@ -201,17 +203,19 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
                                                     Wait wait_tile, Next next_tile) {
   const bool has_bias = g.ep.bias != nullptr;
   const float* bias = g.ep.bias + bias_off;
-  if constexpr (EPI == EPI_BF16 || EPI == EPI_GELU || EPI == EPI_MUL) {
-    // one store group: 64 bf16 columns = 128-byte rows, 128B swizzle.  The aux tile of EPI_MUL
-    // lies in the staging tile already, in the same layout.
+  if constexpr (EPI == EPI_BF16 || EPI == EPI_GELU || EPI == EPI_MUL || EPI == EPI_DOT) {
+    // one store group: 64 bf16 columns = 128-byte rows, 128B swizzle.  The aux tile of EPI_MUL and
+    // EPI_DOT lies in the staging tile already, in the same layout.
+    constexpr bool AUX = EPI == EPI_MUL || EPI == EPI_DOT;
     uint8_t* rowp = stg + lane * 128;
     const int sw = lane & 7;
+    uint64_t dot = 0;                    // EPI_DOT: two partial sums
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       uint32_t r[32];
       tmem_ld32(taddr + half * 32, r);
       if (half == 0) {
-        if constexpr (EPI == EPI_MUL) {
+        if constexpr (AUX) {
           if (!wait_tile()) return false;
         } else {
           if (lane == 0) tma_store_wait_read<0>();        // staging tile free again
@@ -223,7 +227,7 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
       for (int c = 0; c < 4; ++c) {
         const int n = nbase + half * 32 + c * 8;
         uint64_t v[4];
-        epi_load8(r + c * 8, v, bias, n, EPI != EPI_MUL && has_bias && n < g.N);
+        epi_load8(r + c * 8, v, bias, n, !AUX && has_bias && n < g.N);
         uint4* chunk = reinterpret_cast<uint4*>(rowp + (((half * 4 + c) ^ sw) << 4));
         if constexpr (EPI == EPI_GELU) {
 #pragma unroll
@@ -238,6 +242,13 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
         }
         uint4 o = epi_pack8(v);
         if (MASK_ROWS && !row_ok) o = make_uint4(0, 0, 0, 0);
+        if constexpr (EPI == EPI_DOT) {
+          const uint4 q = *chunk;
+          dot = f2_fma(f2_pack(bf16_lo(o.x), bf16_hi(o.x)), f2_pack(bf16_lo(q.x), bf16_hi(q.x)), dot);
+          dot = f2_fma(f2_pack(bf16_lo(o.y), bf16_hi(o.y)), f2_pack(bf16_lo(q.y), bf16_hi(q.y)), dot);
+          dot = f2_fma(f2_pack(bf16_lo(o.z), bf16_hi(o.z)), f2_pack(bf16_lo(q.z), bf16_hi(q.z)), dot);
+          dot = f2_fma(f2_pack(bf16_lo(o.w), bf16_hi(o.w)), f2_pack(bf16_lo(q.w), bf16_hi(q.w)), dot);
+        }
         *chunk = o;
       }
     }
@@ -246,7 +257,38 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
     if (lane == 0) {
       tma_store_2d(&tmOut, stg, nbase, m0w);
       tma_store_commit();
-      if constexpr (EPI == EPI_MUL) {
+    }
+    if constexpr (EPI == EPI_MUL) {
+      if (g.ep.colsum) {
+        // Column sums of the tile just staged (rows past M are zeros): each lane adds up two columns, a
+        // row of shared memory per load, while the store leaves.  The issue slots are free: the tensor
+        // core needs 8192 clocks per 256 x 256 tile at K = 1024, this takes 600 of the epilogue's.  A
+        // pass of its own over 32768 x 4096 took 55 us.
+        uint64_t s2[2] = {0ull, 0ull};
+#pragma unroll 8
+        for (int row = 0; row < 32; ++row) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(
+              stg + row * 128 + (((lane >> 2) ^ (row & 7)) << 4) + (lane & 3) * 4);
+          s2[row & 1] = f2_add(s2[row & 1], f2_pack(bf16_lo(w), bf16_hi(w)));
+        }
+        float a0, a1;
+        f2_unpack(f2_add(s2[0], s2[1]), a0, a1);
+        const int n = nbase + lane * 2;
+        if (n < g.N)
+          asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(g.ep.colsum + n), "f"(a0), "f"(a1) : "memory");
+        __syncwarp();                      // all lanes have read the tile
+      }
+    }
+    if constexpr (EPI == EPI_DOT) {
+      float a0, a1;
+      f2_unpack(dot, a0, a1);
+      if (m < g.M) {
+        const int seq = m / g.ep.dot_T;
+        g.ep.dot_out[(static_cast<long long>(seq) * (g.N >> 6) + (nbase >> 6)) * g.ep.dot_T + (m - seq * g.ep.dot_T)] = a0 + a1;
+      }
+    }
+    if constexpr (AUX) {
+      if (lane == 0) {
         tma_store_wait_read<0>();          // the store has read the staging tile
         next_tile(0);
       }

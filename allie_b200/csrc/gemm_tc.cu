@@ -485,7 +485,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     // (aux_tma == 2) do the same with 32 x 32 fp32 tiles: the second of a unit's two tiles follows
     // when the first has left, the next unit's first one unit ahead.
     static_assert(COLS_PER_WARP == 64, "the staged aux tile is one 64-column store group");
-    const bool stage_aux = EPI == EPI_RESID || EPI == EPI_MUL || (EPI == EPI_ANY && g.aux_tma != 0);
+    const bool stage_aux = EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT || (EPI == EPI_ANY && g.aux_tma != 0);
     uint32_t aux_phase = 0;
     auto fetch_aux = [&](int u, int grp) {          // lane 0; the staging tile must be free
       if (u >= num_units) return;
@@ -544,7 +544,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           if (!epilogue_drain_kind<EPI, false>(g, tmOut, tmAux, taddr, m, m0w, nbase, true, my_stage, lane, 0,
                                                wait_aux, next_tile))
             break;
-        } else if ((EPI == EPI_RESID || EPI == EPI_MUL) && lane == 0) {
+        } else if ((EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT) && lane == 0) {
           fetch_aux(u + num_pairs, 0);
         }
       }
@@ -592,7 +592,7 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   if (ep.act == 1) {
     rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 32, 2, 64);
     if (rc) return rc;
-  } else if (ep.act == 2 && !ep.out_fp32 && !ep.accumulate && g.k_splits == 1 &&
+  } else if ((ep.act == 2 || ep.act == 4) && !ep.out_fp32 && !ep.accumulate && g.k_splits == 1 &&
              (reinterpret_cast<uintptr_t>(ep.aux) & 15) == 0 && (ep.ldaux * 2) % 16 == 0) {
     // the aux tiles travel by TMA in the geometry of the output tiles (see the kernel)
     rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 64, 2, 128);
@@ -623,7 +623,7 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
     launch_chained(kern, dim3(2 * pairs), dim3(NUM_THREADS), SMEM, stream, tmA, tmB, tmOut, tmAux, ga);
     return static_cast<int>(cudaGetLastError());
   };
-  static PerDeviceOnce attr[EPI_ACCUM + 1];      // one per kernel of this operand layout
+  static PerDeviceOnce attr[EPI_DOT + 1];      // one per kernel of this operand layout
   const EpiKind kind = epi_kind(ga);
   // forward layers: [in][out] weights; input gradients: the same weights read K-major; weight
   // gradients: both operands MN-major
@@ -637,10 +637,12 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   }
   if constexpr (!A_MN && !B_MN) {
     if (kind == EPI_MUL) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_MUL>, attr[EPI_MUL]);
+    if (kind == EPI_DOT) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_DOT>, attr[EPI_DOT]);
   }
   if constexpr (A_MN && B_MN) {
     if (kind == EPI_ACCUM) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_ACCUM>, attr[EPI_ACCUM]);
   }
+  if (ep.colsum) return -7;                      // only EPI_MUL adds column sums
   if (ga.aux_tma == 2) ga.aux_tma = 0;           // EPI_ANY reads the residual row by row
   return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_ANY>, attr[EPI_ANY]);
 }
@@ -699,6 +701,11 @@ static int launch(const void* A, long long lda, const void* B, long long ldb, co
 
 }  // namespace ab
 
+extern "C" int ab_colsum_bf16(const void* x, long long ld, int M, int N, float* out, const int* m_limit,
+                              cudaStream_t stream);
+extern "C" int ab_attn_delta(const void* o, const void* dout, float* delta, int B, int T, int H, int hd,
+                             cudaStream_t stream);
+
 extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
                             long long ldb, int M, int N, int K, const AbGemmEpilogue* ep,
                             int k_splits, int max_ctas, int* status, cudaStream_t stream) {
@@ -713,12 +720,40 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
     return -3;
   if ((ep->ldo * (ep->out_fp32 ? 4 : 2)) & 15) return -4;   // TMA row pitch: multiple of 16 bytes
   if (ep->act == 1 && (ep->ldaux & 7)) return -4;
+  // CTA pairs for the large shapes; the single-CTA kernel keeps the device-sized problems
+  // (m_limit / k_limit) and anything a caller pins with AB_GEMM_NO_PAIR=1 in the environment
+  static const bool no_pair = [] {
+    const char* v = getenv("AB_GEMM_NO_PAIR");
+    return v && v[0] == '1';
+  }();
+  if (max_ctas <= 0) max_ctas = 148;
+  const bool pair = !no_pair && !ep->m_limit && !ep->k_limit && M >= 512 && N >= 256 && max_ctas >= 2;
+  const bool aux_by_tma = ep->aux && !ep->out_fp32 && !ep->accumulate && k_splits == 1 && (ep->ldaux & 7) == 0;
+  if (ep->act == 4) {
+    if (!ep->aux || !ep->dot_out || ep->dot_T < 1 || M % ep->dot_T || (N & 63) || ep->out_fp32 || ep->ldo != N ||
+        ep->ldaux != N || ep->m_limit || ep->resid)
+      return -5;
+    if (!(pair && aux_by_tma && !a_mn && !b_mn && ep->alpha == 1.f && !ep->bias)) {
+      AbGemmEpilogue plain = *ep;
+      plain.act = 0;
+      const int rc = ab_gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, &plain, k_splits, max_ctas, status, stream);
+      return rc ? rc : ab_attn_delta(ep->aux, ep->out, ep->dot_out, M / ep->dot_T, ep->dot_T, N / 64, 64, stream);
+    }
+  }
+  if (ep->colsum && !(pair && aux_by_tma && !a_mn && !b_mn && ep->act == 2 && ep->aux_grad && ep->alpha == 1.f &&
+                      !ep->bias && !ep->resid)) {
+    // every other form: a pass of its own over the finished output
+    if (ep->out_fp32) return -6;
+    AbGemmEpilogue plain = *ep;
+    plain.colsum = nullptr;
+    const int rc = ab_gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, &plain, k_splits, max_ctas, status, stream);
+    return rc ? rc : ab_colsum_bf16(ep->out, ep->ldo, M, N, ep->colsum, ep->m_limit, stream);
+  }
   GemmArgs g;
   g.M = M; g.N = N; g.K = K; g.k_splits = k_splits; g.ep = *ep; g.status = status; g.salt = seed_salt_ptr(); g.aux_tma = 0;
   // programmatic dependent launch: single-CTA kernels only, never with device-side limits (those
   // are values of earlier kernels, read before any wait)
   g.pdl = (ep->pdl && !ep->m_limit && !ep->k_limit) ? 1 : 0;
-  if (max_ctas <= 0) max_ctas = 148;
   // narrow tiles also for skinny problems (decode steps with a few hundred rows): twice the CTAs
   const bool narrow = (N <= 128) || (M <= 256);
   // A few hundred rows against a wide weight matrix (decode steps): the time goes into streaming
@@ -733,13 +768,7 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
     if (a_mn && !b_mn) return launch<128, 6, true, false>(A, lda, B, ldb, g, max_ctas, stream);
     return launch<128, 6, true, true>(A, lda, B, ldb, g, max_ctas, stream);
   }
-  // CTA pairs for the large shapes; the single-CTA kernel keeps the device-sized problems
-  // (m_limit / k_limit) and anything a caller pins with AB_GEMM_NO_PAIR=1 in the environment
-  static const bool no_pair = [] {
-    const char* v = getenv("AB_GEMM_NO_PAIR");
-    return v && v[0] == '1';
-  }();
-  if (!no_pair && !ep->m_limit && !ep->k_limit && M >= 512 && N >= 256 && max_ctas >= 2) {
+  if (pair) {
     if (!a_mn && !b_mn) return launch_pair<false, false>(A, lda, B, ldb, g, max_ctas, stream);
     if (!a_mn && b_mn) return launch_pair<false, true>(A, lda, B, ldb, g, max_ctas, stream);
     if (a_mn && !b_mn) return launch_pair<true, false>(A, lda, B, ldb, g, max_ctas, stream);

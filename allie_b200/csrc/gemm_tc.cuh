@@ -13,6 +13,8 @@ extern "C" {
 //   act == 3:  v = gelu_new(v)            (no pre-activation kept: inference)
 //   aux_grad:  act == 1 stores aux[m][n] = bf16(gelu_new'(v)) instead of bf16(v), and act == 2
 //              multiplies by aux[m][n] as it is (forward and backward must agree on the flag)
+//   act == 4:  v stays as it is; dot_out receives, for every row and group of 64 columns (an attention
+//              head), the sum of bf16(v) * aux over the group (see dot_out)
 //   resid != null:  v = resid[m][n] + dropout(v)   (dropout only when drop_thr16 > 0)
 //   out_fp32 ? (accumulate ? out[m][n] += v (atomic) : out[m][n] = v) : out[m][n] = bf16(v)
 struct AbGemmEpilogue {
@@ -40,6 +42,12 @@ struct AbGemmEpilogue {
   // tiles overlap that kernel; `B` must not be something it writes.
   int pdl;
   int aux_grad;
+  // optional fp32 [N]: the column sums of the bf16 output are added to it (bias gradients)
+  float* colsum;
+  // act == 4: fp32 [rows / dot_T][N / 64][dot_T]; row m is (m / dot_T, m % dot_T).  N a multiple of 64,
+  // out and aux dense.  From the epilogue on CTA pairs with K-major operands, else by a pass of its own.
+  float* dot_out;
+  int dot_T;
 };
 
 // C[M,N] = A[M,K] * B[K,N] on the 5th-generation tensor cores.

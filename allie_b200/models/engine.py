@@ -388,12 +388,14 @@ class B200Engine:
         attention_fwd(qkv, out, lse, B, T, self.cfg.n_head, self.cfg.head_dim, p_drop, seed, stream_id,
                       drop_mask if p_drop > 0 else None)
 
-    def _attention_bwd(self, qkv, out, lse, dout, dqkv, B, T, p_drop, seed, stream_id, drop_mask=None):
+    def _attention_bwd(self, qkv, out, lse, dout, dqkv, B, T, p_drop, seed, stream_id, drop_mask=None,
+                       delta_ready=False):
         from ..ops.attention import attention_bwd
 
         buf = self._buffers(B, T, True)
         attention_bwd(qkv, out, lse, dout, dqkv, buf["delta"], B, T, self.cfg.n_head, self.cfg.head_dim,
-                      p_drop, seed, stream_id, drop_mask if p_drop > 0 else None, buf.get("dq_acc"))
+                      p_drop, seed, stream_id, drop_mask if p_drop > 0 else None, buf.get("dq_acc"),
+                      delta_ready)
 
     # -------------------------------------------------------------- forward
     def _drop(self, train: bool):
@@ -510,18 +512,19 @@ class B200Engine:
                 self._moe(l, B * T, True).backward(dyb, buf["ln2"][l], dsmall, self._aux_coef())
             else:
                 gemm(buf["act"][l], dyb, a_mn=True, b_mn=True, out=L["pr_w"][2], accumulate=True)
-                gemm(dyb, L["pr_w"][1], b_mn=False, out=dpre, act=2, aux=buf["pre"][l], aux_grad=True)
+                gemm(dyb, L["pr_w"][1], b_mn=False, out=dpre, act=2, aux=buf["pre"][l], aux_grad=True,
+                     colsum=L["fc_b"][2])
                 gemm(buf["ln2"][l], dpre, a_mn=True, b_mn=True, out=L["fc_w"][2], accumulate=True)
-                K.colsum_bf16(dpre, L["fc_b"][2])
                 gemm(dpre, L["fc_w"][1], b_mn=False, out=dsmall)
             K.layernorm_bwd(dsmall, buf["xmid"][l], buf["mean2"][l], buf["rstd2"][l], L["ln2_w"][0], dx, dx,
                             dyb, L["ln2_w"][2], L["ln2_b"][2], rms=self.rms, drop_seed=seed,
                             drop_stream=1 + 3 * l, drop_p=p_res, dbias=L["o_b"][2])
             # ---- attention
             gemm(buf["attn"][l], dyb, a_mn=True, b_mn=True, out=L["o_w"][2], accumulate=True)
-            gemm(dyb, L["o_w"][1], b_mn=False, out=dsmall)
+            dot = dict(act=4, aux=buf["attn"][l], dot=(buf["delta"], T)) if cfg.head_dim == 64 else {}
+            gemm(dyb, L["o_w"][1], b_mn=False, out=dsmall, **dot)      # and delta = row sums of dO * O
             self._attention_bwd(buf["qkv"][l], buf["attn"][l], buf["lse"][l], dsmall, dqkv, B, T, p_att,
-                                seed, 3 + 3 * l, buf["dmask"][l] if "dmask" in buf else None)
+                                seed, 3 + 3 * l, buf["dmask"][l] if "dmask" in buf else None, bool(dot))
             gemm(buf["ln1"][l], dqkv, a_mn=True, b_mn=True, out=L["qkv_w"][2], accumulate=True)
             K.colsum_bf16(dqkv, L["qkv_b"][2])
             gemm(dqkv, L["qkv_w"][1], b_mn=False, out=dsmall)

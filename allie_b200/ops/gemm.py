@@ -60,14 +60,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          drop_p: float = 0.0, drop_seed: int = 0, drop_stream: int = 0,
          alpha: float = 1.0, k_splits: int | None = None, m_limit: torch.Tensor | None = None,
          k_limit: torch.Tensor | None = None, dependent: bool = False,
-         aux_grad: bool = False) -> torch.Tensor:
+         aux_grad: bool = False, colsum: torch.Tensor | None = None,
+         dot: tuple[torch.Tensor, int] | None = None) -> torch.Tensor:
     """``dependent``: launch as a programmatic dependent of the previous kernel in the stream
     (honoured by the small-M kernel): its set-up and first weight tiles overlap that kernel.  ``b``
     must then be data the previous kernel does not write (weights).
     ``aux_grad``: with ``act=1`` store GELU'(pre-activation) in ``aux`` instead of the
     pre-activation, with ``act=2`` multiply by ``aux`` as it is: the derivative is computed once,
     beside the activation it shares its tanh with, and the backward epilogue (bound by instruction
-    issue) shrinks to a multiply."""
+    issue) shrinks to a multiply.
+    ``colsum`` (fp32 [N]): the column sums of a bf16 ``out`` are added to it (bias gradients), from the
+    epilogue where ``act=2`` with ``aux_grad`` runs on CTA pairs, else by a pass over ``out``.
+    ``dot=(dst, T)`` with ``act=4``: ``dst`` fp32 [M/T, N/64, T] receives each row's dot product with
+    ``aux`` per 64 columns (``out`` and ``aux`` dense)."""
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     if a_mn:
@@ -107,7 +112,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert bias.dtype == torch.float32 and bias.numel() == N
         ep.bias = bias.data_ptr()
     ep.act = act            # 1: GELU, pre-activation saved in aux; 2: times GELU'(aux); 3: GELU, nothing saved
-    if act in (1, 2):
+    if act in (1, 2, 4):
         assert aux is not None and aux.dtype == torch.bfloat16 and aux.shape == (M, N)
         ep.aux = aux.data_ptr()
         ep.ldaux = aux.stride(0)
@@ -125,6 +130,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         ep.k_limit = k_limit.data_ptr()
     ep.pdl = int(dependent)
     ep.aux_grad = int(aux_grad)
+    if colsum is not None:
+        assert colsum.dtype == torch.float32 and colsum.numel() == N and not out_fp32
+        ep.colsum = colsum.data_ptr()
+    if dot is not None:
+        dst, ep.dot_T = dot
+        assert act == 4 and dst.dtype == torch.float32 and dst.numel() * 64 == M * N and M % ep.dot_T == 0
+        ep.dot_out = dst.data_ptr()
     rc = _lib.cuda().ab_gemm_bf16(
         _lib.ptr(a), c_int(int(a_mn)), c_longlong(a.stride(0)),
         _lib.ptr(b), c_int(int(b_mn)), c_longlong(b.stride(0)),
