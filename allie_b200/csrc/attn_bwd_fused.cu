@@ -6,12 +6,16 @@
 // double-buffered).  The 16 math warps turn S/dP into P/dS exactly once per pair - half the
 // exponentials and dropout work of the two-kernel scheme - and push each dQ_ij tile to an fp32
 // accumulator in global memory with TMA reduce-add, one 32x16 box per warp, so no atomics are
-// issued by threads.  A trailing kernel converts the fp32 dQ to bf16 into the packed dQKV
-// activation and clears the accumulator for the next layer.
+// issued by threads.  With one key tile per CTA (and for ragged lengths) a trailing kernel converts
+// the fp32 dQ to bf16 into the packed dQKV activation and the accumulator is cleared for the next
+// layer; the persistent walk does both by itself.
 //
 // TMEM columns (512): S 0-127 | dP 128-255 | dV 256-319 | dK 320-383 | dQ 384-447, 448-511.
 #include "attn_common.cuh"
 #include <cstdlib>
+
+extern "C" int ab_colsum_bf16(const void* x, long long ld, int M, int N, float* out, const int* m_limit,
+                              cudaStream_t stream);
 
 namespace ab {
 
@@ -350,11 +354,14 @@ struct FbWalk {
   }
 };
 
+// WHOLE: T is a multiple of 128 (see drain_dq)
+template <bool WHOLE>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
                                    const __grid_constant__ CUtensorMap tmDO,
                                    const __grid_constant__ CUtensorMap tmDQ,
-                                   const __grid_constant__ CUtensorMap tmDKV, const AttnBwdArgs a) {
+                                   const __grid_constant__ CUtensorMap tmDKV,
+                                   const __grid_constant__ CUtensorMap tmDQB, const AttnBwdArgs a) {
   griddep_enter();
   constexpr int HD = 64;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
@@ -518,17 +525,82 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     uint8_t* my_dq = sDQ + warp * 2048;
     bool ok = true;
 
-    // drains the dQ tile of pair g (query rows starting at global row `row0` of head h, this
-    // warp's 16 columns) into the global fp32 accumulator with one TMA reduce-add
-    auto drain_dq = [&](int g, int row0, int h) {
+    // Whole tiles (T % 128 == 0): the dQ sums of a slice live in the place of this CTA's FIRST slice in
+    // dq_acc and nowhere else, so 148 slices stay in L2 instead of every slice passing through memory
+    // twice, and no pass converts or clears them: key tile 0 stores its contributions, later ones add,
+    // and the last one of a query tile (its diagonal pair) reads the sum back, adds its own part from
+    // TMEM and stores bf16 into dQKV.  The same warp does all of it for its rows and columns.
+    const int s_row0 = (start.bh / a.H) * a.T + quad * 32, s_col = (start.bh % a.H) * HD + cb * 16;
+    // adds the column sums of a staged bf16 tile (32 rows of `cols` columns) to dst: a lane takes two
+    // columns of every (64 / cols)-th row, so each load of the warp reads 128 contiguous bytes
+    auto add_colsum = [&](const uint8_t* tile, int cols, float* dst) {
+      const int pairs = cols >> 1, cp = lane % pairs, rows = 32 / pairs;
+      uint64_t sum = 0ull;
+      for (int row = lane / pairs; row < 32; row += rows) {
+        const int sw = cols == 32 ? ((row >> 1) & 3) : ((row >> 2) & 1);
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + row * cols * 2 + (((cp >> 2) ^ sw) << 4) + (cp & 3) * 4);
+        sum = f2_add(sum, f2_pack(bf16_lo(w), bf16_hi(w)));
+      }
+      float s0, s1;
+      f2_unpack(sum, s0, s1);
+      for (int o = pairs; o < 32; o <<= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      }
+      if (lane < pairs)
+        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst + cp * 2), "f"(s0), "f"(s1) : "memory");
+    };
+
+    // drains the dQ tile of pair g (query tile own + it of head h of sequence b, this warp's 16 columns)
+    auto drain_dq = [&](int g, int b, int h, int own, int it) {
       if (!mbar_wait(&dq_full[g & 1], (g >> 1) & 1, abort_flag)) return false;
       tc_fence_after();
       uint32_t v[16];
       tmem_ld16(tDQ + (g & 1) * 64 + lane_addr + cb * 16, v);
-      if (lane == 0) tma_store_wait_read<0>();
+      const bool last = WHOLE && it == 0;
+      if (lane == 0) {
+        if (last && own > 0) {
+          tma_store_wait<0>();                   // this warp's earlier contributions are in memory
+          asm volatile("fence.proxy.async;" ::: "memory");
+        } else {
+          tma_store_wait_read<0>();
+        }
+      }
       __syncwarp();
       tmem_ld_wait();
       tc_fence_before();
+      const int qrow = (own + it) * 128;
+      if (last) {
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+        if (own > 0) {
+          const float4* src = reinterpret_cast<const float4*>(
+              a.dq_acc + (static_cast<long long>(s_row0) + qrow + lane) * d_model + s_col);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float4 t = __ldcg(src + c);
+            f[c * 4 + 0] += t.x; f[c * 4 + 1] += t.y; f[c * 4 + 2] += t.z; f[c * 4 + 3] += t.w;
+          }
+        }
+        // 16 bf16 columns = 32-byte rows, 32B swizzle
+        uint8_t* rowp = my_dq + lane * 32;
+        const int sw = (lane >> 2) & 1;
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) =
+              make_uint4(pack_bf16x2(f[c * 8 + 0], f[c * 8 + 1]), pack_bf16x2(f[c * 8 + 2], f[c * 8 + 3]),
+                         pack_bf16x2(f[c * 8 + 4], f[c * 8 + 5]), pack_bf16x2(f[c * 8 + 6], f[c * 8 + 7]));
+        asm volatile("fence.proxy.async;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&dq_empty[g & 1]);
+          tma_store_2d(&tmDQB, my_dq, h * HD + cb * 16, b * a.T + qrow + quad * 32);
+          tma_store_commit();
+        }
+        if (a.dbias) add_colsum(my_dq, 16, a.dbias + h * HD + cb * 16);
+        return true;
+      }
       uint8_t* rowp = my_dq + lane * 64;       // 16 fp32 columns = 64-byte rows, 64B swizzle
       const int sw = (lane >> 1) & 3;
 #pragma unroll
@@ -540,7 +612,10 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&dq_empty[g & 1]);
-        tma_reduce_add_2d(&tmDQ, my_dq, h * HD + cb * 16, row0 + quad * 32);
+        if (!WHOLE)        tma_reduce_add_2d(&tmDQ, my_dq, h * HD + cb * 16, b * a.T + qrow + quad * 32);
+        else if (own == 0) tma_store_2d(&tmDQ, my_dq, s_col, s_row0 + qrow);
+        // (own == 1 adds to what own == 0 stored: those stores were waited for at its diagonal pair)
+        else               tma_reduce_add_2d(&tmDQ, my_dq, s_col, s_row0 + qrow);
         tma_store_commit();
       }
       return true;
@@ -557,7 +632,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty);
-      if ((a.T & 127) == 0) {
+      if (WHOLE) {
         // 32 rows x 32 bf16 columns per warp: staged with 64-byte swizzle, one TMA store.  (Plain
         // stores of 64-byte row pieces 6 KB apart kept the load/store unit busy for thousands of
         // cycles per key tile and delayed every other warp's shared-memory traffic with them.)
@@ -581,6 +656,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
                        b * a.T + own * 128 + quad * 32);
           tma_store_commit();
         }
+        if (a.dbias) add_colsum(my_dq, 32, a.dbias + (cb < 2 ? 2 * d_model : d_model) + h * HD + (cb & 1) * 32);
         return true;
       }
       // ragged last tile: rows past T belong to the next sequence, so store row by row
@@ -601,7 +677,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       return true;
     };
 
-    int prev_row0 = 0, prev_h = 0, prev_b = 0, prev_own = 0;     // pair g - 1 / its key tile
+    int prev_h = 0, prev_b = 0, prev_own = 0, prev_it = 0;       // pair g - 1 / its key tile
     // per-row inputs of a pair: log-sum-exp, delta and the 32 dropout keep bits of this thread's
     // columns.  They are fetched one pair ahead so their latency never sits in the pair's chain.
     // Addresses advance by fixed strides from one query tile to the next, so they are rebuilt from
@@ -706,15 +782,28 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       if (lane == 0) mbar_arrive(pds_full);
       // work left over from the previous pair, done while the tensor core runs this one
       if (p.g > 0) {
-        ok = drain_dq(p.g - 1, prev_row0, prev_h);
+        ok = drain_dq(p.g - 1, prev_b, prev_h, prev_own, prev_it);
         if (ok && p.first()) ok = finish_tile(p.w - 1, prev_b, prev_h, prev_own);
       }
-      prev_row0 = b * a.T + qi * 128; prev_h = h; prev_b = b; prev_own = p.own;
+      prev_h = h; prev_b = b; prev_own = p.own; prev_it = p.it;
       lse_raw = n_lse; dlt = n_dlt; keep32 = n_keep;
     }
     if (ok && p.g > 0) {
-      ok = drain_dq(p.g - 1, prev_row0, prev_h);
+      ok = drain_dq(p.g - 1, prev_b, prev_h, prev_own, prev_it);
       if (ok) ok = finish_tile(p.w - 1, prev_b, prev_h, prev_own);
+      if (WHOLE && ok && nt > 1) {
+        // hand the accumulator back all zero (query tile 0 never went through it)
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(my_dq + lane * 64 + c * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          for (int i = 1; i < nt; ++i) tma_store_2d(&tmDQ, my_dq, s_col, s_row0 + i * 128);
+          tma_store_commit();
+        }
+      }
     }
     if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
     if (lane == 0) tma_store_wait<0>();
@@ -766,6 +855,9 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
   // the persistent walk hands whole (batch, head) slices to CTAs, which only balances with several
   // slices per SM; few, long slices go to the one-tile-per-CTA grid
   const int mode = attn_bwd_schedule_mode();
+  const bool whole = (a.T & 127) == 0;
+  AttnBwdArgs p = a;
+  if (!whole) p.dbias = nullptr;
   if (mode == 1 || (mode == 0 && a.B * a.H < 4 * 148)) {
     constexpr int SMEM = 6 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
     static PerDeviceOnce attr;
@@ -779,26 +871,31 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
     launch_chained(attn_bwd_fused64_kernel, dim3(grid), dim3(FB_THREADS), SMEM, stream, tq, td, tdq, a);
   } else {
     constexpr int SMEM = 8 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
-    static PerDeviceOnce attr;
-    if (attr.first_use_on_device()) {
-      cudaError_t e = cudaFuncSetAttribute(attn_bwd_fused64_persistent_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    auto kern = whole ? attn_bwd_fused64_persistent_kernel<true> : attn_bwd_fused64_persistent_kernel<false>;
+    static PerDeviceOnce attr[2];
+    if (attr[whole].first_use_on_device()) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
       if (e != cudaSuccess) return (int)e;
-      attr.mark_device();
+      attr[whole].mark_device();
     }
     CUtensorMap tdkv;     // the packed dQKV activation, boxes of 32 rows x 32 columns for dK / dV
     rc = make_tmap_2d_sw(&tdkv, a.dqkv, rows, 3 * d, 3 * d, 32, 32, 2, 64);
     if (rc) return rc;
+    CUtensorMap tdqb;     // the same, boxes of 32 rows x 16 columns for dQ
+    rc = make_tmap_2d_sw(&tdqb, a.dqkv, rows, 3 * d, 3 * d, 32, 16, 2, 32);
+    if (rc) return rc;
     const int bh = a.B * a.H;
-    launch_chained(attn_bwd_fused64_persistent_kernel, dim3(bh < 148 ? bh : 148), dim3(FB_THREADS), SMEM, stream, tq, td, tdq,
-                                                                                          tdkv, a);
+    launch_chained(kern, dim3(bh < 148 ? bh : 148), dim3(FB_THREADS), SMEM, stream, tq, td, tdq, tdkv, tdqb, p);
+    if (whole) return (int)cudaGetLastError();       // dQ, its bias sums and the clearing are done
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   launch_chained(attn_dq_convert_kernel, dim3(148 * 16), dim3(256), 0, stream, a.dq_acc, a.dqkv, (int)rows, d);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  return (int)cudaMemsetAsync(a.dq_acc, 0, sizeof(float) * rows * d, stream);
+  e = cudaMemsetAsync(a.dq_acc, 0, sizeof(float) * rows * d, stream);
+  if (e != cudaSuccess || !a.dbias) return (int)e;
+  return ab_colsum_bf16(a.dqkv, 3 * d, (int)rows, 3 * d, a.dbias, nullptr, stream);
 }
 
 }  // namespace ab

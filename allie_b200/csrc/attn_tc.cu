@@ -767,6 +767,8 @@ static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& td, const A
 
 extern "C" {
 
+int ab_colsum_bf16(const void* x, long long ld, int M, int N, float* out, const int* m_limit, cudaStream_t stream);
+
 // delta[b][h][t] = sum over the head's columns of dO * O (o, dout: bf16 [B*T, H*hd])
 int ab_attn_delta(const void* o, const void* dout, float* delta, int B, int T, int H, int hd, cudaStream_t stream) {
   using namespace ab;
@@ -816,11 +818,12 @@ int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T
 // delta: fp32 scratch [B,H,T] owned by the caller.  drop_mask (optional): the keep bits the forward
 // pass wrote.  dq_acc (optional, hd == 64): fp32 [B*T, H*hd] accumulator that must be all zero on
 // entry and is all zero again on return; when given, the single-kernel backward runs.
-// delta_ready: delta already holds the row sums of dO * O.
+// dbias (optional, fp32 [3*H*hd]): the column sums of dqkv are added to it (the bias gradient of the
+// QKV projection).  delta_ready: delta already holds the row sums of dO * O.
 int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* dout, void* dqkv,
                 float* delta, const unsigned int* drop_mask, float* dq_acc, int B, int T, int H, int hd,
                 float scale, unsigned long long seed, unsigned int stream_id, unsigned int thr16,
-                int delta_ready, int* status, cudaStream_t stream) {
+                float* dbias, int delta_ready, int* status, cudaStream_t stream) {
   using namespace ab;
   if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || (thr16 && (T & 7))) return -1;
   if (drop_mask && (T & 31)) return -1;
@@ -834,16 +837,13 @@ int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* 
   a.B = B; a.T = T; a.H = H; a.hd = hd; a.scale = scale; a.seed = seed; a.stream_id = stream_id;
   a.thr16 = thr16; a.lse = lse; a.delta = delta; a.dqkv = (__nv_bfloat16*)dqkv; a.status = status;
   a.salt = seed_salt_ptr();
-  a.drop_mask = drop_mask; a.dq_acc = dq_acc;
+  a.drop_mask = drop_mask; a.dq_acc = dq_acc; a.dbias = dbias;
   if (hd == 64 && dq_acc) return launch_attn_bwd_fused64(tq, td, a, stream);
-  if (hd == 64) {
-    rc = launch_attn_bwd<64, 0>(tq, td, a, stream);
-    if (rc) return rc;
-    return launch_attn_bwd<64, 1>(tq, td, a, stream);
-  }
-  rc = launch_attn_bwd<128, 0>(tq, td, a, stream);
+  rc = hd == 64 ? launch_attn_bwd<64, 0>(tq, td, a, stream) : launch_attn_bwd<128, 0>(tq, td, a, stream);
   if (rc) return rc;
-  return launch_attn_bwd<128, 1>(tq, td, a, stream);
+  rc = hd == 64 ? launch_attn_bwd<64, 1>(tq, td, a, stream) : launch_attn_bwd<128, 1>(tq, td, a, stream);
+  if (rc || !dbias) return rc;
+  return ab_colsum_bf16(dqkv, 3ll * H * hd, B * T, 3 * H * hd, dbias, nullptr, stream);
 }
 }
 
@@ -884,5 +884,5 @@ extern "C" int ab_attn_bwd_static(const void* qkv, const void* out, const float*
     g_attn_static_ptr[dev].store(scratch, std::memory_order_release);
   }
   return ab_attn_bwd(qkv, out, lse, dout, dqkv, scratch, drop_mask, nullptr, B, T, H, hd,
-                     scale, seed, stream_id, thr16, 0, status, stream);
+                     scale, seed, stream_id, thr16, nullptr, 0, status, stream);
 }

@@ -389,13 +389,13 @@ class B200Engine:
                       drop_mask if p_drop > 0 else None)
 
     def _attention_bwd(self, qkv, out, lse, dout, dqkv, B, T, p_drop, seed, stream_id, drop_mask=None,
-                       delta_ready=False):
+                       delta_ready=False, dbias=None):
         from ..ops.attention import attention_bwd
 
         buf = self._buffers(B, T, True)
         attention_bwd(qkv, out, lse, dout, dqkv, buf["delta"], B, T, self.cfg.n_head, self.cfg.head_dim,
                       p_drop, seed, stream_id, drop_mask if p_drop > 0 else None, buf.get("dq_acc"),
-                      delta_ready)
+                      delta_ready, dbias)
 
     # -------------------------------------------------------------- forward
     def _drop(self, train: bool):
@@ -524,9 +524,8 @@ class B200Engine:
             dot = dict(act=4, aux=buf["attn"][l], dot=(buf["delta"], T)) if cfg.head_dim == 64 else {}
             gemm(dyb, L["o_w"][1], b_mn=False, out=dsmall, **dot)      # and delta = row sums of dO * O
             self._attention_bwd(buf["qkv"][l], buf["attn"][l], buf["lse"][l], dsmall, dqkv, B, T, p_att,
-                                seed, 3 + 3 * l, buf["dmask"][l] if "dmask" in buf else None, bool(dot))
+                                seed, 3 + 3 * l, buf["dmask"][l] if "dmask" in buf else None, bool(dot), L["qkv_b"][2])
             gemm(buf["ln1"][l], dqkv, a_mn=True, b_mn=True, out=L["qkv_w"][2], accumulate=True)
-            K.colsum_bf16(dqkv, L["qkv_b"][2])
             gemm(dqkv, L["qkv_w"][1], b_mn=False, out=dsmall)
             K.layernorm_bwd(dsmall, buf["x"][l], buf["mean1"][l], buf["rstd1"][l], L["ln1_w"][0], dx, dx,
                             dyb if l > 0 else None, L["ln1_w"][2], L["ln1_b"][2], rms=self.rms,

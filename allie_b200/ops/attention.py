@@ -26,16 +26,17 @@ def attention_fwd(qkv, out, lse, B: int, T: int, H: int, hd: int, p_drop: float,
 
 
 def attention_bwd(qkv, out, lse, dout, dqkv, delta, B: int, T: int, H: int, hd: int, p_drop: float,
-                  seed: int, stream_id: int, drop_mask=None, dq_acc=None, delta_ready: bool = False) -> None:
+                  seed: int, stream_id: int, drop_mask=None, dq_acc=None, delta_ready: bool = False, dbias=None) -> None:
     """``delta`` is fp32 scratch [B, H, T] (row sums of dO*O, filled here).  ``dq_acc``: optional
     all-zero fp32 [B*T, H*hd] accumulator (head_dim 64 only) that selects the single-kernel
     backward; it is handed back all zero.  ``delta_ready``: ``delta`` holds the row sums already (see
-    ``act=4`` of :func:`~allie_b200.ops.gemm.gemm`)."""
+    ``act=4`` of :func:`~allie_b200.ops.gemm.gemm`).  ``dbias``: optional fp32 [3*H*hd] to which the column
+    sums of ``dqkv`` are added (the bias gradient of the projection in front)."""
     rc = _lib.cuda().ab_attn_bwd(ptr(qkv), ptr(out), ptr(lse), ptr(dout), ptr(dqkv), ptr(delta),
                                  ptr(drop_mask), ptr(dq_acc), c_int(B), c_int(T),
                                  c_int(H), c_int(hd), c_float(1.0 / hd ** 0.5), c_ulonglong(seed),
                                  c_uint(stream_id), c_uint(_lib.dropout_thr16(p_drop)),
-                                 c_int(int(delta_ready)), ptr(_lib.status_word()), stream_ptr())
+                                 ptr(dbias), c_int(int(delta_ready)), ptr(_lib.status_word()), stream_ptr())
     if rc != 0:
         raise RuntimeError(f"ab_attn_bwd failed with code {rc} (B={B} T={T} H={H} hd={hd})")
     _lib.count_launches(3)  # delta + (two backward kernels | fused backward + dQ conversion)

@@ -125,3 +125,41 @@ def test_attention_dropout_mask_consistency():
         rel = (dqkv.float() - leaf.grad).norm() / leaf.grad.norm()
         assert rel < 3e-2, (rel.item(), use_bits, fused)
     set_backward_schedule(0)
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(2, 128, 2, 64), (160, 256, 1, 64), (40, 512, 4, 64), (3, 200, 2, 64), (2, 256, 2, 128)])
+def test_attention_bwd_bias_sums_and_accumulator(B, T, H, hd):
+    """The column sums of dQKV that the backward adds, from its own tiles (persistent walk over whole
+    tiles: one tile, a CTA with one slice and with two, the sums of a slice kept in place) and by the pass
+    that stands in elsewhere; the accumulator comes back all zero; the schedules agree.  Sums of B*T fp32
+    terms: any order is within B*T * 2^-23 * sum|terms|."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.attention import attention_bwd, attention_fwd, set_backward_schedule
+
+    torch.manual_seed(3)
+    d = H * hd
+    dev = "cuda"
+    qkv = (torch.randn(B * T, 3 * d, device=dev) * 0.7).bfloat16()
+    out = torch.zeros(B * T, d, device=dev, dtype=torch.bfloat16)
+    lse, delta = torch.zeros(B, H, T, device=dev), torch.zeros(B, H, T, device=dev)
+    attention_fwd(qkv, out, lse, B, T, H, hd, 0.0, 0, 0)
+    dout = torch.randn(B * T, d, device=dev).bfloat16()
+    grads = []
+    for schedule in (1, 2) if hd == 64 else (0,):
+        set_backward_schedule(schedule)
+        acc = torch.zeros(B * T, d, device=dev) if hd == 64 else None
+        for _ in range(2):
+            dqkv = torch.full((B * T, 3 * d), float("nan"), device=dev, dtype=torch.bfloat16)
+            dbias = torch.full((3 * d,), 0.5, device=dev)
+            attention_bwd(qkv, out, lse, dout, dqkv, delta, B, T, H, hd, 0.0, 0, 0, None, acc, dbias=dbias)
+            torch.cuda.synchronize()
+            _lib.check_status()
+            terms = dqkv.double()
+            bound = 1e-6 + B * T * 2.0 ** -23 * (terms.abs().sum(0) + 0.5)
+            assert ((dbias.double() - 0.5 - terms.sum(0)).abs() <= bound).all()
+            assert acc is None or not acc.any()
+        grads.append(dqkv.float())
+    set_backward_schedule(0)
+    # the schedules add a query tile's parts in different orders: single bf16 roundings flip
+    for g in grads[1:]:
+        assert (g - grads[0]).norm() / grads[0].norm() < 1e-3
