@@ -20,7 +20,7 @@ namespace ab {
 // each (chunk, head)'s K and V rows into a shared-memory ring with bulk asynchronous copies
 // (cp.async.bulk global -> shared, completion counted on the stage's mbarrier): the prompt slots
 // [0, prefix_len) of a (tree, head) are contiguous in the cache, so a chunk of them is ONE copy of
-// up to 8 KB for K and one for V; ancestor slots are scattered single rows (one 128/256-byte copy
+// up to 4 KB for K and one for V; ancestor slots are scattered single rows (one 128/256-byte copy
 // each, issued by the producer warp's lanes in parallel), and the token's own key / value come from
 // the packed QKV row they are appended from.  Up to DA_STAGES stages per CTA are in flight, with no
 // registers or load instructions of the consumers tied up, which is what lets a kernel whose CTAs
@@ -29,9 +29,16 @@ namespace ab {
 // key (each a quarter of the head dimension), eight keys per round, one online-softmax state per
 // key group, merged across the groups with shuffles at the end.
 // Every wait is bounded; on expiry the CTA records ST_TIMEOUT_MISC and leaves.
-constexpr int DA_HEADS = 4;
-constexpr int DA_CHUNK = 64;
-constexpr int DA_STAGES = 6;
+// Every head has a ring of its own.  With one ring for all heads, a consumer that was done early could
+// wait for a stage's phase k + 1 while the load of phase k (another head's) had not landed yet; a parity
+// wait takes that for phase k + 1.
+// Small CTAs (32 KB of ring at head_dim 64, seven per SM): a tree's keys are few, so a CTA's start-up
+// is a good part of its life and has to be covered by other CTAs.  256 trees of 4 to 300 keys, 16 heads:
+// 43.5 us with four heads and 64-key chunks, 36.9 with two and 32 (25 at memory speed).
+constexpr int DA_HEADS = 2;
+constexpr int DA_CHUNK = 32;
+constexpr int DA_RING = 2;                 // stages per head
+constexpr int DA_STAGES = DA_HEADS * DA_RING;
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -70,23 +77,22 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
   const int* anc_t = anc + static_cast<long long>(t) * anc_stride;
   const __nv_bfloat16* row = qkv + static_cast<long long>(t) * 3 * d;
   const int h0 = hg * DA_HEADS;
-  const int nh = min(H - h0, DA_HEADS);          // heads of this CTA; item (chunk c, head i) = c * nh + i
+  const int nh = min(H - h0, DA_HEADS);          // heads of this CTA
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     // Launched as a programmatic dependent, the chunks that hold prompt slots only are fetched while
     // the kernel before (the QKV projection) is still running: the cache rows of earlier positions
     // do not depend on it.  The first chunk that needs the token's own row waits for it.
-    int item = 0;
     bool waited = false;
     for (int c = 0; c < n_chunks; ++c) {
       const int i0 = c * DA_CHUNK, i1 = min(n, i0 + DA_CHUNK);
       const int pre = max(0, min(P, i1) - i0);         // keys of this chunk that are prompt slots
       if (!waited && pre < i1 - i0) { griddep_wait(); waited = true; }
-      for (int hi = 0; hi < nh; ++hi, ++item) {
+      for (int hi = 0; hi < nh; ++hi) {
         const int h = h0 + hi;
-        const int stage = item % DA_STAGES;
-        const uint32_t parity = ((item / DA_STAGES) & 1) ^ 1;
+        const int stage = hi * DA_RING + c % DA_RING;
+        const uint32_t parity = ((c / DA_RING) & 1) ^ 1;
         const long long cache_base = (static_cast<long long>(t) * H + h) * S * HD;
         int okw = 1;
         if (lane == 0) okw = mbar_wait(&empty[stage], parity, abort_flag) ? 1 : 0;
@@ -148,9 +154,8 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
 #pragma unroll
   for (int e = 0; e < DPL; ++e) acc[e] = 0.f;
   for (int ch = 0; ch < n_chunks; ++ch) {
-    const int item = ch * nh + hi;
-    const int stage = item % DA_STAGES;
-    const uint32_t parity = (item / DA_STAGES) & 1;
+    const int stage = hi * DA_RING + ch % DA_RING;
+    const uint32_t parity = (ch / DA_RING) & 1;
     const int cnt = min(n, (ch + 1) * DA_CHUNK) - ch * DA_CHUNK;
     if (!mbar_wait(&full[stage], parity, abort_flag)) {
       *abort_flag = 1;
