@@ -18,10 +18,12 @@ import torch
 
 from ..ops import _lib, kernels as K
 from ..ops._lib import ptr, stream_ptr
-from ..ops.gemm import gemm
+from ..ops.gemm import gemm, num_sms
 
 
 class KVLeafEvaluator:
+    FEW_TREES = 16
+
     def __init__(self, engine, n_trees: int, max_prefix: int = 320, max_nodes: int = 512,
                  anc_max: int = 128, legal_max: int = 224, use_graph: bool = True):
         self.eng = engine
@@ -52,6 +54,16 @@ class KVLeafEvaluator:
         self.stat = [e(n, dt=f32) for _ in range(2)]
         self.value, self.time = e(n, dt=f32), e(n, dt=f32)
         self.resign_id = 1992
+        # a handful of trees: all layers in one kernel (csrc/decode_few.cu), which reads the layers'
+        # addresses from this table and keeps its accumulators in this scratch
+        self.few = n_trees <= self.FEW_TREES and engine.dense
+        if self.few:
+            addr = lambda t: 0 if t is None else t.data_ptr()
+            table = [[addr(Ly[k][0]) for k in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_b", "o_b", "fc_b", "pr_b")]
+                     + [addr(Ly[k][1]) for k in ("qkv_w", "o_w", "fc_w", "pr_w")] + [addr(self.kc[l]), addr(self.vc[l])]
+                     for l, Ly in enumerate(engine.layers)]
+            self.layer_table = torch.tensor(table, dtype=torch.int64, device=dev)
+            self.few_work = torch.zeros(256 + n * (3 * d + F), dtype=f32, device=dev)
         self.graph = None
         self.use_graph = use_graph
         self.steps = 0
@@ -123,7 +135,8 @@ class KVLeafEvaluator:
         # set-up and first ring of weight tiles, the attention kernel's prompt-slot chunks and every
         # launch overlap the previous kernel (ALLIE_DECODE_PDL=0 turns it off)
         pdl = os.environ.get("ALLIE_DECODE_PDL", "1") != "0"
-        for l, Ly in enumerate(eng.layers):
+        few = self.few and self._launch_few(x)
+        for l, Ly in enumerate(eng.layers if not few else ()):
             K.layernorm_fwd(x, Ly["ln1_w"][0], Ly["ln1_b"][0], self.ln, self.stat[0], self.stat[1], eps, eng.rms,
                             dependent=pdl)
             gemm(self.ln, Ly["qkv_w"][1], b_mn=True, out=self.qkv, bias=Ly["qkv_b"][0], dependent=pdl)
@@ -156,6 +169,20 @@ class KVLeafEvaluator:
                                     c_int(self.out_stride), c_int(n), stream_ptr())
         assert rc == 0
         _lib.count_launches(1)
+
+    def _launch_few(self, x) -> bool:
+        """All layers of the step as one kernel; False (nothing launched) for shapes it does not take."""
+        cfg, rd = self.eng.cfg, self.req_dev
+        rc = _lib.cuda().ab_decode_few(
+            ptr(self.layer_table), c_int(cfg.n_layer), c_int(self.n), c_int(cfg.n_embd), c_int(cfg.n_head),
+            c_int(cfg.ffn_dim), c_int(self.S), c_int(int(self.eng.rms)), c_float(cfg.layer_norm_epsilon), ptr(x),
+            ptr(self.att), ptr(self.view(rd, "active")), ptr(self.view(rd, "slot")), ptr(self.view(rd, "prefix_len")),
+            ptr(self.view(rd, "anc")), c_int(self.anc_max), ptr(self.view(rd, "n_anc")), ptr(self.few_work),
+            c_int(num_sms()), ptr(_lib.status_word()), stream_ptr())
+        if rc < 0:
+            raise RuntimeError(f"ab_decode_few failed with code {rc}")
+        _lib.count_launches(int(rc == 0))
+        return rc == 0
 
     @torch.no_grad()
     def step(self) -> np.ndarray:

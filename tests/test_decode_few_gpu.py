@@ -1,0 +1,63 @@
+"""One-kernel search step for a handful of trees against the chain of kernels."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,d,heads,inner,norm", [
+    (1, 256, 4, 1024, "layernorm"), (4, 1024, 16, 4096, "layernorm"), (16, 768, 12, 3072, "layernorm"),
+    (3, 1280, 20, 5120, "rmsnorm"), (7, 384, 3, 640, "layernorm"), (2, 128, 2, 128, "layernorm"),
+])
+def test_few_tree_step_matches_the_chain(n, d, heads, inner, norm):
+    """Fewer units than SMs and several per SM, contractions split and whole, heads of 64 and 128, tree
+    counts up to the limit; prompts shorter and longer than one round of keys; an inactive tree.  Both
+    forms round to bf16 at the same places, so they differ by the order of fp32 sums, which flips single
+    bf16 roundings: well under 1 % of the logits' size after three layers."""
+    from allie_b200.data import Game, UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.moves import CHESS_MOVES
+    from allie_b200.ops import _lib
+    from allie_b200.search.batched import KVStepEvaluator
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=256, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=3, n_embd=d,
+                             n_head=heads, n_inner=inner, n_positions=256, norm_type=norm)
+    eng = B200Engine(model, "cuda")
+    rng = np.random.default_rng(3)
+    plies = [int(v) for v in rng.integers(0, 180, size=n)]
+    games = [Game("180+0", 1500, 1600, None, False, [CHESS_MOVES[i] for i in rng.integers(0, 1968, size=k)], [1] * k)
+             for k in plies]
+    results = []
+    for few in (True, False):
+        ev = KVStepEvaluator(eng, tok, n, anc_max=16, legal_max=64, max_prefix=200, max_nodes=64)
+        assert ev.kv.few
+        ev.kv.few = few
+        ev.prefill(games)
+        prefix = [len(tok.tokenize(g)) for g in games]
+        steps = np.random.default_rng(5)
+        out = []
+        anc = np.zeros((n, 16), np.int32)
+        for s in range(3):
+            req = dict(need_eval=np.ones(n, np.int32), tok=steps.integers(0, 1968, size=n).astype(np.int32),
+                       pos=np.array([p + s for p in prefix], np.int32), slot=np.array([p + s for p in prefix], np.int32),
+                       n_anc=np.full(n, s + 1, np.int32), n_legal=np.full(n, 40, np.int32), anc=anc,
+                       legal=steps.integers(0, 1968, size=(n, 64)).astype(np.int32))
+            anc[:, s] = req["slot"]
+            if n > 1 and s == 1:
+                req["need_eval"][n - 1] = 0
+            p, v = ev.step(req)
+            live = req["need_eval"] != 0
+            out.append((p[live, :40].copy(), v[live].copy(), ev.kv.logits[torch.from_numpy(live).cuda()].float().cpu()))
+        torch.cuda.synchronize()
+        _lib.check_status()
+        results.append(out)
+        if few:
+            assert int(ev.kv.few_work[:1].view(torch.int32).item()) > 0      # arrivals were counted: the kernel ran
+    for (pa, va, la), (pb, vb, lb) in zip(*results):
+        assert float((la - lb).norm() / lb.norm()) < 1e-2
+        assert np.abs(va - vb).max() < 1e-2
+        assert np.abs(pa - pb).max() < 1e-2
