@@ -83,6 +83,7 @@ struct LnBwdArgs {
   int M, d, rms;
   unsigned long long drop_seed; unsigned int drop_stream, drop_thr16;
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into drop_seed when not null
+  int* status;
 };
 
 // Backward kernel.  A group of threads owns a row and every thread of it the same eight columns of
@@ -91,14 +92,18 @@ struct LnBwdArgs {
 // many rows are in flight: bound by bytes (16 per element with a residual and a masked copy).  The
 // form before kept a warp per row and the sums of every warp in shared memory (96 bytes per column of
 // a block): 16 warps per SM at d <= 1024, 8 above.
-//   LNB_ROWS rows are loaded together (one memory round trip, one exchange of row sums through shared
-//   memory per LNB_ROWS rows).  A block holds as many groups as fit 512 threads (the registers of an
+//   LNB_ROWS rows are handled together (one exchange of row sums through shared memory for all of them).
+//   They come in by bulk copies, LNB_STAGES pairs of rows ahead per group (160 KB in flight on an SM): with
+//   loads into registers nothing was on its way while a block computed (32768 x 1024: 113 us).
+//   RING = false is the form with plain loads, for tensors that bulk copies cannot address (16 bytes).
+//    A block holds as many groups as fit 512 threads (the registers of an
 //   SM) and folds their sums before its atomics: with a block per group, 740 blocks adding to the same
 //   2304 addresses cost 12136 x 768 more than the register sums gain.
 // The eight columns of a thread belong to two dropout groups of eight; neighbouring lanes share both,
 // so each lane draws one and they swap.
 constexpr int LNB_ROWS = 2;
 constexpr int LNB_THREADS = 512;
+constexpr int LNB_STAGES = 2;
 
 __device__ __forceinline__ float4 ln_unpack4(uint2 p) {
   return make_float4(bf16_lo(p.x), bf16_hi(p.x), bf16_lo(p.y), bf16_hi(p.y));
@@ -108,11 +113,20 @@ __device__ __forceinline__ void ln_red4(float* dst, const float4& v) {
                : "memory");
 }
 
+__device__ __forceinline__ void ln_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+template <bool RING>
 __global__ void __launch_bounds__(LNB_THREADS, 1)
 ln_bwd_kernel(const LnBwdArgs a) {
   griddep_enter();
   constexpr int R = LNB_ROWS;
-  extern __shared__ __align__(16) float ln_fold[];          // [groups][3][d] when a block has several groups
+  // RING: [groups][stages][R rows of x | dres_in | dy]; at the end, and without it, [groups][3][d]
+  extern __shared__ __align__(16) float ln_fold[];
+  __shared__ uint64_t full[LNB_THREADS / 32][LNB_STAGES];
+  __shared__ int abort_word;
   __shared__ __align__(16) float red[2][LNB_THREADS / 32][2 * R];
   const int gt = blockDim.x;                                // threads of a row group (multiple of 32)
   const int t = threadIdx.x, grp = threadIdx.y, groups = blockDim.y;
@@ -131,8 +145,38 @@ ln_bwd_kernel(const LnBwdArgs a) {
   for (int u = 0; u < 2; ++u) gam[u] = own ? __ldg(reinterpret_cast<const float4*>(a.gamma) + c[u]) : zero;
 
   int par = 0;
-  const int step = gridDim.x * groups * R;
-  for (int row0 = (blockIdx.x * groups + grp) * R; row0 < a.M; row0 += step, par ^= 1) {
+  const int step = gridDim.x * groups * R, first = (blockIdx.x * groups + grp) * R;
+  uint8_t* ring = reinterpret_cast<uint8_t*>(ln_fold) + static_cast<size_t>(grp) * LNB_STAGES * R * 10 * d;
+  // rows row0 .. row0 + R - 1 (those below M) into stage st; one thread of the group
+  auto fetch = [&](int row0, int st) {
+    if (row0 >= a.M) return;
+    uint8_t* dst = ring + static_cast<size_t>(st) * R * 10 * d;
+    const uint32_t n = (a.M - row0 < R ? a.M - row0 : R) * d;           // elements
+    const long long off = static_cast<long long>(row0) * d;
+    mbar_expect_tx(&full[grp][st], n * (4 + (has_r ? 4 : 0) + (has_dy ? 2 : 0)));
+    ln_bulk_load(dst, a.x + off, n * 4, &full[grp][st]);
+    if (has_r) ln_bulk_load(dst + R * 4 * d, a.dres_in + off, n * 4, &full[grp][st]);
+    if (has_dy) ln_bulk_load(dst + R * 8 * d, a.dy + off, n * 2, &full[grp][st]);
+  };
+  if (RING) {
+    if (t == 0) {
+      for (int i = 0; i < LNB_STAGES; ++i) mbar_init(&full[grp][i], 1);
+      if (grp == 0) abort_word = 0;
+      mbar_fence_init();
+    }
+    __syncthreads();
+    if (t == 0)
+      for (int i = 0; i < LNB_STAGES; ++i) fetch(first + i * step, i);
+  }
+  int stage = 0;
+  uint32_t phase = 0;
+  for (int row0 = first; row0 < a.M; row0 += step, par ^= 1) {
+    const uint8_t* src = ring + static_cast<size_t>(stage) * R * 10 * d;
+    if (RING && !mbar_wait(&full[grp][stage], phase, &abort_word)) {
+      // every thread goes on (the group meets at barriers); the waits that follow end at once
+      *static_cast<volatile int*>(&abort_word) = 1;
+      if (a.status) atomicCAS(a.status, 0, ST_TIMEOUT_FULL);
+    }
     float4 xh[R][2], rv[R][2], dy[R][2];
     uint2 dyp[R][2];
     float mean[R], rstd[R];
@@ -150,9 +194,15 @@ ln_bwd_kernel(const LnBwdArgs a) {
       for (int u = 0; u < 2; ++u) {
         xh[i][u] = zero; rv[i][u] = zero; dyp[i][u] = make_uint2(0u, 0u);
         if (live) {
-          xh[i][u] = reinterpret_cast<const float4*>(a.x + (long long)row * d)[c[u]];
-          if (has_dy) dyp[i][u] = reinterpret_cast<const uint2*>(a.dy + (long long)row * d)[c[u]];
-          if (has_r) rv[i][u] = reinterpret_cast<const float4*>(a.dres_in + (long long)row * d)[c[u]];
+          if (RING) {
+            xh[i][u] = reinterpret_cast<const float4*>(src + i * 4 * d)[c[u]];
+            if (has_r) rv[i][u] = reinterpret_cast<const float4*>(src + (R + i) * 4 * d)[c[u]];
+            if (has_dy) dyp[i][u] = reinterpret_cast<const uint2*>(src + R * 8 * d + i * 2 * d)[c[u]];
+          } else {
+            xh[i][u] = reinterpret_cast<const float4*>(a.x + (long long)row * d)[c[u]];
+            if (has_dy) dyp[i][u] = reinterpret_cast<const uint2*>(a.dy + (long long)row * d)[c[u]];
+            if (has_r) rv[i][u] = reinterpret_cast<const float4*>(a.dres_in + (long long)row * d)[c[u]];
+          }
         }
       }
     }
@@ -201,6 +251,12 @@ ln_bwd_kernel(const LnBwdArgs a) {
       for (int w = 0; w < gwarps; ++w)
 #pragma unroll
         for (int k = 0; k < 2 * R; ++k) part[k] += red[par][grp * gwarps + w][k];
+    } else {
+      __syncwarp();
+    }
+    if (RING) {                                             // the group has read the stage
+      if (t == 0) fetch(row0 + LNB_STAGES * step, stage);
+      if (++stage == LNB_STAGES) { stage = 0; phase ^= 1; }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -240,6 +296,7 @@ ln_bwd_kernel(const LnBwdArgs a) {
   }
   if (!a.dgamma) return;
   if (groups > 1) {                                         // block-uniform
+    if (RING) __syncthreads();                              // the sums take the place of the ring
     float4* f = reinterpret_cast<float4*>(ln_fold);
     const int d4 = d >> 2;
     if (own && grp > 0)
@@ -310,12 +367,10 @@ int ab_layernorm_fwd(const float* x, const float* gamma, const float* beta, void
   if (d % 128 != 0 || d > 2048 || M <= 0) return -1;
   int grid = (M + LN_WARPS - 1) / LN_WARPS;
   if (grid > 148 * 8) grid = 148 * 8;
-  if (d <= 1024)
-    launch_chained(ln_fwd_kernel<8>, dim3(grid), dim3(LN_WARPS * 32), 0, stream, x, gamma, beta, (__nv_bfloat16*)y, mean,
-                                                         rstd, M, d, eps, rms);
-  else
-    launch_chained(ln_fwd_kernel<16>, dim3(grid), dim3(LN_WARPS * 32), 0, stream, x, gamma, beta, (__nv_bfloat16*)y, mean,
-                                                          rstd, M, d, eps, rms);
+  // 1280 columns in ten register groups: 72 registers and three blocks per SM, with sixteen 96 and two
+  auto kern = d <= 1024 ? ln_fwd_kernel<8> : d <= 1280 ? ln_fwd_kernel<10> : ln_fwd_kernel<16>;
+  launch_chained(kern, dim3(grid), dim3(LN_WARPS * 32), 0, stream, x, gamma, beta, (__nv_bfloat16*)y, mean, rstd, M, d,
+                 eps, rms);
   return (int)cudaGetLastError();
 }
 
@@ -324,14 +379,14 @@ int ab_layernorm_bwd(const void* dy, const float* x, const float* mean, const fl
                      float* dgamma, float* dbeta, float* dbias, const float* s0, const float* w0,
                      const float* s1, const float* w1, int M, int d, int rms,
                      unsigned long long drop_seed, unsigned int drop_stream,
-                     unsigned int drop_thr16, cudaStream_t stream) {
+                     unsigned int drop_thr16, int* status, cudaStream_t stream) {
   using namespace ab;
   if (d % 128 != 0 || d > 2048 || M <= 0) return -1;
   LnBwdArgs a;
   a.dy = (const __nv_bfloat16*)dy; a.x = x; a.mean = mean; a.rstd = rstd; a.gamma = gamma;
   a.dres_in = dres_in; a.dx = dx; a.dbranch = (__nv_bfloat16*)dbranch; a.dgamma = dgamma;
   a.dbeta = dbeta; a.dbias = dbias; a.s0 = s0; a.w0 = w0; a.s1 = s1; a.w1 = w1; a.M = M; a.d = d; a.rms = rms;
-  a.drop_seed = drop_seed; a.drop_stream = drop_stream; a.drop_thr16 = drop_thr16; a.salt = seed_salt_ptr();
+  a.drop_seed = drop_seed; a.drop_stream = drop_stream; a.drop_thr16 = drop_thr16; a.salt = seed_salt_ptr(); a.status = status;
   const int gt = ((d >> 3) + 31) / 32 * 32;                 // threads of a row group
   // groups per block: what 512 threads hold, but no more than leaves every SM a block
   const int want = (M + 148 * LNB_ROWS - 1) / (148 * LNB_ROWS);
@@ -339,16 +394,18 @@ int ab_layernorm_bwd(const void* dy, const float* x, const float* mean, const fl
   const int rows = groups * LNB_ROWS;
   int grid = (M + rows - 1) / rows;
   if (grid > 148) grid = 148;
-  const size_t smem = groups > 1 ? sizeof(float) * groups * 3 * d : 0;
-  static PerDeviceOnce attr_set;
-  if (attr_set.first_use_on_device()) {
-    // groups * d <= LNB_THREADS / gt * 8 * gt
-    cudaError_t e = cudaFuncSetAttribute(ln_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         LNB_THREADS * 8 * 3 * (int)sizeof(float));
+  const bool ring = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dres_in)) & 15) == 0;
+  const size_t smem = ring ? (size_t)groups * LNB_STAGES * LNB_ROWS * 10 * d : groups > 1 ? sizeof(float) * groups * 3 * d : 0;
+  auto kern = ring ? ln_bwd_kernel<true> : ln_bwd_kernel<false>;
+  static PerDeviceOnce attr_set[2];
+  if (attr_set[ring].first_use_on_device()) {
+    // groups * d <= LNB_THREADS / gt * 8 * gt columns
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         LNB_THREADS * 8 * (ring ? LNB_STAGES * LNB_ROWS * 10 : 3 * (int)sizeof(float)));
     if (e != cudaSuccess) return (int)e;
-    attr_set.mark_device();
+    attr_set[ring].mark_device();
   }
-  launch_chained(ln_bwd_kernel, dim3(grid), dim3(gt, groups), smem, stream, a);
+  launch_chained(kern, dim3(grid), dim3(gt, groups), smem, stream, a);
   return (int)cudaGetLastError();
 }
 }

@@ -37,7 +37,7 @@ def layernorm_bwd(dy, x, mean, rstd, gamma, dres_in, dx, dbranch, dgamma, dbeta,
         ptr(dy), ptr(x), ptr(mean), ptr(rstd), ptr(gamma), ptr(dres_in), ptr(dx), ptr(dbranch),
         ptr(dgamma), ptr(dbeta), ptr(dbias), ptr(s0), ptr(w0), ptr(s1), ptr(w1), c_int(M), c_int(d),
         c_int(int(rms)), c_ulonglong(drop_seed), c_uint(drop_stream),
-        c_uint(_lib.dropout_thr16(drop_p)), stream_ptr()), "ab_layernorm_bwd")
+        c_uint(_lib.dropout_thr16(drop_p)), ptr(_lib.status_word()), stream_ptr()), "ab_layernorm_bwd")
 
 
 # -------------------------------------------------------------- embedding ---

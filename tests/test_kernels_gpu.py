@@ -169,6 +169,24 @@ def test_layernorm_backward_column_sums_and_mask_at_row_group_edges(M, d):
         assert ((got.double() - terms.sum(0)).abs() <= 1e-6 + M * 2.0 ** -22 * terms.abs().sum(0)).all()
 
 
+def test_layernorm_backward_without_bulk_copies():
+    """A gradient at 8 bytes (bulk copies need 16) takes the form with plain loads: the same values."""
+    from allie_b200.ops import kernels as K
+
+    torch.manual_seed(9)
+    M, d = 301, 768
+    x, g, dres = torch.randn(M, d, device=DEV), torch.randn(d, device=DEV), torch.randn(M, d, device=DEV)
+    mean, rstd = x.mean(-1), (x.var(-1, unbiased=False) + 1e-5).rsqrt()
+    room = torch.randn(M * d + 4, device=DEV).bfloat16()
+    results = []
+    for dy in (room[4:].view(M, d), room[4:].view(M, d).clone()):
+        dx, db = torch.empty(M, d, device=DEV), torch.empty(M, d, device=DEV, dtype=torch.bfloat16)
+        K.layernorm_bwd(dy, x, mean, rstd, g, dres, dx, db, torch.zeros(d, device=DEV), torch.zeros(d, device=DEV))
+        _done()
+        results.append((dx, db))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 def _thr16(p):
     from allie_b200.ops import _lib
 
