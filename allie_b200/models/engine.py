@@ -21,6 +21,7 @@ from __future__ import annotations
 import math
 import os
 import re
+from functools import cached_property
 
 import numpy as np
 import torch
@@ -319,6 +320,22 @@ class B200Engine:
             self.bv = self._views(self.reg.value_head[0].bias)
             self.wt = self._views(self.reg.time_head[0].weight)
             self.bt = self._views(self.reg.time_head[0].bias)
+
+    @cached_property
+    def _infer_layers(self):
+        """The layers' addresses for the native inference schedule.  They are views of the arenas that
+        this engine holds for its lifetime (240 us of attribute stores per pass otherwise).  GEMM weights
+        are read as bf16, norms and biases as fp32."""
+        from ..ops.infer import InferLayer
+
+        layers = (InferLayer * self.cfg.n_layer)()
+        for dst, L in zip(layers, self.layers):
+            for name in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_b", "o_b", "fc_b", "pr_b"):
+                t = L[name][0]
+                setattr(dst, name, 0 if t is None else t.data_ptr())
+            for name in ("qkv_w", "o_w", "fc_w", "pr_w"):
+                setattr(dst, name, L[name][1].data_ptr())
+        return layers
 
     # -------------------------------------------------------------- buffers
     def _buffers(self, B: int, T: int, train: bool) -> dict:
@@ -693,7 +710,7 @@ class B200Engine:
         ``kv``: optional ``(k, v)`` caches [layer, sequence, head, slot, head_dim] that receive the keys
         and values of all positions.  Dense models only."""
         from ..ops.gemm import num_sms
-        from ..ops.infer import Infer, InferLayer, infer_last
+        from ..ops.infer import Infer, infer_last
 
         cfg, dev = self.cfg, self.device
         assert self.dense
@@ -725,24 +742,16 @@ class B200Engine:
             setattr(a, name, t.data_ptr())
         for name, off in (("ids", 0), ("pos", M), ("row0", 2 * M), ("last", 2 * M + n + 1)):
             setattr(a, name, batch.data_ptr() + 4 * off)
-        address = lambda t: 0 if t is None else t.data_ptr()
         for name, t in (("wte", self.wte[0]), ("wpe", self.wpe[0]), ("ctrl", self.ctrl_w[0]), ("lnf_w", self.lnf_w[0]),
                         ("lnf_b", self.lnf_b[0]), ("wte_bf16", self.wte[1])):
-            setattr(a, name, address(t))
+            setattr(a, name, 0 if t is None else t.data_ptr())
         if self.reg is not None:
             for name, t in (("wv", self.wv[0]), ("bv", self.bv[0]), ("wt", self.wt[0]), ("bt", self.bt[0])):
                 setattr(a, name, t.data_ptr())
         if kv is not None:
             k, v = kv
             a.kc, a.vc, a.kv_layer, a.S = k.data_ptr(), v.data_ptr(), k.stride(0), k.shape[3]
-        # GEMM weights are read as bf16, norms and biases as fp32
-        layers = (InferLayer * cfg.n_layer)()
-        for dst, L in zip(layers, self.layers):
-            for name in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_b", "o_b", "fc_b", "pr_b"):
-                setattr(dst, name, address(L[name][0]))
-            for name in ("qkv_w", "o_w", "fc_w", "pr_w"):
-                setattr(dst, name, L[name][1].data_ptr())
-        infer_last(a, layers)
+        infer_last(a, self._infer_layers)
         return scratch["logits"], scratch.get("value"), scratch.get("time")
 
     def zero_grad(self) -> None:

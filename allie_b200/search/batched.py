@@ -136,7 +136,7 @@ class KVStepEvaluator:
             if g is None:
                 rows.append(np.array([self.tok.bos_token_id], dtype=np.int64))
             else:
-                rows.append((self.tok.tokenize(g)[: self.tok.max_length] & 0x3FFF).astype(np.int64))
+                rows.append(self.tok.token_ids(g)[: self.tok.max_length])
         return self.kv.prefill(rows)
 
     def step(self, req: dict) -> tuple[np.ndarray, np.ndarray]:

@@ -89,9 +89,12 @@ class EngineRunner(ModelRunner):
         self.calls += 1
         games, eng, n = list(games), self.engine, len(games)
         if eng.dense and games and not isinstance(games[0], np.ndarray):
-            words = [self.tokenizer.tokenize(g)[: self.tokenizer.max_length] for g in games]
-            assert all(int(((w & 0xFFFF) >> 14).max()) < 3 for w in words)
-            logits, value, time = eng.infer_last([w & 0x3FFF for w in words])
+            tok = self.tokenizer
+            rows = [tok.token_ids(g)[: tok.max_length] for g in games]
+            if any(e + len(tok) > 0x3FFF for g in games for e in (g.white_elo, g.black_elo)):
+                # ratings that run into the outcome bits of a word: refused where the padded batch does
+                assert all(int(((tok.tokenize(g)[: tok.max_length] & 0xFFFF) >> 14).max()) < 3 for g in games)
+            logits, value, time = eng.infer_last(rows)
         else:      # experts are laid out for a fixed number of rows; arrays come as equal windows already
             batch = self.tokenizer.pad_and_collate(games, return_labels=False)
             out = eng.evaluate_batch(batch, with_loss=False)

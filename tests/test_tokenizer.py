@@ -1,5 +1,6 @@
 """Tokenizer / vocabulary golden tests (CPU)."""
 import numpy as np
+import pytest
 import torch
 from hypothesis import given, settings, strategies as st
 
@@ -101,3 +102,22 @@ def test_time_normalisation_and_json():
     p = json_to_partial_game(row, 1)
     assert p.moves == ["e2e4"] and p.next_move_seconds == 2 and p.outcome is None
     assert Game.from_dict(g.to_dict()) == g
+
+
+@pytest.mark.parametrize("outcome,resigned,secs", [(None, False, [1, 0, 9]), ("1-0", True, [65534, 3, -1]),
+                                                   ("0-1", False, [True, 2, 3]), (None, True, [])])
+def test_token_ids_are_the_ids_of_the_words(outcome, resigned, secs):
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    g = Game("180+0", 1500, 2900, outcome, resigned, ["e2e4", "nonsense", "g1f3"][:len(secs)], secs)
+    want = tok.tokenize(g) & 0x3FFF
+    got = tok.token_ids(g)
+    assert got.dtype == np.uint32 and (got == want).all()
+
+
+@pytest.mark.parametrize("secs,error", [([65535], AssertionError), ([0.5], TypeError), ([], AssertionError)])
+def test_token_ids_refuses_what_tokenize_refuses(secs, error):
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    g = Game("180+0", 1500, 2900, None, False, ["e2e4"], secs)
+    for f in (tok.tokenize, tok.token_ids):
+        with pytest.raises(error):
+            f(g)
