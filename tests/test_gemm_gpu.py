@@ -188,6 +188,7 @@ def test_gemm_gelu_derivative_kept_in_aux():
 @pytest.mark.parametrize("M,N,K", [(512, 256, 64),      # one tile per pair, both column groups of every warp
                                    (520, 264, 72),      # rows past a tile, eight columns in the last tile
                                    (1100, 800, 256),    # last column tile ends inside a warp's first group
+                                   (4744, 808, 72),     # the same edges beyond one wave of smaller tiles: on pairs
                                    (20000, 512, 128)])  # several units per pair: tiles fetched one unit ahead
 def test_gemm_pair_residual_tiles(M, N, K, drop_p):
     """CTA-pair kernel with a fp32 residual: its tiles travel by TMA through the output staging tile."""
@@ -215,7 +216,8 @@ def test_gemm_pair_residual_tiles(M, N, K, drop_p):
         assert torch.allclose(out, ref, rtol=1e-4, atol=1e-4 * K ** 0.5)
 
 
-@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (520, 264, 72), (1100, 800, 256), (20000, 512, 128)])
+@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (520, 264, 72), (1100, 800, 256), (20000, 512, 128),
+                                   (4744, 1032, 136), (5000, 808, 72)])
 def test_gemm_pair_specialised_epilogues(M, N, K):
     """Every specialised drain of the CTA-pair kernel at tile edges: rows and columns past a tile, a last
     column tile that ends inside a warp's columns, several units per pair."""
