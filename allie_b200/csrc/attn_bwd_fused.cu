@@ -726,9 +726,6 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     if (p.valid()) fetch(p, lse_raw, dlt, keep32);
     for (; p.valid() && ok; p.next()) {
       if (p.it == 0 && p.own == 0) { b = p.bh / a.H; h = p.bh - b * a.H; }
-      const int qi = p.own + p.it;
-      const int q_idx = qi * 128 + r;
-      const bool q_ok = q_idx < a.T;
       const bool diag = p.it == 0;
       float n_lse = 0.f, n_dlt = 0.f;
       uint32_t n_keep = 0xffffffffu;
