@@ -254,14 +254,16 @@ kv_store_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict
 }
 
 // out row: [0, max_legal) priors over the legal moves in list order, then value, time, resign logit,
-// best legal logit.  One warp per tree.
+// best legal logit.  Behind the last row: the status word, so that the copy which brings the results to the
+// host also tells whether a wait of this pass ran out.  One warp per tree.
 __global__ void __launch_bounds__(32)
 policy_epilogue_kernel(const __nv_bfloat16* __restrict__ logits, long long ld,
                        const int* __restrict__ active, const int* __restrict__ legal, int legal_stride,
                        const int* __restrict__ n_legal, const float* __restrict__ value,
                        const float* __restrict__ time, int resign_id, float inv_temperature,
-                       float* __restrict__ out, int out_stride) {
+                       float* __restrict__ out, int out_stride, const int* __restrict__ status) {
   const int t = blockIdx.x, lane = threadIdx.x;
+  if (t == 0 && lane == 0) out[static_cast<long long>(gridDim.x) * out_stride] = __int_as_float(*status);
   if (!active[t]) return;
   const int n = min(n_legal[t], legal_stride);
   const __nv_bfloat16* lr = logits + static_cast<long long>(t) * ld;
@@ -324,13 +326,14 @@ int ab_kv_store(const void* qkv, void* kc, void* vc, const int* len, int n_trees
   return (int)cudaGetLastError();
 }
 
+// out: n_trees rows of out_stride values and one more word, which receives *status
 int ab_policy_epilogue(const void* logits, long long ld, const int* active, const int* legal,
                        int legal_stride, const int* n_legal, const float* value, const float* time,
                        int resign_id, float inv_temperature, float* out, int out_stride, int n_trees,
-                       cudaStream_t stream) {
+                       const int* status, cudaStream_t stream) {
   ab::policy_epilogue_kernel<<<n_trees, 32, 0, stream>>>((const __nv_bfloat16*)logits, ld, active, legal,
                                                          legal_stride, n_legal, value, time, resign_id,
-                                                         inv_temperature, out, out_stride);
+                                                         inv_temperature, out, out_stride, status);
   return (int)cudaGetLastError();
 }
 }

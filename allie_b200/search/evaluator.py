@@ -45,8 +45,11 @@ class KVLeafEvaluator:
         self.req_host = torch.zeros(o, dtype=i32, pin_memory=True)
         self.req_dev = torch.zeros(o, dtype=i32, device=dev)
         self.out_stride = legal_max + 4
-        self.out_dev = torch.zeros(n, self.out_stride, dtype=f32, device=dev)
-        self.out_host = torch.zeros(n, self.out_stride, dtype=f32, pin_memory=True)
+        # result rows, and the status word behind them (written by the step's last kernel)
+        self.out_flat = torch.zeros(n * self.out_stride + 1, dtype=f32, device=dev)
+        self.out_flat_host = torch.zeros(n * self.out_stride + 1, dtype=f32, pin_memory=True)
+        self.out_host = self.out_flat_host[:-1].view(n, self.out_stride)
+        self.status_host = self.out_flat_host[-1:].view(i32)
         e = lambda *s, dt=bf: torch.empty(*s, dtype=dt, device=dev)
         self.x = [e(n, d, dt=f32), e(n, d, dt=f32)]
         self.ln, self.qkv, self.att = e(n, d), e(n, 3 * d), e(n, d)
@@ -91,11 +94,13 @@ class KVLeafEvaluator:
             logits, value, time = self._prefill_padded(token_rows, lens)
         # one device-to-host copy
         V = logits.size(1)
-        out = torch.zeros(n, V + 2, dtype=torch.float32, device=eng.device)
+        out, flat = _lib.rows_and_status(n, V + 2, eng.device)
         out[:, :V] = logits
         if eng.reg is not None:
             out[:, V], out[:, V + 1] = value, time
-        out = out.cpu()
+        else:
+            out[:, V:] = 0
+        out = _lib.fetch_rows(out, flat)
         self.view(self.req_host, "prefix_len").copy_(torch.tensor(lens, dtype=torch.int32))
         return out[:, :V], out[:, V], out[:, V + 1]
 
@@ -165,8 +170,8 @@ class KVLeafEvaluator:
                                     ptr(self.view(rd, "active")), ptr(self.view(rd, "legal")),
                                     c_int(self.legal_max), ptr(self.view(rd, "n_legal")),
                                     ptr(self.value if has_heads else None), ptr(self.time if has_heads else None),
-                                    c_int(self.resign_id), c_float(1.0), ptr(self.out_dev),
-                                    c_int(self.out_stride), c_int(n), stream_ptr())
+                                    c_int(self.resign_id), c_float(1.0), ptr(self.out_flat),
+                                    c_int(self.out_stride), c_int(n), ptr(_lib.status_word()), stream_ptr())
         assert rc == 0
         _lib.count_launches(1)
 
@@ -187,7 +192,8 @@ class KVLeafEvaluator:
     @torch.no_grad()
     def step(self) -> np.ndarray:
         """Evaluates the requests currently in ``req_host``; returns the packed result rows
-        (host, [n, legal_max + 4]: priors..., value, time, resign logit, best legal logit)."""
+        (host, [n, legal_max + 4]: priors..., value, time, resign logit, best legal logit).  Raises if a
+        wait of one of the step's kernels ran out."""
         self.req_dev.copy_(self.req_host, non_blocking=True)
         if self.use_graph:
             if self.graph is None:
@@ -200,7 +206,8 @@ class KVLeafEvaluator:
             self.graph.replay()
         else:
             self._launch_step()
-        self.out_host.copy_(self.out_dev, non_blocking=True)
+        self.out_flat_host.copy_(self.out_flat, non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        _lib.raise_on_status(int(self.status_host))
         self.steps += 1
         return self.out_host.numpy()

@@ -16,6 +16,7 @@ import torch
 
 from ..data import Game, UCITokenizer
 from ..models import unwrap
+from ..ops import _lib
 
 
 @dataclass
@@ -104,14 +105,14 @@ class EngineRunner(ModelRunner):
             value, time = ((out["value_logits"][rows, idx], out["time_logits"][rows, idx]) if self.has_value_head
                            else (None, None))
         V = logits.size(-1)
-        packed = torch.empty(n, V + 2, dtype=torch.float32, device=eng.device)
+        packed, flat = _lib.rows_and_status(n, V + 2, eng.device)
         packed[:, :V] = logits
         if self.has_value_head:
             packed[:, V] = value
             packed[:, V + 1] = time
         else:
             packed[:, V:] = 0
-        host = packed.cpu()          # the one device-to-host copy of this evaluation
+        host = _lib.fetch_rows(packed, flat)     # the one device-to-host copy of this evaluation
         return Evaluation(host[:, :V], host[:, V], host[:, V + 1])
 
 
