@@ -53,6 +53,7 @@ struct DecodeFewArgs {
   int slices[4];                                   // of the contraction, per matrix
   int pitch;                                       // bytes per row of the operand buffer
   unsigned int* arrivals;                          // zero at launch
+  long long max_wait;                              // clock cycles at a meeting
   int* status;
 };
 
@@ -279,7 +280,7 @@ decode_few_kernel(const DecodeFewArgs g) {
   float* sM = reinterpret_cast<float*>(sA + DF_MAX_N * g.pitch);     // 8 x (HD + 2): attention's merge
   DecodeLayer* sL = reinterpret_cast<DecodeLayer*>(sM + DF_WARPS * (HD + 2));
   __shared__ uint64_t full[DF_STAGES], empty[DF_STAGES];
-  __shared__ int abort_word;
+  __shared__ int abort_word, met;
   volatile int* abort_flag = &abort_word;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cta = blockIdx.x, ctas = gridDim.x;
@@ -340,7 +341,9 @@ decode_few_kernel(const DecodeFewArgs g) {
   bool good = true;     // of this warp: after a wait that ran out it goes through the motions up to the barrier
   // All CTAs have finished the phase and see its results (read through L2 afterwards).  One addition and
   // one watching thread per CTA; the release and the acquire order the CTA's other accesses.  (A flag per
-  // CTA that threads of all CTAs watch keeps 148 x 148 loads in flight and takes longer.)
+  // CTA that threads of all CTAs watch keeps 148 x 148 loads in flight and takes longer.)  The verdict is one
+  // thread's: were each warp to read the abort flag, which the producer may set at any time, those that saw
+  // it would leave and the others wait at the next df_sync for good.
   auto grid_barrier = [&]() {
     target += ctas;
     df_sync();
@@ -351,15 +354,16 @@ decode_few_kernel(const DecodeFewArgs g) {
       while (true) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(g.arrivals) : "memory");
         if (static_cast<int>(seen - target) >= 0) break;
-        if ((++spins & 0xff) == 0 && (*abort_flag || clock64() - t0 > AB_SPIN_CYCLES)) {
+        if ((++spins & 0xf) == 0 && (*abort_flag || clock64() - t0 > g.max_wait)) {
           *abort_flag = ST_TIMEOUT_MISC;
           atomicCAS(g.status, 0, ST_TIMEOUT_MISC);
           break;
         }
       }
+      met = *abort_flag == 0;
     }
     df_sync();
-    return *abort_flag == 0;
+    return met != 0;                               // rewritten behind the next meeting's first df_sync
   };
   // Vectors (norms, biases) and cached keys / values are read once per step, so they come from memory:
   // a latency in the middle of a phase, unless they are asked for a phase or a layer ahead.
@@ -439,7 +443,8 @@ decode_few_kernel(const DecodeFewArgs g) {
         uint32_t a_addr = smem_u32(sA) + (lane & 15) * g.pitch + (lane >> 4) * 16 + a_col * 2;
         const uint32_t w_off = lane * 128 + ((warp ^ (lane & 7)) << 4);
         for (int c = 0; c < p.k / DF_CHUNK; ++c) {
-          if (good && !mbar_wait(&full[slot], par, abort_flag)) {
+          // one answer per warp: its lanes go through ldmatrix and the MMAs together
+          if (good && !__all_sync(0xffffffffu, mbar_wait(&full[slot], par, abort_flag))) {
             good = false;
             *abort_flag = ST_TIMEOUT_FULL;
             atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
@@ -480,12 +485,13 @@ decode_few_kernel(const DecodeFewArgs g) {
 }  // namespace ab
 
 // Layers of one search step for n <= 16 trees.  `layers`: device array of DecodeLayer.  `work`: device
-// scratch of 256 + n * (3 * d + F) words, cleared here.  Returns 1, with nothing launched, for shapes that
-// the chain of kernels serves.
+// scratch of 256 + n * (3 * d + F) words, cleared here.  `max_wait`: clock cycles after which a CTA gives up
+// at a meeting (0: the usual second).  Returns 1, with nothing launched, for shapes that the chain of
+// kernels serves.
 extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int H, int F, int S, int rms, float eps,
                              float* x, void* att, const int* active, const int* slot, const int* prefix_len,
-                             const int* anc, int anc_stride, const int* n_anc, void* work, int max_ctas, int* status,
-                             cudaStream_t stream) {
+                             const int* anc, int anc_stride, const int* n_anc, void* work, int max_ctas,
+                             long long max_wait, int* status, cudaStream_t stream) {
   using namespace ab;
   const int hd = H > 0 ? d / H : 0;
   if (n < 1 || n > DF_MAX_N || n_layer < 1 || n_layer > DF_MAX_LAYERS || d % 128 || F % 128 || d > DF_MAX_K ||
@@ -520,6 +526,7 @@ extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int 
   g.fc = g.qkv + static_cast<long long>(n) * 3 * d;
   g.active = active; g.slot = slot; g.prefix_len = prefix_len; g.anc = anc; g.anc_stride = anc_stride; g.n_anc = n_anc;
   g.pitch = longest * 2 + 16;                      // eight rows fall on different banks
+  g.max_wait = max_wait > 0 ? max_wait : AB_SPIN_CYCLES;
   g.status = status;
   const int smem = DF_STAGES * DF_SLOT + DF_MAX_N * g.pitch + DF_WARPS * (hd + 2) * 4 + n_layer * (int)sizeof(DecodeLayer);
   auto kern = hd == 64 ? decode_few_kernel<64> : decode_few_kernel<128>;

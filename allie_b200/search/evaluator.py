@@ -60,6 +60,7 @@ class KVLeafEvaluator:
         # a handful of trees: all layers in one kernel (csrc/decode_few.cu), which reads the layers'
         # addresses from this table and keeps its accumulators in this scratch
         self.few = n_trees <= self.FEW_TREES and engine.dense
+        self.few_max_wait = 0           # clock cycles at a meeting of that kernel's CTAs; 0: about a second
         if self.few:
             addr = lambda t: 0 if t is None else t.data_ptr()
             table = [[addr(Ly[k][0]) for k in ("ln1_w", "ln1_b", "ln2_w", "ln2_b", "qkv_b", "o_b", "fc_b", "pr_b")]
@@ -183,7 +184,7 @@ class KVLeafEvaluator:
             c_int(cfg.ffn_dim), c_int(self.S), c_int(int(self.eng.rms)), c_float(cfg.layer_norm_epsilon), ptr(x),
             ptr(self.att), ptr(self.view(rd, "active")), ptr(self.view(rd, "slot")), ptr(self.view(rd, "prefix_len")),
             ptr(self.view(rd, "anc")), c_int(self.anc_max), ptr(self.view(rd, "n_anc")), ptr(self.few_work),
-            c_int(num_sms()), ptr(_lib.status_word()), stream_ptr())
+            c_int(num_sms()), c_longlong(self.few_max_wait), ptr(_lib.status_word()), stream_ptr())
         if rc < 0:
             raise RuntimeError(f"ab_decode_few failed with code {rc}")
         _lib.count_launches(int(rc == 0))

@@ -61,3 +61,35 @@ def test_few_tree_step_matches_the_chain(n, d, heads, inner, norm):
         assert float((la - lb).norm() / lb.norm()) < 1e-2
         assert np.abs(va - vb).max() < 1e-2
         assert np.abs(pa - pb).max() < 1e-2
+
+
+def test_few_tree_step_ends_when_meetings_run_out():
+    """One tree with a very long prompt: the CTAs that hold its heads read keys for hundreds of microseconds
+    while the others wait at the meeting, longer than the limit set here.  All leave together (a verdict
+    per CTA), the step raises, and with the usual limit it works again."""
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.ops import _lib
+    from allie_b200.search.evaluator import KVLeafEvaluator
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=3, n_embd=256,
+                             n_head=4, n_positions=64)
+    keys = 40000
+    ev = KVLeafEvaluator(B200Engine(model, "cuda"), 1, max_prefix=keys, max_nodes=8, anc_max=4, legal_max=8, use_graph=False)
+    for name, v in (("active", 1), ("tok", 5), ("pos", 9), ("slot", keys), ("prefix_len", keys), ("n_anc", 1),
+                    ("n_legal", 8)):
+        ev.view(ev.req_host, name).fill_(v)
+    ev.view(ev.req_host, "anc").fill_(keys)
+    ev.view(ev.req_host, "legal").copy_(torch.arange(8))
+    want = ev.step().copy()
+    for _ in range(5):
+        ev.few_max_wait = 20000                  # about ten microseconds
+        with pytest.raises(RuntimeError, match="timeout"):
+            ev.step()
+        ev.few_max_wait = 0
+        got = ev.step()
+        _lib.check_status()
+        assert np.allclose(got, want, rtol=1e-2, atol=1e-3)
