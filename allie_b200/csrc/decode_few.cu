@@ -530,8 +530,18 @@ extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int 
   g.status = status;
   const int smem = DF_STAGES * DF_SLOT + DF_MAX_N * g.pitch + DF_WARPS * (hd + 2) * 4 + n_layer * (int)sizeof(DecodeLayer);
   auto kern = hd == 64 ? decode_few_kernel<64> : decode_few_kernel<128>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return -static_cast<int>(e);
+  // the most any model needs, once: set to each call's own size, one thread's call lowers the limit between
+  // another's setting and its launch
+  constexpr int SMEM_MAX = DF_STAGES * DF_SLOT + DF_MAX_N * (DF_MAX_K * 2 + 16) + DF_WARPS * (128 + 2) * 4 +
+                           DF_MAX_LAYERS * (int)sizeof(DecodeLayer);
+  static PerDeviceOnce attr[2];
+  PerDeviceOnce& once = attr[hd == 128];
+  cudaError_t e = cudaSuccess;
+  if (once.first_use_on_device()) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+    if (e != cudaSuccess) return -static_cast<int>(e);
+    once.mark_device();
+  }
   e = cudaMemsetAsync(work, 0, sizeof(float) * (DF_WORK_HEAD + static_cast<size_t>(n) * (3 * d + F)), stream);
   if (e != cudaSuccess) return -static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};

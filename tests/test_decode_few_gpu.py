@@ -93,3 +93,44 @@ def test_few_tree_step_ends_when_meetings_run_out():
         got = ev.step()
         _lib.check_status()
         assert np.allclose(got, want, rtol=1e-2, atol=1e-3)
+
+
+def _idle_evaluator(n_layer, n=1):
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.search.evaluator import KVLeafEvaluator
+
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=n_layer, n_embd=128,
+                             n_head=2, n_inner=128, n_positions=64)
+    ev = KVLeafEvaluator(B200Engine(model, "cuda"), n, max_prefix=16, max_nodes=8, anc_max=4, legal_max=8, use_graph=False)
+    ev.x[0].zero_()
+    return ev
+
+
+def test_few_tree_launches_of_two_threads_with_different_models():
+    """A deep and a shallow model need different amounts of shared memory; neither thread's launches may
+    depend on what the other set last."""
+    import threading
+
+    from allie_b200.ops import _lib
+
+    evs = [_idle_evaluator(60), _idle_evaluator(1)]
+    errors = []
+
+    def loop(ev):
+        try:
+            for _ in range(400):
+                assert ev._launch_few(ev.x[0])
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=loop, args=(ev,)) for ev in evs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert not errors, errors
