@@ -486,8 +486,8 @@ decode_few_kernel(const DecodeFewArgs g) {
 
 // Layers of one search step for n <= 16 trees.  `layers`: device array of DecodeLayer.  `work`: device
 // scratch of 256 + n * (3 * d + F) words, cleared here.  `max_wait`: clock cycles after which a CTA gives up
-// at a meeting (0: the usual second).  Returns 1, with nothing launched, for shapes that the chain of
-// kernels serves.
+// at a meeting (0: the usual second).  Returns 1, with no kernel launched, for shapes that the chain of
+// kernels serves and where max_ctas CTAs cannot all be resident (a process that has part of the SMs).
 extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int H, int F, int S, int rms, float eps,
                              float* x, void* att, const int* active, const int* slot, const int* prefix_len,
                              const int* anc, int anc_stride, const int* n_anc, void* work, int max_ctas,
@@ -542,6 +542,12 @@ extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int 
     if (e != cudaSuccess) return -static_cast<int>(e);
     once.mark_device();
   }
+  int per_sm = 0, sms = 0, dev = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DF_THREADS, smem);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return -static_cast<int>(e);
+  if (per_sm * sms < max_ctas) return 1;
   e = cudaMemsetAsync(work, 0, sizeof(float) * (DF_WORK_HEAD + static_cast<size_t>(n) * (3 * d + F)), stream);
   if (e != cudaSuccess) return -static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};
@@ -554,5 +560,10 @@ extern "C" int ab_decode_few(const void* layers, int n_layer, int n, int d, int 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return -static_cast<int>(cudaLaunchKernelEx(&cfg, kern, g));
+  e = cudaLaunchKernelEx(&cfg, kern, g);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {   // nothing was launched, and nothing is wrong otherwise
+    cudaGetLastError();
+    return 1;
+  }
+  return -static_cast<int>(e);
 }

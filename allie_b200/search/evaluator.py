@@ -177,7 +177,8 @@ class KVLeafEvaluator:
         _lib.count_launches(1)
 
     def _launch_few(self, x) -> bool:
-        """All layers of the step as one kernel; False (nothing launched) for shapes it does not take."""
+        """All layers of the step as one kernel; False (nothing launched) for shapes it does not take and
+        where its CTAs cannot all be resident."""
         cfg, rd = self.eng.cfg, self.req_dev
         rc = _lib.cuda().ab_decode_few(
             ptr(self.layer_table), c_int(cfg.n_layer), c_int(self.n), c_int(cfg.n_embd), c_int(cfg.n_head),

@@ -134,3 +134,26 @@ def test_few_tree_launches_of_two_threads_with_different_models():
     torch.cuda.synchronize()
     _lib.check_status()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_few_tree_step_that_cannot_be_resident_takes_the_chain(monkeypatch, use_graph):
+    """More CTAs than can be resident at once (here by asking for three per SM): the step is served by the
+    chain of kernels, captured or not, with the chain's results."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import num_sms
+    from allie_b200.search import evaluator
+
+    ev = _idle_evaluator(2, n=2)
+    ev.use_graph = use_graph
+    for name, v in (("active", 1), ("tok", 5), ("pos", 0), ("slot", 0), ("prefix_len", 0), ("n_anc", 1), ("n_legal", 8)):
+        ev.view(ev.req_host, name).fill_(v)
+    ev.view(ev.req_host, "legal").copy_(torch.arange(8).expand(2, 8))
+    ev.few = False
+    want = ev.step().copy()
+    ev.few, ev.graph = True, None
+    monkeypatch.setattr(evaluator, "num_sms", lambda: 3 * num_sms())
+    got = ev.step()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert np.array_equal(got, want)
