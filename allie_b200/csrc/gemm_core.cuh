@@ -361,7 +361,7 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
     uint8_t* rowp = stg + lane * 128;
     const int sw = lane & 7;
     const uint32_t thr16 = g.ep.drop_thr16;
-    const float s = dropout_scale(thr16);
+    const uint64_t s2 = f2_bcast(dropout_scale(thr16));
 #pragma unroll 1
     for (int grp = 0; grp < 2; ++grp) {
       const int gn0 = nbase + grp * 32;
@@ -390,9 +390,11 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
         float o[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          if (thr16)
-            v[j] = f2_mul(v[j], f2_pack(((keep >> (c * 8 + 2 * j)) & 1u) ? s : 0.f,
-                                        ((keep >> (c * 8 + 2 * j + 1)) & 1u) ? s : 0.f));
+          if (thr16) {               // selected, not multiplied by zero: a dropped Inf or NaN is a zero
+            float x0, x1;
+            f2_unpack(f2_mul(v[j], s2), x0, x1);
+            v[j] = f2_pack(((keep >> (c * 8 + 2 * j)) & 1u) ? x0 : 0.f, ((keep >> (c * 8 + 2 * j + 1)) & 1u) ? x1 : 0.f);
+          }
           f2_unpack(f2_add(v[j], res[j]), o[2 * j], o[2 * j + 1]);
         }
         *s0 = make_float4(o[0], o[1], o[2], o[3]);

@@ -285,3 +285,29 @@ def test_gemm_column_sums_and_head_products(M, N, K):
         assert torch.equal(out, gemm(a, w))
         prod = (out.double() * aux.double()).view(M // T, T, N // 64, 64).permute(0, 2, 1, 3)
         assert ((dot.double() - prod.sum(-1)).abs() <= 1e-6 + 64 * 2.0 ** -23 * prod.abs().sum(-1)).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(4744, 808, 72), (512, 256, 64)])     # CTA pairs; one wave of smaller tiles
+def test_gemm_residual_drops_non_finite_values(M, N, K):
+    """A dropped element adds nothing to the residual, whatever it was: Inf and NaN of one row of the product
+    stay out of its dropped columns."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(7)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w = torch.rand(K, N, device="cuda").add_(1.0).bfloat16()
+    resid = torch.randn(M, N, device="cuda")
+    kw = dict(b_mn=True, drop_p=0.25, drop_seed=5, drop_stream=2)
+    kept = gemm(torch.ones_like(a), w, out=torch.empty_like(resid), resid=torch.zeros_like(resid), **kw) != 0
+    a[3] = float("inf")
+    a[M - 1] = float("nan")
+    out = gemm(a, w, out=torch.empty_like(resid), resid=resid, **kw)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert 0.7 < float(kept.float().mean()) < 0.8
+    assert torch.equal(out[~kept], resid[~kept])
+    assert torch.isinf(out[3][kept[3]]).all() and torch.isnan(out[M - 1][kept[M - 1]]).all()
+    keep = torch.ones(M, dtype=torch.bool, device="cuda")
+    keep[[3, M - 1]] = False
+    assert out[keep].isfinite().all()
