@@ -127,6 +127,7 @@ ln_bwd_kernel(const LnBwdArgs a) {
   extern __shared__ __align__(16) float ln_fold[];
   __shared__ uint64_t full[LNB_THREADS / 32][LNB_STAGES];
   __shared__ int abort_word;
+  __shared__ int late[LNB_THREADS / 32][3];                 // first wait of a group's thread 0 that ran out
   __shared__ __align__(16) float red[2][LNB_THREADS / 32][2 * R];
   const int gt = blockDim.x;                                // threads of a row group (multiple of 32)
   const int t = threadIdx.x, grp = threadIdx.y, groups = blockDim.y;
@@ -162,6 +163,7 @@ ln_bwd_kernel(const LnBwdArgs a) {
     if (t == 0) {
       for (int i = 0; i < LNB_STAGES; ++i) mbar_init(&full[grp][i], 1);
       if (grp == 0) abort_word = 0;
+      late[grp][0] = -1;
       mbar_fence_init();
     }
     __syncthreads();
@@ -176,6 +178,7 @@ ln_bwd_kernel(const LnBwdArgs a) {
       // every thread goes on (the group meets at barriers); the waits that follow end at once
       *static_cast<volatile int*>(&abort_word) = 1;
       if (a.status) atomicCAS(a.status, 0, ST_TIMEOUT_FULL);
+      if (t == 0 && late[grp][0] < 0) { late[grp][0] = row0; late[grp][1] = stage; late[grp][2] = phase; }
     }
     float4 xh[R][2], rv[R][2], dy[R][2];
     uint2 dyp[R][2];
@@ -255,7 +258,7 @@ ln_bwd_kernel(const LnBwdArgs a) {
       __syncwarp();
     }
     if (RING) {                                             // the group has read the stage
-      if (t == 0) fetch(row0 + LNB_STAGES * step, stage);
+      if (t == 0 && late[grp][0] < 0) fetch(row0 + LNB_STAGES * step, stage);
       if (++stage == LNB_STAGES) { stage = 0; phase ^= 1; }
     }
 #pragma unroll
@@ -292,6 +295,14 @@ ln_bwd_kernel(const LnBwdArgs a) {
           sc[u].x += o.x; sc[u].y += o.y; sc[u].z += o.z; sc[u].w += o.w;
         }
       }
+    }
+  }
+  if (RING && t == 0 && late[grp][0] >= 0) {
+    // The thread that fetches has stopped there; what it had under way lands before the block reuses or
+    // leaves its shared memory.
+    for (int i = 0; i < LNB_STAGES; ++i) {
+      const int row0 = late[grp][0] + i * step, st = (late[grp][1] + i) % LNB_STAGES;
+      if (row0 < a.M) mbar_wait_landed(&full[grp][st], late[grp][2] ^ (late[grp][1] + i >= LNB_STAGES));
     }
   }
   if (!a.dgamma) return;

@@ -130,6 +130,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return true;
 }
 
+// The same for a copy that has to land before its shared memory is given up (a block on its way out):
+// another thread's trouble does not end this wait, only the clock does.
+__device__ __forceinline__ bool mbar_wait_landed(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait_suspend(bar, parity, AB_MBAR_SUSPEND_NS))
+    if (clock64() - t0 > AB_SPIN_CYCLES) return false;
+  return true;
+}
+
 // Makes generic-proxy writes to shared memory visible to the async proxy
 // (TMA, tcgen05.mma operand fetch).
 __device__ __forceinline__ void fence_proxy_async_smem() {
