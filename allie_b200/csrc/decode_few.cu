@@ -193,14 +193,14 @@ __device__ __forceinline__ void df_attention(const DecodeFewArgs& g, const Decod
         kv[r][u] = make_uint4(0u, 0u, 0u, 0u);
         vv[r][u] = kv[r][u];
       }
-      if (j < n - 1) {
+      if (j < n && (j < P || j < n - 1)) {
         const long long off = base + static_cast<long long>(j < P ? j : anc[j - P]) * HD + c4 * DPL;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           kv[r][u] = __ldcg(reinterpret_cast<const uint4*>(L.kc + off + u * 8));
           vv[r][u] = __ldcg(reinterpret_cast<const uint4*>(L.vc + off + u * 8));
         }
-      } else if (j == n - 1) {                     // the last entry is the token itself
+      } else if (j == n - 1) {                     // the last entry of the list is the token itself
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           kv[r][u] = own(1, c4 * DPL + u * 8);

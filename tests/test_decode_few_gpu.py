@@ -157,3 +157,31 @@ def test_few_tree_step_that_cannot_be_resident_takes_the_chain(monkeypatch, use_
     torch.cuda.synchronize()
     _lib.check_status()
     assert np.array_equal(got, want)
+
+
+def test_few_tree_step_with_an_empty_list_reads_the_prompt_only():
+    """A token whose list of slots is empty attends to the prompt slots, all of them from the cache, as in
+    the chain of kernels."""
+    from allie_b200.ops import _lib
+
+    ev = _idle_evaluator(2, n=3)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    prompt = [1, 7, 16]
+    for cache in (ev.kc, ev.vc):
+        cache.copy_(torch.randn(cache.shape, device="cuda", generator=g))
+    kc, vc = ev.kc.clone(), ev.vc.clone()
+    for name, v in (("active", 1), ("tok", 5), ("pos", 3), ("n_anc", 0), ("n_legal", 8)):
+        ev.view(ev.req_host, name).fill_(v)
+    ev.view(ev.req_host, "prefix_len").copy_(torch.tensor(prompt))
+    ev.view(ev.req_host, "slot").copy_(torch.tensor(prompt))
+    ev.view(ev.req_host, "legal").copy_(torch.arange(8).expand(3, 8))
+    logits = []
+    for few in (False, True):
+        ev.few = few
+        ev.kc.copy_(kc)
+        ev.vc.copy_(vc)
+        ev.step()
+        logits.append(ev.logits.float().cpu())
+    _lib.check_status()
+    # two blocks, single flipped bf16 roundings (see above)
+    assert float((logits[1] - logits[0]).norm() / logits[0].norm()) < 1e-2
