@@ -132,6 +132,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 #pragma unroll
       for (int p = 0; p < PANELS; ++p)
         tma_load_2d(sQ + p * 16384, &tmQKV, q_full, h * HD + p * 64, first + qt * AT_BM);
+      int nk = 0, nv = 0;                        // tiles asked for
       for (int j = 0; j < nkv; ++j) {
         const int st = j % STAGES;
         const uint32_t par = ((j / STAGES) & 1) ^ 1;
@@ -142,13 +143,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         for (int p = 0; p < PANELS; ++p)
           tma_load_2d(sK + st * TILE_BYTES + p * 16384, &tmQKV, &k_full[st],
                       d_model + h * HD + p * 64, row_k);
+        nk = j + 1;
         if (!mbar_wait(&v_empty[st], par, abort_flag)) { *abort_flag = ST_TIMEOUT_EMPTY; atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY); break; }
         mbar_expect_tx(&v_full[st], TILE_BYTES);
 #pragma unroll
         for (int p = 0; p < PANELS; ++p)
           tma_load_2d(sV + st * TILE_BYTES + p * 16384, &tmQKV, &v_full[st],
                       2 * d_model + h * HD + p * 64, row_k);
+        nv = j + 1;
       }
+      // when a wait ran out, nobody has waited for these: they land before the block leaves
+      mbar_wait_landed(q_full, 0);
+      for (int j = nk > STAGES ? nk - STAGES : 0; j < nk; ++j) mbar_wait_landed(&k_full[j % STAGES], (j / STAGES) & 1);
+      for (int j = nv > STAGES ? nv - STAGES : 0; j < nv; ++j) mbar_wait_landed(&v_full[j % STAGES], (j / STAGES) & 1);
     }
   } else if (warp == FWD_MMA_WARP) {
     // -------------------------------------------------------------- MMA issuer

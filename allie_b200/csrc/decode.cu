@@ -85,6 +85,14 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
     // the kernel before (the QKV projection) is still running: the cache rows of earlier positions
     // do not depend on it.  The first chunk that needs the token's own row waits for it.
     bool waited = false;
+    // before this warp leaves, early or not: the last `DA_RING` chunks fetched for each head (`done` for
+    // heads below `hi`, one fewer for the others) have landed, so none arrives in another block's memory
+    auto landed = [&](int done, int hi) {
+      if (lane) return;
+      for (int i = 0; i < nh; ++i)
+        for (int k = max(0, done - (i >= hi) - DA_RING); k < done - (i >= hi); ++k)
+          mbar_wait_landed(&full[i * DA_RING + k % DA_RING], (k / DA_RING) & 1);
+    };
     for (int c = 0; c < n_chunks; ++c) {
       const int i0 = c * DA_CHUNK, i1 = min(n, i0 + DA_CHUNK);
       const int pre = max(0, min(P, i1) - i0);         // keys of this chunk that are prompt slots
@@ -99,6 +107,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
         okw = __shfl_sync(0xffffffffu, okw, 0);
         if (!okw) {
           if (lane == 0) { *abort_flag = 1; atomicCAS(status, 0, ST_TIMEOUT_MISC); }
+          landed(c + 1, hi);
           return;
         }
         uint8_t* sk = ring + stage * STAGE;
@@ -125,6 +134,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
         }
       }
     }
+    landed(n_chunks, nh);
     return;
   }
   // -------------------------------------------------------------------- consumers

@@ -508,20 +508,22 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
       const int m = m0w + lane;
       const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
+      const bool staged = stage_aux && m0w < g.M && nbase < g.N;
       if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
+        if (staged) mbar_wait_landed(&aux_bar[e], aux_phase);     // before the warp leaves
         break;
       }
       acc_phase ^= 1u << ab;
       tc_fence_after();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
-      const bool staged = stage_aux && m0w < g.M && nbase < g.N;
       auto wait_aux = [&]() {
         if (!mbar_wait(&aux_bar[e], aux_phase, abort_flag)) {
           *abort_flag = ST_TIMEOUT_FULL;
           atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
+          mbar_wait_landed(&aux_bar[e], aux_phase);
           return false;
         }
         aux_phase ^= 1;
