@@ -87,6 +87,12 @@ class MoEContext:
         # within one layer's forward, so the layers share them)
         self.ready_fwd, self.p_ready_fwd = self.shared(self.rows // 128, torch.int32)
         self.dgate, self.dlogits = e(M * 2, dt=f32), e(M, self.E)
+        # Rows of the router's operands are 16 bytes or a multiple: expert counts that are no multiple of
+        # eight go through copies with zero experts at the end, which the routing kernels never see.
+        self.E8 = -(-self.E // 8) * 8
+        if self.E8 != self.E:
+            self.router_pad, self.drouter_pad = e(self.E8, self.d), e(self.E8, self.d, dt=f32)
+            self.logits_pad, self.dlogits_pad = e(M, self.E8, dt=f32), e(M, self.E8)
         self.aux_total = torch.zeros((), dtype=f32, device=dev)
         if self.R > 1:
             torch.cuda.synchronize()
@@ -142,7 +148,12 @@ class MoELayer:
     def forward(self, ln2, resid, out, seed: int, stream_id: int, p_drop: float) -> None:
         c, v, lib = self.ctx, self.v, _lib.cuda()
         st = _lib.status_word()
-        gemm(ln2, v["router_w"][1], b_mn=False, out=self.logits)
+        if c.E8 == c.E:
+            gemm(ln2, v["router_w"][1], b_mn=False, out=self.logits)
+        else:
+            c.router_pad[:c.E].copy_(v["router_w"][1])
+            gemm(ln2, c.router_pad, b_mn=False, out=c.logits_pad)
+            self.logits.copy_(c.logits_pad[:, :c.E])
         self.cnt_ps.zero_()
         ep = c.next_epoch(PH_COUNTS)
         _ck(lib.ab_moe_route_plan_dispatch(
@@ -187,7 +198,15 @@ class MoELayer:
         _ck(lib.ab_moe_router_bwd(ptr(self.probs), ptr(self.topi), ptr(self.gates), ptr(c.dgate), ptr(self.counts),
                                   c_float(aux_scale), c_float(1.0), c_int(c.M), c_int(c.E), ptr(c.dlogits),
                                   stream_ptr()), "ab_moe_router_bwd")
-        gemm(c.dlogits, ln2, a_mn=True, b_mn=True, out=v["router_w"][2], accumulate=True)
-        gemm(c.dlogits, v["router_w"][1], b_mn=True, out=dln2_out)
+        if c.E8 == c.E:
+            gemm(c.dlogits, ln2, a_mn=True, b_mn=True, out=v["router_w"][2], accumulate=True)
+            gemm(c.dlogits, v["router_w"][1], b_mn=True, out=dln2_out)
+        else:
+            c.dlogits_pad[:, :c.E].copy_(c.dlogits)
+            c.drouter_pad.zero_()
+            gemm(c.dlogits_pad, ln2, a_mn=True, b_mn=True, out=c.drouter_pad, accumulate=True)
+            v["router_w"][2].add_(c.drouter_pad[:c.E])
+            c.router_pad[:c.E].copy_(v["router_w"][1])
+            gemm(c.dlogits_pad, c.router_pad, b_mn=True, out=dln2_out)
         _ck(lib.ab_moe_dx_sum(ptr(dln2_out), ptr(c.dxcomb), ptr(self.dest), c_int(c.M), c_int(c.d), ptr(c.flags),
                               c_int(PH_BWD_RETURN), c_int(c.R), c_uint(ep), ptr(st), stream_ptr()), "ab_moe_dx_sum")

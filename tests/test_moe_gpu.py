@@ -9,7 +9,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def test_moe_engine_matches_oracle():
+# 8: rows of 16 bytes; the others are padded to them.  (Counts for which no token's second choice is a near
+# tie: one that flips for the rounding of the logits moves the router's gradient by several per cent.)
+@pytest.mark.parametrize("experts", [8, 4, 5])
+def test_moe_engine_matches_oracle(experts):
     from allie_b200.data import UCITokenizer
     from allie_b200.models import initialize_model
     from allie_b200.models.engine import B200Engine
@@ -19,7 +22,8 @@ def test_moe_engine_matches_oracle():
     T, B = 128, 8
     tok = UCITokenizer(max_length=T, vocab_size_multiple_of=128)
     kw = dict(n_layer=3, n_embd=256, n_head=4, n_positions=T, resid_pdrop=0.0, embd_pdrop=0.0, attn_pdrop=0.0,
-              num_experts=8, moe_top_k=2, moe_ffn=512, moe_layer_freq=3, aux_loss_coef=0.05, capacity_factor=8.0)
+              num_experts=experts, moe_top_k=2, moe_ffn=512, moe_layer_freq=3, aux_loss_coef=0.05,
+              capacity_factor=float(experts))
     m = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, **kw)
     with torch.no_grad():       # spread the router so that top-2 choices are not razor-edge ties
         for n, p in m.named_parameters():
