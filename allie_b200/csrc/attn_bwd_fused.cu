@@ -844,7 +844,7 @@ static int attn_bwd_schedule_mode() {
 }
 
 int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const AttnBwdArgs& a,
-                            cudaStream_t stream) {
+                            int* launched, cudaStream_t stream) {
   CUtensorMap tdq;
   const long long rows = static_cast<long long>(a.B) * a.T;
   const int d = a.H * 64;
@@ -867,6 +867,7 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
     }
     dim3 grid((a.T + 127) / 128, a.H, a.B);
     launch_chained(attn_bwd_fused64_kernel, dim3(grid), dim3(FB_THREADS), SMEM, stream, tq, td, tdq, a);
+    ++*launched;
   } else {
     constexpr int SMEM = 8 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
     auto kern = whole ? attn_bwd_fused64_persistent_kernel<true> : attn_bwd_fused64_persistent_kernel<false>;
@@ -884,15 +885,18 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
     if (rc) return rc;
     const int bh = a.B * a.H;
     launch_chained(kern, dim3(bh < 148 ? bh : 148), dim3(FB_THREADS), SMEM, stream, tq, td, tdq, tdkv, tdqb, p);
+    ++*launched;
     if (whole) return (int)cudaGetLastError();       // dQ, its bias sums and the clearing are done
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   launch_chained(attn_dq_convert_kernel, dim3(148 * 16), dim3(256), 0, stream, a.dq_acc, a.dqkv, (int)rows, d);
+  ++*launched;
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   e = cudaMemsetAsync(a.dq_acc, 0, sizeof(float) * rows * d, stream);
   if (e != cudaSuccess || !a.dbias) return (int)e;
+  ++*launched;
   return ab_colsum_bf16(a.dqkv, 3 * d, (int)rows, 3 * d, a.dbias, nullptr, stream);
 }
 

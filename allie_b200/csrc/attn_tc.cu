@@ -715,7 +715,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 // ------------------------------------------------------------------------------------ host side
 namespace ab {
 int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const AttnBwdArgs& a,
-                            cudaStream_t stream);   // attn_bwd_fused.cu
+                            int* launched, cudaStream_t stream);   // attn_bwd_fused.cu
 
 template <int HD>
 static int launch_attn_fwd(const CUtensorMap& tm, const AttnArgs& a, uint64_t rows, int dependent,
@@ -826,12 +826,16 @@ int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T
 // pass wrote.  dq_acc (optional, hd == 64): fp32 [B*T, H*hd] accumulator that must be all zero on
 // entry and is all zero again on return; when given, the single-kernel backward runs.
 // dbias (optional, fp32 [3*H*hd]): the column sums of dqkv are added to it (the bias gradient of the
-// QKV projection).  delta_ready: delta already holds the row sums of dO * O.
+// QKV projection).  delta_ready: delta already holds the row sums of dO * O.  launched (optional, host):
+// receives the number of kernels launched.
 int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* dout, void* dqkv,
                 float* delta, const unsigned int* drop_mask, float* dq_acc, int B, int T, int H, int hd,
                 float scale, unsigned long long seed, unsigned int stream_id, unsigned int thr16,
-                float* dbias, int delta_ready, int* status, cudaStream_t stream) {
+                float* dbias, int delta_ready, int* launched, int* status, cudaStream_t stream) {
   using namespace ab;
+  int count = 0;
+  if (!launched) launched = &count;
+  *launched = 0;
   if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || (thr16 && (T & 7))) return -1;
   if (drop_mask && (T & 31)) return -1;
   CUtensorMap tq, td;
@@ -839,17 +843,23 @@ int ab_attn_bwd(const void* qkv, const void* out, const float* lse, const void* 
   if (rc) return rc;
   rc = make_tmap_2d(&td, dout, (uint64_t)B * T, (uint64_t)H * hd, (uint64_t)H * hd, 128, 64, 2, true);
   if (rc) return rc;
-  if (!delta_ready && (rc = ab_attn_delta(out, dout, delta, B, T, H, hd, stream)) != 0) return rc;
+  if (!delta_ready) {
+    if ((rc = ab_attn_delta(out, dout, delta, B, T, H, hd, stream)) != 0) return rc;
+    ++*launched;
+  }
   AttnBwdArgs a;
   a.B = B; a.T = T; a.H = H; a.hd = hd; a.scale = scale; a.seed = seed; a.stream_id = stream_id;
   a.thr16 = thr16; a.lse = lse; a.delta = delta; a.dqkv = (__nv_bfloat16*)dqkv; a.status = status;
   a.salt = seed_salt_ptr();
   a.drop_mask = drop_mask; a.dq_acc = dq_acc; a.dbias = dbias;
-  if (hd == 64 && dq_acc) return launch_attn_bwd_fused64(tq, td, a, stream);
+  if (hd == 64 && dq_acc) return launch_attn_bwd_fused64(tq, td, a, launched, stream);
   rc = hd == 64 ? launch_attn_bwd<64, 0>(tq, td, a, stream) : launch_attn_bwd<128, 0>(tq, td, a, stream);
   if (rc) return rc;
   rc = hd == 64 ? launch_attn_bwd<64, 1>(tq, td, a, stream) : launch_attn_bwd<128, 1>(tq, td, a, stream);
-  if (rc || !dbias) return rc;
+  if (rc) return rc;
+  *launched += 2;
+  if (!dbias) return 0;
+  ++*launched;
   return ab_colsum_bf16(dqkv, 3ll * H * hd, B * T, 3 * H * hd, dbias, nullptr, stream);
 }
 }
@@ -891,5 +901,5 @@ extern "C" int ab_attn_bwd_static(const void* qkv, const void* out, const float*
     g_attn_static_ptr[dev].store(scratch, std::memory_order_release);
   }
   return ab_attn_bwd(qkv, out, lse, dout, dqkv, scratch, drop_mask, nullptr, B, T, H, hd,
-                     scale, seed, stream_id, thr16, nullptr, 0, status, stream);
+                     scale, seed, stream_id, thr16, nullptr, 0, nullptr, status, stream);
 }

@@ -739,7 +739,9 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
       AbGemmEpilogue plain = *ep;
       plain.act = 0;
       const int rc = ab_gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, &plain, k_splits, max_ctas, status, stream);
-      return rc ? rc : ab_attn_delta(ep->aux, ep->out, ep->dot_out, M / ep->dot_T, ep->dot_T, N / 64, 64, stream);
+      if (rc) return rc;
+      if (ep->passes) ++*ep->passes;
+      return ab_attn_delta(ep->aux, ep->out, ep->dot_out, M / ep->dot_T, ep->dot_T, N / 64, 64, stream);
     }
   }
   if (ep->colsum && !(pair && aux_by_tma && !a_mn && !b_mn && ep->act == 2 && ep->aux_grad && ep->alpha == 1.f &&
@@ -749,7 +751,9 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
     AbGemmEpilogue plain = *ep;
     plain.colsum = nullptr;
     const int rc = ab_gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, &plain, k_splits, max_ctas, status, stream);
-    return rc ? rc : ab_colsum_bf16(ep->out, ep->ldo, M, N, ep->colsum, ep->m_limit, stream);
+    if (rc) return rc;
+    if (ep->passes) ++*ep->passes;
+    return ab_colsum_bf16(ep->out, ep->ldo, M, N, ep->colsum, ep->m_limit, stream);
   }
   // A problem that fits one wave of smaller tiles takes them: a 256 x 256 tile keeps two SMs for the whole
   // contraction and its epilogue while the others are idle.  128 x 64 tiles where they fit, else 128 x 128

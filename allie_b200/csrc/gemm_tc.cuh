@@ -48,6 +48,8 @@ struct AbGemmEpilogue {
   // out and aux dense.  From the epilogue on CTA pairs with K-major operands, else by a pass of its own.
   float* dot_out;
   int dot_T;
+  // optional host counter: increased by every pass that was launched beside the GEMM itself
+  int* passes;
 };
 
 // C[M,N] = A[M,K] * B[K,N] on the 5th-generation tensor cores.

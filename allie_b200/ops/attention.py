@@ -6,7 +6,7 @@ reads.  ``lse`` [B, H, T] keeps the log-sum-exp of each row for the backward pas
 """
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_uint, c_ulonglong
+from ctypes import byref, c_float, c_int, c_uint, c_ulonglong
 
 from . import _lib
 from ._lib import ptr, stream_ptr
@@ -32,14 +32,16 @@ def attention_bwd(qkv, out, lse, dout, dqkv, delta, B: int, T: int, H: int, hd: 
     backward; it is handed back all zero.  ``delta_ready``: ``delta`` holds the row sums already (see
     ``act=4`` of :func:`~allie_b200.ops.gemm.gemm`).  ``dbias``: optional fp32 [3*H*hd] to which the column
     sums of ``dqkv`` are added (the bias gradient of the projection in front)."""
+    launched = c_int(0)
     rc = _lib.cuda().ab_attn_bwd(ptr(qkv), ptr(out), ptr(lse), ptr(dout), ptr(dqkv), ptr(delta),
                                  ptr(drop_mask), ptr(dq_acc), c_int(B), c_int(T),
                                  c_int(H), c_int(hd), c_float(1.0 / hd ** 0.5), c_ulonglong(seed),
                                  c_uint(stream_id), c_uint(_lib.dropout_thr16(p_drop)),
-                                 ptr(dbias), c_int(int(delta_ready)), ptr(_lib.status_word()), stream_ptr())
+                                 ptr(dbias), c_int(int(delta_ready)), byref(launched), ptr(_lib.status_word()),
+                                 stream_ptr())
     if rc != 0:
         raise RuntimeError(f"ab_attn_bwd failed with code {rc} (B={B} T={T} H={H} hd={hd})")
-    _lib.count_launches(3)  # delta + (two backward kernels | fused backward + dQ conversion)
+    _lib.count_launches(launched.value)
 
 
 def set_backward_schedule(mode: int) -> None:
