@@ -570,6 +570,31 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   }
 }
 
+// What an epilogue warp of the pair kernel fetches by TMA (GemmArgs::aux_tma)
+static int pair_aux_tma(const AbGemmEpilogue& ep, int k_splits) {
+  if (ep.act == 1 || ep.accumulate || k_splits != 1) return 0;
+  // aux tiles travel in the geometry of the output tiles (see the kernel)
+  if ((ep.act == 2 || ep.act == 4) && !ep.out_fp32)
+    return (reinterpret_cast<uintptr_t>(ep.aux) & 15) == 0 && (ep.ldaux * 2) % 16 == 0 ? 1 : 0;
+  // residual tiles likewise, in the geometry of the fp32 output tiles
+  if (ep.resid && ep.out_fp32 && ep.act == 0)
+    return (reinterpret_cast<uintptr_t>(ep.resid) & 15) == 0 && (ep.ldr & 3) == 0 ? 2 : 0;
+  return 0;
+}
+
+// The specialised drain that an epilogue takes where it is compiled.  Forward layers: [in][out] weights;
+// input gradients: the same weights read K-major; weight gradients: both operands MN-major.
+static EpiKind pair_kind(bool a_mn, bool b_mn, const GemmArgs& g) {
+  const EpiKind kind = epi_kind(g);
+  switch (kind) {
+    case EPI_BF16: return !a_mn ? kind : EPI_ANY;
+    case EPI_GELU: case EPI_GELU_GRAD: case EPI_RESID: return !a_mn && b_mn ? kind : EPI_ANY;
+    case EPI_MUL: case EPI_DOT: return !a_mn && !b_mn ? kind : EPI_ANY;
+    case EPI_ACCUM: return a_mn && b_mn ? kind : EPI_ANY;
+    default: return EPI_ANY;
+  }
+}
+
 template <bool A_MN, bool B_MN>
 static int launch_pair(const void* A, long long lda, const void* B, long long ldb, const GemmArgs& g,
                        int max_ctas, cudaStream_t stream) {
@@ -590,25 +615,12 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   else                   rc = make_tmap_2d_sw(&tmOut, ep.out, g.M, g.N, ep.ldo, 32, 64, 2, 128);
   if (rc) return rc;
   GemmArgs ga = g;
-  ga.aux_tma = 0;
-  if (ep.act == 1) {
-    rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 32, 2, 64);
-    if (rc) return rc;
-  } else if ((ep.act == 2 || ep.act == 4) && !ep.out_fp32 && !ep.accumulate && g.k_splits == 1 &&
-             (reinterpret_cast<uintptr_t>(ep.aux) & 15) == 0 && (ep.ldaux * 2) % 16 == 0) {
-    // the aux tiles travel by TMA in the geometry of the output tiles (see the kernel)
-    rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 64, 2, 128);
-    if (rc) return rc;
-    ga.aux_tma = 1;
-  } else if (ep.resid && ep.out_fp32 && !ep.accumulate && ep.act == 0 && g.k_splits == 1 &&
-             (reinterpret_cast<uintptr_t>(ep.resid) & 15) == 0 && (ep.ldr & 3) == 0) {
-    // residual tiles likewise, in the geometry of the fp32 output tiles
-    rc = make_tmap_2d_sw(&tmAux, ep.resid, g.M, g.N, ep.ldr, 32, 32, 4, 128);
-    if (rc) return rc;
-    ga.aux_tma = 2;
-  } else {
-    tmAux = tmOut;
-  }
+  ga.aux_tma = pair_aux_tma(ep, g.k_splits);
+  if (ep.act == 1)            rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 32, 2, 64);
+  else if (ga.aux_tma == 1)   rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 64, 2, 128);
+  else if (ga.aux_tma == 2)   rc = make_tmap_2d_sw(&tmAux, ep.resid, g.M, g.N, ep.ldr, 32, 32, 4, 128);
+  else                        tmAux = tmOut;
+  if (rc) return rc;
   constexpr int SMEM = 1024 + PAIR_STAGES * (BM * BK * 2 + HALF_N * BK * 2) +
                        NUM_EPI_WARPS * PAIR_WARP_STAGING + 256;
   const int m_tiles = (g.M + 2 * BM - 1) / (2 * BM), n_tiles = (g.N + PAIR_BN - 1) / PAIR_BN;
@@ -626,9 +638,7 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
     return static_cast<int>(cudaGetLastError());
   };
   static PerDeviceOnce attr[EPI_DOT + 1];      // one per kernel of this operand layout
-  const EpiKind kind = epi_kind(ga);
-  // forward layers: [in][out] weights; input gradients: the same weights read K-major; weight
-  // gradients: both operands MN-major
+  const EpiKind kind = pair_kind(A_MN, B_MN, ga);
   if constexpr (!A_MN) {
     if (kind == EPI_BF16) return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_BF16>, attr[EPI_BF16]);
   }
@@ -708,6 +718,57 @@ extern "C" int ab_colsum_bf16(const void* x, long long ld, int M, int N, float* 
 extern "C" int ab_attn_delta(const void* o, const void* dout, float* delta, int B, int T, int H, int hd,
                              cudaStream_t stream);
 
+namespace ab {
+
+// Which kernel serves a problem, and whether column sums or head products come from passes of their own
+struct GemmPlan {
+  int kernel;                  // columns of the single-CTA kernel's tile (64, 128, 256), or PLAN_PAIR
+  bool dot_pass, colsum_pass;
+};
+constexpr int PLAN_PAIR = 512;
+
+static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue& ep, int k_splits, int max_ctas) {
+  // CTA pairs for the large shapes; the single-CTA kernel keeps the device-sized problems
+  // (m_limit / k_limit) and anything a caller pins with AB_GEMM_NO_PAIR=1 in the environment
+  static const bool no_pair = [] {
+    const char* v = getenv("AB_GEMM_NO_PAIR");
+    return v && v[0] == '1';
+  }();
+  bool pair = !no_pair && !ep.m_limit && !ep.k_limit && M >= 512 && N >= 256 && max_ctas >= 2;
+  const bool aux_by_tma = pair && ep.aux && pair_aux_tma(ep, k_splits) == 1 && !a_mn && !b_mn && ep.alpha == 1.f && !ep.bias;
+  const bool dot = ep.act == 4 && aux_by_tma;
+  const bool sums = ep.colsum && aux_by_tma && ep.act == 2 && ep.aux_grad && !ep.resid;
+  GemmPlan p = {0, ep.act == 4 && !dot, ep.colsum && !sums};
+  // A problem that fits one wave of smaller tiles takes them: a 256 x 256 tile keeps two SMs for the whole
+  // contraction and its epilogue while the others are idle.  128 x 64 tiles where they fit, else 128 x 128
+  // (2048 x 256 x 256 with residual and dropout: 11.7 us on pairs, 9.4 with 128 x 128, 7.3 with 128 x 64;
+  // 2048 x 1024 x 256: 11.9, 9.6, 9.8 in two waves; 4096 x 1024 x 1024, two waves: 16.3, 19.9, 27.7).
+  auto tiles = [&](int bn) { return static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn); };
+  const bool one_wave = pair && !a_mn && !sums && !dot && k_splits == 1 && tiles(128) <= max_ctas;
+  // narrow tiles also for skinny problems (decode steps with a few hundred rows): twice the CTAs
+  const bool narrow = (N <= 128) || (M <= 256);
+  // A few hundred rows against a wide weight matrix (decode steps): the time goes into streaming
+  // the weights, so the columns are cut into 64-wide tiles to put twice as many SMs on them.
+  if (M <= 256 && N >= 1024 && k_splits == 1 && !a_mn) p.kernel = 64;
+  else if (one_wave) p.kernel = tiles(64) <= max_ctas ? 64 : 128;
+  else if (narrow)   p.kernel = 128;
+  else               p.kernel = pair ? PLAN_PAIR : 256;
+  return p;
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_plan(int kernel, const void* A, long long lda, const void* B, long long ldb, const GemmArgs& g,
+                       int max_ctas, cudaStream_t stream) {
+  if (kernel == PLAN_PAIR) return launch_pair<A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+  if (kernel == 256) return launch<256, 4, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+  if constexpr (!A_MN) {
+    if (kernel == 64) return launch<64, 8, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+  }
+  return launch<128, 6, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+}
+
+}  // namespace ab
+
 extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
                             long long ldb, int M, int N, int K, const AbGemmEpilogue* ep,
                             int k_splits, int max_ctas, int* status, cudaStream_t stream) {
@@ -722,20 +783,13 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
     return -3;
   if ((ep->ldo * (ep->out_fp32 ? 4 : 2)) & 15) return -4;   // TMA row pitch: multiple of 16 bytes
   if (ep->act == 1 && (ep->ldaux & 7)) return -4;
-  // CTA pairs for the large shapes; the single-CTA kernel keeps the device-sized problems
-  // (m_limit / k_limit) and anything a caller pins with AB_GEMM_NO_PAIR=1 in the environment
-  static const bool no_pair = [] {
-    const char* v = getenv("AB_GEMM_NO_PAIR");
-    return v && v[0] == '1';
-  }();
   if (max_ctas <= 0) max_ctas = 148;
-  bool pair = !no_pair && !ep->m_limit && !ep->k_limit && M >= 512 && N >= 256 && max_ctas >= 2;
-  const bool aux_by_tma = ep->aux && !ep->out_fp32 && !ep->accumulate && k_splits == 1 && (ep->ldaux & 7) == 0;
+  const GemmPlan plan = gemm_plan(a_mn, b_mn, M, N, *ep, k_splits, max_ctas);
   if (ep->act == 4) {
     if (!ep->aux || !ep->dot_out || ep->dot_T < 1 || M % ep->dot_T || (N & 63) || ep->out_fp32 || ep->ldo != N ||
         ep->ldaux != N || ep->m_limit || ep->resid)
       return -5;
-    if (!(pair && aux_by_tma && !a_mn && !b_mn && ep->alpha == 1.f && !ep->bias)) {
+    if (plan.dot_pass) {
       AbGemmEpilogue plain = *ep;
       plain.act = 0;
       const int rc = ab_gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, &plain, k_splits, max_ctas, status, stream);
@@ -744,9 +798,7 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
       return ab_attn_delta(ep->aux, ep->out, ep->dot_out, M / ep->dot_T, ep->dot_T, N / 64, 64, stream);
     }
   }
-  if (ep->colsum && !(pair && aux_by_tma && !a_mn && !b_mn && ep->act == 2 && ep->aux_grad && ep->alpha == 1.f &&
-                      !ep->bias && !ep->resid)) {
-    // every other form: a pass of its own over the finished output
+  if (plan.colsum_pass) {
     if (ep->out_fp32) return -6;
     AbGemmEpilogue plain = *ep;
     plain.colsum = nullptr;
@@ -755,43 +807,31 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
     if (ep->passes) ++*ep->passes;
     return ab_colsum_bf16(ep->out, ep->ldo, M, N, ep->colsum, ep->m_limit, stream);
   }
-  // A problem that fits one wave of smaller tiles takes them: a 256 x 256 tile keeps two SMs for the whole
-  // contraction and its epilogue while the others are idle.  128 x 64 tiles where they fit, else 128 x 128
-  // (2048 x 256 x 256 with residual and dropout: 11.7 us on pairs, 9.4 with 128 x 128, 7.3 with 128 x 64;
-  // 2048 x 1024 x 256: 11.9, 9.6, 9.8 in two waves; 4096 x 1024 x 1024, two waves: 16.3, 19.9, 27.7).
-  auto tiles = [&](int bn) { return static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn); };
-  const bool one_wave = pair && !a_mn && !ep->colsum && ep->act != 4 && k_splits == 1 && tiles(128) <= max_ctas;
-  if (one_wave) pair = false;
   GemmArgs g;
   g.M = M; g.N = N; g.K = K; g.k_splits = k_splits; g.ep = *ep; g.status = status; g.salt = seed_salt_ptr(); g.aux_tma = 0;
   // programmatic dependent launch: single-CTA kernels only, never with device-side limits (those
   // are values of earlier kernels, read before any wait)
   g.pdl = (ep->pdl && !ep->m_limit && !ep->k_limit) ? 1 : 0;
-  // narrow tiles also for skinny problems (decode steps with a few hundred rows): twice the CTAs
-  const bool narrow = (N <= 128) || (M <= 256);
-  // A few hundred rows against a wide weight matrix (decode steps): the time goes into streaming
-  // the weights, so the columns are cut into 64-wide tiles to put twice as many SMs on them.
-  if (M <= 256 && N >= 1024 && k_splits == 1) {
-    if (!a_mn && !b_mn) return launch<64, 8, false, false>(A, lda, B, ldb, g, max_ctas, stream);
-    if (!a_mn && b_mn) return launch<64, 8, false, true>(A, lda, B, ldb, g, max_ctas, stream);
-  }
-  if (one_wave && tiles(64) <= max_ctas)
-    return b_mn ? launch<64, 8, false, true>(A, lda, B, ldb, g, max_ctas, stream)
-                : launch<64, 8, false, false>(A, lda, B, ldb, g, max_ctas, stream);
-  if (narrow || one_wave) {
-    if (!a_mn && !b_mn) return launch<128, 6, false, false>(A, lda, B, ldb, g, max_ctas, stream);
-    if (!a_mn && b_mn) return launch<128, 6, false, true>(A, lda, B, ldb, g, max_ctas, stream);
-    if (a_mn && !b_mn) return launch<128, 6, true, false>(A, lda, B, ldb, g, max_ctas, stream);
-    return launch<128, 6, true, true>(A, lda, B, ldb, g, max_ctas, stream);
-  }
-  if (pair) {
-    if (!a_mn && !b_mn) return launch_pair<false, false>(A, lda, B, ldb, g, max_ctas, stream);
-    if (!a_mn && b_mn) return launch_pair<false, true>(A, lda, B, ldb, g, max_ctas, stream);
-    if (a_mn && !b_mn) return launch_pair<true, false>(A, lda, B, ldb, g, max_ctas, stream);
-    return launch_pair<true, true>(A, lda, B, ldb, g, max_ctas, stream);
-  }
-  if (!a_mn && !b_mn) return launch<256, 4, false, false>(A, lda, B, ldb, g, max_ctas, stream);
-  if (!a_mn && b_mn) return launch<256, 4, false, true>(A, lda, B, ldb, g, max_ctas, stream);
-  if (a_mn && !b_mn) return launch<256, 4, true, false>(A, lda, B, ldb, g, max_ctas, stream);
-  return launch<256, 4, true, true>(A, lda, B, ldb, g, max_ctas, stream);
+  if (!a_mn && !b_mn) return launch_plan<false, false>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
+  if (!a_mn && b_mn) return launch_plan<false, true>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
+  if (a_mn && !b_mn) return launch_plan<true, false>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
+  return launch_plan<true, true>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
+}
+
+// What ab_gemm_bf16 would run for the same arguments, without running it: the columns of the single-CTA
+// kernel's tile, or 512 + EpiKind on CTA pairs.  Passes beside the GEMM: see `passes`.
+extern "C" int ab_gemm_route(const void*, int a_mn, long long, const void*, int b_mn, long long, int M, int N, int,
+                             const AbGemmEpilogue* ep, int k_splits, int max_ctas, int*, cudaStream_t) {
+  using namespace ab;
+  if (k_splits < 1) k_splits = 1;
+  if (max_ctas <= 0) max_ctas = 148;
+  AbGemmEpilogue e = *ep;
+  GemmPlan plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas);
+  if (plan.dot_pass) { e.act = 0; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
+  if (plan.colsum_pass) { e.colsum = nullptr; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
+  if (plan.kernel != PLAN_PAIR) return plan.kernel;
+  GemmArgs g;
+  g.ep = e;
+  g.aux_tma = pair_aux_tma(e, k_splits);
+  return PLAN_PAIR + pair_kind(a_mn, b_mn, g);
 }

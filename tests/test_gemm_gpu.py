@@ -5,6 +5,30 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+PAIR = 512        # ab_gemm_route on CTA pairs, plus the kind of the epilogue (EpiKind in csrc/gemm_core.cuh)
+ANY, BF16, GELU, GELU_GRAD, MUL, RESID, ACCUM, DOT = range(8)
+
+
+@pytest.fixture
+def routes(monkeypatch):
+    """What each GEMM of a test was dispatched to: 64, 128 or 256 (tile columns of the single-CTA kernel), or
+    PAIR + kind."""
+    from allie_b200.ops import _lib
+
+    lib, seen = _lib.cuda(), []
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def ab_gemm_bf16(self, *args):
+            seen.append(lib.ab_gemm_route(*args))
+            return lib.ab_gemm_bf16(*args)
+
+    monkeypatch.setattr(_lib, "_cuda_lib", Spy())
+    return seen
+
+
 def _ref(a, b, a_mn, b_mn):
     A = a.float().t() if a_mn else a.float()
     B = b.float() if b_mn else b.float().t()
@@ -14,10 +38,12 @@ def _ref(a, b, a_mn, b_mn):
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 512, 320), (384, 768, 1024), (200, 264, 136),
                                    (1000, 128, 512), (64, 64, 64),
-                                   # large enough for the CTA-pair kernel, with ragged edges
+                                   # CTA pairs where A is MN-major, else one wave of smaller tiles
                                    (1000, 264, 136), (640, 768, 320), (2304, 1024, 192),
-                                   (512, 256, 64), (768, 512, 40)])      # one K block; ragged K
-def test_gemm_layouts(a_mn, b_mn, M, N, K):
+                                   (512, 256, 64), (768, 512, 40),       # one K block; ragged K
+                                   # beyond one wave: CTA pairs in every layout, with ragged edges
+                                   (4744, 808, 136), (2440, 1032, 40)])
+def test_gemm_layouts(routes, a_mn, b_mn, M, N, K):
     from allie_b200.ops import _lib
     from allie_b200.ops.gemm import gemm
 
@@ -28,6 +54,7 @@ def test_gemm_layouts(a_mn, b_mn, M, N, K):
     out = gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32)
     torch.cuda.synchronize()
     _lib.check_status()
+    assert (routes == [PAIR + ANY]) == (M >= 2440 or (M >= 512 and N >= 256 and a_mn))
     ref = _ref(a, b, a_mn, b_mn)
     err = (out - ref).abs().max().item()
     assert err < 2e-2 * (K ** 0.5), (err, M, N, K)
@@ -135,8 +162,9 @@ def test_gemm_skinny_residual_update_in_place():
         assert torch.allclose(x, want, rtol=1e-3, atol=3e-2), (M, N, K, (x - want).abs().max().item())
 
 
-@pytest.mark.parametrize("M,N,K", [(1000, 328, 192), (2048, 1024, 256), (640, 72, 128)])
-def test_gemm_gelu_backward_epilogue_ragged(M, N, K):
+@pytest.mark.parametrize("M,N,K,route", [(1000, 328, 192, 64), (2048, 1024, 256, 128), (640, 72, 128, 128),
+                                         (4744, 808, 72, PAIR + ANY), (20000, 520, 128, PAIR + ANY)])
+def test_gemm_gelu_backward_epilogue_ragged(routes, M, N, K, route):
     """out = (dy @ w^T) * gelu'(pre) on shapes with ragged row / column tiles (the CTA-pair kernel
     fetches the pre-activation tiles by TMA one tile ahead)."""
     from allie_b200.ops import _lib
@@ -150,6 +178,7 @@ def test_gemm_gelu_backward_epilogue_ragged(M, N, K):
     out = gemm(dy, wt, act=2, aux=pre)
     torch.cuda.synchronize()
     _lib.check_status()
+    assert routes == [route]
     x = pre.float().requires_grad_(True)
     torch.nn.functional.gelu(x, approximate="tanh").backward(dy.float() @ wt.float().t())
     assert torch.allclose(out.float(), x.grad, rtol=3e-2, atol=3e-2), (out.float() - x.grad).abs().max().item()
@@ -185,13 +214,15 @@ def test_gemm_gelu_derivative_kept_in_aux():
 
 
 @pytest.mark.parametrize("drop_p", [0.0, 0.1])
-@pytest.mark.parametrize("M,N,K", [(512, 256, 64),      # one tile per pair, both column groups of every warp
-                                   (520, 264, 72),      # rows past a tile, eight columns in the last tile
-                                   (1100, 800, 256),    # last column tile ends inside a warp's first group
-                                   (4744, 808, 72),     # the same edges beyond one wave of smaller tiles: on pairs
-                                   (20000, 512, 128)])  # several units per pair: tiles fetched one unit ahead
-def test_gemm_pair_residual_tiles(M, N, K, drop_p):
-    """CTA-pair kernel with a fp32 residual: its tiles travel by TMA through the output staging tile."""
+@pytest.mark.parametrize("M,N,K,route", [
+    (512, 256, 64, 64), (520, 264, 72, 64), (1100, 800, 256, 64),        # one wave of smaller tiles
+    (2560, 1024, 64, PAIR + RESID),      # one tile per pair, both column groups of every warp
+    (2440, 1032, 72, PAIR + RESID),      # rows past a tile, eight columns in the last tile
+    (4744, 800, 256, PAIR + RESID),      # last column tile ends behind a warp's first group
+    (4744, 808, 72, PAIR + RESID),       # and inside its second
+    (20000, 512, 128, PAIR + RESID)])    # several units per pair: tiles fetched one unit ahead
+def test_gemm_pair_residual_tiles(routes, M, N, K, route, drop_p):
+    """A fp32 residual.  On CTA pairs its tiles travel by TMA through the output staging tile."""
     from allie_b200.ops import _lib
     from allie_b200.ops.gemm import gemm
 
@@ -207,6 +238,7 @@ def test_gemm_pair_residual_tiles(M, N, K, drop_p):
     gemm(a, w, out=inplace, resid=inplace, **kw)
     torch.cuda.synchronize()
     _lib.check_status()
+    assert routes == [route] * 3
     # the same accumulators and mask: only the last addition of the residual rounds differently (half
     # an ulp of values below 16)
     assert torch.equal(out, inplace)
@@ -216,11 +248,13 @@ def test_gemm_pair_residual_tiles(M, N, K, drop_p):
         assert torch.allclose(out, ref, rtol=1e-4, atol=1e-4 * K ** 0.5)
 
 
-@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (520, 264, 72), (1100, 800, 256), (20000, 512, 128),
-                                   (4744, 1032, 136), (5000, 808, 72)])
-def test_gemm_pair_specialised_epilogues(M, N, K):
-    """Every specialised drain of the CTA-pair kernel at tile edges: rows and columns past a tile, a last
-    column tile that ends inside a warp's columns, several units per pair."""
+@pytest.mark.parametrize("M,N,K,pair", [(512, 256, 64, False), (520, 264, 72, False), (1100, 800, 256, False),
+                                        (2440, 1032, 64, True), (4744, 800, 72, True), (20000, 512, 128, True),
+                                        (4744, 1032, 136, True), (5000, 808, 72, True)])
+def test_gemm_pair_specialised_epilogues(routes, M, N, K, pair):
+    """The specialised drains of the CTA-pair kernel at tile edges (rows and columns past a tile, a last
+    column tile that ends inside a warp's columns, several units per pair), and the same epilogues where one
+    wave of smaller tiles takes them."""
     from allie_b200.ops import _lib
     from allie_b200.ops.gemm import gemm
 
@@ -243,6 +277,10 @@ def test_gemm_pair_specialised_epilogues(M, N, K):
     assert close(aux, x.grad)
     wt = w.t().contiguous()
     assert close(gemm(a, wt, act=2, aux=aux, aux_grad=True), (ref - bias) * aux.float())
+    if pair:
+        assert routes == [PAIR + kind for kind in (BF16, BF16, GELU, GELU_GRAD, MUL)]
+    else:
+        assert max(routes) < PAIR
     dy = torch.randn(M, N, device="cuda").bfloat16()
     dw = torch.full((K, N), 3.0, device="cuda")
     for splits in (1, 3):
@@ -256,8 +294,51 @@ def test_gemm_pair_specialised_epilogues(M, N, K):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("T", [650, 4096])
+@pytest.mark.parametrize("I,O", [(1000, 808), (512, 256)])
+def test_gemm_pair_accumulate_drain(routes, I, O, T):
+    """Weight gradients on CTA pairs, whole and split contractions, rows and columns past a tile."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(8)
+    x, dy = torch.randn(T, I, device="cuda").bfloat16(), torch.randn(T, O, device="cuda").bfloat16()
+    dw = torch.full((I, O), 3.0, device="cuda")
+    for splits in (1, 3):
+        gemm(x, dy, a_mn=True, b_mn=True, out=dw, accumulate=True, k_splits=splits)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert routes == [PAIR + ACCUM] * 2
+    bound = 2 * (T / 16) * 2 ** -23 * 6 * T ** 0.5 + 1e-5      # as above
+    assert ((dw.double() - 3.0 - 2 * (x.double().t() @ dy.double())).abs() <= bound).all()
+
+
+def test_gemm_pair_general_drain(routes):
+    """What no specialised drain of the CTA-pair kernel takes: a scaled product, a kept pre-activation, a
+    residual with weights read K-major."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(9)
+    M, N, K = 4744, 808, 72
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(K, N, device="cuda") * K ** -0.5).bfloat16()
+    bias, resid = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda")
+    ref = a.float() @ w.float()
+    close = lambda x, y: torch.allclose(x.float(), y, rtol=2 ** -8, atol=2 ** -9)     # as above
+    assert close(gemm(a, w, b_mn=True, alpha=0.5), 0.5 * ref)
+    pre = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    assert close(gemm(a, w, b_mn=True, bias=bias, act=1, aux=pre), torch.nn.functional.gelu(ref + bias, approximate="tanh"))
+    assert close(pre, ref + bias)
+    out = gemm(a, w.t().contiguous(), bias=bias, resid=resid, out=torch.empty_like(resid))
+    assert torch.allclose(out, ref + bias + resid, rtol=1e-4, atol=1e-4 * K ** 0.5)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert routes == [PAIR + ANY] * 3
+
+
 @pytest.mark.parametrize("M,N,K", [(512, 256, 64), (520, 264, 72), (1100, 832, 256), (20000, 512, 128), (96, 256, 128)])
-def test_gemm_column_sums_and_head_products(M, N, K):
+def test_gemm_column_sums_and_head_products(routes, M, N, K):
     """The column sums that the derivative epilogue adds (and the pass that stands in below 512 rows) at
     tile edges, and the per-head products with a second tensor.  Both are fp32 sums of the bf16 values
     that were stored: any order is within terms * 2^-23 * sum|terms|."""
@@ -273,6 +354,7 @@ def test_gemm_column_sums_and_head_products(M, N, K):
     plain = gemm(a, w, act=2, aux=aux, aux_grad=True)
     torch.cuda.synchronize()
     _lib.check_status()
+    assert routes[0] == (PAIR + MUL if M >= 512 else 128)
     assert torch.equal(out, plain)
     terms = out.double()
     assert ((sums.double() - 0.25 - terms.sum(0)).abs() <= 1e-6 + M * 2.0 ** -23 * (terms.abs().sum(0) + 0.25)).all()
@@ -282,13 +364,14 @@ def test_gemm_column_sums_and_head_products(M, N, K):
         out = gemm(a, w, act=4, aux=aux, dot=(dot, T))
         torch.cuda.synchronize()
         _lib.check_status()
+        assert routes[-1] == (PAIR + DOT if M >= 512 else 128)
         assert torch.equal(out, gemm(a, w))
         prod = (out.double() * aux.double()).view(M // T, T, N // 64, 64).permute(0, 2, 1, 3)
         assert ((dot.double() - prod.sum(-1)).abs() <= 1e-6 + 64 * 2.0 ** -23 * prod.abs().sum(-1)).all()
 
 
-@pytest.mark.parametrize("M,N,K", [(4744, 808, 72), (512, 256, 64)])     # CTA pairs; one wave of smaller tiles
-def test_gemm_residual_drops_non_finite_values(M, N, K):
+@pytest.mark.parametrize("M,N,K,route", [(4744, 808, 72, PAIR + RESID), (512, 256, 64, 64)])
+def test_gemm_residual_drops_non_finite_values(routes, M, N, K, route):
     """A dropped element adds nothing to the residual, whatever it was: Inf and NaN of one row of the product
     stay out of its dropped columns."""
     from allie_b200.ops import _lib
@@ -305,6 +388,7 @@ def test_gemm_residual_drops_non_finite_values(M, N, K):
     out = gemm(a, w, out=torch.empty_like(resid), resid=resid, **kw)
     torch.cuda.synchronize()
     _lib.check_status()
+    assert routes == [route] * 2
     assert 0.7 < float(kept.float().mean()) < 0.8
     assert torch.equal(out[~kept], resid[~kept])
     assert torch.isinf(out[3][kept[3]]).all() and torch.isnan(out[M - 1][kept[M - 1]]).all()
