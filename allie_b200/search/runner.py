@@ -89,12 +89,14 @@ class EngineRunner(ModelRunner):
     def evaluate(self, games: list[Game]) -> Evaluation:
         self.calls += 1
         games, eng, n = list(games), self.engine, len(games)
+        tok, rows = self.tokenizer, None
         if eng.dense and games and not isinstance(games[0], np.ndarray):
-            tok = self.tokenizer
             rows = [tok.token_ids(g)[: tok.max_length] for g in games]
             if any(e + len(tok) > 0x3FFF for g in games for e in (g.white_elo, g.black_elo)):
                 # ratings that run into the outcome bits of a word: refused where the padded batch does
                 assert all(int(((tok.tokenize(g)[: tok.max_length] & 0xFFFF) >> 14).max()) < 3 for g in games)
+        # a padding token inside a game takes no position of its own, which the padded batch knows
+        if rows is not None and not (np.concatenate(rows) == tok.pad_token_id).any():
             logits, value, time = eng.infer_last(rows)
         else:      # experts are laid out for a fixed number of rows; arrays come as equal windows already
             batch = self.tokenizer.pad_and_collate(games, return_labels=False)

@@ -66,3 +66,27 @@ def test_packed_inference_refuses_overlong_and_counts_launches():
     before = _lib.LAUNCHES
     eng.infer_last([np.arange(64)])
     assert _lib.LAUNCHES - before == 1 + 2 * 7 + 1 + 3
+
+
+def test_padding_token_inside_a_game():
+    """A padding token among the moves takes no position and is not counted for the last index: such games
+    go through the padded batch, with its results."""
+    from allie_b200.data import Game, UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.search.runner import EngineRunner
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=2, n_embd=128,
+                             n_head=2, n_positions=64)
+    game = lambda moves: Game("180+0", 1500, 1600, None, False, moves, [1] * len(moves))
+    games = [game(["e2e4", tok.pad_token, "e7e5", "g1f3"]), game(["d2d4"]), game(["e2e4", "e7e5", tok.pad_token])]
+    runner = EngineRunner(model, tok)
+    got = runner.evaluate(games)
+    batch = tok.pad_and_collate(games, return_labels=False)
+    out = runner.engine.evaluate_batch(batch, with_loss=False)
+    last = batch["attention_mask"].sum(-1).long() - 1
+    assert last.tolist() == [5, 3, 4]
+    for i, j in enumerate(last.tolist()):
+        assert torch.equal(got.logits[i], out["logits"][i, j].float().cpu())
+        assert float(got.value[i]) == float(out["value_logits"][i, j])
