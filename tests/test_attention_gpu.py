@@ -163,3 +163,88 @@ def test_attention_bwd_bias_sums_and_accumulator(B, T, H, hd):
     # the schedules add a query tile's parts in different orders: single bf16 roundings flip
     for g in grads[1:]:
         assert (g - grads[0]).norm() / grads[0].norm() < 1e-3
+
+
+def _inputs(kind, B, T, H, hd):
+    """plain; later keys score higher, so that the running maximum of a row grows in every key tile; values
+    of one sign, whose sums lose most to rounding."""
+    x = torch.randn(B, T, 3, H, hd, device="cuda") * 0.7
+    if kind == "late":
+        x[:, :, 0, :, :] = x[:, :, 0].abs()
+        x[:, :, 1] = x[:, :, 1].abs() * torch.linspace(-3, 1, T, device="cuda").exp2()[None, :, None, None]
+    elif kind == "mean":
+        x[:, :, 2] += 1.0
+    return x.reshape(B * T, 3 * H * hd).bfloat16()
+
+
+@pytest.mark.parametrize("hd,T", [(64, 129), (64, 384), (64, 1000), (128, 129), (128, 384), (128, 520), (128, 1000)])
+@pytest.mark.parametrize("kind", ["plain", "late", "mean"])
+@pytest.mark.parametrize("p", [0.0, 0.1])
+def test_attention_fwd_against_64_bits(hd, T, kind, p):
+    """Two to eight key tiles (at heads of 128 every stage is used again, O is rescaled in place).  Bound,
+    element by element: P and the stored result are rounded to bf16 (eight significant bits, so up to 2^-8 of
+    each term, twice), exponentials and fp32 sums (the tensor core cuts them off) are good for 2^-13 together at
+    these lengths."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.attention import attention_fwd
+
+    if p and T % 32:
+        T = T // 32 * 32                    # keep bits are kept for whole words
+    torch.manual_seed(0)
+    B, H = 2, 2
+    d, dev = H * hd, "cuda"
+    qkv = _inputs(kind, B, T, H, hd)
+    out = torch.full((B * T, d), float("nan"), device=dev, dtype=torch.bfloat16)
+    lse = torch.zeros(B, H, T, device=dev)
+    bits = torch.zeros(B, H, T, T // 32, device=dev, dtype=torch.int32) if p else None
+    attention_fwd(qkv, out, lse, B, T, H, hd, p, 77, 3, bits)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    q, k, v = (qkv.view(B, T, 3, H, hd)[:, :, i].transpose(1, 2).double() for i in range(3))
+    s = (q @ k.transpose(-1, -2)) / math.sqrt(hd)
+    s = s.masked_fill(~torch.ones(T, T, dtype=torch.bool, device=dev).tril(), float("-inf"))
+    probs = s.softmax(-1)
+    if kind == "late":                     # the maximum does grow, tile after tile
+        tops = torch.stack([s[:, :, T - 1, j:j + 128].amax(-1) for j in range(0, T, 128)], -1)
+        assert (tops[..., 1:-1] > tops[..., :-2]).all()
+    assert torch.allclose(lse.double(), torch.logsumexp(s, -1), rtol=1e-5, atol=1e-4)
+    if p:
+        keep = ((bits.unsqueeze(-1) >> torch.arange(32, device=dev)) & 1).view(B, H, T, T)
+        probs = probs * keep * (65536.0 / (65536 - _lib.dropout_thr16(p)))
+    want = (probs @ v).transpose(1, 2).reshape(B * T, d)
+    size = (probs @ v.abs()).transpose(1, 2).reshape(B * T, d)
+    err = (out.double() - want).abs()
+    assert (err <= (2 * 2 ** -8 + 2 ** -13) * size + 1e-7).all(), float((err / (size + 1e-9)).max())
+
+
+@pytest.mark.parametrize("B,T,H,hd,p", [(2, 384, 2, 128, 0.1), (1, 520, 2, 128, 0.0), (2, 1000, 1, 128, 0.0), (2, 416, 2, 64, 0.1)])
+def test_attention_bwd_over_several_key_tiles(B, T, H, hd, p):
+    """Gradients against autograd in 64 bits with the stored mask, three key tiles and more.  P, dS and the
+    results are rounded to bf16: under 1 % in the 2-norm."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.attention import attention_bwd, attention_fwd
+
+    torch.manual_seed(2)
+    d, dev = H * hd, "cuda"
+    qkv = (torch.randn(B * T, 3 * d, device=dev) * 0.7).bfloat16()
+    out = torch.zeros(B * T, d, device=dev, dtype=torch.bfloat16)
+    lse, delta = torch.zeros(B, H, T, device=dev), torch.zeros(B, H, T, device=dev)
+    bits = torch.zeros(B, H, T, T // 32, device=dev, dtype=torch.int32) if p else None
+    attention_fwd(qkv, out, lse, B, T, H, hd, p, 5, 1, bits)
+    dout = torch.randn(B * T, d, device=dev).bfloat16()
+    leaf = qkv.double().requires_grad_(True)
+    q, k, v = (leaf.view(B, T, 3, H, hd)[:, :, i].transpose(1, 2) for i in range(3))
+    s = (q @ k.transpose(-1, -2)) / math.sqrt(hd)
+    probs = s.masked_fill(~torch.ones(T, T, dtype=torch.bool, device=dev).tril(), float("-inf")).softmax(-1)
+    if p:
+        keep = ((bits.unsqueeze(-1) >> torch.arange(32, device=dev)) & 1).view(B, H, T, T)
+        probs = probs * keep * (65536.0 / (65536 - _lib.dropout_thr16(p)))
+    (probs @ v).transpose(1, 2).reshape(B * T, d).backward(dout.double())
+    dqkv = torch.full((B * T, 3 * d), float("nan"), device=dev, dtype=torch.bfloat16)
+    acc = torch.zeros(B * T, d, device=dev) if hd == 64 else None
+    attention_bwd(qkv, out, lse, dout, dqkv, delta, B, T, H, hd, p, 5, 1, bits, acc)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for i in range(3):
+        a, b = dqkv[:, i * d:(i + 1) * d].double(), leaf.grad[:, i * d:(i + 1) * d]
+        assert float((a - b).norm() / b.norm()) < 1e-2, "qkv"[i]

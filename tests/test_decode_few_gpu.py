@@ -63,6 +63,53 @@ def test_few_tree_step_matches_the_chain(n, d, heads, inner, norm):
         assert np.abs(pa - pb).max() < 1e-2
 
 
+@pytest.mark.parametrize("n", [2, 16, 17])         # one kernel up to 16 trees, the chain from 17 on
+def test_steps_against_the_plain_model(n):
+    """A line of five nodes per tree (and one second child of the root): the logits of each node's token are
+    those of the plain fp32 model over the whole sequence.  bf16 operands, three blocks: under 1 %."""
+    from allie_b200.data import Game, UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.moves import CHESS_MOVES
+    from allie_b200.ops import _lib
+    from allie_b200.search.batched import KVStepEvaluator
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=256, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=3, n_embd=512,
+                             n_head=8, n_inner=2048, n_positions=256)
+    model.eval()
+    eng = B200Engine(model, "cuda")
+    rng = np.random.default_rng(4)
+    games = [Game("180+0", 1500, 1600, None, False, [CHESS_MOVES[i] for i in rng.integers(0, 1968, size=k)], [1] * k)
+             for k in (int(v) for v in rng.integers(0, 150, size=n))]
+    ev = KVStepEvaluator(eng, tok, n, anc_max=16, legal_max=64, max_prefix=200, max_nodes=64)
+    assert ev.kv.few == (n <= 16)
+    ev.prefill(games)
+    prefix = [tok.token_ids(g).astype(np.int64) for g in games]
+    tokens = rng.integers(0, 1968, size=(6, n)).astype(np.int32)
+    anc = np.zeros((n, 16), np.int32)
+    for s in range(6):
+        depth = s if s < 5 else 0                  # the sixth hangs below the root again
+        slot = np.array([len(p) + s for p in prefix], np.int32)
+        anc[:, depth] = slot
+        req = dict(need_eval=np.ones(n, np.int32), tok=tokens[s], pos=np.array([len(p) + depth for p in prefix], np.int32),
+                   slot=slot, n_anc=np.full(n, depth + 1, np.int32), n_legal=np.full(n, 40, np.int32), anc=anc,
+                   legal=np.tile(np.arange(64, dtype=np.int32), (n, 1)))
+        _, value = ev.step(req)
+        path = tokens[:s + 1] if s < 5 else tokens[5:6]
+        for t in range(n):
+            ids = torch.from_numpy(np.concatenate([prefix[t], path[:, t]])).cuda()[None]
+            with torch.no_grad():
+                out = model(input_ids=ids, position_ids=torch.arange(ids.shape[1], device="cuda")[None])
+            want = out["logits"][0, -1].float()
+            assert float((ev.kv.logits[t].float() - want).norm() / want.norm()) < 2e-2, (s, t)
+            assert abs(float(value[t]) - float(out["value_logits"][0, -1])) < 2e-2
+    if n <= 16:
+        assert int(ev.kv.few_work[:1].view(torch.int32).item()) > 0      # the one kernel ran
+    _lib.check_status()
+
+
 def test_few_tree_step_ends_when_meetings_run_out():
     """One tree with a very long prompt: the CTAs that hold its heads read keys for hundreds of microseconds
     while the others wait at the meeting, longer than the limit set here.  All leave together (a verdict

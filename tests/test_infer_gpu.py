@@ -52,6 +52,66 @@ def test_packed_last_positions_and_cache(heads, d, lens):
                 assert not cache[l, i, :, len(r):].any()        # slots of later nodes stay as they were
 
 
+@pytest.mark.parametrize("heads,d", [(4, 256), (2, 256)])
+def test_packed_sequences_of_several_key_tiles(heads, d):
+    """Three to eight key tiles, heads of 64 and 128, beside short sequences; bound as above."""
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.ops import _lib
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=1000, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=2, n_embd=d,
+                             n_head=heads, n_positions=1000)
+    model.eval()
+    eng = B200Engine(model, "cuda")
+    rng = np.random.default_rng(1)
+    rows = [rng.integers(0, 1968, size=n) for n in (300, 5, 513, 1000, 385)]
+    logits, value, _ = eng.infer_last(rows)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for i, r in enumerate(rows):
+        with torch.no_grad():
+            out = model(input_ids=torch.from_numpy(r).cuda()[None], position_ids=torch.arange(len(r), device="cuda")[None])
+        want = out["logits"][0, -1].float()
+        assert float((logits[i].float() - want).norm() / want.norm()) < 2e-2, len(r)
+        assert abs(float(value[i]) - float(out["value_logits"][0, -1])) < 2e-2
+
+
+def test_evaluation_does_not_depend_on_the_games_beside_it():
+    """Alone, among a few (programmatic launches, small tiles) and among many (CTA pairs): the same bits, in
+    the results and in the cache."""
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.ops import _lib
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=400, vocab_size_multiple_of=128)
+    eng = B200Engine(initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=4,
+                                      n_embd=1024, n_head=16, n_positions=400), "cuda")
+    rng = np.random.default_rng(2)
+    picked = [rng.integers(0, 1968, size=n) for n in (1, 90, 130, 300)]
+    others = [rng.integers(0, 1968, size=int(n)) for n in rng.integers(1, 400, size=120)]
+
+    def run(rows):
+        k = torch.zeros(4, len(rows), 16, 400, 64, dtype=torch.bfloat16, device="cuda")
+        v = torch.zeros_like(k)
+        return (*eng.infer_last(rows, (k, v)), k, v)
+
+    alone = [run([r]) for r in picked]
+    for n in (3, 12, 120):
+        rows = [others[0], picked[0], picked[1], *others[1:n], picked[2], picked[3]]
+        at = [next(i for i, r in enumerate(rows) if r is p) for p in picked]
+        logits, value, time, k, v = run(rows)
+        for i, (l1, v1, t1, k1, vc1) in zip(at, alone):
+            assert torch.equal(logits[i], l1[0]) and torch.equal(value[i], v1[0]) and torch.equal(time[i], t1[0])
+            assert torch.equal(k[:, i], k1[:, 0]) and torch.equal(v[:, i], vc1[:, 0])
+    torch.cuda.synchronize()
+    _lib.check_status()
+
+
 def test_packed_inference_refuses_overlong_and_counts_launches():
     from allie_b200.data import UCITokenizer
     from allie_b200.models import initialize_model
