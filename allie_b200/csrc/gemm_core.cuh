@@ -194,15 +194,14 @@ __device__ __forceinline__ uint4 epi_pack8(const uint64_t* v) {
 }
 
 // One epilogue warp drains its 32 rows x 64 columns.  Rows past the end of the output are clipped by
-// the TMA store; with MASK_ROWS (grouped kernels, whose regions are padded) rows with !row_ok are
-// written as zeros.  `wait_tile` / `next_tile`: see EPI_RESID.  Returns false when a wait ran out.
-template <int EPI, bool MASK_ROWS, typename Wait, typename Next>
+// the TMA store.  `wait_tile` / `next_tile`: see EPI_RESID.  Returns false when a wait ran out.
+template <int EPI, typename Wait, typename Next>
 __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUtensorMap& tmOut,
                                                     const CUtensorMap& tmAux, uint32_t taddr, int m, int m0w,
-                                                    int nbase, bool row_ok, uint8_t* stg, int lane, int bias_off,
-                                                    Wait wait_tile, Next next_tile) {
-  const bool has_bias = g.ep.bias != nullptr;
-  const float* bias = g.ep.bias + bias_off;
+                                                    int nbase, uint8_t* stg, int lane, Wait wait_tile,
+                                                    Next next_tile) {
+  const float* bias = g.ep.bias;
+  const bool has_bias = bias != nullptr;
   if constexpr (EPI == EPI_BF16 || EPI == EPI_GELU || EPI == EPI_MUL || EPI == EPI_DOT) {
     // one store group: 64 bf16 columns = 128-byte rows, 128B swizzle.  The aux tile of EPI_MUL and
     // EPI_DOT lies in the staging tile already, in the same layout.
@@ -240,8 +239,7 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
           v[2] = f2_mul(v[2], f2_pack(bf16_lo(q.z), bf16_hi(q.z)));
           v[3] = f2_mul(v[3], f2_pack(bf16_lo(q.w), bf16_hi(q.w)));
         }
-        uint4 o = epi_pack8(v);
-        if (MASK_ROWS && !row_ok) o = make_uint4(0, 0, 0, 0);
+        const uint4 o = epi_pack8(v);
         if constexpr (EPI == EPI_DOT) {
           const uint4 q = *chunk;
           dot = f2_fma(f2_pack(bf16_lo(o.x), bf16_hi(o.x)), f2_pack(bf16_lo(q.x), bf16_hi(q.x)), dot);
@@ -312,11 +310,9 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
         epi_load8(r + c * 8, v, bias, n, has_bias && n < g.N);
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = f2_gelu_tanh_with_grad(v[j], d[j]);
-        uint4 o = epi_pack8(v), p = epi_pack8(d);
-        if (MASK_ROWS && !row_ok) { o = make_uint4(0, 0, 0, 0); p = o; }
         uint8_t* dst = stg + lane * 64 + ((c ^ sw) << 4);
-        *reinterpret_cast<uint4*>(dst) = o;
-        *reinterpret_cast<uint4*>(dst + 2048) = p;
+        *reinterpret_cast<uint4*>(dst) = epi_pack8(v);
+        *reinterpret_cast<uint4*>(dst + 2048) = epi_pack8(d);
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -413,10 +409,10 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
   return true;
 }
 
-// General drain of the CTA-pair kernels (EPI_ANY): the same per-round math as epilogue_drain, but several 16-column rounds are
-// staged side by side in one 4 KB tile per warp and leave in one TMA store with 128-byte rows
-// (64 bf16 or 32 fp32 columns; 64-byte rows when a second bf16 output shares the tile).  Wide
-// rows matter: the store path costs per row segment, not per byte.
+// General drain of the CTA-pair kernels (EPI_ANY, and the grouped kernel): the same per-round math as
+// epilogue_drain, but several 16-column rounds are staged side by side in one 4 KB tile per warp and
+// leave in one TMA store with 128-byte rows (64 bf16 or 32 fp32 columns; 64-byte rows when a second
+// bf16 output shares the tile).  Wide rows matter: the store path costs per row segment, not per byte.
 template <int COLS>
 __device__ __forceinline__ void epilogue_drain_wide(const GemmArgs& g, const CUtensorMap& tmOut,
                                                     const CUtensorMap& tmAux, uint32_t taddr, int m,

@@ -543,8 +543,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           else fetch_aux(u + num_pairs, 0);
         };
         if (m0w < g.M && nbase < g.N) {
-          if (!epilogue_drain_kind<EPI, false>(g, tmOut, tmAux, taddr, m, m0w, nbase, true, my_stage, lane, 0,
-                                               wait_aux, next_tile))
+          if (!epilogue_drain_kind<EPI>(g, tmOut, tmAux, taddr, m, m0w, nbase, my_stage, lane, wait_aux, next_tile))
             break;
         } else if ((EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT) && lane == 0) {
           fetch_aux(u + num_pairs, 0);

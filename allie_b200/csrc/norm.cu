@@ -5,7 +5,7 @@
 //           incoming residual gradient; optionally also emits the bf16, dropout-masked copy of
 //           dx that the previous branch's projection GEMMs consume, and accumulates
 //           dgamma/dbeta into the fp32 gradient buffers with one atomic per column per block.
-// One warp owns one row; a lane owns float4 columns lane*4 + 128*i.
+// Forward: one warp owns one row; a lane owns float4 columns lane*4 + 128*i.  Backward: see ln_bwd_kernel.
 #include "ptx.cuh"
 
 namespace ab {
@@ -94,11 +94,11 @@ struct LnBwdArgs {
 // a block): 16 warps per SM at d <= 1024, 8 above.
 //   LNB_ROWS rows are handled together (one exchange of row sums through shared memory for all of them).
 //   They come in by bulk copies, LNB_STAGES pairs of rows ahead per group (160 KB in flight on an SM): with
-//   loads into registers nothing was on its way while a block computed (32768 x 1024: 113 us).
+//   loads into registers nothing was on its way while a block computed (32768 x 1024: 113 us, now 105).
 //   RING = false is the form with plain loads, for tensors that bulk copies cannot address (16 bytes).
-//    A block holds as many groups as fit 512 threads (the registers of an
-//   SM) and folds their sums before its atomics: with a block per group, 740 blocks adding to the same
-//   2304 addresses cost 12136 x 768 more than the register sums gain.
+//   A block holds as many groups as fit 512 threads (the registers of an SM) and folds their sums before
+//   its atomics: with a block per group, 740 blocks adding to the same 2304 addresses cost 12136 x 768
+//   more than the register sums gain.
 // The eight columns of a thread belong to two dropout groups of eight; neighbouring lanes share both,
 // so each lane draws one and they swap.
 constexpr int LNB_ROWS = 2;
