@@ -11,6 +11,8 @@ TFLOP/s or GB/s against the measured peaks of the machine (``MEASURED_PEAKS.json
     python -m allie_b200.utils.kbench nvl --n 300000000      # gradient-path kernels with the rank as its own only peer
     python -m allie_b200.utils.kbench moe --rows 16384 --d 2048 --experts 8   # routing / dispatch / combine, one rank
     python -m allie_b200.utils.kbench decode_attn --batch 256 --heads 16 --hd 64 --seq 160
+    python -m allie_b200.utils.kbench decode_few --batch 4 --layers 24 --d 1024 --seq 60   # all layers of a step of few trees
+    python -m allie_b200.utils.kbench infer --batch 64 --layers 24 --d 1024 --seq 300     # packed inference, half-full on average
 
 Also the workload to put under ``ncu`` (``--iters`` small).  Inputs are sized beyond the 126 MB L2.
 """
@@ -51,7 +53,7 @@ def main(argv=None) -> dict:
 
     ap = argparse.ArgumentParser()
     ap.add_argument("kernel", choices=["gemm", "attn", "layernorm", "adamw", "colsum", "lmhead_ce", "gemm_grouped",
-                                       "nvl", "moe", "decode_attn"])
+                                       "nvl", "moe", "decode_attn", "decode_few", "infer"])
     ap.add_argument("--groups", type=int, default=8); ap.add_argument("--cap", type=int, default=8192)
     ap.add_argument("--live", type=int, default=4096); ap.add_argument("--experts", type=int, default=8)
     ap.add_argument("--m", type=int, default=32768); ap.add_argument("--n", type=int, default=4096)
@@ -63,6 +65,7 @@ def main(argv=None) -> dict:
     ap.add_argument("--batch", type=int, default=64); ap.add_argument("--seq", type=int, default=512)
     ap.add_argument("--heads", type=int, default=16); ap.add_argument("--hd", type=int, default=64)
     ap.add_argument("--dropout", type=float, default=0.0); ap.add_argument("--bwd", action="store_true")
+    ap.add_argument("--layers", type=int, default=24)
     ap.add_argument("--rows", type=int, default=32768); ap.add_argument("--d", type=int, default=1024)
     ap.add_argument("--iters", type=int, default=20); ap.add_argument("--warmup", type=int, default=3)
     a = ap.parse_args(argv)
@@ -240,6 +243,42 @@ def main(argv=None) -> dict:
         s = _time(fn, a.iters, a.warmup)
         nbytes = n * H * (P + 8) * hd * 2 * 2
         out.update(shape=[n, H, hd, P], seconds=s, gbs=nbytes / s / 1e9, frac_of_measured_hbm=nbytes / s / 1e9 / peaks["hbm_gbs"])
+    elif a.kernel in ("decode_few", "infer"):
+        import numpy as np
+
+        from ..data import UCITokenizer
+        from ..models import initialize_model
+        from ..models.engine import B200Engine
+        from ..search.evaluator import KVLeafEvaluator
+
+        tok = UCITokenizer(max_length=512, vocab_size_multiple_of=128)
+        with torch.device(dev):
+            model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=a.layers,
+                                     n_embd=a.d, n_head=a.d // a.hd, n_positions=512)
+        eng = B200Engine(model, dev)
+        weights = a.layers * 12 * a.d * a.d * 2           # bytes of the layers' matrices
+        if a.kernel == "infer":
+            rng = np.random.default_rng(0)
+            rows = [rng.integers(0, 1968, size=int(n)) for n in np.linspace(4, a.seq, a.batch)]
+            fn = lambda: eng.infer_last(rows)
+            s = _time(fn, a.iters, a.warmup)
+            tf = 2.0 * sum(map(len, rows)) * 12 * a.layers * a.d * a.d / s / 1e12
+            out.update(sequences=a.batch, rows=sum(map(len, rows)), seconds=s, tflops=tf,
+                       frac_of_measured_bf16=tf / peaks["bf16_tflops"])
+        else:
+            ev = KVLeafEvaluator(eng, a.batch, max_prefix=a.seq, max_nodes=64, use_graph=False)
+            for name, v in (("active", 1), ("pos", a.seq), ("slot", a.seq), ("prefix_len", a.seq), ("n_anc", 1)):
+                ev.view(ev.req_dev, name).fill_(v)
+            ev.view(ev.req_dev, "anc").fill_(a.seq)
+            ev.x[0].normal_()
+
+            def fn():
+                assert ev._launch_few(ev.x[0])
+
+            s = _time(fn, a.iters, a.warmup)
+            nbytes = weights + a.batch * a.seq * a.layers * 4 * a.d
+            out.update(trees=a.batch, keys=a.seq, seconds=s, gbs=nbytes / s / 1e9,
+                       frac_of_measured_hbm=nbytes / s / 1e9 / peaks["hbm_gbs"])
     else:
         n = a.n if a.n > 1 << 20 else 300_000_000
         n -= n % 4
