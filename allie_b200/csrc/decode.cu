@@ -5,6 +5,7 @@
 //   decode_attn     : q_len = 1 attention of every tree's new token over that tree's prompt slots
 //                     [0, prefix_len) plus the cache slots of the leaf's ancestors (an index list);
 //                     also appends the new token's key/value to the cache
+//   result_rows     : logits, values and times of an inference pass as the rows that go to the host
 //   policy_epilogue : per tree, softmax over the logits of the leaf's legal moves only, plus value,
 //                     think time and the resign logit, packed into one row for a single
 //                     device-to-host copy
@@ -297,9 +298,33 @@ policy_epilogue_kernel(const __nv_bfloat16* __restrict__ logits, long long ld,
   }
 }
 
+// Results of an inference pass in the form they leave in: n rows of V logits, value and time in fp32, and the
+// status word behind the last row.  One block per row; a few MB at most.
+__global__ void __launch_bounds__(256)
+result_rows_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ value,
+                   const float* __restrict__ time, int V, float* __restrict__ out, const int* __restrict__ status) {
+  const long long r = blockIdx.x;
+  const __nv_bfloat16* src = logits + r * V;
+  float* dst = out + r * (V + 2);
+  for (int i = threadIdx.x; i < V; i += 256) dst[i] = __bfloat162float(src[i]);
+  if (threadIdx.x == 0) {
+    dst[V] = value ? value[r] : 0.f;
+    dst[V + 1] = time ? time[r] : 0.f;
+    if (r == 0) out[static_cast<long long>(gridDim.x) * (V + 2)] = __int_as_float(*status);
+  }
+}
+
 }  // namespace ab
 
 extern "C" {
+
+// out: fp32 [n * (V + 2) + 1]; value / time may be null
+int ab_result_rows(const void* logits, const float* value, const float* time, int n, int V, float* out,
+                   const int* status, cudaStream_t stream) {
+  if (n < 1 || V < 1 || !logits || !out || !status) return -1;
+  ab::result_rows_kernel<<<n, 256, 0, stream>>>((const __nv_bfloat16*)logits, value, time, V, out, status);
+  return (int)cudaGetLastError();
+}
 
 int ab_decode_attn(const void* qkv, void* kc, void* vc, const int* active, const int* slot,
                    const int* prefix_len, const int* anc, int anc_stride, const int* n_anc, void* out,

@@ -703,12 +703,13 @@ class B200Engine:
         return out
 
     @torch.no_grad()
-    def infer_last(self, rows: list, kv=None) -> tuple[torch.Tensor, torch.Tensor | None, torch.Tensor | None]:
+    def infer_last(self, rows: list, kv=None, ids=None) -> tuple[torch.Tensor, torch.Tensor | None, torch.Tensor | None]:
         """Inference over token sequences of different lengths (integer arrays of raw ids): logits [n, V]
         bf16 and, with the scalar heads, value and time [n] fp32 of every sequence's LAST position, on
         the device.  The sequences lie packed behind one another, so no row is computed for padding.
         ``kv``: optional ``(k, v)`` caches [layer, sequence, head, slot, head_dim] that receive the keys
-        and values of all positions.  Dense models only."""
+        and values of all positions.  ``ids``: the concatenation of ``rows``, where a caller has it.  Dense
+        models only."""
         from ..ops.gemm import num_sms
         from ..ops.infer import Infer, infer_last
 
@@ -725,7 +726,10 @@ class B200Engine:
         d, F, V = cfg.n_embd, cfg.ffn_dim, cfg.vocab_size
         host = torch.empty(2 * M + 2 * n + 1, dtype=torch.int32, pin_memory=True)
         block = host.numpy()
-        np.concatenate(rows, out=block[:M], casting="unsafe")
+        if ids is None:
+            np.concatenate(rows, out=block[:M], casting="unsafe")
+        else:
+            block[:M] = ids
         block[M:2 * M] = np.arange(M, dtype=np.int32) - np.repeat(row0[:-1], lens)
         block[2 * M:2 * M + n + 1] = row0
         block[2 * M + n + 1:] = row0[1:] - 1

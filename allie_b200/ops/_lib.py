@@ -112,22 +112,6 @@ def check_status() -> None:
     raise_on_status(int(status_word()[0].item()))
 
 
-def rows_and_status(n: int, width: int, device) -> tuple[torch.Tensor, torch.Tensor]:
-    """fp32 rows [n, width] on the device and the flat buffer they lie in, which has room for
-    the status word at its end: see :func:`fetch_rows`."""
-    flat = torch.empty(n * width + 1, dtype=torch.float32, device=device)
-    return flat[:-1].view(n, width), flat
-
-
-def fetch_rows(rows: torch.Tensor, flat: torch.Tensor) -> torch.Tensor:
-    """The rows of :func:`rows_and_status` on the host, in one copy; raises if a wait of a kernel ran out
-    before it (what was computed behind such a kernel is not to be used)."""
-    flat[-1:].view(torch.int32).copy_(status_word()[:1])
-    host = flat.cpu()
-    raise_on_status(int(host[-1:].view(torch.int32)))
-    return host[:-1].view(rows.shape)
-
-
 def dropout_thr16(p: float) -> int:
     t = p * 65536.0
     if t <= 0:

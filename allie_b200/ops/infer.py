@@ -1,12 +1,14 @@
-"""Binding of the native inference schedule (``csrc/infer.cu``): one forward pass over a packed batch
-whose last positions are the only outputs."""
+"""Bindings of the native inference schedule (``csrc/infer.cu``): one forward pass over a packed batch
+whose last positions are the only outputs, and of the kernel that lays its results out for the host."""
 from __future__ import annotations
 
 import ctypes
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
+import torch
+
 from . import _lib
-from ._lib import stream_ptr
+from ._lib import ptr, stream_ptr
 
 
 class InferLayer(ctypes.Structure):
@@ -30,3 +32,21 @@ def infer_last(args: Infer, layers) -> None:
     if rc < 0:
         raise RuntimeError(f"ab_infer_last failed with code {rc} (n={args.n} M={args.M} T={args.T})")
     _lib.count_launches(rc)
+
+
+def results_to_host(logits: torch.Tensor, value: torch.Tensor | None, time: torch.Tensor | None) -> torch.Tensor:
+    """bf16 logits [n, V] and fp32 value and time [n] (zeros without them) -> host fp32 [n, V + 2], in one
+    copy.  The status word comes along: raises if a wait of a kernel ran out before (what was computed
+    behind such a kernel is not to be used)."""
+    n, V = logits.shape
+    assert logits.dtype == torch.bfloat16 and logits.is_contiguous()
+    assert all(t is None or (t.dtype == torch.float32 and t.is_contiguous()) for t in (value, time))
+    out = torch.empty(n * (V + 2) + 1, dtype=torch.float32, device=logits.device)
+    rc = _lib.cuda().ab_result_rows(ptr(logits), ptr(value), ptr(time), c_int(n), c_int(V), ptr(out),
+                                    ptr(_lib.status_word()), stream_ptr())
+    if rc != 0:
+        raise RuntimeError(f"ab_result_rows failed with code {rc}")
+    _lib.count_launches(1)
+    host = out.cpu()
+    _lib.raise_on_status(int(host.numpy()[-1:].view("int32")[0]))
+    return host[:-1].view(n, V + 2)

@@ -19,6 +19,7 @@ import torch
 from ..ops import _lib, kernels as K
 from ..ops._lib import ptr, stream_ptr
 from ..ops.gemm import gemm, num_sms
+from ..ops.infer import results_to_host
 
 
 class KVLeafEvaluator:
@@ -49,7 +50,7 @@ class KVLeafEvaluator:
         self.out_flat = torch.zeros(n * self.out_stride + 1, dtype=f32, device=dev)
         self.out_flat_host = torch.zeros(n * self.out_stride + 1, dtype=f32, pin_memory=True)
         self.out_host = self.out_flat_host[:-1].view(n, self.out_stride)
-        self.status_host = self.out_flat_host[-1:].view(i32)
+        self.status_host = self.out_flat_host[-1:].view(i32).numpy()
         e = lambda *s, dt=bf: torch.empty(*s, dtype=dt, device=dev)
         self.x = [e(n, d, dt=f32), e(n, d, dt=f32)]
         self.ln, self.qkv, self.att = e(n, d), e(n, 3 * d), e(n, d)
@@ -93,15 +94,8 @@ class KVLeafEvaluator:
             logits, value, time = eng.infer_last(token_rows, (self.kc.view(shape), self.vc.view(shape)))
         else:
             logits, value, time = self._prefill_padded(token_rows, lens)
-        # one device-to-host copy
+        out = results_to_host(logits, value, time)
         V = logits.size(1)
-        out, flat = _lib.rows_and_status(n, V + 2, eng.device)
-        out[:, :V] = logits
-        if eng.reg is not None:
-            out[:, V], out[:, V + 1] = value, time
-        else:
-            out[:, V:] = 0
-        out = _lib.fetch_rows(out, flat)
         self.view(self.req_host, "prefix_len").copy_(torch.tensor(lens, dtype=torch.int32))
         return out[:, :V], out[:, V], out[:, V + 1]
 
@@ -210,6 +204,6 @@ class KVLeafEvaluator:
             self._launch_step()
         self.out_flat_host.copy_(self.out_flat, non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        _lib.raise_on_status(int(self.status_host))
+        _lib.raise_on_status(int(self.status_host[0]))
         self.steps += 1
         return self.out_host.numpy()

@@ -16,7 +16,7 @@ import torch
 
 from ..data import Game, UCITokenizer
 from ..models import unwrap
-from ..ops import _lib
+from ..ops.infer import results_to_host
 
 
 @dataclass
@@ -96,8 +96,9 @@ class EngineRunner(ModelRunner):
                 # ratings that run into the outcome bits of a word: refused where the padded batch does
                 assert all(int(((tok.tokenize(g)[: tok.max_length] & 0xFFFF) >> 14).max()) < 3 for g in games)
         # a padding token inside a game takes no position of its own, which the padded batch knows
-        if rows is not None and not (np.concatenate(rows) == tok.pad_token_id).any():
-            logits, value, time = eng.infer_last(rows)
+        ids = None if rows is None else np.concatenate(rows)
+        if rows is not None and not (ids == tok.pad_token_id).any():
+            logits, value, time = eng.infer_last(rows, ids=ids)
         else:      # experts are laid out for a fixed number of rows; arrays come as equal windows already
             batch = self.tokenizer.pad_and_collate(games, return_labels=False)
             out = eng.evaluate_batch(batch, with_loss=False)
@@ -106,15 +107,8 @@ class EngineRunner(ModelRunner):
             logits = out["logits"][rows, idx]
             value, time = ((out["value_logits"][rows, idx], out["time_logits"][rows, idx]) if self.has_value_head
                            else (None, None))
+        host = results_to_host(logits, value, time)     # the one device-to-host copy of this evaluation
         V = logits.size(-1)
-        packed, flat = _lib.rows_and_status(n, V + 2, eng.device)
-        packed[:, :V] = logits
-        if self.has_value_head:
-            packed[:, V] = value
-            packed[:, V + 1] = time
-        else:
-            packed[:, V:] = 0
-        host = _lib.fetch_rows(packed, flat)     # the one device-to-host copy of this evaluation
         return Evaluation(host[:, :V], host[:, V], host[:, V + 1])
 
 
