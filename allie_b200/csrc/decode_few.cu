@@ -338,7 +338,7 @@ decode_few_kernel(const DecodeFewArgs g) {
   uint32_t par = 0;
   unsigned int target = 0;
   bool ok = true;       // uniform over the computing warps
-  bool good = true;     // of this warp: after a wait that ran out it goes through the motions up to the barrier
+  bool good = true;     // of this lane: after a wait that ran out it goes through the motions up to the meeting
   // All CTAs have finished the phase and see its results (read through L2 afterwards).  One addition and
   // one watching thread per CTA; the release and the acquire order the CTA's other accesses.  (A flag per
   // CTA that threads of all CTAs watch keeps 148 x 148 loads in flight and takes longer.)  The verdict is one
@@ -443,13 +443,14 @@ decode_few_kernel(const DecodeFewArgs g) {
         uint32_t a_addr = smem_u32(sA) + (lane & 15) * g.pitch + (lane >> 4) * 16 + a_col * 2;
         const uint32_t w_off = lane * 128 + ((warp ^ (lane & 7)) << 4);
         for (int c = 0; c < p.k / DF_CHUNK; ++c) {
-          // one answer per warp: its lanes go through ldmatrix and the MMAs together
-          if (good && !__all_sync(0xffffffffu, mbar_wait(&full[slot], par, abort_flag))) {
+          // After a wait that ran out a lane goes on like the others, with whatever the slot holds: ldmatrix and
+          // the MMAs are the whole warp's.  (A vote on the answer costs 7 us of a step's 640.)
+          if (good && !mbar_wait(&full[slot], par, abort_flag)) {
             good = false;
             *abort_flag = ST_TIMEOUT_FULL;
             atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
           }
-          if (!good) break;
+          __syncwarp();
           const uint32_t w_addr = smem_u32(ring + slot * DF_SLOT) + w_off;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {            // 32 rows each: two contraction steps
