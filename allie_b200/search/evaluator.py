@@ -196,10 +196,13 @@ class KVLeafEvaluator:
                 self._launch_step()                      # warm-up outside capture (first-launch set-up)
                 torch.cuda.synchronize()
                 g = torch.cuda.CUDAGraph()
+                before = _lib.LAUNCHES
                 with torch.cuda.graph(g):
                     self._launch_step()
-                self.graph = g
+                self.graph, self.graph_launches = g, _lib.LAUNCHES - before
+                _lib.count_launches(-self.graph_launches)     # nothing ran yet: counted per replay
             self.graph.replay()
+            _lib.count_launches(self.graph_launches)
         else:
             self._launch_step()
         self.out_flat_host.copy_(self.out_flat, non_blocking=True)

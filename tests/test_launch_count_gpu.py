@@ -65,3 +65,25 @@ def test_gemm_with_column_sums_and_head_products(M, N):
         kernels, counted = _kernels_and_count(lambda: gemm(a, w, out=out, **kw))
         assert kernels == counted > 0, kw
     _lib.check_status()
+
+
+@pytest.mark.parametrize("n", [2, 20])            # all layers in one kernel / the chain of kernels
+def test_replayed_search_step(n):
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import initialize_model
+    from allie_b200.models.engine import B200Engine
+    from allie_b200.ops import _lib
+    from allie_b200.search.evaluator import KVLeafEvaluator
+
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    eng = B200Engine(initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=2, n_embd=128,
+                                      n_head=2, n_positions=64), "cuda")
+    counts = []
+    for use_graph in (False, True):
+        ev = KVLeafEvaluator(eng, n, max_prefix=16, max_nodes=8, anc_max=4, legal_max=8, use_graph=use_graph)
+        ev.step()
+        before = _lib.LAUNCHES
+        ev.step()
+        counts.append(_lib.LAUNCHES - before)
+    # embedding, layers, final norm, logits, heads, policy
+    assert counts[0] == counts[1] == 5 + (1 if n == 2 else 7 * 2)
