@@ -137,8 +137,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         dst, ep.dot_T = dot
         assert act == 4 and dst.dtype == torch.float32 and dst.numel() * 64 == M * N and M % ep.dot_T == 0
         ep.dot_out = dst.data_ptr()
-    passes = c_int(0)
-    ep.passes = ctypes.addressof(passes)
+    passes = None
+    if colsum is not None or dot is not None:       # only these can take a pass of their own
+        passes = c_int(0)
+        ep.passes = ctypes.addressof(passes)
     rc = _lib.cuda().ab_gemm_bf16(
         _lib.ptr(a), c_int(int(a_mn)), c_longlong(a.stride(0)),
         _lib.ptr(b), c_int(int(b_mn)), c_longlong(b.stride(0)),
@@ -146,7 +148,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         _lib.ptr(_lib.status_word()), _lib.stream_ptr())
     if rc != 0:
         raise RuntimeError(f"ab_gemm_bf16 failed with code {rc} for M={M} N={N} K={K}")
-    _lib.count_launches(1 + passes.value)
+    _lib.count_launches(1 if passes is None else 1 + passes.value)
     return out
 
 

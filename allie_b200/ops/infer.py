@@ -34,13 +34,15 @@ def infer_last(args: Infer, layers) -> None:
     _lib.count_launches(rc)
 
 
-def results_to_host(logits: torch.Tensor, value: torch.Tensor | None, time: torch.Tensor | None) -> torch.Tensor:
-    """bf16 logits [n, V] and fp32 value and time [n] (zeros without them) -> host fp32 [n, V + 2], in one
+def results_to_host(logits: torch.Tensor, value: torch.Tensor | None,
+                    time: torch.Tensor | None) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """bf16 logits [n, V] and fp32 value and time [n] (zeros without them) as fp32 on the host, in one
     copy.  The status word comes along: raises if a wait of a kernel ran out before (what was computed
     behind such a kernel is not to be used)."""
     n, V = logits.shape
     assert logits.dtype == torch.bfloat16 and logits.is_contiguous()
-    assert all(t is None or (t.dtype == torch.float32 and t.is_contiguous()) for t in (value, time))
+    for t in (value, time):
+        assert t is None or (t.dtype == torch.float32 and t.is_contiguous())
     out = torch.empty(n * (V + 2) + 1, dtype=torch.float32, device=logits.device)
     rc = _lib.cuda().ab_result_rows(ptr(logits), ptr(value), ptr(time), c_int(n), c_int(V), ptr(out),
                                     ptr(_lib.status_word()), stream_ptr())
@@ -49,4 +51,5 @@ def results_to_host(logits: torch.Tensor, value: torch.Tensor | None, time: torc
     _lib.count_launches(1)
     host = out.cpu()
     _lib.raise_on_status(int(host.numpy()[-1:].view("int32")[0]))
-    return host[:-1].view(n, V + 2)
+    row = V + 2
+    return host.as_strided((n, V), (row, 1)), host.as_strided((n,), (row,), V), host.as_strided((n,), (row,), V + 1)

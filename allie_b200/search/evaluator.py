@@ -95,9 +95,8 @@ class KVLeafEvaluator:
         else:
             logits, value, time = self._prefill_padded(token_rows, lens)
         out = results_to_host(logits, value, time)
-        V = logits.size(1)
         self.view(self.req_host, "prefix_len").copy_(torch.tensor(lens, dtype=torch.int32))
-        return out[:, :V], out[:, V], out[:, V + 1]
+        return out
 
     def _prefill_padded(self, token_rows, lens):
         """The same for models with experts, whose buffers are laid out for a fixed number of rows."""

@@ -107,9 +107,8 @@ class EngineRunner(ModelRunner):
             logits = out["logits"][rows, idx]
             value, time = ((out["value_logits"][rows, idx], out["time_logits"][rows, idx]) if self.has_value_head
                            else (None, None))
-        host = results_to_host(logits, value, time)     # the one device-to-host copy of this evaluation
-        V = logits.size(-1)
-        return Evaluation(host[:, :V], host[:, V], host[:, V + 1])
+        # the one device-to-host copy of this evaluation
+        return Evaluation(*results_to_host(logits, value, time))
 
 
 PRECISIONS = (None, "float32", "bfloat16")
