@@ -17,7 +17,7 @@
 //     next phase rounds as the chain of kernels does;
 //   * every CTA normalises the residual rows for itself (n x d values through L2);
 //   * attention: a CTA takes a (tree, head), its warps split the keys.
-// Measured (24 layers of 1024 / 4096, cold weights): 600 us with 1 or 4 trees, 780 with 16; 16 us of a
+// Measured (24 layers of 1024 / 4096, cold weights): 640 us with 1 or 4 trees, 840 with 16; 16 us of a
 // layer's 25 are the five meetings and the first loads behind each (what a layer of width 128 takes),
 // which is what bounds it now.  From 17 trees on the chain of kernels is used: its tiles hold 128 rows.
 #include "ptx.cuh"

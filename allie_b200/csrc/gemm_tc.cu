@@ -742,6 +742,8 @@ static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue
   // contraction and its epilogue while the others are idle.  128 x 64 tiles where they fit, else 128 x 128
   // (2048 x 256 x 256 with residual and dropout: 11.7 us on pairs, 9.4 with 128 x 128, 7.3 with 128 x 64;
   // 2048 x 1024 x 256: 11.9, 9.6, 9.8 in two waves; 4096 x 1024 x 1024, two waves: 16.3, 19.9, 27.7).
+  // Over M 512 to 4096, N 256 to 4096, K 128 to 4096 with bias, GELU, residual or plain outputs, wherever the rule
+  // holds: 0.64 to 0.77 of the pairs' time on average, 0.89 at most.
   auto tiles = [&](int bn) { return static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn); };
   const bool one_wave = pair && !a_mn && !sums && !dot && k_splits == 1 && tiles(128) <= max_ctas;
   // narrow tiles also for skinny problems (decode steps with a few hundred rows): twice the CTAs

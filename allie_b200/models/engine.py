@@ -597,7 +597,7 @@ class B200Engine:
 
     # ------------------------------------------------------- captured micro-step
     def enable_step_graph(self, on: bool = True) -> bool:
-        """Replays the micro-step (window unpack, forward, backward: a few thousand launches for
+        """Replays the micro-step (window unpack, forward, backward: a few hundred launches for
         the medium model) as one CUDA graph per batch shape instead of launching its kernels one
         by one.  A captured launch freezes the arguments it was given by value, and the dropout seed
         is one of them, so while capturing, every kernel that draws a mask is also handed the address

@@ -159,7 +159,7 @@ class Trainer:
         ``expert_parallel`` (MoE models on several ranks): true spreads the experts over the ranks,
         false replicates them and averages their gradients like any other parameter.
         ``cuda_graph``: replay the micro-step (unpack, forward, backward) as one CUDA graph instead of
-        a few thousand launches; default (None): on for dense models (1.4x on the tiny config, 7-10 %
+        a few hundred launches; default (None): on for dense models (1.4x on the tiny config, 7-10 %
         on small ones, under 1 % on the medium config, where it mainly frees the host thread: 53 ms of
         launch calls per 82 ms micro-step become 0.04 ms); MoE models keep the ordinary launches."""
         self.expert_parallel_requested = expert_parallel
