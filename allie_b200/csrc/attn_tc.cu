@@ -642,8 +642,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
             const uint64_t e0 = row_elem0 + hf * 16 + g * 8;
+            // keys past the end of the sequence have no bits: their words are the next row's, or past the mask
             const uint32_t keep = a.drop_mask
-                ? (q_ok ? (a.drop_mask[e0 >> 5] >> (e0 & 31)) & 0xffu : 0u)
+                ? (q_ok && kj * 128 + col0 < a.T ? (a.drop_mask[e0 >> 5] >> (e0 & 31)) & 0xffu : 0u)
                 : dropout_keep8(salted(a.seed, a.salt), a.stream_id, e0 >> 3, a.thr16);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {

@@ -283,3 +283,35 @@ def test_persistent_backward_of_ragged_sequences(B, H, T, p):
         assert ((dbias.double() - sums).abs() <= 1e-5 * dqkv.double().abs().sum(0) + 1e-6).all()
     assert float((got[1] - got[2]).norm() / got[1].norm()) < 2e-3
     assert ((got[1] - got[2]).abs() <= 2 ** -7 * got[1].abs() + 1e-2 * got[1].pow(2).mean().sqrt()).all()
+
+
+@pytest.mark.parametrize("T", [96, 160, 448])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_two_kernel_backward_reads_no_keep_bits_past_a_sequence(T, hd):
+    """The last key tile reaches past the sequence, where the mask's words are another row's or not the mask's at
+    all.  Values that are not finite there (the next sequence's V) would reach dQ through such a bit: P is zero,
+    but zero times infinity is not."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.attention import attention_bwd, attention_fwd
+
+    torch.manual_seed(T)
+    B, H = 2, 2
+    d, dev = H * hd, "cuda"
+    qkv = torch.randn(B * T, 3 * d, device=dev).bfloat16()
+    dout = torch.randn(B * T, d, device=dev).bfloat16()
+    out, lse, delta = torch.zeros_like(dout), torch.zeros(B, H, T, device=dev), torch.zeros(B, H, T, device=dev)
+    words = B * H * T * (T // 32)
+    store = torch.full((words + 64,), -1, device=dev, dtype=torch.int32)      # ones behind the mask
+    bits = store[:words].view(B, H, T, T // 32)
+    attention_fwd(qkv, out, lse, B, T, H, hd, 0.1, 5, 1, bits)
+    got = []
+    for last_v in (None, float("inf")):
+        x = qkv.clone()
+        if last_v is not None:
+            x[T:, 2 * d:] = last_v
+        dqkv = torch.zeros_like(qkv)
+        attention_bwd(x, out, lse, dout, dqkv, delta, B, T, H, hd, 0.1, 5, 1, bits)
+        got.append(dqkv[:T])
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert got[0].isfinite().all() and torch.equal(got[0], got[1])
