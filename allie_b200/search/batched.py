@@ -131,6 +131,7 @@ class KVStepEvaluator:
         self.positions = 0
 
     def prefill(self, games: list[Game | None]):
+        games = list(games)
         rows = iter(self.tok.token_rows([g for g in games if g is not None]))
         return self.kv.prefill([np.array([self.tok.bos_token_id], dtype=np.int64) if g is None else next(rows)
                                 for g in games])

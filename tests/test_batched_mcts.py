@@ -94,3 +94,16 @@ def test_search_refuses_positions_beyond_the_table(tok_model):
     with pytest.raises(ValueError, match="positions"):
         bm2.search([game])
     assert ev.runner.calls == 1 + 4 + 0        # the refused search evaluated nothing
+
+
+@pytest.mark.parametrize("form", [list, tuple, iter])
+def test_key_value_prompts_of_games_in_any_iterable(form):
+    """Games and empty trees (None) as a sequence or as what can be walked only once: one row each, in order."""
+    from allie_b200.search.batched import KVStepEvaluator
+
+    tok = UCITokenizer(max_length=64, vocab_size_multiple_of=128)
+    ev = object.__new__(KVStepEvaluator)
+    ev.tok, ev.kv = tok, type("Cache", (), {"prefill": staticmethod(lambda rows: [list(map(int, r)) for r in rows])})()
+    games = [Game("180+0", 1500, 1600, None, False, ["e2e4"] * n, [1] * n) for n in (1, 3)]
+    want = [tok.token_ids(games[0]).tolist(), [tok.bos_token_id], tok.token_ids(games[1]).tolist()]
+    assert ev.prefill(form([games[0], None, games[1]])) == want
