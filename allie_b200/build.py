@@ -12,6 +12,7 @@ Run ``python -m allie_b200.build`` or call :func:`build_all`.
 """
 from __future__ import annotations
 
+import logging
 import os
 import shutil
 import subprocess
@@ -103,17 +104,24 @@ def build_host(force: bool = False) -> Path | None:
 
 
 def build_py(force: bool = False) -> Path | None:
-    """``csrc/py``: code that walks Python objects, for this interpreter.  Without its headers (None) the
-    Python statements of the same rules serve."""
+    """``csrc/py``: code that walks Python objects, for this interpreter.  Optional: where it cannot be built (None;
+    no interpreter headers, no source, no compiler) the Python statements of the same rules serve."""
     src = CSRC / "py" / "tokens.cpp"
     include = Path(sysconfig.get_paths()["include"])
+    out = LIB / "liballie_py.so"
+    if not src.exists():                 # a copy without it keeps what was built elsewhere
+        return out if out.exists() else None
     if not (include / "Python.h").exists():
         return None
     OBJ.mkdir(parents=True, exist_ok=True)
-    out = LIB / "liballie_py.so"
     if force or not out.exists() or out.stat().st_mtime < src.stat().st_mtime:
         cxx = os.environ.get("CXX", "g++")
-        _compile([cxx, *CXX_FLAGS, "-shared", "-I", str(include), "-o", str(out), str(src)], OBJ / "py.log")
+        try:
+            _compile([cxx, *CXX_FLAGS, "-shared", "-I", str(include), "-o", str(out), str(src)], OBJ / "py.log")
+        except (RuntimeError, OSError) as e:
+            out.unlink(missing_ok=True)  # what an older source gave is not served either
+            logging.getLogger(__name__).warning("optional %s not built: %s", out.name, e)
+            return None
     return out
 
 

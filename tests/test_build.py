@@ -1,0 +1,45 @@
+"""The build of the native libraries (CPU): what is optional stops nothing."""
+import shutil
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+from allie_b200 import build
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+def test_an_installed_copy_has_every_source(tmp_path):
+    tree = tmp_path / "tree"
+    tree.mkdir()
+    for name in ("allie_b200", "src"):
+        shutil.copytree(ROOT / name, tree / name, ignore=shutil.ignore_patterns("lib", "__pycache__"))
+    for name in ("setup.py", "pyproject.toml"):
+        shutil.copy(ROOT / name, tree / name)
+    subprocess.run([sys.executable, "setup.py", "-q", "build_py", "--build-lib", str(tmp_path / "out")], cwd=tree, check=True,
+                   capture_output=True)
+    sources = [p.relative_to(ROOT) for p in build.CSRC.rglob("*") if p.is_file()]
+    assert sources and all((tmp_path / "out" / p).is_file() for p in sources)
+
+
+@pytest.mark.parametrize("trouble", ["no source", "no source, built before", "does not compile", "no compiler"])
+def test_the_optional_library_does_not_stop_the_build(trouble, tmp_path, monkeypatch):
+    csrc, lib = tmp_path / "csrc", tmp_path / "lib"
+    (csrc / "py").mkdir(parents=True)
+    lib.mkdir()
+    if not trouble.startswith("no source"):
+        (csrc / "py" / "tokens.cpp").write_text("not C++\n")
+    for name, value in (("CSRC", csrc), ("LIB", lib), ("OBJ", lib / "obj")):
+        monkeypatch.setattr(build, name, value)
+    if trouble == "no source, built before":
+        (lib / "liballie_py.so").write_bytes(b"")
+    if trouble == "no compiler":
+        monkeypatch.setenv("CXX", str(tmp_path / "none"))
+    built = []
+    monkeypatch.setattr(build, "build_host", lambda *a: built.append("host"))
+    monkeypatch.setattr(build, "build_cuda", lambda *a: built.append("cuda"))
+    build.build_all()
+    assert built == ["host", "cuda"]
+    assert (build.build_py() is None) == (trouble != "no source, built before")
