@@ -5,8 +5,8 @@ Every ``csrc/*.cu`` file is compiled for sm_100a only
 ``allie_b200/lib/liballie_b200.so``, with a plain C ABI that the Python side
 binds through ``ctypes``.  Host-only C++ (chess move generation, MCTS) goes
 into ``allie_b200/lib/liballie_host.so`` with g++, code on Python objects
-into ``allie_b200/lib/liballie_py.so``.  Objects are rebuilt only when their source (or a header)
-is newer.
+into ``allie_b200/lib/liballie_py<interpreter's suffix>.so``.  Objects are rebuilt only when their source (or a
+header) is newer.
 
 Run ``python -m allie_b200.build`` or call :func:`build_all`.
 """
@@ -103,12 +103,18 @@ def build_host(force: bool = False) -> Path | None:
     return out
 
 
+def py_library() -> str:
+    """Name of the library of code on Python objects.  Object layouts are compiled in and differ between
+    interpreters (a str's at 3.12), so each has a file of its own."""
+    return "liballie_py" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
+
+
 def build_py(force: bool = False) -> Path | None:
     """``csrc/py``: code that walks Python objects, for this interpreter.  Optional: where it cannot be built (None;
     no interpreter headers, no source, no compiler) the Python statements of the same rules serve."""
     src = CSRC / "py" / "tokens.cpp"
     include = Path(sysconfig.get_paths()["include"])
-    out = LIB / "liballie_py.so"
+    out = LIB / py_library()
     if not src.exists():                 # a copy without it keeps what was built elsewhere
         return out if out.exists() else None
     if not (include / "Python.h").exists():

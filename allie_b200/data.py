@@ -28,7 +28,6 @@ from array import array
 from dataclasses import dataclass
 from functools import cached_property, lru_cache
 from itertools import repeat
-from pathlib import Path
 from typing import Any, Sequence
 
 import numpy as np
@@ -149,8 +148,10 @@ def json_to_partial_game(d: dict, halfmove: int) -> Game:
 
 @lru_cache(maxsize=None)
 def _native_tokens():
-    """The native tokenizer call, or None where ``liballie_py.so`` has not been built."""
-    path = Path(__file__).resolve().parent / "lib" / "liballie_py.so"
+    """The native tokenizer call, or None where it has not been built for this interpreter."""
+    from . import build
+
+    path = build.LIB / build.py_library()
     if not path.exists():
         return None
     fn = ctypes.PyDLL(str(path)).allie_token_rows

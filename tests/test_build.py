@@ -34,7 +34,7 @@ def test_the_optional_library_does_not_stop_the_build(trouble, tmp_path, monkeyp
     for name, value in (("CSRC", csrc), ("LIB", lib), ("OBJ", lib / "obj")):
         monkeypatch.setattr(build, name, value)
     if trouble == "no source, built before":
-        (lib / "liballie_py.so").write_bytes(b"")
+        (lib / build.py_library()).write_bytes(b"")
     if trouble == "no compiler":
         monkeypatch.setenv("CXX", str(tmp_path / "none"))
     built = []
@@ -43,3 +43,20 @@ def test_the_optional_library_does_not_stop_the_build(trouble, tmp_path, monkeyp
     build.build_all()
     assert built == ["host", "cuda"]
     assert (build.build_py() is None) == (trouble != "no source, built before")
+
+
+@pytest.mark.parametrize("suffix", [".cpython-311-x86_64-linux-gnu.so", ".cpython-313t-x86_64-linux-gnu.so"])
+def test_a_library_of_another_interpreter_is_not_loaded(suffix, monkeypatch):
+    """It reads object layouts that are compiled in; the Python statement of the rules serves until there is one."""
+    from allie_b200 import data
+
+    if build.build_py() is None:
+        pytest.skip("no interpreter headers")
+    data._native_tokens.cache_clear()
+    try:
+        assert data._native_tokens() is not None
+        data._native_tokens.cache_clear()
+        monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name: suffix)
+        assert data._native_tokens() is None
+    finally:
+        data._native_tokens.cache_clear()
