@@ -6,7 +6,12 @@ cheap): ``UCITokenizer``, ``Game``, ``load_data``, ``load_config``, ``initialize
 ``ops`` (kernel bindings), ``parallel`` (NVLink gradient path, expert parallelism), ``train``,
 ``search`` (decode strategies, batched MCTS), ``evaluation``, ``serve``, ``etl``, ``chess``.
 """
+from importlib.machinery import EXTENSION_SUFFIXES
+
 __version__ = "0.1.0"
+# The library of code on Python objects (csrc/py).  Object layouts are compiled in and differ between interpreters (a
+# str's at 3.12), so each has a file of its own.
+PY_LIBRARY = "liballie_py" + EXTENSION_SUFFIXES[0]
 
 _EXPORTS = {
     "UCITokenizer": "allie_b200.data", "Game": "allie_b200.data", "load_data": "allie_b200.data",

@@ -21,6 +21,8 @@ import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
+import allie_b200
+
 ROOT = Path(__file__).resolve().parent
 CSRC = ROOT / "csrc"
 LIB = ROOT / "lib"
@@ -103,18 +105,12 @@ def build_host(force: bool = False) -> Path | None:
     return out
 
 
-def py_library() -> str:
-    """Name of the library of code on Python objects.  Object layouts are compiled in and differ between
-    interpreters (a str's at 3.12), so each has a file of its own."""
-    return "liballie_py" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
-
-
 def build_py(force: bool = False) -> Path | None:
     """``csrc/py``: code that walks Python objects, for this interpreter.  Optional: where it cannot be built (None;
     no interpreter headers, no source, no compiler) the Python statements of the same rules serve."""
     src = CSRC / "py" / "tokens.cpp"
     include = Path(sysconfig.get_paths()["include"])
-    out = LIB / py_library()
+    out = LIB / allie_b200.PY_LIBRARY
     if not src.exists():                 # a copy without it keeps what was built elsewhere
         return out if out.exists() else None
     if not (include / "Python.h").exists():

@@ -28,10 +28,13 @@ from array import array
 from dataclasses import dataclass
 from functools import cached_property, lru_cache
 from itertools import repeat
+from pathlib import Path
 from typing import Any, Sequence
 
 import numpy as np
 import torch
+
+import allie_b200
 
 from .moves import CHESS_MOVES
 
@@ -149,9 +152,7 @@ def json_to_partial_game(d: dict, halfmove: int) -> Game:
 @lru_cache(maxsize=None)
 def _native_tokens():
     """The native tokenizer call, or None where it has not been built for this interpreter."""
-    from . import build
-
-    path = build.LIB / build.py_library()
+    path = Path(allie_b200.__file__).resolve().parent / "lib" / allie_b200.PY_LIBRARY
     if not path.exists():
         return None
     fn = ctypes.PyDLL(str(path)).allie_token_rows

@@ -6,7 +6,7 @@ from pathlib import Path
 
 import pytest
 
-from allie_b200 import build
+from allie_b200 import PY_LIBRARY, build
 
 ROOT = Path(__file__).resolve().parent.parent
 
@@ -34,7 +34,7 @@ def test_the_optional_library_does_not_stop_the_build(trouble, tmp_path, monkeyp
     for name, value in (("CSRC", csrc), ("LIB", lib), ("OBJ", lib / "obj")):
         monkeypatch.setattr(build, name, value)
     if trouble == "no source, built before":
-        (lib / build.py_library()).write_bytes(b"")
+        (lib / PY_LIBRARY).write_bytes(b"")
     if trouble == "no compiler":
         monkeypatch.setenv("CXX", str(tmp_path / "none"))
     built = []
@@ -56,7 +56,7 @@ def test_a_library_of_another_interpreter_is_not_loaded(suffix, monkeypatch):
     try:
         assert data._native_tokens() is not None
         data._native_tokens.cache_clear()
-        monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name: suffix)
+        monkeypatch.setattr("allie_b200.PY_LIBRARY", "liballie_py" + suffix)
         assert data._native_tokens() is None
     finally:
         data._native_tokens.cache_clear()
