@@ -3,8 +3,8 @@
 // UCITokenizer.token_ids: 17 us per game of 150 plies against 2 here, which is what a batch of a few hundred
 // prompts waits for before its first kernel.
 //
-// A move of the usual form (two squares, an optional promotion piece) is looked up by its squares in a
-// table that the tokenizer lays out once; any other string through the tokenizer's dictionary.  A game
+// Ids come from the tokenizer's dictionary as it is at the call.  Where a call has many moves, those of the usual form
+// (two squares, an optional promotion piece) are looked up by their squares in a table laid out from it.  A game
 // that is not plain (other types than the usual ones, anything the Python rules would refuse) is
 // left to the Python statement: its entry of `lens` is -1 and it adds nothing to the ids.
 #define PY_SSIZE_T_CLEAN
@@ -36,10 +36,29 @@ inline int move_index(const Py_UCS1* s, Py_ssize_t n) {
   return promo * 4096 + static_cast<int>((a * 8 + b) * 64 + c * 8 + d);
 }
 
+constexpr long TABLE_FROM = 2048;          // moves looked up one by one before a table is worth its layout
+
 struct Tokens {
   PyObject *ids, *outcomes;                // dictionaries: token -> id, outcome -> mask
-  const int32_t* table;
   long unk, vocab, resigned, eos;
+  std::vector<int32_t> table;              // by move_index; -1: ask the dictionary
+  long asked = 0;                          // moves so far
+
+  // (Left empty when a key is no plain string: one equal to a move could be among those.)
+  void lay_out() {
+    std::vector<int32_t> t(5 * 4096, static_cast<int32_t>(unk));
+    PyObject *k, *v;
+    Py_ssize_t at = 0;
+    while (PyDict_Next(ids, &at, &k, &v)) {
+      if (!PyUnicode_CheckExact(k)) return;
+      const int m = PyUnicode_IS_COMPACT_ASCII(k) ? move_index(PyUnicode_1BYTE_DATA(k), PyUnicode_GET_LENGTH(k)) : -1;
+      if (m < 0) continue;
+      const long x = PyLong_CheckExact(v) ? PyLong_AsLong(v) : -1;
+      if (x == -1) PyErr_Clear();
+      t[m] = x < 0 || x > 0x7fffffff ? -1 : static_cast<int32_t>(x);
+    }
+    table.swap(t);
+  }
 
   // id of a token in the dictionary, `unk` without one; false when Python raised or the id is no small int
   bool lookup(PyObject* token, uint32_t* out) const {
@@ -66,7 +85,7 @@ struct Tokens {
   }
 
   // appends the ids of a plain game; false (and possibly a pending exception) for any other
-  bool game(PyObject* g, std::vector<uint32_t>& row) const {
+  bool game(PyObject* g, std::vector<uint32_t>& row) {
     if (!rating(g, "white_elo", row) || !rating(g, "black_elo", row)) return false;
     Ref tc(PyObject_GetAttrString(g, "time_control"));
     uint32_t id;
@@ -83,8 +102,10 @@ struct Tokens {
       int overflow = 0;
       const long long sec = PyLong_AsLongLongAndOverflow(t, &overflow);
       if (overflow > 0 || (overflow == 0 && sec >= 0xFFFF)) return false;
-      const int k = PyUnicode_IS_COMPACT_ASCII(m) ? move_index(PyUnicode_1BYTE_DATA(m), PyUnicode_GET_LENGTH(m)) : -1;
-      if (k >= 0) id = static_cast<uint32_t>(table[k]);
+      if (++asked == TABLE_FROM) lay_out();
+      const int k = !table.empty() && PyUnicode_IS_COMPACT_ASCII(m)
+                        ? move_index(PyUnicode_1BYTE_DATA(m), PyUnicode_GET_LENGTH(m)) : -1;
+      if (k >= 0 && table[k] >= 0) id = static_cast<uint32_t>(table[k]);
       else if (!lookup(m, &id)) return false;
       row.push_back(id);
     }
@@ -106,14 +127,14 @@ struct Tokens {
 // games: list.  Returns (ids, lens): the ids & 0x3fff of all plain games behind one another, each cut to
 // max_length, as bytes of uint32; and a count per game as bytes of int32 (-1: not plain).  Null with an
 // exception set when memory runs out.
-extern "C" PyObject* allie_token_rows(PyObject* games, PyObject* ids, PyObject* outcomes, const int32_t* table,
-                                      long unk, long vocab, long resigned, long eos, long max_length) {
+extern "C" PyObject* allie_token_rows(PyObject* games, PyObject* ids, PyObject* outcomes, long unk,
+                                      long vocab, long resigned, long eos, long max_length) {
   if (!PyList_CheckExact(games) || !PyDict_CheckExact(ids) || !PyDict_CheckExact(outcomes) || max_length < 0) {
     PyErr_SetString(PyExc_TypeError, "a list of games and two dictionaries expected");
     return nullptr;
   }
   try {
-    const Tokens tok{ids, outcomes, table, unk, vocab, resigned, eos};
+    Tokens tok{ids, outcomes, unk, vocab, resigned, eos};
     std::vector<uint32_t> all, row;
     std::vector<int32_t> lens;
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(games); ++i) {      // attribute access may run Python code

@@ -157,15 +157,8 @@ def _native_tokens():
         return None
     fn = ctypes.PyDLL(str(path)).allie_token_rows
     fn.restype = ctypes.py_object
-    fn.argtypes = [ctypes.py_object] * 3 + [ctypes.c_void_p] + [ctypes.c_long] * 5
+    fn.argtypes = [ctypes.py_object] * 3 + [ctypes.c_long] * 5
     return fn
-
-
-@lru_cache(maxsize=None)
-def _move_indices() -> np.ndarray:
-    square = {f + r: 8 * i + j for i, f in enumerate("abcdefgh") for j, r in enumerate("12345678")}
-    piece = {"": 0, "q": 1, "r": 2, "b": 3, "n": 4}
-    return np.array([4096 * piece[m[4:]] + 64 * square[m[:2]] + square[m[2:4]] for m in CHESS_MOVES])
 
 
 class UCITokenizer:
@@ -248,13 +241,16 @@ class UCITokenizer:
     def token_rows(self, games: Sequence[Game]) -> list[np.ndarray]:
         """``[token_ids(g)[:max_length] for g in games]``, read-only, from one native call
         (``csrc/py/tokens.cpp``); games it does not take go through :meth:`token_ids`."""
-        usual = type(self) is UCITokenizer and type(self.max_length) is int and self.max_length >= 0
+        own_ids = self.unk_token_id, self.resigned_token_id, self.eos_token_id
+        usual = (type(self) is UCITokenizer and type(self.max_length) is int and self.max_length >= 0
+                 and type(self.token_to_id) is dict and all(type(i) is int and 0 <= i < 1 << 31 for i in own_ids))
         native = _native_tokens() if usual else None
         if native is None:
             return [self.token_ids(g)[: self.max_length] for g in games]
         games = list(games)
-        ids, lens = native(games, self.token_to_id, OUTCOME_MASKS, self._move_table.ctypes.data, self.unk_token_id,
-                           len(self), self.resigned_token_id, self.eos_token_id, self.max_length)
+        unk, resigned, eos = own_ids
+        ids, lens = native(games, self.token_to_id, OUTCOME_MASKS, unk, len(self), resigned, eos,
+                           min(self.max_length, (1 << 31) - 1))
         ids, rows, o = np.frombuffer(ids, dtype=np.uint32), [], 0
         for g, n in zip(games, np.frombuffer(lens, dtype=np.int32).tolist()):
             if n < 0:
@@ -263,14 +259,6 @@ class UCITokenizer:
                 rows.append(ids[o:o + n])
                 o += n
         return rows
-
-    @cached_property
-    def _move_table(self) -> np.ndarray:
-        """Ids of all strings of two squares and an optional promotion piece, in the order of ``move_index``
-        (``csrc/py/tokens.cpp``); the moves are the only tokens of that form and their ids the first."""
-        table = np.full(5 * 4096, self.unk_token_id, dtype=np.int32)
-        table[_move_indices()] = np.arange(len(CHESS_MOVES), dtype=np.int32)
-        return table
 
     def pad(self, seq: list[int]) -> list[int]:
         out = seq + [self.pad_token_id] * (self.max_length - len(seq))

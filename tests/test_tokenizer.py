@@ -163,3 +163,47 @@ def test_native_token_rows_match_the_python_rules(odd, length):
         return
     got = tok.token_rows(games)
     assert [g.tolist() for g in got] == [w.tolist() for w in want] and all(g.dtype == np.uint32 for g in got)
+
+
+class _Dict(dict):
+    pass
+
+
+def _edited(tok):
+    tok.token_rows([_game(["e2e4"], [1])])           # nothing of an earlier call is kept
+    tok.token_to_id["e2e4"] = 7
+
+
+_TOKENIZERS = {
+    "plain": ({}, None), "no cut": (dict(max_length=1 << 70), None), "unknown token is a move": (dict(unk_token="e2e4"), None),
+    "special token of a move's form": (dict(bos_token="a1a1", pad_token="a1a1q"), None), "edited ids": ({}, _edited),
+    "dictionary subclass": ({}, lambda t: setattr(t, "token_to_id", _Dict(t.token_to_id))),
+    "a key that is no string": ({}, lambda t: t.token_to_id.update({3: 5, _Str("b2b2"): 6})),
+    "ids of other types": ({}, lambda t: setattr(t, "token_to_id", {k: np.int64(v) for k, v in t.token_to_id.items()})),
+    "wide id": ({}, lambda t: t.token_to_id.update(e2e4=1 << 31)), "wide special id": ({}, lambda t: setattr(t, "eos_token_id", 1 << 70)),
+}
+
+
+@pytest.mark.parametrize("games", [1, 40])
+@pytest.mark.parametrize("form", _TOKENIZERS)
+def test_native_token_rows_follow_the_tokenizer(form, games):
+    """Whatever the vocabulary looks like, for a few moves (looked up one by one) and many (by table)."""
+    from allie_b200 import build, data
+
+    if build.build_py() is None:
+        pytest.skip("no interpreter headers")
+    data._native_tokens.cache_clear()
+    kw, change = _TOKENIZERS[form]
+    tok = UCITokenizer(**{**dict(max_length=512, vocab_size_multiple_of=128), **kw})
+    if change:
+        change(tok)
+    rng = np.random.default_rng(games)
+    odd = ["e2e4", "a1a1", "a1a1q", "b2b2", "z9z9", "h2h1n"]
+    rows = [_game(odd + [CHESS_MOVES[i] for i in rng.integers(0, NUM_CHESS_MOVES, size=90)] + odd, [1] * 102) for _ in range(games)]
+    try:
+        want = [tok.token_ids(g)[: tok.max_length].tolist() for g in rows]
+    except Exception as e:
+        with pytest.raises(type(e)):
+            tok.token_rows(rows)
+        return
+    assert [r.tolist() for r in tok.token_rows(rows)] == want
