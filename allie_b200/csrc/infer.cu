@@ -82,8 +82,8 @@ struct AbInfer {
 };
 
 int ab_layernorm_fwd(const float*, const float*, const float*, void*, float*, float*, int, int, float, int, cudaStream_t);
-int ab_layernorm_fwd_dependent(const float*, const float*, const float*, void*, float*, float*, int, int, float, int,
-                               cudaStream_t);
+int ab_layernorm_fwd_ahead(const float*, const float*, const float*, void*, float*, float*, int, int, float, int,
+                           cudaStream_t);
 int ab_embed_fwd(const int*, const int*, const float*, const float*, const float*, float*, int, int, int,
                  unsigned long long, unsigned int, unsigned int, cudaStream_t);
 int ab_heads_fwd(const void*, const float*, const float*, const float*, const float*, const float*, const float*,
@@ -103,8 +103,7 @@ int ab_infer_last(const AbInfer* p, const AbInferLayer* layers, cudaStream_t str
   const int dep = a.M <= 256;
   auto norm = [&](const float* x, const float* w, const float* b, void* y, int M) {
     ++launched;
-    return (dep ? ab_layernorm_fwd_dependent : ab_layernorm_fwd)(x, w, b, y, nullptr, nullptr, M, a.d, a.eps, a.rms,
-                                                                 stream);
+    return (dep ? ab_layernorm_fwd_ahead : ab_layernorm_fwd)(x, w, b, y, nullptr, nullptr, M, a.d, a.eps, a.rms, stream);
   };
   // No contraction is split: each output is one chain of products whatever the batch, so a game's
   // evaluation does not depend on the games beside it.

@@ -13,8 +13,8 @@ namespace ab {
 constexpr int LN_WARPS = 8;
 
 // NV = d / 128 float4s per lane, known at compile time: with a bound checked per float4 every load waited for
-// the one before it.  AHEAD (dependent launches of a few hundred rows): gamma and beta, which are weights and may
-// lie in memory, are fetched while the kernel before is still running.
+// the one before it.  AHEAD (dependent launches of a few hundred rows whose caller says that the kernel before does not
+// write gamma and beta): these, which may lie in memory, are fetched while that kernel is still running.
 template <int NV, bool AHEAD>
 __global__ void __launch_bounds__(LN_WARPS * 32)
 ln_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
@@ -350,6 +350,7 @@ static int ln_block_warps(int M) {
   return want < ab::LN_WARPS ? want : ab::LN_WARPS;
 }
 
+// dependent: 1 = programmatic dependent, 2 = and gamma and beta may be read before the kernel before has finished
 template <int NV>
 static int launch_ln_fwd(int dependent, const float* x, const float* gamma, const float* beta, void* y, float* mean,
                          float* rstd, int M, int d, float eps, int rms, cudaStream_t stream) {
@@ -375,18 +376,26 @@ static int launch_ln_fwd(int dependent, const float* x, const float* gamma, cons
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, ln_fwd_kernel<NV, true>, x, gamma, beta, (__nv_bfloat16*)y, mean, rstd, M, eps, rms);
+  auto kern = dependent == 2 ? ln_fwd_kernel<NV, true> : ln_fwd_kernel<NV, false>;
+  return (int)cudaLaunchKernelEx(&cfg, kern, x, gamma, beta, (__nv_bfloat16*)y, mean, rstd, M, eps, rms);
 }
 
 extern "C" {
 
 // d must be a multiple of 128 and at most 2048.
 // Same as ab_layernorm_fwd, launched as a programmatic dependent of the kernel before it in the
-// stream (its launch overlaps that kernel's tail; it waits for it before reading x).
+// stream (its launch overlaps that kernel's tail; it waits for it before reading anything).
 int ab_layernorm_fwd_dependent(const float* x, const float* gamma, const float* beta, void* y, float* mean,
                                float* rstd, int M, int d, float eps, int rms, cudaStream_t stream) {
   if (d < 128 || d % 128 != 0 || d > 2048 || M <= 0) return -1;
   return launch_ln_fwd<1>(1, x, gamma, beta, y, mean, rstd, M, d, eps, rms, stream);
+}
+
+// The same for gamma and beta that the kernel before does not write: they are read while it is still running.
+int ab_layernorm_fwd_ahead(const float* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
+                           int M, int d, float eps, int rms, cudaStream_t stream) {
+  if (d < 128 || d % 128 != 0 || d > 2048 || M <= 0) return -1;
+  return launch_ln_fwd<1>(2, x, gamma, beta, y, mean, rstd, M, d, eps, rms, stream);
 }
 
 int ab_layernorm_fwd(const float* x, const float* gamma, const float* beta, void* y, float* mean,

@@ -18,11 +18,15 @@ def _ck(rc: int, name: str) -> None:
 
 
 # ------------------------------------------------------------------ norms ---
-def layernorm_fwd(x, gamma, beta, y, mean, rstd, eps: float, rms: bool = False, dependent: bool = False) -> None:
+def layernorm_fwd(x, gamma, beta, y, mean, rstd, eps: float, rms: bool = False, dependent: bool = False,
+                  weights_ready: bool = False) -> None:
     """``dependent``: launch as a programmatic dependent of the previous kernel in the stream (the
-    launch overlaps that kernel's tail; the kernel waits for it before it reads ``x``)."""
+    launch overlaps that kernel's tail; the kernel waits for it before it reads anything).  ``weights_ready``, with
+    it: the previous kernel does not write ``gamma`` and ``beta``, which are then read before that wait."""
     M, d = x.shape
-    fn = _lib.cuda().ab_layernorm_fwd_dependent if dependent else _lib.cuda().ab_layernorm_fwd
+    lib = _lib.cuda()
+    fn = (lib.ab_layernorm_fwd if not dependent else
+          lib.ab_layernorm_fwd_ahead if weights_ready else lib.ab_layernorm_fwd_dependent)
     _ck(fn(ptr(x), ptr(gamma), ptr(beta), ptr(y), ptr(mean), ptr(rstd),
            c_int(M), c_int(d), c_float(eps), c_int(int(rms)), stream_ptr()), "ab_layernorm_fwd")
 

@@ -137,7 +137,7 @@ class KVLeafEvaluator:
         few = self.few and self._launch_few(x)
         for l, Ly in enumerate(eng.layers if not few else ()):
             K.layernorm_fwd(x, Ly["ln1_w"][0], Ly["ln1_b"][0], self.ln, self.stat[0], self.stat[1], eps, eng.rms,
-                            dependent=pdl)
+                            dependent=pdl, weights_ready=True)
             gemm(self.ln, Ly["qkv_w"][1], b_mn=True, out=self.qkv, bias=Ly["qkv_b"][0], dependent=pdl,
                  then=Ly["o_w"][1])
             rc = lib.ab_decode_attn(ptr(self.qkv), ptr(self.kc[l]), ptr(self.vc[l]), ptr(self.view(rd, "active")),
@@ -152,13 +152,13 @@ class KVLeafEvaluator:
             gemm(self.att, Ly["o_w"][1], b_mn=True, out=x, bias=Ly["o_b"][0], resid=x, dependent=pdl,
                  then=Ly["fc_w"][1])
             K.layernorm_fwd(x, Ly["ln2_w"][0], Ly["ln2_b"][0], self.ln, self.stat[0], self.stat[1], eps, eng.rms,
-                            dependent=pdl)
+                            dependent=pdl, weights_ready=True)
             gemm(self.ln, Ly["fc_w"][1], b_mn=True, out=self.act, bias=Ly["fc_b"][0], act=3, dependent=pdl,
                  then=Ly["pr_w"][1])
             gemm(self.act, Ly["pr_w"][1], b_mn=True, out=x, bias=Ly["pr_b"][0], resid=x, dependent=pdl,
                  then=eng.layers[l + 1]["qkv_w"][1] if l + 1 < cfg.n_layer else eng.wte[1])
         K.layernorm_fwd(x, eng.lnf_w[0], eng.lnf_b[0], self.h, self.stat[0], self.stat[1], eps, eng.rms,
-                        dependent=pdl)
+                        dependent=pdl, weights_ready=True)
         gemm(self.h, eng.wte[1], b_mn=False, out=self.logits, dependent=pdl)
         has_heads = eng.reg is not None
         if has_heads:

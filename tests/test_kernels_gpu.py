@@ -308,10 +308,10 @@ def test_fused_lmhead_cross_entropy_matches_fp32(M, V, K):
     assert (dlogits[labels < 0].float() == 0).all()
 
 
-@pytest.mark.parametrize("dependent", [False, True])
+@pytest.mark.parametrize("dependent,ready", [(False, False), (True, False), (True, True)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("d", list(range(128, 2049, 128)))
-def test_layernorm_forward_widths(d, rms, dependent):
+def test_layernorm_forward_widths(d, rms, dependent, ready):
     """Every width, with and without the parameters fetched ahead; one row, more rows than SMs, two rows for a
     block's last warp and none.  bf16 results: half a unit in the last place of a value of up to 6."""
     from allie_b200.ops import kernels as K
@@ -322,7 +322,8 @@ def test_layernorm_forward_widths(d, rms, dependent):
         g, b = torch.randn(d, device=DEV), torch.randn(d, device=DEV)
         y = torch.empty(M, d, device=DEV, dtype=torch.bfloat16)
         mean, rstd = torch.empty(M, device=DEV), torch.empty(M, device=DEV)
-        K.layernorm_fwd(x, g, None if rms else b, y, mean, rstd, 1e-5, rms, dependent=dependent)
+        _done()                                  # with `ready`, no kernel in flight may be writing g and b
+        K.layernorm_fwd(x, g, None if rms else b, y, mean, rstd, 1e-5, rms, dependent=dependent, weights_ready=ready)
         _done()
         x64 = x.double()
         mu = torch.zeros(M, 1, device=DEV, dtype=torch.float64) if rms else x64.mean(1, keepdim=True)
@@ -330,3 +331,27 @@ def test_layernorm_forward_widths(d, rms, dependent):
         want = (x64 - mu) * r * g.double() + (0 if rms else b.double())
         assert ((y.double() - want).abs() <= want.abs() * 2 ** -8 + 1e-5).all()
         assert torch.allclose(rstd.double(), r[:, 0], rtol=1e-5) and torch.allclose(mean.double(), mu[:, 0], atol=1e-5)
+
+
+@pytest.mark.parametrize("d", [128, 1024, 2048])
+def test_dependent_layernorm_waits_for_its_weights(d):
+    """Gamma and beta that the kernel before writes (a long contraction that lets its dependents start at once)
+    are read when it has written them."""
+    from allie_b200.ops import kernels as K
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(d)
+    a, w = torch.randn(2, 16384, device=DEV).bfloat16(), (torch.randn(16384, d, device=DEV) * 0.01).bfloat16()
+    x = torch.randn(64, d, device=DEV)
+    gb = torch.zeros(2, d, device=DEV)
+    y, want = (torch.empty(64, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    mean, rstd = torch.empty(64, device=DEV), torch.empty(64, device=DEV)
+    for _ in range(3):
+        gb.zero_()
+        gemm(a, w, b_mn=True, out=gb)
+        K.layernorm_fwd(x, gb[0], gb[1], y, mean, rstd, 1e-5, dependent=True)
+    _done()
+    assert float(gb.abs().min(0).values.max()) > 0
+    K.layernorm_fwd(x, gb[0], gb[1], want, mean, rstd, 1e-5)
+    _done()
+    assert torch.equal(y, want)
