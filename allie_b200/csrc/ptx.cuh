@@ -276,30 +276,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc], bf16 inputs, fp32 accumulate.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Same with A in TMEM (lane = row, two K-adjacent bf16 values per 32-bit column).
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+// D[tmem] (+)= A[smem desc] * B[smem desc], bf16 inputs, fp32 accumulate; by the warp's elected lane.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -312,6 +289,7 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
+// Same with A in TMEM (lane = row, two K-adjacent bf16 values per 32-bit column).
 __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -324,6 +302,7 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, u
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
+// Arrive on `bar` once every tcgen05.mma issued so far by the elected lane is done.
 __device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t lead) {
   asm volatile(
       "{\n\t"
@@ -332,13 +311,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t lead) {
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
       "}\n"
       ::"r"(smem_u32(bar)), "r"(lead)
-      : "memory");
-}
-// Arrive on `bar` once every tcgen05.mma issued so far by this thread is done.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
       : "memory");
 }
 // Each thread of the warp reads 32 consecutive fp32 columns of its own TMEM
@@ -434,26 +406,6 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                               uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrive on the barrier at `bar_cluster_addr` (either CTA of the pair) once every pair MMA issued
-// so far by this thread is done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          bar_cluster_addr)
-      : "memory");
-}
-
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int x, int y,
                                                  uint32_t lead) {
   asm volatile(
@@ -475,6 +427,8 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, 
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
+// Arrive on the barrier at `bar_cluster_addr` (either CTA of the pair) once every pair MMA issued
+// so far by the elected lane is done.
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr, uint32_t lead) {
   asm volatile(
       "{\n\t"
@@ -491,18 +445,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr, uint
 // a TMA load with CU_TENSOR_MAP_SWIZZLE_128B produces).  Field positions:
 // start>>4 [0,14), LBO>>4 [16,30), SBO>>4 [32,46), version=1 [46,48),
 // layout type [61,64) with 2 = SWIZZLE_128B.
-__device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_t lbo_bytes,
-                                                     uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-// The same for `base` + `off`, both multiples of 16: neighbouring descriptors differ by one addition to the low
-// word (shared memory ends below 2^18, so nothing carries out of the address field).
+// For `base` + `off`, both multiples of 16: neighbouring descriptors differ by one addition to the low word (shared
+// memory ends below 2^18, so nothing carries out of the address field).
 __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t base, uint32_t off, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   const uint32_t lo = (base >> 4) + ((off >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16));
   const uint32_t hi = ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) | (2u << 29);
