@@ -217,10 +217,12 @@ def test_attention_fwd_against_64_bits(hd, T, kind, p):
     assert (err <= (2 * 2 ** -8 + 2 ** -13) * size + 1e-7).all(), float((err / (size + 1e-9)).max())
 
 
-@pytest.mark.parametrize("B,T,H,hd,p", [(2, 384, 2, 128, 0.1), (1, 520, 2, 128, 0.0), (2, 1000, 1, 128, 0.0), (2, 416, 2, 64, 0.1)])
+@pytest.mark.parametrize("B,T,H,hd,p", [(2, 384, 2, 128, 0.1), (1, 520, 2, 128, 0.0), (2, 1000, 1, 128, 0.0), (2, 416, 2, 64, 0.1),
+                                        # sequences that end inside a tile, enough slices for the persistent walk
+                                        (20, 160, 16, 64, 0.1), (20, 330, 16, 64, 0.0), (20, 416, 16, 64, 0.1)])
 def test_attention_bwd_over_several_key_tiles(B, T, H, hd, p):
-    """Gradients against autograd in 64 bits with the stored mask, three key tiles and more.  P, dS and the
-    results are rounded to bf16: under 1 % in the 2-norm."""
+    """Gradients against autograd in 64 bits with the stored mask, several key tiles, by all three
+    schedules.  P, dS and the results are rounded to bf16: under 1 % in the 2-norm."""
     from allie_b200.ops import _lib
     from allie_b200.ops.attention import attention_bwd, attention_fwd
 
@@ -242,9 +244,12 @@ def test_attention_bwd_over_several_key_tiles(B, T, H, hd, p):
     (probs @ v).transpose(1, 2).reshape(B * T, d).backward(dout.double())
     dqkv = torch.full((B * T, 3 * d), float("nan"), device=dev, dtype=torch.bfloat16)
     acc = torch.zeros(B * T, d, device=dev) if hd == 64 else None
+    launched = _lib.LAUNCHES
     attention_bwd(qkv, out, lse, dout, dqkv, delta, B, T, H, hd, p, 5, 1, bits, acc)
     torch.cuda.synchronize()
     _lib.check_status()
+    # row sums of dO * O, and the walk; two kernels for heads of 128; a grid of key tiles and its conversion
+    assert _lib.LAUNCHES - launched == (2 if B == 20 else 3)
     for i in range(3):
         a, b = dqkv[:, i * d:(i + 1) * d].double(), leaf.grad[:, i * d:(i + 1) * d]
         assert float((a - b).norm() / b.norm()) < 1e-2, "qkv"[i]
