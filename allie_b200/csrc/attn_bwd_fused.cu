@@ -858,7 +858,10 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
   // x 12 heads 138 and 90, 16 x 512 x 16 118 and 84, 25 x 400 x 12 138 and 132, 8 x 256 x 4 32 and 22.
   const long long slice = static_cast<long long>(nt) * (nt + 1) / 2;
   const long long grid_pairs = std::max(nt + 2ll, bh * (slice + 2 * nt) / 148) + 4;
-  // (Measured from 32 slices up.  A tenth in favour of the grid: 30 x 1000 x 10, level by this count, 360 and 387.)
+  // A tenth in favour of the grid: 30 x 1000 x 10, level by this count, 360 and 387 (it also leaves 4 x 512 x 16 there,
+  // 48 and 45).  Under 32 slices the grid whatever the count says, which is wrong for three key tiles: 384 keys
+  // and 1 to 5 slices 28 and 31 us, level from 16 on.  For one and two tiles the walk would be the faster there, too,
+  // as above the line: 4 slices of 128 keys 24 and 12, of 256 keys 26 and 21.
   const bool walk = bh >= 32 && 10 * ((bh + 147) / 148 * slice + 1) <= 9 * grid_pairs;
   if (mode == 1 || !fits || (mode == 0 && !walk)) {
     constexpr int SMEM = 6 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;

@@ -540,7 +540,7 @@ decode_few_kernel(const DecodeFewArgs g) {
         for (int c = 0; c < chunks; ++c) {
           if ((c & 1) == (warp >> 2)) {            // warp-uniform
             // After a wait that ran out a lane goes on like the others, with whatever the slot holds: ldmatrix and
-            // the MMAs are the whole warp's.  (A vote on the answer costs 7 us of a step's 640.)
+            // the MMAs are the whole warp's.  (A vote on the answer cost a step 7 us.)
             if (good && !mbar_wait(&full[slot], par, abort_flag)) {
               good = false;
               *abort_flag = ST_TIMEOUT_FULL;

@@ -771,7 +771,9 @@ static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue
   // narrow tiles also for skinny problems (decode steps with a few hundred rows): twice the CTAs
   const bool narrow = (N <= 128) || (M <= 256);
   // A few hundred rows against a wide weight matrix (decode steps): the time goes into streaming
-  // the weights, so the columns are cut into 64-wide tiles to put twice as many SMs on them.
+  // the weights, so the columns are cut into 64-wide tiles to put twice as many SMs on them.  Not for a
+  // contraction whose length is a device value: it ends with a whole stage, and here that is 128 columns instead of 64
+  // that have to be zero past the limit.
   if (M <= 256 && N >= 1024 && !a_mn && !ep.k_limit) p.kernel = 64;
   else if (one_wave) p.kernel = tiles(64) <= max_ctas ? 64 : 128;
   else if (narrow)   p.kernel = 128;

@@ -11,8 +11,9 @@
 // Larger vocabularies (lmhead_ce_kernel): a CTA walks the vocabulary in tiles of 256 columns, TWICE: the first
 // sweep keeps a running maximum and sum of exponentials per row (online softmax across the N tiles) and picks
 // up the label's logit; the second recomputes every tile on the tensor cores.  2048 columns, rows x width, that
-// form and the cluster: 300 x 512 75 and 28 us, 2048 x 256 58 and 24, 12136 x 768 106 and 87, 32768 x 1024 261
-// and 242.
+// form (as it was before the cluster, its loads and MMAs issued by one lane) and the cluster: 300 x 512 70 and 25 us,
+// 2048 x 256 53 and 21, 12136 x 768 99 and 72, 32768 x 1024 248 and 202.  Where the line lies, both as they
+// are: 2048 x 256 with 4096 columns by cluster 39 us, with 4104 by two sweeps 98.
 //
 // Same pipeline as the plain GEMM (gemm_tc.cu): warp 0 TMA producer, warp 1 MMA issuer, 16 epilogue
 // warps (four per TMEM lane quarter, 64 columns each), two accumulators in TMEM so the epilogue of
@@ -583,7 +584,8 @@ static int launch_lmhead_cluster(const CUtensorMap& tmA, const CUtensorMap& tmB,
 }  // namespace ab
 
 // h: [M, K] bf16 (final hidden states), wte: [V, K] bf16, labels: [M] int (already shifted, < 0 =
-// ignored), dlogits: [M, V] bf16 out.  K, V multiples of 8.
+// ignored), dlogits: [M, V] bf16 out.  K, V multiples of 8.  max_ctas bounds the CTAs of the two-sweep form; the
+// clusters, one per 128 rows, are launched all at once.
 extern "C" int ab_lmhead_ce(const void* h, long long ldh, const void* wte, long long ldw, const int* labels,
                             const int* n_valid, float coef, void* dlogits, long long ldo, float* loss_acc,
                             int M, int V, int K, int max_ctas, int* status, cudaStream_t stream) {

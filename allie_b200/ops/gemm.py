@@ -97,7 +97,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             and act == 0 and M <= 512 and m_limit is None and k_limit is None):
         # Skinny in-place residual update (decode steps): x += a @ b + bias.  A few output tiles
         # with a long K loop leave most SMs idle, so the contraction is split over more CTAs and
-        # the partial products are reduce-added into x; the first split adds the bias.
+        # the partial products are reduce-added into x; the first split adds the bias.  128 units are aimed at,
+        # counted in 128-column tiles; where the launch takes 64-column ones (M <= 256, N >= 1024) these are twice as
+        # many, two waves.  Per launch of a chain, us, so and with 128 units of those: 256 x 1024 x 4096 7.25 and 7.42,
+        # 128 x 1024 x 4096 6.40 and 6.06, 256 x 1280 x 1280 6.14 and 5.46, 200 x 1536 x 6144 11.6 and 12.5,
+        # 17 x 1152 x 4608 5.71 and 6.06: neither is ahead.
         tiles = -(-M // 128) * -(-N // 128)
         ks = max(1, min(K // 256, 128 // max(tiles, 1)))
         if ks > 1:
