@@ -3,8 +3,9 @@
 // UCITokenizer.token_ids: 17 to 23 us per game of 150 plies (strings hashed before or not) against 3 to 4 here in a
 // batch of 256, which is what a batch of a few hundred prompts waits for before its first kernel.
 //
-// Ids come from the tokenizer's dictionary as it is at the call.  Where a call has many moves, those of the usual form
-// (two squares, an optional promotion piece) are looked up by their squares in a table laid out from it.  A game
+// Ids are the tokenizer's dictionary's as it is at the call.  Moves of the usual form (two squares, an optional promotion
+// piece) come from a table by their squares, laid out again whenever the dictionary has changed; any other string is
+// looked up.  (All of them looked up, a batch of 30 games waits 30 us longer: the dictionary is not in the caches.)  A game
 // that is not plain (other types than the usual ones, anything the Python rules would refuse) is
 // left to the Python statement: its entry of `lens` is -1 and it adds nothing to the ids.
 #define PY_SSIZE_T_CLEAN
@@ -36,30 +37,42 @@ inline int move_index(const Py_UCS1* s, Py_ssize_t n) {
   return promo * 4096 + static_cast<int>((a * 8 + b) * 64 + c * 8 + d);
 }
 
-// Moves looked up one by one before a table is worth its layout: that takes 20 us, and a move 25 ns one by one (twice
-// that where its string was never hashed) and 13 by table.
-constexpr long TABLE_FROM = 2048;
+// A number that no other dictionary of this process and no other state of this one has; 0 where the interpreter keeps none
+inline uint64_t dict_version(PyObject* d) {
+#if PY_VERSION_HEX < 0x030D0000
+#pragma GCC diagnostic push
+#pragma GCC diagnostic ignored "-Wdeprecated-declarations"
+  return reinterpret_cast<PyDictObject*>(d)->ma_version_tag;
+#pragma GCC diagnostic pop
+#else
+  return 0;
+#endif
+}
+
+// Kept by the tokenizer between calls, all zero at first.
+struct MoveTable {
+  uint64_t version;                        // dict_version that the ids are of
+  int32_t id[5 * 4096];                    // by move_index; -1: ask the dictionary
+};
 
 struct Tokens {
   PyObject *ids, *outcomes;                // dictionaries: token -> id, outcome -> mask
   long unk, vocab, resigned, eos;
-  std::vector<int32_t> table;              // by move_index; -1: ask the dictionary
-  long asked = 0;                          // moves so far
+  MoveTable* table;
 
-  // (Left empty when a key is no plain string: one equal to a move could be among those.)
-  void lay_out() {
-    std::vector<int32_t> t(5 * 4096, static_cast<int32_t>(unk));
+  // 20 us
+  void lay_out(uint64_t version) const {
+    table->version = version;
+    for (int32_t& x : table->id) x = -1;
     PyObject *k, *v;
     Py_ssize_t at = 0;
     while (PyDict_Next(ids, &at, &k, &v)) {
-      if (!PyUnicode_CheckExact(k)) return;
-      const int m = PyUnicode_IS_COMPACT_ASCII(k) ? move_index(PyUnicode_1BYTE_DATA(k), PyUnicode_GET_LENGTH(k)) : -1;
-      if (m < 0) continue;
-      const long x = PyLong_CheckExact(v) ? PyLong_AsLong(v) : -1;
-      if (x == -1) PyErr_Clear();
-      t[m] = x < 0 || x > 0x7fffffff ? -1 : static_cast<int32_t>(x);
+      if (!PyUnicode_CheckExact(k) || !PyUnicode_IS_COMPACT_ASCII(k) || !PyLong_CheckExact(v)) continue;
+      const int m = move_index(PyUnicode_1BYTE_DATA(k), PyUnicode_GET_LENGTH(k));
+      int overflow = 0;
+      const long x = PyLong_AsLongAndOverflow(v, &overflow);
+      if (m >= 0 && !overflow && x >= 0 && x <= 0x7fffffff) table->id[m] = static_cast<int32_t>(x);
     }
-    table.swap(t);
   }
 
   // id of a token in the dictionary, `unk` without one; false when Python raised or the id is no small int
@@ -87,7 +100,7 @@ struct Tokens {
   }
 
   // appends the ids of a plain game; false (and possibly a pending exception) for any other
-  bool game(PyObject* g, std::vector<uint32_t>& row) {
+  bool game(PyObject* g, std::vector<uint32_t>& row) const {
     if (!rating(g, "white_elo", row) || !rating(g, "black_elo", row)) return false;
     Ref tc(PyObject_GetAttrString(g, "time_control"));
     uint32_t id;
@@ -97,6 +110,8 @@ struct Tokens {
     if (!moves.p || !secs.p || !PyList_CheckExact(moves.p) || !PyList_CheckExact(secs.p) ||
         PyList_GET_SIZE(moves.p) != PyList_GET_SIZE(secs.p))
       return false;
+    const uint64_t version = dict_version(ids);
+    if (version && version != table->version) lay_out(version);
     // exact strings and ints only from here on: no Python code runs that could change the lists
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(moves.p); ++i) {
       PyObject *m = PyList_GET_ITEM(moves.p, i), *t = PyList_GET_ITEM(secs.p, i);
@@ -104,10 +119,9 @@ struct Tokens {
       int overflow = 0;
       const long long sec = PyLong_AsLongLongAndOverflow(t, &overflow);
       if (overflow > 0 || (overflow == 0 && sec >= 0xFFFF)) return false;
-      if (++asked == TABLE_FROM) lay_out();
-      const int k = !table.empty() && PyUnicode_IS_COMPACT_ASCII(m)
+      const int k = version && PyUnicode_IS_COMPACT_ASCII(m)
                         ? move_index(PyUnicode_1BYTE_DATA(m), PyUnicode_GET_LENGTH(m)) : -1;
-      if (k >= 0 && table[k] >= 0) id = static_cast<uint32_t>(table[k]);
+      if (k >= 0 && table->id[k] >= 0) id = static_cast<uint32_t>(table->id[k]);
       else if (!lookup(m, &id)) return false;
       row.push_back(id);
     }
@@ -126,17 +140,17 @@ struct Tokens {
 
 }  // namespace
 
-// games: list.  Returns (ids, lens): the ids & 0x3fff of all plain games behind one another, each cut to
+// games: list; table: a MoveTable.  Returns (ids, lens): the ids & 0x3fff of all plain games behind one another, each cut to
 // max_length, as bytes of uint32; and a count per game as bytes of int32 (-1: not plain).  Null with an
 // exception set when memory runs out.
-extern "C" PyObject* allie_token_rows(PyObject* games, PyObject* ids, PyObject* outcomes, long unk,
-                                      long vocab, long resigned, long eos, long max_length) {
+extern "C" PyObject* allie_token_rows(PyObject* games, PyObject* ids, PyObject* outcomes, void* table,
+                                      long unk, long vocab, long resigned, long eos, long max_length) {
   if (!PyList_CheckExact(games) || !PyDict_CheckExact(ids) || !PyDict_CheckExact(outcomes) || max_length < 0) {
     PyErr_SetString(PyExc_TypeError, "a list of games and two dictionaries expected");
     return nullptr;
   }
   try {
-    Tokens tok{ids, outcomes, unk, vocab, resigned, eos};
+    const Tokens tok{ids, outcomes, unk, vocab, resigned, eos, static_cast<MoveTable*>(table)};
     std::vector<uint32_t> all, row;
     std::vector<int32_t> lens;
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(games); ++i) {      // attribute access may run Python code

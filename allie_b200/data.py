@@ -157,7 +157,7 @@ def _native_tokens():
         return None
     fn = ctypes.PyDLL(str(path)).allie_token_rows
     fn.restype = ctypes.py_object
-    fn.argtypes = [ctypes.py_object] * 3 + [ctypes.c_long] * 5
+    fn.argtypes = [ctypes.py_object] * 3 + [ctypes.c_void_p] + [ctypes.c_long] * 5
     return fn
 
 
@@ -249,8 +249,8 @@ class UCITokenizer:
             return [self.token_ids(g)[: self.max_length] for g in games]
         games = list(games)
         unk, resigned, eos = own_ids
-        ids, lens = native(games, self.token_to_id, OUTCOME_MASKS, unk, len(self), resigned, eos,
-                           min(self.max_length, (1 << 31) - 1))
+        ids, lens = native(games, self.token_to_id, OUTCOME_MASKS, self._move_table.ctypes.data, unk, len(self), resigned,
+                           eos, min(self.max_length, (1 << 31) - 1))
         ids, rows, o = np.frombuffer(ids, dtype=np.uint32), [], 0
         for g, n in zip(games, np.frombuffer(lens, dtype=np.int32).tolist()):
             if n < 0:
@@ -259,6 +259,14 @@ class UCITokenizer:
                 rows.append(ids[o:o + n])
                 o += n
         return rows
+
+    @cached_property
+    def _move_table(self) -> np.ndarray:
+        """What the native call keeps of ``token_to_id`` in this process (``MoveTable`` in ``csrc/py/tokens.cpp``)."""
+        return np.zeros(1 + 5 * 4096 // 2, dtype=np.uint64)
+
+    def __getstate__(self) -> dict:
+        return {k: v for k, v in self.__dict__.items() if k != "_move_table"}
 
     def pad(self, seq: list[int]) -> list[int]:
         out = seq + [self.pad_token_id] * (self.max_length - len(seq))

@@ -1,4 +1,7 @@
 """Tokenizer / vocabulary golden tests (CPU)."""
+import copy
+import pickle
+
 import numpy as np
 import pytest
 import torch
@@ -169,14 +172,18 @@ class _Dict(dict):
     pass
 
 
-def _edited(tok):
-    tok.token_rows([_game(["e2e4"], [1])])           # nothing of an earlier call is kept
-    tok.token_to_id["e2e4"] = 7
+def _edited(change):
+    def edit(tok):
+        tok.token_rows([_game(["e2e4"], [1])])       # the vocabulary changes after a first call
+        change(tok)
+    return edit
 
 
 _TOKENIZERS = {
     "plain": ({}, None), "no cut": (dict(max_length=1 << 70), None), "unknown token is a move": (dict(unk_token="e2e4"), None),
-    "special token of a move's form": (dict(bos_token="a1a1", pad_token="a1a1q"), None), "edited ids": ({}, _edited),
+    "special token of a move's form": (dict(bos_token="a1a1", pad_token="a1a1q"), None), "edited ids": ({}, _edited(lambda t: t.token_to_id.update(e2e4=7))),
+    "removed id": ({}, _edited(lambda t: t.token_to_id.pop("e2e4"))), "added id": ({}, _edited(lambda t: t.token_to_id.setdefault("b2b2", 9))),
+    "other dictionary": ({}, _edited(lambda t: setattr(t, "token_to_id", {**t.token_to_id, "e2e4": 8}))),
     "dictionary subclass": ({}, lambda t: setattr(t, "token_to_id", _Dict(t.token_to_id))),
     "a key that is no string": ({}, lambda t: t.token_to_id.update({3: 5, _Str("b2b2"): 6})),
     "ids of other types": ({}, lambda t: setattr(t, "token_to_id", {k: np.int64(v) for k, v in t.token_to_id.items()})),
@@ -207,3 +214,14 @@ def test_native_token_rows_follow_the_tokenizer(form, games):
             tok.token_rows(rows)
         return
     assert [r.tolist() for r in tok.token_rows(rows)] == want
+
+
+@pytest.mark.parametrize("again", [copy.copy, copy.deepcopy, lambda t: pickle.loads(pickle.dumps(t))])
+def test_a_copied_tokenizer_keeps_no_move_table(again):
+    """What the native call keeps is of one dictionary in one process."""
+    tok = UCITokenizer(max_length=512, vocab_size_multiple_of=128)
+    game = _game(["e2e4", "a1a1"], [1, 1])
+    want = [r.tolist() for r in tok.token_rows([game])]
+    other = again(tok)
+    assert "_move_table" not in vars(other) and vars(other).keys() >= vars(UCITokenizer()).keys()
+    assert [r.tolist() for r in other.token_rows([game])] == want
