@@ -1,7 +1,7 @@
 // Token ids of many games in one call, straight from the Python objects (loaded with ctypes.PyDLL, so
 // the interpreter lock is held throughout).  The Python statement of the same rules is
-// UCITokenizer.token_ids: 17 to 23 us per game of 150 plies (strings hashed before or not) against 3 to 4 here in a
-// batch of 256, which is what a batch of a few hundred prompts waits for before its first kernel.
+// UCITokenizer.token_ids: 12 to 14 us per game of 150 plies (strings hashed before or not) against 2 here, in a batch of
+// 256, which is what a batch of a few hundred prompts waits for before its first kernel.
 //
 // Ids are the tokenizer's dictionary's as it is at the call.  Moves of the usual form (two squares, an optional promotion
 // piece) come from a table by their squares, laid out again whenever the dictionary has changed; any other string is
