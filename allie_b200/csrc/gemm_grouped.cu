@@ -200,7 +200,8 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------- TMA producer (both CTAs)
+    // ------------------------------------------------------- TMA producer (both CTAs): one lane, which also watches
+    // the arrival counters and orders what it saw before its loads
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
