@@ -18,6 +18,7 @@ struct AttnArgs {
   float* lse;               // [B, H, T]
   uint32_t* drop_mask;      // [B, H, T, T/32] keep bits written by the forward pass, or null
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into `seed` when not null
+  int take_over;            // forward: blocks take the place of those that have not started
   int* status;
 };
 

@@ -359,6 +359,31 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// ------------------------------------------------------------- grid scheduling ---
+// A running block takes the place of one of its grid that has not started, and does its work: the set-up is paid
+// once per resident block, loads for the next work go out under the current one, and blocks that run ahead take more.
+// The answer (16 bytes) arrives at `bar` (expect 16 bytes); after a "none left" no block may be asked for again.
+__device__ __forceinline__ void grid_take_block(uint4* answer, uint64_t* bar, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n\t}\n"
+      ::"r"(smem_u32(answer)), "r"(smem_u32(bar)), "r"(lead) : "memory");
+}
+// Whether there was one, and which.  Whole warp; before asking again: fence_proxy_async_smem() and __syncwarp().
+__device__ __forceinline__ bool grid_taken_block(const uint4* answer, uint3& block) {
+  uint32_t yes, x, y, z;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t.reg .b32 w;\n\t"
+      "ld.shared.b128 h, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, w}, h;\n\t}\n"
+      : "=r"(yes), "=r"(x), "=r"(y), "=r"(z) : "r"(smem_u32(answer)) : "memory");
+  block = make_uint3(x, y, z);
+  return __shfl_sync(0xffffffffu, yes, 0) != 0;
+}
+
 // ------------------------------------------------- CTA pairs (cta_group::2) ---
 // Two CTAs of a cluster (ranks 0 and 1) act as one MMA unit: the leader (rank 0) issues
 // tcgen05.mma for both, each CTA stages its own half of A (rows) and of B (columns) in its own

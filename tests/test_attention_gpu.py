@@ -320,3 +320,75 @@ def test_two_kernel_backward_reads_no_keep_bits_past_a_sequence(T, hd):
     torch.cuda.synchronize()
     _lib.check_status()
     assert got[0].isfinite().all() and torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("hd,H,lens", [
+    (64, 16, [300] * 20), (64, 8, [1, 128, 129, 300, 4, 257] * 14), (64, 3, [700, 1, 1, 1, 128] * 20 + [5]),
+    (128, 8, [1, 128, 129, 300, 4, 257] * 14), (128, 5, [384] * 20), (64, 37, [16] * 8), (64, 37, [16] * 9),
+])
+def test_blocks_that_take_over_others(hd, H, lens):
+    """More items than CTAs fit the GPU (and, last, just as many and some more than 296), with blocks in
+    between that have no rows: packed sequences against a call of their own each, to the bit, and against fp32."""
+    import ctypes
+
+    import numpy as np
+
+    from allie_b200.ops import _lib
+
+    torch.manual_seed(3)
+    lib, d = _lib.cuda(), H * hd
+    row0 = torch.from_numpy(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)).cuda()
+    M = int(row0[-1])
+    qkv = (torch.randn(M, 3 * d, device="cuda") * 0.7).bfloat16()
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def packed(rows, starts, n, longest):
+        out = torch.full((rows.shape[0] + 128, d), 7.0, device="cuda", dtype=torch.bfloat16)
+        assert lib.ab_attn_fwd_packed(P(rows), P(out), P(starts), n, longest, rows.shape[0], H, hd,
+                                      ctypes.c_float(hd ** -0.5), 0, P(_lib.status_word()),
+                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        assert (out[rows.shape[0]:] == 7.0).all()
+        return out[:rows.shape[0]]
+
+    outs = [packed(qkv, row0, len(lens), max(lens)) for _ in range(3)]
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    starts = row0.tolist()
+    for i in range(0, len(lens), 7):
+        rows = qkv[starts[i]:starts[i + 1]].contiguous()
+        alone = packed(rows, torch.tensor([0, len(rows)], dtype=torch.int32, device="cuda"), 1, len(rows))
+        assert torch.equal(alone, outs[0][starts[i]:starts[i + 1]]), i
+        ref, _ = _ref(rows, 1, len(rows), H, hd)
+        assert torch.allclose(alone.float(), ref, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(24, 296, 8, 64), (40, 512, 4, 64), (24, 384, 5, 128)])
+def test_dropout_of_blocks_that_take_over_others(B, T, H, hd):
+    """Keep bits of every item as the host draws them, and the outputs as fp32 gives them with these."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.attention import attention_fwd
+
+    torch.manual_seed(4)
+    d, p, seed, stream = H * hd, 0.1, 77, 9
+    qkv = (torch.randn(B * T, 3 * d, device="cuda") * 0.5).bfloat16()
+    out = torch.zeros(B * T, d, device="cuda", dtype=torch.bfloat16)
+    lse = torch.zeros(B, H, T, device="cuda")
+    bits = torch.zeros(B, H, T, T // 32, device="cuda", dtype=torch.int32) if T % 32 == 0 else None
+    attention_fwd(qkv, out, lse, B, T, H, hd, p, seed, stream, bits)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    thr = _lib.dropout_thr16(p)
+    keep = torch.empty(B * H * T * T, dtype=torch.uint8)
+    import ctypes
+
+    assert _lib.cuda().ab_dropout_mask_host(ctypes.c_ulonglong(seed), stream, ctypes.c_longlong(keep.numel()), thr,
+                                            ctypes.c_void_p(keep.data_ptr())) == 0
+    keep = keep.cuda().view(B, H, T, T).bool()
+    if bits is not None:
+        causal = torch.ones(T, T, dtype=torch.bool, device="cuda").tril()
+        unpacked = ((bits.unsqueeze(-1) >> torch.arange(32, device="cuda")) & 1).view(B, H, T, T).bool()
+        assert torch.equal(unpacked & causal, keep & causal)
+    ref, lse_ref = _ref(qkv, B, T, H, hd, keep.float(), 65536.0 / (65536 - thr))
+    assert torch.allclose(out.float(), ref, rtol=3e-2, atol=3e-2)
+    assert torch.allclose(lse, lse_ref, rtol=1e-3, atol=1e-2)
