@@ -14,7 +14,7 @@
 // (64 columns x 128 rows), and O is written in the [B*T, d] layout the projection GEMM reads.
 // V is consumed MN-major (rows = keys), so no transposes exist anywhere.
 //
-// What bounds it: with dropout, instruction issue (17 per element, half of them the generator) and how
+// What bounds it: with dropout, instruction issue (the generator takes 45 of 150 us at 64 x 512 x 16 x 64) and how
 // much of it the warps of an SM can overlap; without, latencies and then the exponential unit (16 per SM
 // and clock).  So: sixteen math warps per SM (with one thread per row, eight, issue was 39 % busy), S
 // is read once, P never passes through shared memory, O stays in TMEM and is rescaled there when the
@@ -26,8 +26,9 @@
 // With a CTA per item (and blocks past the end of their sequence that only leave) an SM had 1.3 of its two CTAs at
 // work and 4700 of a CTA's 7900 clocks over one key tile were set-up, first loads and the way out.  Cold L2, heads of
 // 64, us, a CTA per item and now: 256 prompts of 4 to 300 tokens x 16 heads 192 and 111, 64 of them 58 and 41,
-// 256 x 128 tokens 86 and 61, 64 x 512 x 16 117 and 97, with dropout 176 and 171;
-// heads of 128, 256 prompts x 8 121 and 90.  A tile takes 1650 clocks per SM, of which the exponential unit needs 1024.
+// 256 x 128 tokens 86 and 61, 64 x 512 x 16 117 and 97, with dropout (and with the generator's keys in uniform
+// registers and its bits by carry) 176 and 150, 37 x 328 x 12 with dropout 57 and 51; heads of 128, 256 prompts x 8
+// 121 and 90.  A tile takes 1650 clocks per SM, of which the exponential unit needs 1024.
 #include "attn_common.cuh"
 
 namespace ab {
@@ -284,7 +285,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     };
     const float sl2 = a.scale * LOG2E;
     const uint64_t sl2_2 = f2_bcast(sl2);
-    const uint64_t seed = a.thr16 ? salted(a.seed, a.salt) : 0;
+    const uint64_t seed = uniform64(a.thr16 ? salted(a.seed, a.salt) : 0);
     bool ok = true;
     bool leaving = false;                         // output of the item before, out of its Q tile
     for (int n = 0;; ++n) {
@@ -299,11 +300,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         if (a.thr16) {
           const uint64_t e0 = (static_cast<uint64_t>(it->b * a.H + it->h) * a.T + q_idx) * a.T + hf * 64 + j * AT_BN;
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              keep[c] |= dropout_keep8(seed, a.stream_id, (e0 >> 3) + c * 4 + k, a.thr16) << (8 * k);
-          }
+          for (int c = 0; c < 2; ++c)              // zeros where all 32 rows of the warp are before these keys
+            if (j < it->qt || hf * 64 + c * 32 < quad * 32 + 32)
+              keep[c] = dropout_keep32(seed, a.stream_id, (e0 >> 3) + c * 4, a.thr16);
           const int T = a.T;                       // packed batches have no dropout
           if (a.drop_mask && q_idx < T) {
             uint32_t* dst = a.drop_mask + (e0 >> 5);

@@ -366,11 +366,9 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
       tmem_ld32(taddr + grp * 32, r);
       uint32_t keep = 0xffffffffu;         // does not depend on the accumulator: drawn under the load
       if (thr16) {
-        const uint64_t seed = salted(g.ep.drop_seed, g.salt);
+        const uint64_t seed = uniform64(salted(g.ep.drop_seed, g.salt));
         const uint64_t group0 = (static_cast<uint64_t>(m) * g.N + gn0) >> 3;
-        keep = 0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) keep |= dropout_keep8(seed, g.ep.drop_stream, group0 + c, thr16) << (8 * c);
+        keep = dropout_keep32(seed, g.ep.drop_stream, group0, thr16);
       }
       if (!wait_tile()) return false;
       tmem_ld_wait();

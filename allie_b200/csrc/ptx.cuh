@@ -592,13 +592,6 @@ __device__ __forceinline__ uint64_t f2_gelu_tanh_with_grad(uint64_t x, uint64_t&
 struct Philox4 {
   uint32_t x, y, z, w;
 };
-__host__ __device__ __forceinline__ uint32_t mulhi32(uint32_t a, uint32_t b) {
-#ifdef __CUDA_ARCH__
-  return __umulhi(a, b);
-#else
-  return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
-#endif
-}
 __host__ __device__ __forceinline__ Philox4 philox4x32_7(uint64_t seed, uint32_t stream,
                                                          uint64_t counter) {
   uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
@@ -606,10 +599,11 @@ __host__ __device__ __forceinline__ Philox4 philox4x32_7(uint64_t seed, uint32_t
   uint32_t c2 = stream, c3 = 0x9E3779B9u;
 #pragma unroll
   for (int r = 0; r < 7; ++r) {
-    uint32_t hi0 = mulhi32(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-    uint32_t hi1 = mulhi32(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-    uint32_t n0 = hi1 ^ c1 ^ k0, n2 = hi0 ^ c3 ^ k1;
-    c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
+    const uint64_t p0 = static_cast<uint64_t>(0xD2511F53u) * c0, p1 = static_cast<uint64_t>(0xCD9E8D57u) * c2;
+    c0 = static_cast<uint32_t>(p1 >> 32) ^ c1 ^ k0;
+    c2 = static_cast<uint32_t>(p0 >> 32) ^ c3 ^ k1;
+    c1 = static_cast<uint32_t>(p1);
+    c3 = static_cast<uint32_t>(p0);
     k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
   }
   return Philox4{c0, c1, c2, c3};
@@ -624,6 +618,12 @@ __device__ __forceinline__ unsigned long long salted(unsigned long long seed,
                                                      const unsigned long long* salt) {
   return salt ? (seed ^ __ldg(salt)) : seed;
 }
+// A value that is the same for all lanes of a converged warp, known to be: the generator's seven keys per half then
+// lie in uniform registers instead of being added up for every draw.
+__device__ __forceinline__ uint64_t uniform64(uint64_t v) {
+  const uint32_t hi = __shfl_sync(0xffffffffu, static_cast<uint32_t>(v >> 32), 0);
+  return (static_cast<uint64_t>(hi) << 32) | __shfl_sync(0xffffffffu, static_cast<uint32_t>(v), 0);
+}
 // Dropout decisions come in groups of eight consecutive elements: element
 // index i uses 16 bits of philox(seed, stream, i / 8).  keep iff bits >= thr16.
 __host__ __device__ __forceinline__ uint32_t dropout_thr16(float p) {
@@ -633,19 +633,34 @@ __host__ __device__ __forceinline__ uint32_t dropout_thr16(float p) {
 __host__ __device__ __forceinline__ float dropout_scale(uint32_t thr16) {
   return 65536.f / static_cast<float>(65536u - thr16);
 }
-// keep-mask bits (bit j set = keep element 8*group + j)
-__host__ __device__ __forceinline__ uint32_t dropout_keep8(uint64_t seed, uint32_t stream,
-                                                           uint64_t group, uint32_t thr16) {
-  Philox4 r = philox4x32_7(seed, stream, group);
+// Appends a keep bit to `m`: 1 where the upper 16 bits of `x` are at least the threshold.  `wrap` is
+// -(thr16 << 16): the addition carries out exactly then, and the carry is shifted in (thr16 > 0).
+__host__ __device__ __forceinline__ void push_keep(uint32_t& m, uint32_t x, uint32_t wrap) {
+#ifdef __CUDA_ARCH__
+  asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %1, %2;\n\taddc.u32 %0, %0, %0;\n\t}" : "+r"(m) : "r"(x), "r"(wrap));
+#else
+  m = 2 * m + (static_cast<uint64_t>(x) + wrap > 0xffffffffu);
+#endif
+}
+// the eight bits of a group behind those in `m`, the last element first
+__host__ __device__ __forceinline__ void push_keep8(uint32_t& m, uint64_t seed, uint32_t stream, uint64_t group, uint32_t wrap) {
+  const Philox4 r = philox4x32_7(seed, stream, group);
+  push_keep(m, r.w, wrap); push_keep(m, r.w << 16, wrap);
+  push_keep(m, r.z, wrap); push_keep(m, r.z << 16, wrap);
+  push_keep(m, r.y, wrap); push_keep(m, r.y << 16, wrap);
+  push_keep(m, r.x, wrap); push_keep(m, r.x << 16, wrap);
+}
+// keep-mask bits (bit j set = keep element 8 * group + j); thr16 > 0
+__host__ __device__ __forceinline__ uint32_t dropout_keep8(uint64_t seed, uint32_t stream, uint64_t group, uint32_t thr16) {
   uint32_t m = 0;
-  m |= ((r.x & 0xffffu) >= thr16) << 0;
-  m |= ((r.x >> 16) >= thr16) << 1;
-  m |= ((r.y & 0xffffu) >= thr16) << 2;
-  m |= ((r.y >> 16) >= thr16) << 3;
-  m |= ((r.z & 0xffffu) >= thr16) << 4;
-  m |= ((r.z >> 16) >= thr16) << 5;
-  m |= ((r.w & 0xffffu) >= thr16) << 6;
-  m |= ((r.w >> 16) >= thr16) << 7;
+  push_keep8(m, seed, stream, group, 0u - (thr16 << 16));
+  return m;
+}
+// the same for four groups in a row
+__device__ __forceinline__ uint32_t dropout_keep32(uint64_t seed, uint32_t stream, uint64_t group, uint32_t thr16) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 3; k >= 0; --k) push_keep8(m, seed, stream, group + k, 0u - (thr16 << 16));
   return m;
 }
 
