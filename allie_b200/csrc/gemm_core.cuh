@@ -19,6 +19,36 @@ constexpr int PAIR_STAGES = 5;
 constexpr int PAIR_WARP_STAGING = 4096;   // one wide staging tile per epilogue warp
 constexpr int PAIR_BN = 256;      // instruction N; each CTA stages PAIR_BN / 2 columns of B
 
+// Equal shares of an accumulation for all CTA pairs: `waves` rounds of whole tiles, then `rest` tiles that are cut
+// along the contraction into `slices` parts of `q` steps, a pair each, and what is left of each, `r` steps; the
+// pairs that are over take these, `extra_q` steps each of them all laid end to end.
+struct EvenShare {
+  int on, pairs, waves, rest, slices, q, r, extra_q;
+};
+// i-th unit of a pair: steps [kb0, kb1) of a tile; false when it has no more
+__host__ __device__ inline bool even_unit(const EvenShare& s, int steps, int pair, int i, int& tile, int& kb0, int& kb1) {
+  if (i < s.waves) {
+    tile = i * s.pairs + pair; kb0 = 0; kb1 = steps;
+    return true;
+  }
+  i -= s.waves;
+  const int first = s.waves * s.pairs, main = s.slices * s.rest;
+  if (pair < main) {
+    tile = first + pair % s.rest;
+    kb0 = pair / s.rest * s.q;
+    kb1 = kb0 + s.q < steps ? kb0 + s.q : steps;
+    return i == 0 && kb0 < kb1;
+  }
+  if (s.r == 0) return false;
+  const int x0 = (pair - main) * s.extra_q, all = s.rest * s.r, x1 = x0 + s.extra_q < all ? x0 + s.extra_q : all;
+  const int t = x0 / s.r + i;
+  const int a = t * s.r > x0 ? t * s.r : x0, b = (t + 1) * s.r < x1 ? (t + 1) * s.r : x1;
+  tile = first + t;
+  kb0 = s.slices * s.q + a - t * s.r;
+  kb1 = s.slices * s.q + b - t * s.r;
+  return a < b;
+}
+
 struct GemmArgs {
   int M, N, K;
   int k_splits;
@@ -26,6 +56,8 @@ struct GemmArgs {
   int aux_tma;        // CTA-pair kernel: a second epilogue operand arrives by TMA in the warp's staging tile
                       // (tmAux is a load map) instead of by row loads.  1: the aux tile of act == 2,
                       // 64 bf16 columns; 2: the residual, 32 fp32 columns at a time
+  EvenShare even;     // CTA-pair kernel, EPI_ACCUM
+  int accum_steps;    // likewise: steps that one accumulator sums up
   AbGemmEpilogue ep;
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into ep.drop_seed when not null
   int* status;
@@ -193,6 +225,31 @@ __device__ __forceinline__ uint4 epi_pack8(const uint64_t* v) {
   return make_uint4(f2_to_bf16x2(v[0]), f2_to_bf16x2(v[1]), f2_to_bf16x2(v[2]), f2_to_bf16x2(v[3]));
 }
 
+// EPI_ACCUM: a warp's 32 rows x 64 columns of sums, two to a register pair, are added to the output by the TMA unit;
+// 32 fp32 columns at a time = 128-byte rows, 128B swizzle
+__device__ __forceinline__ void epilogue_add_sums(const CUtensorMap& tmOut, const uint64_t* sum, int nbase, int m0w, int N,
+                                                  uint8_t* stg, int lane) {
+#pragma unroll
+  for (int grp = 0; grp < 2; ++grp) {
+    if (nbase + grp * 32 >= N) break;      // warp-uniform
+    if (lane == 0) tma_store_wait_read<0>();
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float4 v;
+      f2_unpack(sum[grp * 16 + c * 2], v.x, v.y);
+      f2_unpack(sum[grp * 16 + c * 2 + 1], v.z, v.w);
+      *reinterpret_cast<float4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = v;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_reduce_add_2d(&tmOut, stg, nbase + grp * 32, m0w);
+      tma_store_commit();
+    }
+  }
+}
+
 // One epilogue warp drains its 32 rows x 64 columns.  Rows past the end of the output are clipped by
 // the TMA store.  `wait_tile` / `next_tile`: see EPI_RESID.  Returns false when a wait ran out.
 template <int EPI, typename Wait, typename Next>
@@ -319,29 +376,6 @@ __device__ __forceinline__ bool epilogue_drain_kind(const GemmArgs& g, const CUt
       if (lane == 0) {
         tma_store_2d(&tmOut, stg, gn0, m0w);
         tma_store_2d(&tmAux, stg + 2048, gn0, m0w);
-        tma_store_commit();
-      }
-    }
-  } else if constexpr (EPI == EPI_ACCUM) {
-    // 32 fp32 columns = 128-byte rows, 128B swizzle, added to the output by the TMA unit
-    uint8_t* rowp = stg + lane * 128;
-    const int sw = lane & 7;
-#pragma unroll
-    for (int grp = 0; grp < 2; ++grp) {
-      const int gn0 = nbase + grp * 32;
-      if (gn0 >= g.N) break;               // warp-uniform
-      uint32_t r[32];
-      tmem_ld32(taddr + grp * 32, r);
-      if (lane == 0) tma_store_wait_read<0>();
-      __syncwarp();
-      tmem_ld_wait();
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = make_uint4(r[c * 4], r[c * 4 + 1], r[c * 4 + 2], r[c * 4 + 3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        tma_reduce_add_2d(&tmOut, stg, gn0, m0w);
         tma_store_commit();
       }
     }

@@ -322,6 +322,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 //   tempty[b]  leader only, 2 x NUM_EPI_WARPS arrivals: the epilogue warps of both CTAs
 // Loads are plain unicast TMA loads whose completion is counted on the leader's barrier.
 
+// An accumulation (EPI_ACCUM) hands its accumulator over every few 64-wide steps (GemmArgs::accum_steps), and the
+// epilogue warps add these up in registers.  The tensor core cuts its sums off after every 16 products instead of
+// rounding them, so the error of a chain grows with its length: 1024 x 4096 outputs over 32768 rows, 2-norm
+// against 64 bits, one chain 3.8e-5, of 64 steps 4.4e-6, of 32 2.1e-6, of 16 1.0e-6, of 8 4.8e-7.  It costs 0.5 % of the
+// time every 32 steps and 2.5 % every 8, and is never longer than a part of `k_splits` equal ones.
+constexpr int ACCUM_STEPS = 32;
+
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -394,6 +401,15 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   const int num_units = num_tiles * g.k_splits;
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
+  // i-th work unit of this pair, for accumulations: steps [kb0, kb1) of an output tile
+  auto accum_unit = [&](int i, int& tile, int& kb0, int& kb1) {
+    if (g.even.on) return even_unit(g.even, kb_total, pair_id, i, tile, kb0, kb1);
+    const int u = pair_id + i * num_pairs, ks = u / num_tiles;
+    tile = u - ks * num_tiles;
+    kb0 = ks * kb_per;
+    kb1 = min(kb_total, kb0 + kb_per);
+    return u < num_units;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer (both CTAs)
@@ -401,13 +417,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int u = pair_id; u < num_units && ok; u += num_pairs) {
-      const int ks = u / num_tiles;
-      const int tile = u % num_tiles;
+    auto load_unit = [&](int tile, int kb0, int kb1) {
       const int m0 = (tile / n_tiles) * (2 * BM) + rank * BM;
       const int n0 = (tile % n_tiles) * BN + rank * HALF_N;
-      const int kb0 = ks * kb_per;
-      const int kb1 = min(kb_total, kb0 + kb_per);
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_EMPTY;
@@ -436,6 +448,15 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+    };
+    if constexpr (EPI == EPI_ACCUM) {
+      int tile, kb0, kb1;
+      for (int i = 0; ok && accum_unit(i, tile, kb0, kb1); ++i) load_unit(tile, kb0, kb1);
+    } else {
+      for (int u = pair_id; u < num_units && ok; u += num_pairs) {
+        const int ks = u / num_tiles, kb0 = ks * kb_per;
+        load_unit(u % num_tiles, kb0, min(kb_total, kb0 + kb_per));
+      }
     }
   } else if (warp == 1) {
     // --------------------------------------------------------- MMA issuer (leader only)
@@ -448,19 +469,13 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
-      int it = 0;
-      bool ok = true;
-      for (int u = pair_id; u < num_units && ok; u += num_pairs, ++it) {
-        const int ks = u / num_tiles;
-        const int kb0 = ks * kb_per;
-        const int kb1 = min(kb_total, kb0 + kb_per);
-        if (kb0 >= kb1) continue;
-        const int ab = it & 1;
-        if (!mbar_wait_warp(&tempty_bar[ab], ((acc_phase >> ab) & 1) ^ 1, abort_flag)) {
+      uint32_t n_acc = 0;                 // accumulators handed over, the two in turn
+      auto accumulate = [&](int kb0, int kb1) {
+        const int ab = n_acc & 1;
+        if (!mbar_wait_warp(&tempty_bar[ab], ((n_acc >> 1) & 1) ^ 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_EMPTY;
           if (lead) atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_EMPTY);
-          break;
+          return false;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * BN;
@@ -468,8 +483,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) {
             *abort_flag = ST_TIMEOUT_FULL;
             if (lead) atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
-            ok = false;
-            break;
+            return false;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
@@ -485,11 +499,22 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           umma_commit_pair(mapa_shared(eb, 1), lead);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
         const uint32_t tb = smem_u32(&tfull_bar[ab]);
         umma_commit_pair(mapa_shared(tb, 0), lead);     // accumulator complete -> both epilogues
         umma_commit_pair(mapa_shared(tb, 1), lead);
-        acc_phase ^= 1u << ab;
+        ++n_acc;
+        return true;
+      };
+      bool ok = true;
+      if constexpr (EPI == EPI_ACCUM) {
+        int tile, kb0, kb1;
+        for (int i = 0; ok && accum_unit(i, tile, kb0, kb1); ++i)
+          for (; ok && kb0 < kb1; kb0 += g.accum_steps) ok = accumulate(kb0, min(kb1, kb0 + g.accum_steps));
+      } else {
+        for (int u = pair_id; u < num_units && ok; u += num_pairs) {
+          const int kb0 = u / num_tiles * kb_per, kb1 = min(kb_total, kb0 + kb_per);
+          if (kb0 < kb1) ok = accumulate(kb0, kb1);
+        }
       }
     }
   } else {
@@ -499,7 +524,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     const int part = e >> 2;
     constexpr int COLS_PER_WARP = BN / 4;
     uint8_t* my_stage = stage_out + e * PAIR_WARP_STAGING;
-    uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
+    uint32_t n_acc = 0;                 // accumulators taken over, the two in turn
     // GELU backward (aux_tma == 1): the warp's 32 x 64 tile of aux values is fetched by TMA into its
     // staging tile one unit ahead (right after the store of the unit before has read the tile), so
     // the loads that the epilogue math depends on are in flight while the accumulator is still
@@ -509,74 +534,113 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     static_assert(COLS_PER_WARP == 64, "the staged aux tile is one 64-column store group");
     const bool stage_aux = EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT || (EPI == EPI_ANY && g.aux_tma != 0);
     uint32_t aux_phase = 0;
-    auto fetch_aux = [&](int u, int grp) {          // lane 0; the staging tile must be free
-      if (u >= num_units) return;
-      const int tile = u % num_tiles;
-      const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
-      const int n = (tile % n_tiles) * BN + part * COLS_PER_WARP + grp * 32;
-      if (m0w >= g.M || n >= g.N) return;           // the same test skips the drain below
-      mbar_expect_tx(&aux_bar[e], 32 * 128);
-      tma_load_2d(my_stage, &tmAux, &aux_bar[e], n, m0w);
-    };
-    if (stage_aux && lane == 0) fetch_aux(pair_id, 0);
-    int it = 0;
-    for (int u = pair_id; u < num_units; u += num_pairs, ++it) {
-      const int ks = u / num_tiles;
-      const int tile = u % num_tiles;
-      const int kb0 = ks * kb_per;
-      const int kb1 = min(kb_total, kb0 + kb_per);
-      if (kb0 >= kb1) continue;
-      const int ab = it & 1;
-      const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
-      const int m = m0w + lane;
-      const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
-      const bool staged = stage_aux && m0w < g.M && nbase < g.N;
-      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
-        *abort_flag = ST_TIMEOUT_TMEM_FULL;
-        atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
-        if (staged) mbar_wait_landed(&aux_bar[e], aux_phase);     // before the warp leaves
-        break;
-      }
-      acc_phase ^= 1u << ab;
-      tc_fence_after();
-      const uint32_t taddr =
-          tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
-      auto wait_aux = [&]() {
-        if (!mbar_wait(&aux_bar[e], aux_phase, abort_flag)) {
-          *abort_flag = ST_TIMEOUT_FULL;
-          atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
-          mbar_wait_landed(&aux_bar[e], aux_phase);
-          return false;
-        }
-        aux_phase ^= 1;
-        return true;
-      };
-      // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
-      // from zero-filled loads); it still hands the buffer back
-      if constexpr (EPI == EPI_ANY) {
-        if (staged && !wait_aux()) break;
-        if (m0w < g.M)
-          epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
-                                             ks == 0, 0, staged);
-      } else {
-        // past the last staged tile of this unit: the first one of the next
-        auto next_tile = [&](int grp) {
-          if (EPI == EPI_RESID && grp == 0 && nbase + 32 < g.N) fetch_aux(u, 1);
-          else fetch_aux(u + num_pairs, 0);
-        };
-        if (m0w < g.M && nbase < g.N) {
-          if (!epilogue_drain_kind<EPI>(g, tmOut, tmAux, taddr, m, m0w, nbase, my_stage, lane, wait_aux, next_tile))
+    if constexpr (EPI == EPI_ACCUM) {
+      int tile, kb0, kb1;
+      bool ok = true;
+      for (int i = 0; ok && accum_unit(i, tile, kb0, kb1); ++i) {
+        if (kb0 >= kb1) continue;
+        const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
+        const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
+        const bool live = m0w < g.M && nbase < g.N;
+        uint64_t sum[COLS_PER_WARP / 2];
+#pragma unroll
+        for (int c = 0; c < COLS_PER_WARP / 2; ++c) sum[c] = 0;
+        for (; kb0 < kb1; kb0 += g.accum_steps) {
+          const int ab = n_acc & 1;
+          if (!mbar_wait(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
+            *abort_flag = ST_TIMEOUT_TMEM_FULL;
+            atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
+            ok = false;
             break;
-        } else if ((EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT) && lane == 0) {
+          }
+          ++n_acc;
+          tc_fence_after();
+          if (live) {
+#pragma unroll
+            for (int c = 0; c < COLS_PER_WARP / 16; ++c) {
+              uint32_t r[16];
+              tmem_ld16(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP + c * 16, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                sum[c * 8 + k] = f2_add(sum[c * 8 + k], f2_pack(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1])));
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
+        }
+        if (ok && live) epilogue_add_sums(tmOut, sum, nbase, m0w, g.N, my_stage, lane);
+      }
+    } else {
+      auto fetch_aux = [&](int u, int grp) {          // lane 0; the staging tile must be free
+        if (u >= num_units) return;
+        const int tile = u % num_tiles;
+        const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
+        const int n = (tile % n_tiles) * BN + part * COLS_PER_WARP + grp * 32;
+        if (m0w >= g.M || n >= g.N) return;           // the same test skips the drain below
+        mbar_expect_tx(&aux_bar[e], 32 * 128);
+        tma_load_2d(my_stage, &tmAux, &aux_bar[e], n, m0w);
+      };
+      if (stage_aux && lane == 0) fetch_aux(pair_id, 0);
+      for (int u = pair_id; u < num_units; u += num_pairs) {
+        const int ks = u / num_tiles;
+        const int tile = u % num_tiles;
+        const int kb0 = ks * kb_per;
+        const int kb1 = min(kb_total, kb0 + kb_per);
+        if (kb0 >= kb1) continue;
+        const int ab = n_acc & 1;
+        const int m0w = (tile / n_tiles) * (2 * BM) + rank * BM + quad * 32;
+        const int m = m0w + lane;
+        const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
+        const bool staged = stage_aux && m0w < g.M && nbase < g.N;
+        if (!mbar_wait(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
+          *abort_flag = ST_TIMEOUT_TMEM_FULL;
+          atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
+          if (staged) mbar_wait_landed(&aux_bar[e], aux_phase);     // before the warp leaves
+          break;
+        }
+        ++n_acc;
+        tc_fence_after();
+        const uint32_t taddr =
+            tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
+        auto wait_aux = [&]() {
+          if (!mbar_wait(&aux_bar[e], aux_phase, abort_flag)) {
+            *abort_flag = ST_TIMEOUT_FULL;
+            atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
+            mbar_wait_landed(&aux_bar[e], aux_phase);
+            return false;
+          }
+          aux_phase ^= 1;
+          return true;
+        };
+        // a warp whose 32 rows lie entirely past M has nothing to store (its accumulator rows came
+        // from zero-filled loads); it still hands the buffer back
+        if constexpr (EPI == EPI_ANY) {
+          if (staged && !wait_aux()) break;
+          if (m0w < g.M)
+            epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, m < g.M, my_stage, lane,
+                                               ks == 0, 0, staged);
+        } else {
+          // past the last staged tile of this unit: the first one of the next
+          auto next_tile = [&](int grp) {
+            if (EPI == EPI_RESID && grp == 0 && nbase + 32 < g.N) fetch_aux(u, 1);
+            else fetch_aux(u + num_pairs, 0);
+          };
+          if (m0w < g.M && nbase < g.N) {
+            if (!epilogue_drain_kind<EPI>(g, tmOut, tmAux, taddr, m, m0w, nbase, my_stage, lane, wait_aux, next_tile))
+              break;
+          } else if ((EPI == EPI_RESID || EPI == EPI_MUL || EPI == EPI_DOT) && lane == 0) {
+            fetch_aux(u + num_pairs, 0);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
+        if (EPI == EPI_ANY && stage_aux && lane == 0) {
+          tma_store_wait_read<0>();           // the store just issued has read the staging tile
           fetch_aux(u + num_pairs, 0);
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
-      if (EPI == EPI_ANY && stage_aux && lane == 0) {
-        tma_store_wait_read<0>();           // the store just issued has read the staging tile
-        fetch_aux(u + num_pairs, 0);
       }
     }
     if (lane == 0) tma_store_wait<0>();
@@ -616,6 +680,57 @@ static EpiKind pair_kind(bool a_mn, bool b_mn, const GemmArgs& g) {
   }
 }
 
+// Cuts an accumulation into work units for `max_pairs` CTA pairs: either every tile into `splits` equal parts
+// (`on` = 0), or equal shares of it all.  A unit ends with a pass over its tile that adds 256 KB of fp32 in L2; it runs
+// under the next unit's main loop, which has to be EVEN_COVER steps long for that, and the last one under
+// none.  The cheapest way by that count is taken, a number of equal parts where it is level with the shares (its CTAs
+// read the same rows of the operands at the same time).  us, the equal parts taken before (balanced within 2 %,
+// whatever their length) and now, at 16384 rows: 1280 x 3840 181 and 112, 1280 x 1280 69 and 44, 1280 x 5120 166 and 156;
+// at 32768: 1024 x 4096 206 and 194, 1024 x 1024 67 and 56, 2048 x 1024 109 and 100; 1024 x 3072 (three equal parts
+// either way) 148, and at 12136 rows 768 x 3072 45 and 46, 768 x 768 22.
+constexpr int EVEN_MIN_STEPS = 8;      // of a part
+constexpr int EVEN_COVER = 16;
+constexpr int EVEN_UNIT = 2;           // steps that any unit costs beside its own
+static EvenShare even_share(int tiles, int steps, int max_pairs, int* splits) {
+  auto unit_cost = [](long long n) { return (n > EVEN_COVER ? n : EVEN_COVER) + EVEN_UNIT; };
+  if (max_pairs < 1) max_pairs = 1;
+  const int most = steps / EVEN_MIN_STEPS > 1 ? steps / EVEN_MIN_STEPS : 1;
+  long long best = 0;
+  for (int s = 1; s <= most && s <= 32; ++s) {
+    const long long rounds = (static_cast<long long>(tiles) * s + max_pairs - 1) / max_pairs;
+    const long long len = (steps + s - 1) / s, cost = (rounds - 1) * unit_cost(len) + len + EVEN_UNIT;
+    if (s == 1 || cost < best) { best = cost; *splits = s; }
+  }
+  EvenShare b = {};
+  b.pairs = max_pairs;
+  b.waves = tiles / max_pairs;
+  b.rest = tiles % max_pairs;
+  if (b.rest == 0) return b;
+  const long long before = b.waves * unit_cost(steps);
+  auto take = [&](int q, int r, int extra_q, long long cost) {
+    if ((before + cost) * 65 >= best * 64) return;
+    best = before + cost;
+    b.on = 1; b.q = q; b.r = r; b.extra_q = extra_q;
+  };
+  b.slices = max_pairs / b.rest < most ? max_pairs / b.rest : most;
+  take((steps + b.slices - 1) / b.slices, 0, 0, (steps + b.slices - 1) / b.slices + EVEN_UNIT);
+  const int extra = max_pairs - b.slices * b.rest;
+  if (extra == 0) return b;
+  // a longer main part leaves the other pairs less to do, and these have more and shorter units
+  const int q0 = static_cast<int>((static_cast<long long>(b.rest) * steps + max_pairs - 1) / max_pairs);
+  const int q1 = (steps + b.slices - 1) / b.slices, by = steps / 128 > 1 ? steps / 128 : 1;
+  for (int q = q0; q < q1; q += by) {
+    const int r = steps - b.slices * q;
+    if (r < EVEN_MIN_STEPS) break;
+    const int xq = (b.rest * r + extra - 1) / extra, whole = xq / r, part = xq % r;
+    // part of a tile lies across two more often than not
+    long long cost = part ? whole * unit_cost(r) + part + unit_cost(0) : (whole - 1) * unit_cost(r) + r + EVEN_UNIT;
+    if (q + EVEN_UNIT > cost) cost = q + EVEN_UNIT;
+    take(q, r, xq, cost);
+  }
+  return b;
+}
+
 template <bool A_MN, bool B_MN>
 static int launch_pair(const void* A, long long lda, const void* B, long long ldb, const GemmArgs& g,
                        int max_ctas, cudaStream_t stream) {
@@ -645,9 +760,15 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   constexpr int SMEM = 1024 + PAIR_STAGES * (BM * BK * 2 + HALF_N * BK * 2) +
                        NUM_EPI_WARPS * PAIR_WARP_STAGING + 256;
   const int m_tiles = (g.M + 2 * BM - 1) / (2 * BM), n_tiles = (g.N + PAIR_BN - 1) / PAIR_BN;
-  const int units = m_tiles * n_tiles * g.k_splits;
+  const int steps = (g.K + BK - 1) / BK;
+  ga.accum_steps = (steps + g.k_splits - 1) / g.k_splits;
+  if (ga.accum_steps > ACCUM_STEPS) ga.accum_steps = ACCUM_STEPS;
+  ga.even.on = 0;
+  if (ep.even_k && pair_kind(A_MN, B_MN, ga) == EPI_ACCUM)
+    ga.even = even_share(m_tiles * n_tiles, steps, max_ctas / 2, &ga.k_splits);
+  const int units = m_tiles * n_tiles * ga.k_splits;
   int pairs = max_ctas / 2;
-  if (pairs > units) pairs = units;
+  if (pairs > units && !ga.even.on) pairs = units;
   if (pairs < 1) pairs = 1;
   auto go = [&](auto kern, PerDeviceOnce& attr_set) {
     if (attr_set.first_use_on_device()) {
@@ -842,6 +963,19 @@ extern "C" int ab_gemm_bf16(const void* A, int a_mn, long long lda, const void* 
   if (!a_mn && b_mn) return launch_plan<false, true>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
   if (a_mn && !b_mn) return launch_plan<true, false>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
   return launch_plan<true, true>(plan.kernel, A, lda, B, ldb, g, max_ctas, stream);
+}
+
+// For tests: the units that `pairs` CTA pairs get of `tiles` output tiles of `steps` steps with even_k, four numbers
+// each (pair, tile, first step, end).  Returns how many (no more than `room` are written), or minus the number of
+// equal parts per tile.
+extern "C" int ab_gemm_even_units(int tiles, int steps, int pairs, int* out, int room) {
+  int splits = 1, n = 0, tile, kb0, kb1;
+  const ab::EvenShare s = ab::even_share(tiles, steps, pairs, &splits);
+  if (!s.on) return -splits;
+  for (int p = 0; p < s.pairs; ++p)
+    for (int i = 0; ab::even_unit(s, steps, p, i, tile, kb0, kb1); ++i, ++n)
+      if (n < room) { out[4 * n] = p; out[4 * n + 1] = tile; out[4 * n + 2] = kb0; out[4 * n + 3] = kb1; }
+  return n;
 }
 
 // What ab_gemm_bf16 would run for the same arguments, without running it: the columns of the single-CTA

@@ -54,6 +54,9 @@ struct AbGemmEpilogue {
   // bytes).  They are asked into L2 while this launch runs.
   const void* next_b;
   long long next_bytes;
+  // nonzero: a plain accumulation is cut up for the CTA pairs as suits them; k_splits is then for the kernels that
+  // know equal parts only, and still the least number of partial sums
+  int even_k;
 };
 
 // C[M,N] = A[M,K] * B[K,N] on the 5th-generation tensor cores.

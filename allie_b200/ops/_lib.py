@@ -60,7 +60,7 @@ class GemmEpilogue(ctypes.Structure):
         ("drop_seed", c_ulonglong), ("drop_stream", c_uint), ("drop_thr16", c_uint),
         ("alpha", c_float), ("m_limit", c_void_p), ("k_limit", c_void_p), ("pdl", c_int),
         ("aux_grad", c_int), ("colsum", c_void_p), ("dot_out", c_void_p), ("dot_T", c_int),
-        ("passes", c_void_p), ("next_b", c_void_p), ("next_bytes", c_longlong),
+        ("passes", c_void_p), ("next_b", c_void_p), ("next_bytes", c_longlong), ("even_k", c_int),
     ]
 
 

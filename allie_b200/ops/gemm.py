@@ -33,7 +33,8 @@ def num_sms() -> int:
 
 def pick_k_splits(M: int, N: int, K: int) -> int:
     """Split K when the output alone has too few 128x256 tiles to fill the GPU
-    (the weight-gradient case: small output, very long contraction)."""
+    (the weight-gradient case: small output, very long contraction).  The CTA-pair kernel cuts such a
+    problem up by itself; to it this is the least number of partial sums."""
     bn = 128 if N <= 128 else 256
     tiles = ((M + 127) // 128) * ((N + bn - 1) // bn)
     sms = num_sms()
@@ -106,9 +107,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         ks = max(1, min(K // 256, 128 // max(tiles, 1)))
         if ks > 1:
             accumulate, resid, k_splits = True, None, ks
+    even_k = k_splits is None and accumulate
     if k_splits is None:
         k_splits = pick_k_splits(M, N, K) if (accumulate and out_fp32) else 1
     ep = _lib.GemmEpilogue()
+    ep.even_k = int(even_k)
     ep.out = out.data_ptr()
     ep.ldo = out.stride(0)
     ep.out_fp32 = int(out_fp32)

@@ -411,3 +411,29 @@ def test_gemm_asks_for_the_next_weights(M, nbytes):
     got = gemm(a, w, b_mn=True, dependent=True, then=nxt)
     torch.cuda.synchronize()
     assert torch.equal(want, got)
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1280, 3840, 16384),            # 75 tiles: a round of whole ones and one cut into 32 parts
+    (1280, 1280, 16384),            # 25: two parts each, 24 pairs take what is left
+    (1280, 5120, 4104),             # 100: a round, 26 in two parts and the rest; a last step of 8
+    (1000, 1096, 8200), (2048, 1024, 12000), (520, 264, 40000), (1024, 4096, 8192),
+])
+def test_weight_gradients_in_equal_shares(routes, M, N, K):
+    """Shares of the contraction that are no equal parts, edges of tiles, and sums handed over every few steps:
+    no accumulator sums up more than 32 steps of 64, of 16 products each addition, which are cut off at
+    2^-23 of a partial sum below 6 sqrt(2048); each of the K / 2048 parts adds one such error at most, the fp32
+    additions of the parts 2^-24 of 6 sqrt(K) each."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(9)
+    a, dy = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    dw = torch.full((M, N), 3.0, device="cuda")
+    gemm(a, dy, a_mn=True, b_mn=True, out=dw, accumulate=True)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert routes == [PAIR + ACCUM]
+    parts = K / 2048 + 1
+    bound = parts * (128 * 2 ** -23 * 6 * 2048 ** 0.5 + 2 ** -24 * 6 * K ** 0.5) + 1e-5
+    assert ((dw.double() - 3.0 - a.double().t() @ dy.double()).abs() <= bound).all()
