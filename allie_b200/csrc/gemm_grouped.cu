@@ -200,74 +200,71 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------- TMA producer (both CTAs): one lane, which also watches
-    // the arrival counters and orders what it saw before its loads
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int u = pair_id; u < num_units && ok; u += num_pairs) {
-        int grp, mrow0, ncol0, kb_total;
-        decode(u, grp, mrow0, ncol0, kb_total);
-        const int n0 = ncol0 + rank * HALF_N;
-        if constexpr (MODE == 1) {
-          if (ga.tile_ready) {
-            // my 128 rows of A: complete once every live row in them has arrived
-            const int first = mrow0 + rank * BM;
-            const int need = max(0, min(BM, s_rows[grp] - first));
-            if (!wait_rows(ga.tile_ready + (grp * ga.cap + first) / BM, need, abort_flag)) {
-              *abort_flag = ST_TIMEOUT_PEER;
-              atomicCAS(g.status, 0, ST_TIMEOUT_PEER);
-              ok = false;
-              break;
-            }
-            fence_proxy_async_all();
-          }
+    // ------------------------------------------------------- TMA producer (both CTAs).  The elected lane also watches
+    // the arrival counters and orders what it saw before its loads.  What comes from shared memory is made known to
+    // be the same for all lanes, or the coordinates would be moved to the uniform registers load by load.
+    const uint32_t lead = elect_one();
+    auto known = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    // the rows of a 128-row block from `first` on have arrived
+    auto arrived = [&](int grp, int first) {
+      int seen = 1;
+      if (lead) {
+        const int need = max(0, min(BM, s_rows[grp] - first));
+        seen = wait_rows(ga.tile_ready + (grp * ga.cap + first) / BM, need, abort_flag);
+        if (seen) {
+          fence_proxy_async_all();
+        } else {
+          *abort_flag = ST_TIMEOUT_PEER;
+          atomicCAS(g.status, 0, ST_TIMEOUT_PEER);
         }
-        for (int kb = 0; kb < kb_total; ++kb) {
-          const int k0 = kb * BK;
-          if constexpr (MODE == 2) {
-            if (ga.tile_ready && (k0 % BM) == 0) {
-              const int need = max(0, min(BM, s_rows[grp] - k0));
-              if (!wait_rows(ga.tile_ready + (grp * ga.cap + k0) / BM, need, abort_flag)) {
-                *abort_flag = ST_TIMEOUT_PEER;
-                atomicCAS(g.status, 0, ST_TIMEOUT_PEER);
-                ok = false;
-                break;
-              }
-              fence_proxy_async_all();
-            }
-          }
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
-            *abort_flag = ST_TIMEOUT_EMPTY;
-            atomicCAS(g.status, 0, ST_TIMEOUT_EMPTY);
-            ok = false;
-            break;
-          }
-          uint8_t* sa = smem + stage * STAGE_BYTES;
-          uint8_t* sb = sa + A_BYTES;
-          const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
-          if constexpr (MODE == 1) {
-            tma_load_2d_pair(sa, &tmA, fb, k0, grp * ga.cap + mrow0 + rank * BM);
-            if constexpr (!B_MN) {
-              tma_load_2d_pair(sb, &tmB, fb, k0, grp * g.N + n0);
-            } else {
-#pragma unroll
-              for (int i = 0; i < HALF_N / 64; ++i)
-                tma_load_2d_pair(sb + i * (BK * 128), &tmB, fb, n0 + i * 64, grp * g.K + k0);
-            }
+      }
+      return __all_sync(0xffffffffu, seen) != 0;
+    };
+    for (int u = pair_id; u < num_units && ok; u += num_pairs) {
+      int grp, mrow0, ncol0, kb_total;
+      decode(u, grp, mrow0, ncol0, kb_total);
+      grp = known(grp); mrow0 = known(mrow0); kb_total = known(kb_total);
+      const int n0 = ncol0 + rank * HALF_N;
+      if constexpr (MODE == 1) {
+        if (ga.tile_ready && !(ok = arrived(grp, mrow0 + rank * BM))) break;      // my 128 rows of A
+      }
+      for (int kb = 0; kb < kb_total; ++kb) {
+        const int k0 = kb * BK;
+        if constexpr (MODE == 2) {
+          if (ga.tile_ready && (k0 % BM) == 0 && !(ok = arrived(grp, k0))) break;
+        }
+        if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
+          *abort_flag = ST_TIMEOUT_EMPTY;
+          if (lead) atomicCAS(g.status, 0, ST_TIMEOUT_EMPTY);
+          ok = false;
+          break;
+        }
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        uint8_t* sb = sa + A_BYTES;
+        const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
+        if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE_BYTES, lead);
+        if constexpr (MODE == 1) {
+          tma_load_2d_pair(sa, &tmA, fb, k0, grp * ga.cap + mrow0 + rank * BM, lead);
+          if constexpr (!B_MN) {
+            tma_load_2d_pair(sb, &tmB, fb, k0, grp * g.N + n0, lead);
           } else {
-            const int y = grp * ga.cap + k0;
-#pragma unroll
-            for (int i = 0; i < BM / 64; ++i)
-              tma_load_2d_pair(sa + i * (BK * 128), &tmA, fb, mrow0 + rank * BM + i * 64, y);
 #pragma unroll
             for (int i = 0; i < HALF_N / 64; ++i)
-              tma_load_2d_pair(sb + i * (BK * 128), &tmB, fb, n0 + i * 64, y);
+              tma_load_2d_pair(sb + i * (BK * 128), &tmB, fb, n0 + i * 64, grp * g.K + k0, lead);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        } else {
+          const int y = grp * ga.cap + k0;
+#pragma unroll
+          for (int i = 0; i < BM / 64; ++i)
+            tma_load_2d_pair(sa + i * (BK * 128), &tmA, fb, mrow0 + rank * BM + i * 64, y, lead);
+#pragma unroll
+          for (int i = 0; i < HALF_N / 64; ++i)
+            tma_load_2d_pair(sb + i * (BK * 128), &tmB, fb, n0 + i * 64, y, lead);
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
@@ -373,9 +370,23 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           }
         }
       } else {
-        if (mrow_w < g.M)
-          epilogue_drain_wide<COLS_PER_WARP>(g, tmOut, tmAux, taddr, grp * g.M + mrow, grp * g.M + mrow_w, nbase,
-                                             mrow < g.M, my_stage, lane, true, grp * g.N);
+        // the accumulator is free as soon as it lies in registers (M is a multiple of 32: all rows of a warp or none)
+        uint64_t sum[COLS_PER_WARP / 2];
+        const uint64_t alpha = f2_bcast(g.ep.alpha);
+#pragma unroll
+        for (int c = 0; c < COLS_PER_WARP / 16; ++c) {
+          uint32_t r[16];
+          tmem_ld16(taddr + c * 16, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            sum[c * 8 + k] = f2_mul(f2_pack(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1])), alpha);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[ab]), 0));
+        if (mrow_w < g.M) epilogue_add_sums(tmOut, sum, nbase, grp * g.M + mrow_w, g.N, my_stage, lane);
+        continue;
       }
       tc_fence_before();
       __syncwarp();
