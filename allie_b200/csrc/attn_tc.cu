@@ -118,6 +118,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   const int warp = warp_number(), lane = threadIdx.x & 31;
   const int d_model = a.H * HD;
 
+  int2 first_rows = make_int2(0, 0);         // asked for under the set-up
+  if (a.row0 && warp == FWD_TMA_WARP) first_rows = make_int2(__ldg(a.row0 + blockIdx.z), __ldg(a.row0 + blockIdx.z + 1));
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], FWD_MATH_WARPS);
@@ -164,6 +166,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       return true;
     };
     uint3 block = make_uint3(blockIdx.x, blockIdx.y, blockIdx.z);
+    int2 rows = first_rows;                      // of the block's sequence: first row, and the next one's
     for (int asked = 0; ok; ++asked) {
       // the place of a block that has not started yet; the answer is needed when this one's loads are out
       if (a.take_over) {
@@ -174,8 +177,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       it.qt = (a.T + AT_BM - 1) / AT_BM - 1 - static_cast<int>(block.x);       // heaviest tiles first
       it.h = block.y; it.b = block.z;
       // packed batch: sequence b owns rows [row0[b], row0[b + 1]) of the activation
-      it.first = a.row0 ? __ldg(a.row0 + it.b) : it.b * a.T;
-      it.T = a.row0 ? __ldg(a.row0 + it.b + 1) - it.first : a.T;
+      it.first = a.row0 ? rows.x : it.b * a.T;
+      it.T = a.row0 ? rows.y - rows.x : a.T;
       if (it.qt * AT_BM < it.T) {
         ok = push(it);
         const int qs = n % STAGES;
@@ -209,6 +212,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       // before the block leaves, too: the answer is written to its shared memory
       ok = __all_sync(0xffffffffu, mbar_wait_landed(grid_bar, asked & 1)) && ok;
       if (!grid_taken_block(grid_next, block)) break;       // none left, and none may be asked for after that
+      if (a.row0) rows = make_int2(__ldg(a.row0 + block.z), __ldg(a.row0 + block.z + 1));
       fence_proxy_async_smem();
       __syncwarp();
     }
