@@ -77,7 +77,6 @@ template <int HD>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmO,
                 const AttnArgs a) {
-  griddep_wait();
   using C = FwdCfg<HD>;
   constexpr int PANELS = C::PANELS, TILE_BYTES = C::TILE_BYTES, STAGES = C::STAGES;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
@@ -118,19 +117,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   const int warp = warp_number(), lane = threadIdx.x & 31;
   const int d_model = a.H * HD;
 
-  int2 first_rows = make_int2(0, 0);         // asked for under the set-up
-  if (a.row0 && warp == FWD_TMA_WARP) first_rows = make_int2(__ldg(a.row0 + blockIdx.z), __ldg(a.row0 + blockIdx.z + 1));
+  // The set-up may run under the kernel before; the producer asks for the first item's rows as soon as that is done.
+  int2 first_rows = make_int2(0, 0);
+  if (warp == FWD_TMA_WARP) {
+    griddep_wait();
+    if (a.row0) first_rows = make_int2(__ldg(a.row0 + blockIdx.z), __ldg(a.row0 + blockIdx.z + 1));
+  }
+  if (warp == 0) {                           // a barrier per lane
+    const uint64_t* bar = bars + lane;
+    const uint32_t count = bar == s_empty || bar == p_full || (bar >= q_empty && bar < k_full) ? FWD_MATH_WARPS
+                           : bar >= xchg && bar < item_full       ? 2
+                           : bar >= item_empty && bar < grid_bar ? FWD_MATH_WARPS + 1 : 1;
+    if (bar <= grid_bar) mbar_init(bars + lane, count);
+    __syncwarp();
+  }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], FWD_MATH_WARPS);
-      mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1);
-      mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-    }
-    mbar_init(s_full, 1); mbar_init(s_empty, FWD_MATH_WARPS);
-    mbar_init(p_full, FWD_MATH_WARPS); mbar_init(pv_full, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&xchg[i], 2);
-    for (int i = 0; i < FWD_QUEUE; ++i) { mbar_init(&item_full[i], 1); mbar_init(&item_empty[i], FWD_MATH_WARPS + 1); }
-    mbar_init(grid_bar, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQKV);
@@ -142,6 +143,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   // only now: a dependent GEMM's CTA must not take the TMEM columns that this grid still has to allocate
   if (threadIdx.x == 0) griddep_launch_dependents();
+  griddep_wait();                            // all else that is read or written comes after this
   const uint32_t tS = tmem_base, tP = tmem_base + C::TM_P, tO = tmem_base + C::TM_O;
 
   // n-th item of this CTA, for a whole warp (bounded; null when a wait ran out).  It stays until item_done.
@@ -180,15 +182,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       it.first = a.row0 ? rows.x : it.b * a.T;
       it.T = a.row0 ? rows.y - rows.x : a.T;
       if (it.qt * AT_BM < it.T) {
-        ok = push(it);
         const int qs = n % STAGES;
-        if (ok) ok = mbar_wait_warp(&q_empty[qs], ((n / STAGES) & 1) ^ 1, abort_flag);
-        if (ok) {
+        if ((ok = mbar_wait_warp(&q_empty[qs], ((n / STAGES) & 1) ^ 1, abort_flag))) {
           mbar_expect_tx(&q_full[qs], TILE_BYTES, lead);
 #pragma unroll
           for (int p = 0; p < PANELS; ++p)
             tma_load_2d(sQ + qs * TILE_BYTES + p * 16384, &tmQKV, &q_full[qs], it.h * HD + p * 64, it.first + it.qt * AT_BM, lead);
-          nq = ++n;
+          nq = n + 1;
+          ok = push(it);
+          ++n;
         }
         for (int j = 0; j <= it.qt && ok; ++j, ++g) {                          // causal: key tiles 0..qt
           const int st = g % STAGES;
@@ -295,17 +297,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     for (int n = 0;; ++n) {
       const volatile FwdItem* it = next_item(n);
       if (!(ok = it != nullptr) || it->qt < 0) break;
-      const int q_idx = it->qt * AT_BM + r, qs = n % STAGES;
+      const int qt = it->qt, q_idx = qt * AT_BM + r, qs = n % STAGES;
       float m_ref = 0.f;                          // running maximum, which P and O are scaled to
       float l_run = 0.f;                          // row sum of this half's keys
-      for (int j = 0; j <= it->qt; ++j, tile ^= 1) {
+      for (int j = 0; j <= qt; ++j, tile ^= 1) {
         // dropout keep bits of this thread's 64 keys; they are also what the backward pass reads back
         uint32_t keep[2] = {0u, 0u};
         if (a.thr16) {
           const uint64_t e0 = (static_cast<uint64_t>(it->b * a.H + it->h) * a.T + q_idx) * a.T + hf * 64 + j * AT_BN;
 #pragma unroll
           for (int c = 0; c < 2; ++c)              // zeros where all 32 rows of the warp are before these keys
-            if (j < it->qt || hf * 64 + c * 32 < quad * 32 + 32)
+            if (j < qt || hf * 64 + c * 32 < quad * 32 + 32)
               keep[c] = dropout_keep32(seed, a.stream_id, (e0 >> 3) + c * 4, a.thr16);
           const int T = a.T;                       // packed batches have no dropout
           if (a.drop_mask && q_idx < T) {
@@ -330,7 +332,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           __syncwarp();
           if (lane == 0) mbar_arrive(s_empty);     // the next S may be computed
         }
-        if (j == it->qt) {                         // diagonal tile: keys after the row's own position
+        if (j == qt) {                             // diagonal tile: keys after the row's own position
 #pragma unroll
           for (int i = 0; i < 64; ++i) v[i] = hf * 64 + i <= r ? v[i] : 0xff800000u;
         }
@@ -412,15 +414,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         leaving = false;
         l_run = l_run * grow + rs;
       }
-      if (!ok || !(ok = mbar_wait(pv_full, tile ^ 1, abort_flag))) break;
+      if (!ok) break;
+      const int T = it->T, h = it->h, b = it->b, row = it->first + qt * AT_BM + quad * 32;    // this warp's first row
+      item_done(n);
+      if (!(ok = mbar_wait(pv_full, tile ^ 1, abort_flag))) break;
       tc_fence_after();
       float* slot = s_row + met * 256;
       slot[hf * 128 + r] = l_run;
       if (!(ok = pair_sync())) break;
       const float l = slot[r] + slot[128 + r];
       const float inv = dropout_scale(a.thr16) / l;
-      const int qt = it->qt, T = it->T, h = it->h, b = it->b, row = it->first + qt * AT_BM + quad * 32;    // this warp's first row
-      item_done(n);
       // The warps' 32 rows leave through the (now idle) Q tile with one TMA store per 64 columns; warps
       // with rows past the end of the sequence store row by row.
       const bool whole = qt * AT_BM + quad * 32 + 32 <= T;

@@ -61,18 +61,21 @@ int make_tmap_2d_sw(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
 
 // KSUB: 64-wide steps of the contraction per stage.  Two for the 64-column tiles, whose four MMAs a step take no longer
 // than the waits and commits around them (chain of 90 x 1024 x 1024 launches: 5.8 us with one, 5.45 with two).
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
+template <int TM, int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmOut,
                          const __grid_constant__ CUtensorMap tmAux, const GemmArgs g) {
-  constexpr int A_BYTES = BM * BK * 2;
+  static_assert(TM == 128 || (TM == 64 && !A_MN), "rows of a tile");
+  constexpr int A_BYTES = TM * BK * 2;
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int SUB_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KSUB * SUB_BYTES;
   constexpr int BKS = KSUB * BK;          // contraction columns of a stage
   constexpr int TMEM_COLS = 2 * BN;  // 256 or 512, power of two
-  static_assert(TMEM_COLS == 256 || TMEM_COLS == 512 || TMEM_COLS == 128, "bad BN");
+  static_assert(TMEM_COLS == 256 || TMEM_COLS == 512 || TMEM_COLS == 128 || TMEM_COLS == 64, "bad BN");
+  // 32 columns of an MN-major B: rows of 64 bytes, swizzled over 64 (else panels of 64 columns, over 128)
+  constexpr bool B_HALF_PANEL = B_MN && BN == 32;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -132,7 +135,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 
   const int Meff = g.ep.m_limit ? min(g.M, __ldg(g.ep.m_limit)) : g.M;
   const int Keff = g.ep.k_limit ? min(g.K, __ldg(g.ep.k_limit)) : g.K;
-  const int m_tiles = (Meff + BM - 1) / BM;
+  const int m_tiles = (Meff + TM - 1) / TM;
   const int n_tiles = (g.N + BN - 1) / BN;
   const int kb_total = (Keff + BKS - 1) / BKS;
   const int kb_per = (kb_total + g.k_splits - 1) / g.k_splits;
@@ -152,7 +155,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         tma_load_2d(sb, &tmB, bar, k0, n0, lead);
       } else {
 #pragma unroll
-        for (int i = 0; i < BN / 64; ++i) tma_load_2d(sb + i * (BK * 128), &tmB, bar, n0 + i * 64, k0, lead);
+        for (int i = 0; i < (BN + 63) / 64; ++i) tma_load_2d(sb + i * (BK * 128), &tmB, bar, n0 + i * 64, k0, lead);
       }
     };
     // dependent launch: the first ring-full of weight tiles of my first unit goes out while the
@@ -184,7 +187,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     for (int u = blockIdx.x; u < num_units && ok; u += gridDim.x) {
       const int ks = u / num_tiles;
       const int tile = u % num_tiles;
-      const int m0 = (tile / n_tiles) * BM;
+      const int m0 = (tile / n_tiles) * TM;
       const int n0 = (tile % n_tiles) * BN;
       const int kb0 = ks * kb_per;
       const int kb1 = min(kb_total, kb0 + kb_per);
@@ -206,7 +209,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             tma_load_2d(sa, &tmA, &full_bar[stage], k0, m0, lead);
           } else {
 #pragma unroll
-            for (int i = 0; i < BM / 64; ++i)
+            for (int i = 0; i < TM / 64; ++i)
               tma_load_2d(sa + i * (BK * 128), &tmA, &full_bar[stage], m0 + i * 64, k0, lead);
           }
           if (!b_done) load_b(sa + A_BYTES, &full_bar[stage], k0, n0);
@@ -217,11 +220,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   } else if (warp == 1) {
     // --------------------------------------------------------- MMA issuer
     const uint32_t lead = elect_one();
-    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr uint32_t idesc = make_idesc_bf16(TM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
     constexpr uint32_t A_LBO = A_MN ? BK * 128 : 16;
     constexpr uint32_t B_LBO = B_MN ? BK * 128 : 16;
     constexpr uint32_t A_KADV = A_MN ? UMMA_K * 128 : UMMA_K * 2;  // bytes per UMMA_K step
-    constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * 2;
+    constexpr uint32_t B_KADV = B_HALF_PANEL ? UMMA_K * 64 : B_MN ? UMMA_K * 128 : UMMA_K * 2;
     int stage = 0;
     uint32_t phase = 0;
     uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
@@ -254,7 +257,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         for (int k = 0; k < BKS / UMMA_K; ++k) {
           const int sub = k / (BK / UMMA_K) * SUB_BYTES, kk = k % (BK / UMMA_K);
           const uint64_t adesc = make_sdesc_sw128(sa, sub + kk * A_KADV, A_LBO, 1024);
-          const uint64_t bdesc = make_sdesc_sw128(sb, sub + kk * B_KADV, B_LBO, 1024);
+          const uint64_t bdesc = B_HALF_PANEL ? make_sdesc<4>(sb, sub + kk * B_KADV, B_LBO, 512)
+                                              : make_sdesc_sw128(sb, sub + kk * B_KADV, B_LBO, 1024);
           umma_bf16(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u, lead);
         }
         umma_commit(&empty_bar[stage], lead);  // frees the smem stage once these MMAs retire
@@ -269,7 +273,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     const int e = warp - 2;
     const int quad = warp & 3;           // TMEM lane quarter this warp may read
     const int part = e >> 2;             // which quarter of the BN columns
-    constexpr int COLS_PER_WARP = BN / 4;
+    constexpr int COLS_PER_WARP = BN > 64 ? BN / 4 : 16;      // with 32 columns half of the warps have none
+    constexpr int ROWS = TM / 4;         // of the tile in a TMEM lane quarter, from its first lane on
     uint8_t* my_stage = stage_out + e * 2048;
     uint32_t acc_phase = 0;             // bit ab: phase of accumulator ab
     int it = 0;
@@ -280,7 +285,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       const int kb1 = min(kb_total, kb0 + kb_per);
       if (kb0 >= kb1) continue;
       const int ab = it & 1;
-      const int m = (tile / n_tiles) * BM + quad * 32 + lane;
+      const int m0w = (tile / n_tiles) * TM + quad * ROWS, m = m0w + lane;   // first row of this warp's block
       const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
       if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
@@ -291,9 +296,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       tc_fence_after();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
-      const int m0w = (tile / n_tiles) * BM + quad * 32;   // first row of this warp's block
-      const bool row_ok = m < Meff;
-      epilogue_drain<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, row_ok, my_stage, lane, ks == 0);
+      const bool row_ok = lane < ROWS && m < Meff;
+      if (part * COLS_PER_WARP < BN)
+        epilogue_drain<COLS_PER_WARP>(g, tmOut, tmAux, taddr, m, m0w, nbase, row_ok, my_stage, lane, ks == 0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[ab]);
@@ -801,38 +806,38 @@ static int launch_pair(const void* A, long long lda, const void* B, long long ld
   return go(gemm_bf16_tcgen05_pair_kernel<A_MN, B_MN, EPI_ANY>, attr[EPI_ANY]);
 }
 
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
+template <int TM, int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
 static int launch(const void* A, long long lda, const void* B, long long ldb, const GemmArgs& g,
                   int max_ctas, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
   int rc;
-  if (!A_MN) rc = make_tmap_2d(&tmA, A, g.M, g.K, lda, BM, BK, 2, true);
+  if (!A_MN) rc = make_tmap_2d(&tmA, A, g.M, g.K, lda, TM, BK, 2, true);
   else       rc = make_tmap_2d(&tmA, A, g.K, g.M, lda, BK, 64, 2, true);
   if (rc) return rc;
   if (!B_MN) rc = make_tmap_2d(&tmB, B, g.N, g.K, ldb, BN, BK, 2, true);
-  else       rc = make_tmap_2d(&tmB, B, g.K, g.N, ldb, BK, 64, 2, true);
+  else       rc = make_tmap_2d_sw(&tmB, B, g.K, g.N, ldb, BK, BN < 64 ? BN : 64, 2, BN < 64 ? 64 : 128);
   if (rc) return rc;
-  // output / pre-activation maps for the epilogue's TMA stores: boxes of 32 rows x 16 columns
+  // output / pre-activation maps for the epilogue's TMA stores: boxes of a warp's rows x 16 columns
   CUtensorMap tmOut, tmAux;
   const AbGemmEpilogue& ep = g.ep;
-  if (ep.out_fp32) rc = make_tmap_2d_sw(&tmOut, ep.out, g.M, g.N, ep.ldo, 32, 16, 4, 64);
-  else             rc = make_tmap_2d_sw(&tmOut, ep.out, g.M, g.N, ep.ldo, 32, 16, 2, 32);
+  if (ep.out_fp32) rc = make_tmap_2d_sw(&tmOut, ep.out, g.M, g.N, ep.ldo, TM / 4, 16, 4, 64);
+  else             rc = make_tmap_2d_sw(&tmOut, ep.out, g.M, g.N, ep.ldo, TM / 4, 16, 2, 32);
   if (rc) return rc;
   if (ep.act == 1) {
-    rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, 32, 16, 2, 32);
+    rc = make_tmap_2d_sw(&tmAux, ep.aux, g.M, g.N, ep.ldaux, TM / 4, 16, 2, 32);
     if (rc) return rc;
   } else {
     tmAux = tmOut;
   }
-  constexpr int SMEM = 1024 + STAGES * KSUB * (BM * BK * 2 + BN * BK * 2) + NUM_EPI_WARPS * 2048 + 256;
-  auto kern = gemm_bf16_tcgen05_kernel<BN, STAGES, KSUB, A_MN, B_MN>;
+  constexpr int SMEM = 1024 + STAGES * KSUB * (TM * BK * 2 + BN * BK * 2) + NUM_EPI_WARPS * 2048 + 256;
+  auto kern = gemm_bf16_tcgen05_kernel<TM, BN, STAGES, KSUB, A_MN, B_MN>;
   static PerDeviceOnce attr_set;
   if (attr_set.first_use_on_device()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set.mark_device();
   }
-  const int m_tiles = (g.M + BM - 1) / BM, n_tiles = (g.N + BN - 1) / BN;
+  const int m_tiles = (g.M + TM - 1) / TM, n_tiles = (g.N + BN - 1) / BN;
   const int units = m_tiles * n_tiles * g.k_splits;
   int grid = units < max_ctas ? units : max_ctas;
   if (grid < 1) grid = 1;
@@ -864,10 +869,11 @@ namespace ab {
 
 // Which kernel serves a problem, and whether column sums or head products come from passes of their own
 struct GemmPlan {
-  int kernel;                  // columns of the single-CTA kernel's tile (64, 128, 256), or PLAN_PAIR
+  int kernel;                  // columns of the single-CTA kernel's tile (64, 128, 256), PLAN_64X32 or PLAN_PAIR
   bool dot_pass, colsum_pass;
 };
 constexpr int PLAN_PAIR = 512;
+constexpr int PLAN_64X32 = 32;          // 64 rows
 
 static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue& ep, int k_splits, int max_ctas) {
   // CTA pairs for the large shapes; the single-CTA kernel keeps the device-sized problems
@@ -899,6 +905,15 @@ static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue
   else if (one_wave) p.kernel = tiles(64) <= max_ctas ? 64 : 128;
   else if (narrow)   p.kernel = 128;
   else               p.kernel = pair ? PLAN_PAIR : 256;
+  // 64 x 32 tiles where they fit a wave and 128 x 64 ones leave three quarters of the SMs idle: a step of the
+  // contraction takes 165 clocks (12 KB of operands) instead of 320 (24 KB, and MMAs of 128 rows that take 67 clocks
+  // whatever their columns).  Per launch of a chain, us, before and now: 90 x 1024 x 4096 14.7 and 10.7, 90 x 1024 x 1024
+  // with residual 6.5 and 5.4, 200 x 1024 x 4096 15.0 and 11.2.  With 64 x 64 tiles as well where 64 x 32 are too many
+  // (90 x 3072 x 1024 5.9 and 5.6) neighbouring launches of a pass no longer fit the SMs together, and their
+  // set-up waits: one game 1230 us as it was, 1250 so, 1180 without.
+  if (p.kernel == 64 && k_splits == 1 && !ep.m_limit && !ep.k_limit &&
+      static_cast<long long>((M + 63) / 64) * ((N + 31) / 32) <= max_ctas)
+    p.kernel = PLAN_64X32;
   return p;
 }
 
@@ -906,11 +921,12 @@ template <bool A_MN, bool B_MN>
 static int launch_plan(int kernel, const void* A, long long lda, const void* B, long long ldb, const GemmArgs& g,
                        int max_ctas, cudaStream_t stream) {
   if (kernel == PLAN_PAIR) return launch_pair<A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
-  if (kernel == 256) return launch<256, 4, 1, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+  if (kernel == 256) return launch<128, 256, 4, 1, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
   if constexpr (!A_MN) {
-    if (kernel == 64) return launch<64, 4, 2, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+    if (kernel == 64) return launch<128, 64, 4, 2, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+    if (kernel == PLAN_64X32) return launch<64, 32, 8, 2, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
   }
-  return launch<128, 6, 1, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
+  return launch<128, 128, 6, 1, A_MN, B_MN>(A, lda, B, ldb, g, max_ctas, stream);
 }
 
 }  // namespace ab
@@ -979,7 +995,7 @@ extern "C" int ab_gemm_even_units(int tiles, int steps, int pairs, int* out, int
 }
 
 // What ab_gemm_bf16 would run for the same arguments, without running it: the columns of the single-CTA
-// kernel's tile, or 512 + EpiKind on CTA pairs.  Passes beside the GEMM: see `passes`.
+// kernel's tile (64 also where it takes half of that by half of the rows), or 512 + EpiKind on CTA pairs.  Passes beside the GEMM: see `passes`.
 extern "C" int ab_gemm_route(const void*, int a_mn, long long, const void*, int b_mn, long long, int M, int N, int,
                              const AbGemmEpilogue* ep, int k_splits, int max_ctas, int*, cudaStream_t) {
   using namespace ab;
@@ -989,6 +1005,7 @@ extern "C" int ab_gemm_route(const void*, int a_mn, long long, const void*, int 
   GemmPlan plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas);
   if (plan.dot_pass) { e.act = 0; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
   if (plan.colsum_pass) { e.colsum = nullptr; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
+  if (plan.kernel == PLAN_64X32) return 64;
   if (plan.kernel != PLAN_PAIR) return plan.kernel;
   GemmArgs g;
   g.ep = e;

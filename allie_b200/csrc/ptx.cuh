@@ -469,13 +469,17 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr, uint
 // Shared-memory matrix descriptor for 128-byte-swizzled bf16 tiles (the layout
 // a TMA load with CU_TENSOR_MAP_SWIZZLE_128B produces).  Field positions:
 // start>>4 [0,14), LBO>>4 [16,30), SBO>>4 [32,46), version=1 [46,48),
-// layout type [61,64) with 2 = SWIZZLE_128B.
+// layout type [61,64) with 2 = SWIZZLE_128B, 4 = SWIZZLE_64B.
 // For `base` + `off`, both multiples of 16: neighbouring descriptors differ by one addition to the low word (shared
 // memory ends below 2^18, so nothing carries out of the address field).
-__device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t base, uint32_t off, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+template <uint32_t LAYOUT>
+__device__ __forceinline__ uint64_t make_sdesc(uint32_t base, uint32_t off, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   const uint32_t lo = (base >> 4) + ((off >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16));
-  const uint32_t hi = ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) | (2u << 29);
+  const uint32_t hi = ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) | (LAYOUT << 29);
   return (static_cast<uint64_t>(hi) << 32) | lo;
+}
+__device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t base, uint32_t off, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return make_sdesc<2>(base, off, lbo_bytes, sbo_bytes);
 }
 // Instruction descriptor for kind::f16 with bf16 A/B and fp32 accumulator.
 // a_mn / b_mn: operand is MN-major (1) rather than K-major (0).

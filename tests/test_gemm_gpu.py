@@ -437,3 +437,37 @@ def test_weight_gradients_in_equal_shares(routes, M, N, K):
     parts = K / 2048 + 1
     bound = parts * (128 * 2 ** -23 * 6 * 2048 ** 0.5 + 2 ** -24 * 6 * K ** 0.5) + 1e-5
     assert ((dw.double() - 3.0 - a.double().t() @ dy.double()).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M", [1, 20, 64, 65, 90, 128, 200])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (1024, 72), (264, 520), (40, 4096)])
+@pytest.mark.parametrize("b_mn", [True, False])
+def test_gemm_small_tiles(M, N, K, b_mn):
+    """Tiles of 64 rows x 32 columns: edges, a contraction that ends inside a stage, all epilogues; and the same
+    bits as the tiles give that a larger batch of the same rows takes (contractions are not split)."""
+    from allie_b200.ops import _lib
+    from allie_b200.ops.gemm import gemm
+
+    torch.manual_seed(10)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(K, N, device="cuda") / K ** 0.5).bfloat16()
+    b = w if b_mn else w.t().contiguous()
+    bias, resid = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda")
+    ref = a.double() @ w.double() + bias
+    close = lambda x, y: torch.allclose(x.double(), y, rtol=1e-2, atol=1e-2)      # bf16 results: 2^-9 each
+    plain = gemm(a, b, b_mn=b_mn, bias=bias)
+    assert close(plain, ref)
+    assert close(gemm(a, b, b_mn=b_mn, bias=bias, act=3), torch.nn.functional.gelu(ref, approximate="tanh"))
+    aux = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert close(gemm(a, b, b_mn=b_mn, bias=bias, act=1, aux=aux), torch.nn.functional.gelu(ref, approximate="tanh"))
+    assert close(aux, ref)
+    out = torch.full((M + 1, N), 7.0, device="cuda")
+    gemm(a, b, b_mn=b_mn, bias=bias, resid=resid, out=out[:M])
+    assert ((out[:M].double() - ref - resid).abs() <= 1e-4).all() and (out[M] == 7.0).all()
+    dropped = gemm(a, b, b_mn=b_mn, bias=bias, resid=resid, out_dtype=torch.float32, drop_p=0.25, drop_seed=5, drop_stream=3)
+    kept = dropped != resid
+    assert M * N < 1000 or abs(kept.double().mean() - 0.75) < 0.03
+    assert ((dropped - resid).double()[kept] - (ref / 0.75)[kept]).abs().max() < 1e-3
+    more = torch.cat([a, torch.randn(3000, K, device="cuda").bfloat16()])
+    assert torch.equal(gemm(more, b, b_mn=b_mn, bias=bias)[:M], plain)
+    _lib.check_status()
