@@ -271,30 +271,43 @@ kv_store_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict
 
 // out row: [0, max_legal) priors over the legal moves in list order, then value, time, resign logit,
 // best legal logit.  Behind the last row: the status word, so that the copy which brings the results to the
-// host also tells whether a wait of this pass ran out.  One warp per tree.
+// host also tells whether a wait of this pass ran out.  One warp per tree.  `ahead`: a programmatic dependent, which reads
+// the request (active, legal moves) before it waits.
 __global__ void __launch_bounds__(32)
 policy_epilogue_kernel(const __nv_bfloat16* __restrict__ logits, long long ld,
                        const int* __restrict__ active, const int* __restrict__ legal, int legal_stride,
                        const int* __restrict__ n_legal, const float* __restrict__ value,
                        const float* __restrict__ time, int resign_id, float inv_temperature,
-                       float* __restrict__ out, int out_stride, const int* __restrict__ status) {
+                       float* __restrict__ out, int out_stride, const int* __restrict__ status, int ahead) {
   const int t = blockIdx.x, lane = threadIdx.x;
+  if (!ahead) griddep_wait();
+  const int live = active[t], n = live ? min(n_legal[t], legal_stride) : 0;
+  // the first 64 moves' logits stay in registers; a position rarely has more
+  int move[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) move[k] = lane + 32 * k < n ? legal[t * legal_stride + lane + 32 * k] : 0;
+  if (ahead) griddep_wait();
   if (t == 0 && lane == 0) out[static_cast<long long>(gridDim.x) * out_stride] = __int_as_float(*status);
-  if (!active[t]) return;
-  const int n = min(n_legal[t], legal_stride);
+  if (!live) return;
   const __nv_bfloat16* lr = logits + static_cast<long long>(t) * ld;
+  float near[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) near[k] = __bfloat162float(lr[move[k]]);
+  auto logit = [&](int i) {
+    return i < 32 ? near[0] : i < 64 ? near[1] : __bfloat162float(lr[legal[t * legal_stride + i]]);
+  };
   float mx = -INFINITY;
-  for (int i = lane; i < n; i += 32) mx = fmaxf(mx, __bfloat162float(lr[legal[t * legal_stride + i]]));
+  for (int i = lane; i < n; i += 32) mx = fmaxf(mx, logit(i));
 #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float s = 0.f;
   for (int i = lane; i < n; i += 32)
-    s += __expf((__bfloat162float(lr[legal[t * legal_stride + i]]) - mx) * inv_temperature);
+    s += __expf((logit(i) - mx) * inv_temperature);
 #pragma unroll
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   float* orow = out + static_cast<long long>(t) * out_stride;
   for (int i = lane; i < n; i += 32)
-    orow[i] = __expf((__bfloat162float(lr[legal[t * legal_stride + i]]) - mx) * inv_temperature) / s;
+    orow[i] = __expf((logit(i) - mx) * inv_temperature) / s;
   if (lane == 0) {
     orow[legal_stride] = value ? value[t] : 0.f;
     orow[legal_stride + 1] = time ? time[t] : 0.f;
@@ -366,14 +379,19 @@ int ab_kv_store(const void* qkv, void* kc, void* vc, const int* len, int n_trees
   return (int)cudaGetLastError();
 }
 
-// out: n_trees rows of out_stride values and one more word, which receives *status
+// out: n_trees rows of out_stride values and one more word, which receives *status.  `dependent`: launched as a
+// programmatic dependent of the kernel before it, which must not write active, legal or n_legal
 int ab_policy_epilogue(const void* logits, long long ld, const int* active, const int* legal,
                        int legal_stride, const int* n_legal, const float* value, const float* time,
                        int resign_id, float inv_temperature, float* out, int out_stride, int n_trees,
-                       const int* status, cudaStream_t stream) {
-  ab::policy_epilogue_kernel<<<n_trees, 32, 0, stream>>>((const __nv_bfloat16*)logits, ld, active, legal,
-                                                         legal_stride, n_legal, value, time, resign_id,
-                                                         inv_temperature, out, out_stride, status);
+                       const int* status, int dependent, cudaStream_t stream) {
+  const auto* lg = (const __nv_bfloat16*)logits;
+  if (dependent)
+    return (int)ab::launch_dependent(ab::policy_epilogue_kernel, dim3(n_trees), dim3(32), 0, stream, lg, ld, active, legal,
+                                     legal_stride, n_legal, value, time, resign_id, inv_temperature, out, out_stride,
+                                     status, 1);
+  ab::policy_epilogue_kernel<<<n_trees, 32, 0, stream>>>(lg, ld, active, legal, legal_stride, n_legal, value, time,
+                                                         resign_id, inv_temperature, out, out_stride, status, 0);
   return (int)cudaGetLastError();
 }
 }

@@ -88,6 +88,8 @@ int ab_embed_fwd(const int*, const int*, const float*, const float*, const float
                  unsigned long long, unsigned int, unsigned int, cudaStream_t);
 int ab_heads_fwd(const void*, const float*, const float*, const float*, const float*, const float*, const float*,
                  const int*, float, float, float*, float*, float*, float*, float*, int, int, cudaStream_t);
+int ab_heads_fwd_ahead(const void*, const float*, const float*, const float*, const float*, float*, float*, int, int,
+                       cudaStream_t);
 int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
                        int dependent, int* status, cudaStream_t stream);
 
@@ -157,8 +159,9 @@ int ab_infer_last(const AbInfer* p, const AbInferLayer* layers, cudaStream_t str
   AB_TRY(norm(x, a.lnf_w, a.lnf_b, a.h, M));
   AB_TRY(gemm(a.h, a.d, a.wte_bf16, 0, nullptr, 0, a.logits, 0, M, a.V));
   if (a.wv) {
-    AB_TRY(ab_heads_fwd(a.h, a.wv, a.bv, a.wt, a.bt, nullptr, nullptr, nullptr, 0.f, 0.f, a.value, a.time, nullptr,
-                        nullptr, nullptr, M, a.d, stream));
+    AB_TRY(dep ? ab_heads_fwd_ahead(a.h, a.wv, a.bv, a.wt, a.bt, a.value, a.time, M, a.d, stream)
+               : ab_heads_fwd(a.h, a.wv, a.bv, a.wt, a.bt, nullptr, nullptr, nullptr, 0.f, 0.f, a.value, a.time, nullptr,
+                              nullptr, nullptr, M, a.d, stream));
     ++launched;
   }
 #undef AB_TRY

@@ -103,6 +103,13 @@ def heads_fwd(h, wv, bv, wt, bt, value_labels, time_labels, counts, value_coef: 
                                  ptr(acc), c_int(M), c_int(d), stream_ptr()), "ab_heads_fwd")
 
 
+def heads_fwd_ahead(h, wv, bv, wt, bt, value_out, time_out) -> None:
+    """Without labels, as a programmatic dependent of the kernel before it (which must not write the weights)."""
+    M, d = h.shape
+    _ck(_lib.cuda().ab_heads_fwd_ahead(ptr(h), ptr(wv), ptr(bv), ptr(wt), ptr(bt), ptr(value_out), ptr(time_out),
+                                       c_int(M), c_int(d), stream_ptr()), "ab_heads_fwd_ahead")
+
+
 def heads_bwd_w(h, dv, dt, dwv, dbv, dwt, dbt) -> None:
     M, d = h.shape
     _ck(_lib.cuda().ab_heads_bwd_w(ptr(h), ptr(dv), ptr(dt), ptr(dwv), ptr(dbv), ptr(dwt), ptr(dbt),

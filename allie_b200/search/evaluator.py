@@ -161,7 +161,9 @@ class KVLeafEvaluator:
                         dependent=pdl, weights_ready=True)
         gemm(self.h, eng.wte[1], b_mn=False, out=self.logits, dependent=pdl)
         has_heads = eng.reg is not None
-        if has_heads:
+        if has_heads and pdl:
+            K.heads_fwd_ahead(self.h, eng.wv[0], eng.bv[0], eng.wt[0], eng.bt[0], self.value, self.time)
+        elif has_heads:
             K.heads_fwd(self.h, eng.wv[0], eng.bv[0], eng.wt[0], eng.bt[0], None, None, eng.counts, 0.0, 0.0,
                         self.value, self.time, None, None, None)
         rc = lib.ab_policy_epilogue(ptr(self.logits), c_longlong(self.logits.stride(0)),
@@ -169,7 +171,8 @@ class KVLeafEvaluator:
                                     c_int(self.legal_max), ptr(self.view(rd, "n_legal")),
                                     ptr(self.value if has_heads else None), ptr(self.time if has_heads else None),
                                     c_int(self.resign_id), c_float(1.0), ptr(self.out_flat),
-                                    c_int(self.out_stride), c_int(n), ptr(_lib.status_word()), stream_ptr())
+                                    c_int(self.out_stride), c_int(n), ptr(_lib.status_word()), c_int(int(pdl)),
+                                    stream_ptr())
         assert rc == 0
         _lib.count_launches(1)
 

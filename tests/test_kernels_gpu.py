@@ -1,4 +1,6 @@
 """Non-GEMM sm_100a kernels against plain PyTorch fp32 references of the same ops."""
+import ctypes
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -355,3 +357,95 @@ def test_dependent_layernorm_waits_for_its_weights(d):
     K.layernorm_fwd(x, gb[0], gb[1], want, mean, rstd, 1e-5)
     _done()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("M,d", [(1, 128), (5, 96), (7, 384), (3, 1024), (4, 1280), (300, 256), (9, 2048)])
+def test_embedding_rows_of_any_width(M, d):
+    """Several rows to a block, one, and a row in two rounds: control token, dropped and kept elements."""
+    from allie_b200.ops import _lib, kernels as K
+
+    torch.manual_seed(11)
+    V, P, p, seed, stream = 64, 32, 0.25, 5, 3
+    wte, wpe, ctrl = (torch.randn(n, d, device="cuda") for n in (V, P, 2))
+    ids = torch.randint(0, V, (M,), device="cuda", dtype=torch.int32)
+    ids[0] = V + 1500
+    pos = torch.randint(0, P, (M,), device="cuda", dtype=torch.int32)
+    want = wte[ids.clamp(max=V - 1).long()] + wpe[pos.long()]
+    e = (1500 - 500) / 2500
+    want[0] = e * ctrl[0] + (1 - e) * ctrl[1] + wpe[pos[0].long()]
+    x = torch.full((M + 1, d), 7.0, device="cuda")
+    K.embed_fwd(ids, pos, wte, wpe, ctrl, x[:M], V, 0, 0, 0.0)
+    assert torch.allclose(x[:M], want, rtol=1e-6, atol=1e-6) and (x[M] == 7.0).all()
+    K.embed_fwd(ids, pos, wte, wpe, ctrl, x[:M], V, seed, stream, p)
+    n = -(-M * d // 8) * 8
+    keep = torch.empty(n, dtype=torch.uint8)
+    thr = _lib.dropout_thr16(p)
+    assert _lib.cuda().ab_dropout_mask_host(ctypes.c_ulonglong(seed), ctypes.c_uint(stream), ctypes.c_longlong(n),
+                                            ctypes.c_uint(thr), ctypes.c_void_p(keep.data_ptr())) == 0
+    keep = keep[:M * d].view(M, d).cuda()
+    assert torch.allclose(x[:M], want * keep * (65536.0 / (65536 - thr)), rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("M,d", [(1, 128), (9, 1024), (3, 1280), (20, 2048), (5, 100)])
+def test_scalar_heads_with_and_without_waiting(M, d):
+    from allie_b200.ops import kernels as K
+
+    torch.manual_seed(12)
+    h = torch.randn(M, d, device="cuda").bfloat16()
+    wv, wt = (torch.randn(d, device="cuda") * 0.05 for _ in range(2))
+    bv, bt = torch.randn(1, device="cuda"), torch.randn(1, device="cuda")
+    outs = [torch.full((M + 1,), 7.0, device="cuda") for _ in range(4)]
+    K.heads_fwd(h, wv, bv, wt, bt, None, None, torch.zeros(4, dtype=torch.int32, device="cuda"), 0.0, 0.0, outs[0][:M],
+                outs[1][:M], None, None, None)
+    K.heads_fwd_ahead(h, wv, bv, wt, bt, outs[2][:M], outs[3][:M])
+    want_v, want_t = torch.tanh(h.double() @ wv.double() + bv), h.double() @ wt.double() + bt
+    # d products of fp32 rounding, summed to order 1
+    assert torch.allclose(outs[0][:M].double(), want_v, atol=1e-5) and torch.allclose(outs[1][:M].double(), want_t, atol=1e-5)
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3]) and outs[2][M] == 7.0
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 2047, 2500, 20000])
+def test_scalar_head_gradients_over_any_rows(M):
+    from allie_b200.ops import kernels as K
+
+    torch.manual_seed(13)
+    d = 256
+    h = torch.randn(M, d, device="cuda").bfloat16()
+    dv, dt = torch.randn(M, device="cuda"), torch.randn(M, device="cuda")
+    gv, gt = torch.ones(d, device="cuda"), torch.ones(d, device="cuda")
+    bv, bt = torch.ones(1, device="cuda"), torch.ones(1, device="cuda")
+    K.heads_bwd_w(h, dv, dt, gv, bv, gt, bt)
+    tol = 1e-6 * M ** 0.5 * 6 + 1e-5          # sums of M terms of order one in fp32
+    for g, b, x in ((gv, bv, dv), (gt, bt, dt)):
+        assert (g.double() - 1 - x.double() @ h.double()).abs().max() < tol * 6
+        assert abs(float(b) - 1 - float(x.double().sum())) < tol * 6
+
+
+@pytest.mark.parametrize("dependent", [0, 1])
+def test_policy_rows_of_any_number_of_moves(dependent):
+    """None, a warp's worth, the 64 that stay in registers and more."""
+    from allie_b200.ops import _lib
+
+    torch.manual_seed(14)
+    counts, width, V = [0, 1, 31, 32, 33, 63, 64, 65, 100, 224], 224, 2048
+    n = len(counts)
+    logits = torch.randn(n, V, device="cuda").bfloat16()
+    active = torch.ones(n, dtype=torch.int32, device="cuda")
+    active[3] = 0
+    legal = torch.stack([torch.randperm(V, device="cuda")[:width] for _ in counts]).int()
+    n_legal = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    value, time = torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
+    out = torch.full((n * (width + 4) + 1,), 7.0, device="cuda")
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert _lib.cuda().ab_policy_epilogue(P(logits), ctypes.c_longlong(V), P(active), P(legal), width, P(n_legal), P(value),
+                                          P(time), 1992, ctypes.c_float(1.0), P(out), width + 4, n, P(_lib.status_word()),
+                                          dependent, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    rows = out[:-1].view(n, width + 4)
+    for t, c in enumerate(counts):
+        if t == 3:
+            assert (rows[t] == 7.0).all()
+            continue
+        x = logits[t, legal[t, :c].long()].float()
+        assert torch.allclose(rows[t, :c], x.softmax(0), rtol=1e-5, atol=1e-6) and (rows[t, c:width] == 7.0).all()
+        assert rows[t, width] == value[t] and rows[t, width + 1] == time[t] and rows[t, width + 2] == logits[t, 1992].float()
+        assert c == 0 or rows[t, width + 3] == x.max()
