@@ -18,6 +18,9 @@ struct AttnArgs {
   float* lse;               // [B, H, T]
   uint32_t* drop_mask;      // [B, H, T, T/32] keep bits written by the forward pass, or null
   const unsigned long long* salt;   // seed_salt_ptr() at launch: folded into `seed` when not null
+  // key / value cache [sequence][head][slots][hd] that a packed batch's keys and values also go to, or null
+  __nv_bfloat16 *kc, *vc;
+  int slots;
   int take_over;            // forward: blocks take the place of those that have not started
   int* status;
 };

@@ -73,10 +73,19 @@ __device__ __forceinline__ void keep_masks16(uint32_t word, uint32_t* m) {
   }
 }
 
-template <int HD>
+// The caches that keys and values also go to.  A kernel of its own: as an option of the one without, its maps and code
+// cost a pass over one short game 25 of 1180 us.
+template <bool KV>
+struct KvMaps {
+  CUtensorMap k, v;
+};
+template <>
+struct KvMaps<false> {};
+
+template <int HD, bool KV>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmO,
-                const AttnArgs a) {
+                const __grid_constant__ KvMaps<KV> cache, const AttnArgs a) {
   using C = FwdCfg<HD>;
   constexpr int PANELS = C::PANELS, TILE_BYTES = C::TILE_BYTES, STAGES = C::STAGES;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
@@ -160,6 +169,39 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     const uint32_t lead = elect_one();
     int g = 0, n = 0, nq = 0, nk = 0, nv = 0;    // key tiles, items; tiles asked for
     bool ok = true;
+    // An item's last key tile is its own rows' keys and values: they go on to the cache from where they lie, before
+    // the tile's place is loaded again.  32 rows per TMA store; the last rows of a sequence one by one, the
+    // slots behind them belong to others.
+    int keep = -1, keep_rows = 0;                // that tile (keep < 0: none), its rows in the sequence
+    long long keep_slot = 0;                     // and the first one's row of the cache
+    [[maybe_unused]] auto store_kept = [&]() {
+      if constexpr (KV) {
+        const int st = keep % STAGES, par = (keep / STAGES) & 1, whole = keep_rows & ~31;
+        keep = -1;
+        if (!mbar_wait_warp(&k_full[st], par, abort_flag) || !mbar_wait_warp(&v_full[st], par, abort_flag)) return false;
+        const uint8_t* k = sK + st * TILE_BYTES;
+        const uint8_t* v = sV + st * TILE_BYTES;
+        if (lead) {
+          for (int r = 0; r < whole; r += 32)
+#pragma unroll
+            for (int p = 0; p < PANELS; ++p) {
+              tma_store_2d(&cache.k, k + p * 16384 + r * 128, p * 64, static_cast<int>(keep_slot) + r);
+              tma_store_2d(&cache.v, v + p * 16384 + r * 128, p * 64, static_cast<int>(keep_slot) + r);
+            }
+          tma_store_commit();
+        }
+        for (int i = lane; i < (keep_rows - whole) * 8 * PANELS; i += 32) {
+          const int r = whole + i / (8 * PANELS), c = i % (8 * PANELS);          // row, 16-byte chunk of it
+          const uint32_t off = (c >> 3) * 16384 + sw128_chunk(r, c & 7);
+          const long long dst = (keep_slot + r) * HD + c * 8;
+          *reinterpret_cast<uint4*>(a.kc + dst) = *reinterpret_cast<const uint4*>(k + off);
+          *reinterpret_cast<uint4*>(a.vc + dst) = *reinterpret_cast<const uint4*>(v + off);
+        }
+        if (lead) tma_store_wait_read<0>();
+        __syncwarp();
+      }
+      return true;
+    };
     auto push = [&](const FwdItem& it) {
       const int s = n % FWD_QUEUE;
       if (!mbar_wait_warp(&item_empty[s], ((n / FWD_QUEUE) & 1) ^ 1, abort_flag)) return false;
@@ -196,6 +238,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           const int st = g % STAGES;
           const uint32_t par = ((g / STAGES) & 1) ^ 1;
           const int row_k = it.first + j * AT_BN;
+          if (KV && keep >= 0 && keep % STAGES == st && !(ok = store_kept())) break;
           if (!(ok = mbar_wait_warp(&k_empty[st], par, abort_flag))) break;
           mbar_expect_tx(&k_full[st], TILE_BYTES, lead);
 #pragma unroll
@@ -209,6 +252,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             tma_load_2d(sV + st * TILE_BYTES + p * 16384, &tmQKV, &v_full[st], 2 * d_model + it.h * HD + p * 64, row_k, lead);
           nv = g + 1;
         }
+        if (KV && ok) {
+          if (keep >= 0) ok = store_kept();
+          keep = g - 1;
+          keep_rows = min(AT_BM, it.T - it.qt * AT_BM);
+          keep_slot = (static_cast<long long>(it.b) * a.H + it.h) * a.slots + it.qt * AT_BM;
+        }
       }
       if (!a.take_over) break;
       // before the block leaves, too: the answer is written to its shared memory
@@ -219,6 +268,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       __syncwarp();
     }
     if (ok) { FwdItem end = {-1, 0, 0, 0, 0}; ok = push(end); }
+    if (KV && ok && keep >= 0) ok = store_kept();
     if (!ok) { *abort_flag = ST_TIMEOUT_EMPTY; if (lead) atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY); }
     // when a wait ran out, nobody has waited for these: they land before the block leaves
     for (int i = nq > STAGES ? nq - STAGES : 0; i < nq; ++i) mbar_wait_landed(&q_full[i % STAGES], (i / STAGES) & 1);
@@ -820,15 +870,22 @@ namespace ab {
 int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const AttnBwdArgs& a,
                             int* launched, cudaStream_t stream);   // attn_bwd_fused.cu
 
-template <int HD>
+template <int HD, bool KV>
 static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int dependent,
                            cudaStream_t stream) {
   // output map: boxes of 32 rows x 64 columns (half a math warp's rows at head_dim 128)
   CUtensorMap tmo;
-  const int rc_o = make_tmap_2d_sw(&tmo, a.out, rows, (uint64_t)a.H * HD, (uint64_t)a.H * HD, 32, 64, 2, 128);
-  if (rc_o) return rc_o;
+  int rc = make_tmap_2d_sw(&tmo, a.out, rows, (uint64_t)a.H * HD, (uint64_t)a.H * HD, 32, 64, 2, 128);
+  if (rc) return rc;
+  KvMaps<KV> cache;
+  if constexpr (KV) {                            // rows of HD
+    const uint64_t slots = (uint64_t)a.B * a.H * a.slots;
+    if (slots > 0x7fffffffull) return -1;
+    if ((rc = make_tmap_2d_sw(&cache.k, a.kc, slots, HD, HD, 32, 64, 2, 128)) != 0) return rc;
+    if ((rc = make_tmap_2d_sw(&cache.v, a.vc, slots, HD, HD, 32, 64, 2, 128)) != 0) return rc;
+  }
   constexpr int SMEM = FwdCfg<HD>::SMEM;
-  auto kern = attn_fwd_kernel<HD>;
+  auto kern = attn_fwd_kernel<HD, KV>;
   static PerDeviceOnce attr;
   if (attr.first_use_on_device()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -858,9 +915,9 @@ static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kern, tm, tmo, a);
+    return (int)cudaLaunchKernelEx(&cfg, kern, tm, tmo, cache, a);
   }
-  launch_chained(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, a);
+  launch_chained(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, cache, a);
   return (int)cudaGetLastError();
 }
 
@@ -911,25 +968,35 @@ int ab_attn_fwd(const void* qkv, void* out, float* lse, unsigned int* drop_mask,
   AttnArgs a;
   a.B = B; a.T = T; a.H = H; a.hd = hd; a.scale = scale; a.seed = seed; a.stream_id = stream_id;
   a.thr16 = thr16; a.out = (__nv_bfloat16*)out; a.lse = lse; a.status = status; a.salt = seed_salt_ptr();
-  a.drop_mask = drop_mask; a.row0 = nullptr;
+  a.drop_mask = drop_mask; a.row0 = nullptr; a.kc = a.vc = nullptr; a.slots = 0;
   const uint64_t rows = (uint64_t)B * T;
-  return hd == 64 ? launch_attn_fwd<64>(tm, a, rows, 0, stream) : launch_attn_fwd<128>(tm, a, rows, 0, stream);
+  return hd == 64 ? launch_attn_fwd<64, false>(tm, a, rows, 0, stream) : launch_attn_fwd<128, false>(tm, a, rows, 0, stream);
 }
 
 // The same over a packed batch without padding (inference: no dropout, no log-sum-exp): sequence b is
 // rows [row0[b], row0[b+1]) of qkv [rows, 3*H*hd]; T = longest sequence.  `dependent`: launched as a
-// programmatic dependent of the kernel before it.
-int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
-                       int dependent, int* status, cudaStream_t stream) {
+// programmatic dependent of the kernel before it.  kc, vc (optional, bf16 [B, H, slots, hd], 16-byte aligned): receive
+// the keys and values of every sequence in slots 0, 1, ...; T <= slots.
+int ab_attn_fwd_packed_kv(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
+                          void* kc, void* vc, int slots, int dependent, int* status, cudaStream_t stream) {
   using namespace ab;
   if ((hd != 64 && hd != 128) || B <= 0 || T <= 0 || rows < B || !row0) return -1;
+  if ((kc == nullptr) != (vc == nullptr) || (kc && T > slots)) return -1;
   CUtensorMap tm;
   int rc = make_tmap_2d(&tm, qkv, (uint64_t)rows, 3ull * H * hd, 3ull * H * hd, 128, 64, 2, true);
   if (rc) return rc;
   AttnArgs a = {};
   a.B = B; a.T = T; a.row0 = row0; a.H = H; a.hd = hd; a.scale = scale; a.out = (__nv_bfloat16*)out; a.status = status;
-  return hd == 64 ? launch_attn_fwd<64>(tm, a, rows, dependent, stream)
-                  : launch_attn_fwd<128>(tm, a, rows, dependent, stream);
+  a.kc = (__nv_bfloat16*)kc; a.vc = (__nv_bfloat16*)vc; a.slots = slots;
+  if (kc)
+    return hd == 64 ? launch_attn_fwd<64, true>(tm, a, rows, dependent, stream)
+                    : launch_attn_fwd<128, true>(tm, a, rows, dependent, stream);
+  return hd == 64 ? launch_attn_fwd<64, false>(tm, a, rows, dependent, stream)
+                  : launch_attn_fwd<128, false>(tm, a, rows, dependent, stream);
+}
+int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
+                       int dependent, int* status, cudaStream_t stream) {
+  return ab_attn_fwd_packed_kv(qkv, out, row0, B, T, rows, H, hd, scale, nullptr, nullptr, 0, dependent, status, stream);
 }
 
 // delta: fp32 scratch [B,H,T] owned by the caller.  drop_mask (optional): the keep bits the forward

@@ -4,7 +4,6 @@
 //
 //   gather_rows : the last rows of the residual stream and of the attention output, after the last
 //                 layer's attention; everything behind it runs on one row per sequence
-//   kv_store    : keys / values of a packed prompt batch into the per-tree cache of the search
 //   ab_infer_last : the schedule of one such pass.  It is native because a pass of the medium model is
 //                 170 launches: about 15 us each from Python against 3 us from here, and a single short
 //                 game needs less than that on the GPU.
@@ -23,25 +22,6 @@ gather_rows_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict_
     reinterpret_cast<uint4*>(y_out + dst * d)[i] = reinterpret_cast<const uint4*>(y + src * d)[i];
     reinterpret_cast<float4*>(x_out + dst * d)[2 * i] = reinterpret_cast<const float4*>(x + src * d)[2 * i];
     reinterpret_cast<float4*>(x_out + dst * d)[2 * i + 1] = reinterpret_cast<const float4*>(x + src * d)[2 * i + 1];
-  }
-}
-
-// Rows [row0[t], row0[t + 1]) of the packed QKV activation -> slots 0.. of tree t.  Bound by bytes:
-// a block copies KV_ROWS rows, so every thread has several independent 16-byte loads in flight.
-constexpr int KV_ROWS = 8;
-__global__ void __launch_bounds__(256)
-kv_store_packed_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ kc,
-                       __nv_bfloat16* __restrict__ vc, const int* __restrict__ row0, int S, int d, int hd) {
-  griddep_enter();
-  const int t = blockIdx.y, first = row0[t], len = row0[t + 1] - first;
-  const int p0 = blockIdx.x * KV_ROWS, rows = min(KV_ROWS, len - p0);
-  const int n8 = d / 8, hd8 = hd / 8, H = d / hd;
-  for (int i = threadIdx.x; i < rows * 2 * n8; i += 256) {
-    const int r = i / (2 * n8), c = i - r * 2 * n8;             // c < n8: keys, else values
-    const int col = c < n8 ? c : c - n8, h = col / hd8;
-    const uint4 w = reinterpret_cast<const uint4*>(qkv + (static_cast<long long>(first) + p0 + r) * 3 * d)[n8 + c];
-    const long long dst = ((static_cast<long long>(t) * H + h) * S + p0 + r) * hd8 + (col - h * hd8);
-    reinterpret_cast<uint4*>(c < n8 ? kc : vc)[dst] = w;
   }
 }
 
@@ -90,8 +70,8 @@ int ab_heads_fwd(const void*, const float*, const float*, const float*, const fl
                  const int*, float, float, float*, float*, float*, float*, float*, int, int, cudaStream_t);
 int ab_heads_fwd_ahead(const void*, const float*, const float*, const float*, const float*, float*, float*, int, int,
                        cudaStream_t);
-int ab_attn_fwd_packed(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
-                       int dependent, int* status, cudaStream_t stream);
+int ab_attn_fwd_packed_kv(const void* qkv, void* out, const int* row0, int B, int T, int rows, int H, int hd, float scale,
+                          void* kc, void* vc, int slots, int dependent, int* status, cudaStream_t stream);
 
 // Returns the number of kernels launched, or a negative number / minus a cudaError_t.
 int ab_infer_last(const AbInfer* p, const AbInferLayer* layers, cudaStream_t stream) {
@@ -129,16 +109,12 @@ int ab_infer_last(const AbInfer* p, const AbInferLayer* layers, cudaStream_t str
     AB_TRY(norm(x, L.ln1_w, L.ln1_b, a.ln, M));
     const long long dd = static_cast<long long>(a.d) * a.d, df = static_cast<long long>(a.d) * a.F;
     AB_TRY(gemm(a.ln, a.d, L.qkv_w, 1, L.qkv_b, 0, a.qkv, 0, M, 3 * a.d, L.o_w, dd));
-    if (a.kc) {
-      __nv_bfloat16* kc = static_cast<__nv_bfloat16*>(a.kc) + l * a.kv_layer;
-      __nv_bfloat16* vc = static_cast<__nv_bfloat16*>(a.vc) + l * a.kv_layer;
-      kv_store_packed_kernel<<<dim3((a.T + KV_ROWS - 1) / KV_ROWS, a.n), 256, 0, stream>>>(
-          static_cast<const __nv_bfloat16*>(a.qkv), kc, vc, a.row0, a.S, a.d, a.hd);
-      AB_TRY((int)cudaGetLastError());
-      ++launched;
-    }
-    AB_TRY(ab_attn_fwd_packed(a.qkv, a.att, a.row0, a.n, a.T, M, a.H, a.hd, 1.f / sqrtf((float)a.hd), dep, a.status,
-                              stream));
+    // the keys and values of a search's prompts go on to its cache from the attention's shared memory (a kernel of
+    // its own took 59 us per layer for 39000 rows of 1024)
+    __nv_bfloat16* kc = a.kc ? static_cast<__nv_bfloat16*>(a.kc) + l * a.kv_layer : nullptr;
+    __nv_bfloat16* vc = a.kc ? static_cast<__nv_bfloat16*>(a.vc) + l * a.kv_layer : nullptr;
+    AB_TRY(ab_attn_fwd_packed_kv(a.qkv, a.att, a.row0, a.n, a.T, M, a.H, a.hd, 1.f / sqrtf((float)a.hd), kc, vc, a.S, dep,
+                                 a.status, stream));
     ++launched;
     if (l == a.n_layer - 1) {
       launch_chained(gather_rows_kernel, dim3(a.n), dim3(128), 0, stream, (const float*)x,

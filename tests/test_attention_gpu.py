@@ -392,3 +392,46 @@ def test_dropout_of_blocks_that_take_over_others(B, T, H, hd):
     ref, lse_ref = _ref(qkv, B, T, H, hd, keep.float(), 65536.0 / (65536 - thr))
     assert torch.allclose(out.float(), ref, rtol=3e-2, atol=3e-2)
     assert torch.allclose(lse, lse_ref, rtol=1e-3, atol=1e-2)
+
+
+@pytest.mark.parametrize("hd,H,lens", [
+    (64, 16, [300] * 20), (64, 8, [1, 128, 129, 300, 4, 257, 31, 32, 33, 160] * 9), (64, 3, [700, 1, 1, 1, 128] * 20 + [5]),
+    (128, 8, [1, 128, 129, 300, 4, 257, 31, 32, 33, 160] * 9), (128, 5, [384] * 20), (64, 2, [90]), (128, 2, [97, 40]),
+])
+def test_keys_and_values_of_a_packed_batch_in_a_cache(hd, H, lens):
+    """Sequence ends inside and at blocks of 32 rows: the rows as they are, no slot behind a sequence touched."""
+    import ctypes
+
+    import numpy as np
+
+    from allie_b200.ops import _lib
+
+    torch.manual_seed(5)
+    lib, d, S, n = _lib.cuda(), H * hd, max(lens) + 3, len(lens)
+    starts = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    row0 = torch.from_numpy(starts).cuda()
+    M = int(starts[-1])
+    qkv = (torch.randn(M, 3 * d, device="cuda") * 0.7).bfloat16()
+    P = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+
+    def run(kc, vc):
+        out = torch.empty(M, d, device="cuda", dtype=torch.bfloat16)
+        assert lib.ab_attn_fwd_packed_kv(P(qkv), P(out), P(row0), n, max(lens), M, H, hd, ctypes.c_float(hd ** -0.5), P(kc),
+                                         P(vc), S, 0, P(_lib.status_word()),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        return out
+
+    kc, vc = (torch.full((n, H, S, hd), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    out = run(kc, vc)
+    assert torch.equal(out, run(None, None))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for i, (a, b) in enumerate(zip(starts[:-1], starts[1:])):
+        rows = qkv[a:b].view(b - a, 3, H, hd)
+        for cache, part in ((kc, 1), (vc, 2)):
+            assert torch.equal(cache[i, :, :b - a], rows[:, part].transpose(0, 1)), i
+            assert (cache[i, :, b - a:] == 7.0).all(), i
+    args = [P(qkv), P(out), P(row0), n, max(lens), M, H, hd, ctypes.c_float(0.1)]
+    end = [0, P(_lib.status_word()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)]
+    assert lib.ab_attn_fwd_packed_kv(*args, P(kc), P(vc), max(lens) - 1, *end) == -1      # a sequence that has no room
+    assert lib.ab_attn_fwd_packed_kv(*args, P(kc), P(None), S, *end) == -1
