@@ -343,10 +343,17 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
 // blockIdx.x + gridDim.x, ... and, for each, the key tiles 0..nt-1, as ONE pipeline over
 // (query tile, key tile) pairs.  K/V are double-buffered across key tiles, the Q/dO ring and the
 // S/dP, P/dS and dQ hand-offs run on a pair counter that never restarts, and the end-of-tile work
-// of key tile w (last dQ drain, dV/dK read-out and store) is done by the math warps after the
-// P/dS math of the first pair of key tile w + 1, while the tensor core already works on that pair.
+// of key tile w (last dQ drain, dV/dK read-out and store) runs beside the first pair of key tile w + 1.
 // So the per-key-tile prologue (TMEM allocation, barrier set-up, first loads) and tail, which cost
 // as much as two pairs in the one-tile-per-CTA kernel, are paid once per CTA.
+// Four warps of their own, one per TMEM lane quarter, take the results out: the dQ tile of every pair, and dV / dK
+// where a key tile ends.  Done by the math warps between pairs this was 1100 of a pair's 5000 clocks, and these are
+// what a pair waits for (the tensor core is done early, nobody waits for it).  us with
+// dropout 0.1, before and now: 64 x 512 x 16 heads 258 and 191, 32 x 512 x 20 188 and 141, 37 x 328 x 12 90 and 71,
+// 16 x 1000 x 16 267 and 218.
+
+constexpr int FBP_DRAIN_WARPS = 4;
+constexpr int FBP_THREADS = FB_THREADS + FBP_DRAIN_WARPS * 32;
 
 struct FbWalk {
   int bh, own, it, nt, bh_end, step;
@@ -365,12 +372,11 @@ struct FbWalk {
 
 // RAGGED: T is no multiple of 128; the last 32-row blocks of a sequence are stored row by row
 template <bool RAGGED>
-__global__ void __launch_bounds__(FB_THREADS, 1)
+__global__ void __launch_bounds__(FBP_THREADS, 1)
 attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
                                    const __grid_constant__ CUtensorMap tmDO,
                                    const __grid_constant__ CUtensorMap tmDQ,
-                                   const __grid_constant__ CUtensorMap tmDKV,
-                                   const __grid_constant__ CUtensorMap tmDQB, const AttnBwdArgs a) {
+                                   const __grid_constant__ CUtensorMap tmOut, const AttnBwdArgs a) {
   griddep_enter();
   constexpr int HD = 64;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
@@ -389,8 +395,8 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
   uint8_t* sDO = sQ + 2 * FB_TILE;       // 2 stages
   uint8_t* sP = sDO + 2 * FB_TILE;
   uint8_t* sDS = sP + FB_P;
-  uint8_t* sDQ = sDS + FB_P;             // 16 warps x 2 KB staging for the dQ reduce-adds
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDQ + FB_MATH_WARPS * 2048);
+  uint8_t* sDQ = sDS + FB_P;             // staging of the drain warps, 8 KB each
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDQ + FBP_DRAIN_WARPS * 8192);
   uint64_t* kv_full = bars;        // 2
   uint64_t* kv_empty = bars + 2;   // 2
   uint64_t* full = bars + 4;       // 2
@@ -414,17 +420,17 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     for (int i = 0; i < 2; ++i) {
       mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1);
       mbar_init(&full[i], 1); mbar_init(&empty[i], 1);
-      mbar_init(&dq_full[i], 1); mbar_init(&dq_empty[i], FB_MATH_WARPS);
+      mbar_init(&dq_full[i], 1); mbar_init(&dq_empty[i], FBP_DRAIN_WARPS);
     }
     mbar_init(sdp_full, 1); mbar_init(sdp_empty, FB_MATH_WARPS);
     mbar_init(pds_full, FB_MATH_WARPS); mbar_init(pds_empty, 1);
-    mbar_init(acc_full, 1); mbar_init(acc_empty, FB_MATH_WARPS);
+    mbar_init(acc_full, 1); mbar_init(acc_empty, FBP_DRAIN_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQKV);
     tma_prefetch_desc(&tmDO);
     tma_prefetch_desc(&tmDQ);
-    tma_prefetch_desc(&tmDKV);
+    tma_prefetch_desc(&tmOut);
   }
   if (warp == FB_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -526,6 +532,194 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       }
       if (!ok) { *abort_flag = ST_TIMEOUT_FULL; if (lead) atomicCAS(a.status, 0, ST_TIMEOUT_FULL); }
     }
+  } else if (warp > FB_MMA_WARP) {
+    // ----------------------------------------------------------- drain warps
+    const int quad = warp & 3, r = quad * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    // Staging: two tiles of 32 rows of 128 bytes (128B swizzle), 32 fp32 or 64 bf16 columns.  A lane reads and
+    // writes its own row.
+    uint8_t* stg = sDQ + quad * 8192;
+    uint8_t* my_row = stg + lane * 128;
+    auto at = [&](int k) { return ((k ^ (lane & 7)) << 4); };           // 16-byte chunk k of it
+    bool ok = true;
+
+    // The dQ sums of the slice that this CTA works on live in a place of its own in dq_acc (nt - 1 tiles of 128
+    // rows of 64 columns: query tile 0 has one pair and needs none) and nowhere else, so 148 slices stay in L2 instead of every slice passing through
+    // memory twice, and no pass converts or clears them: key tile 0 stores its contributions, later ones
+    // add, and the last one of a query tile (its diagonal pair) reads the sum back, adds its own part from
+    // TMEM and stores bf16 into dQKV.  The same warp does all of it for its rows.
+    const int s_row0 = (static_cast<int>(blockIdx.x) * (nt - 1) - 1) * 128 + quad * 32;    // of query tile 0, if it had one
+    // rows past the end of a sequence are the next one's: P and dS, and so dQ, dK and dV, are zeros there
+    auto whole_rows = [&](int row) { return !RAGGED || row + 32 <= a.T; };
+    // adds the column sums of a staged tile of 64 bf16 columns to dst: a lane takes two columns
+    auto add_colsum = [&](const uint8_t* tile, float* dst) {
+      uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + k * 128 + (((lane >> 2) ^ (k & 7)) << 4) + (lane & 3) * 4);
+        sum[k & 3] = f2_add(sum[k & 3], f2_pack(bf16_lo(w), bf16_hi(w)));
+      }
+      float s0, s1;
+      f2_unpack(f2_add(f2_add(sum[0], sum[1]), f2_add(sum[2], sum[3])), s0, s1);
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst + lane * 2), "f"(s0), "f"(s1) : "memory");
+    };
+
+    // The sum so far of query tile `own`, into the staging tiles, while
+    // the pair that completes it is still computed: behind it, the wait for this warp's earlier contributions and
+    // the trip to L2 were 6000 of 7500 clocks.
+    auto fetch_sum = [&](int own) {
+      if (lane == 0) {
+        // They are in memory: the last was for the second pair of key tile own - 1, behind which came nt - own - 1
+        // pairs and the stores of that tile's dV / dK (a whole tile, so a group of its own).
+        if (nt - own >= 3) tma_store_wait<3>();
+        else if (nt - own == 2) tma_store_wait<2>();
+        else tma_store_wait<1>();
+        tma_store_wait_read<0>();                // and the staging tiles are free
+        asm volatile("fence.proxy.async;" ::: "memory");
+      }
+      __syncwarp();
+      const float* src = a.dq_acc + (static_cast<long long>(s_row0) + own * 128) * HD;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int row = i * 2 + (lane >> 4), k = lane & 15;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                     ::"r"(smem_u32(stg + (k >> 3) * 4096 + row * 128 + (((k & 7) ^ (row & 7)) << 4))), "l"(src + row * HD + k * 4)
+                     : "memory");
+      }
+    };
+    // the dQ tile of pair g (query tile own + it of head h of sequence b)
+    auto drain_dq = [&](int g, int b, int h, int own, int it) {
+      const bool last = it == 0, summed = last && own > 0;
+      if (summed) fetch_sum(own);
+      const bool there = mbar_wait(&dq_full[g & 1], (g >> 1) & 1, abort_flag);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (!there) return false;
+      tc_fence_after();
+      if (lane == 0 && !summed) tma_store_wait_read<0>();
+      __syncwarp();
+      const int qrow = (own + it) * 128;
+      const bool rows_whole = whole_rows(qrow + quad * 32);            // warp-uniform
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {           // 32 columns
+        uint32_t v[32];
+        tmem_ld32(tDQ + (g & 1) * 64 + lane_addr + hf * 32, v);
+        float4 x[8];                             // the sum so far
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          x[k] = summed ? *reinterpret_cast<const float4*>(my_row + hf * 4096 + at(k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        tmem_ld_wait();
+        if (hf == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&dq_empty[g & 1]);
+        }
+        if (last) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 lo = x[2 * k], hi = x[2 * k + 1];
+            const uint32_t* f = v + k * 8;
+            auto f_ = [&](int i) { return __uint_as_float(f[i]); };
+            const uint4 w = make_uint4(pack_bf16x2(f_(0) + lo.x, f_(1) + lo.y), pack_bf16x2(f_(2) + lo.z, f_(3) + lo.w),
+                                       pack_bf16x2(f_(4) + hi.x, f_(5) + hi.y), pack_bf16x2(f_(6) + hi.z, f_(7) + hi.w));
+            *reinterpret_cast<uint4*>(my_row + at(hf * 4 + k)) = w;
+            if (!rows_whole && qrow + r < a.T)
+              *reinterpret_cast<uint4*>(a.dqkv + (static_cast<long long>(b) * a.T + qrow + r) * (3 * d_model) + h * HD + hf * 32 + k * 8) = w;
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            *reinterpret_cast<uint4*>(my_row + hf * 4096 + at(k)) = make_uint4(v[k * 4], v[k * 4 + 1], v[k * 4 + 2], v[k * 4 + 3]);
+        }
+      }
+      // the first store into the slice's place: behind the reads of what was there for the slice before
+      if (own == 0 && it == 1) asm volatile("fence.proxy.async;" ::: "memory");
+      else fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (last) {
+          if (rows_whole) tma_store_2d(&tmOut, stg, h * HD, b * a.T + qrow + quad * 32);
+        } else if (own == 0) {
+          tma_store_2d(&tmDQ, stg, 0, s_row0 + qrow);
+          tma_store_2d(&tmDQ, stg + 4096, 32, s_row0 + qrow);
+        } else {     // (own == 1 adds to what own == 0 stored: those stores were waited for at its diagonal pair)
+          tma_reduce_add_2d(&tmDQ, stg, 0, s_row0 + qrow);
+          tma_reduce_add_2d(&tmDQ, stg + 4096, 32, s_row0 + qrow);
+        }
+        tma_store_commit();
+      }
+      if (last && a.dbias) add_colsum(stg, a.dbias + h * HD);
+      return true;
+    };
+    // reads the finished dV / dK of key tile w out of TMEM, frees them, and stores them
+    auto finish_tile = [&](int w, int b, int h, int own) {
+      if (!mbar_wait(acc_full, w & 1, abort_flag)) return false;
+      tc_fence_after();
+      const bool rows_whole = whole_rows(own * 128 + quad * 32);       // warp-uniform
+      const int t_idx = own * 128 + r;
+      // dV, then dK, one TMA store each.  (Plain stores of 64-byte row pieces 6 KB apart kept the load/store unit
+      // busy for thousands of cycles per key tile and delayed every other warp's shared-memory traffic with them.)
+#pragma unroll 1
+      for (int m = 0; m < 2; ++m) {
+        uint32_t w[32];                                                // 64 columns as bf16 pairs
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t v[32];
+          tmem_ld32((m ? tDK : tDV) + c * 32 + lane_addr, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int k = 0; k < 16; ++k) w[c * 16 + k] = pack_bf16x2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+        }
+        if (m == 1) tc_fence_before();
+        else if (lane == 0) tma_store_wait_read<0>();                  // the staging tiles are free
+        __syncwarp();
+        if (m == 1 && lane == 0) mbar_arrive(acc_empty);
+        const int col = (m ? d_model : 2 * d_model) + h * HD;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint4 wv = make_uint4(w[k * 4], w[k * 4 + 1], w[k * 4 + 2], w[k * 4 + 3]);
+          *reinterpret_cast<uint4*>(my_row + m * 4096 + at(k)) = wv;
+          if (!rows_whole && t_idx < a.T)
+            *reinterpret_cast<uint4*>(a.dqkv + (static_cast<long long>(b) * a.T + t_idx) * (3 * d_model) + col + k * 8) = wv;
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (rows_whole) {
+          tma_store_2d(&tmOut, stg, 2 * d_model + h * HD, b * a.T + own * 128 + quad * 32);
+          tma_store_2d(&tmOut, stg + 4096, d_model + h * HD, b * a.T + own * 128 + quad * 32);
+        }
+        tma_store_commit();
+      }
+      if (a.dbias) {
+        add_colsum(stg, a.dbias + 2 * d_model + h * HD);
+        add_colsum(stg + 4096, a.dbias + d_model + h * HD);
+      }
+      return true;
+    };
+    int b = 0, h = 0;
+    for (FbWalk p = start; p.valid() && ok; p.next()) {
+      if (p.it == 0 && p.own == 0) { b = p.bh / a.H; h = p.bh - b * a.H; }
+      ok = drain_dq(p.g, b, h, p.own, p.it);
+      if (ok && p.last()) ok = finish_tile(p.w, b, h, p.own);
+      __syncwarp();                                // the staging tiles have been read by all lanes
+    }
+    if (ok && start.valid() && nt > 1) {
+      // hand the accumulator back all zero (query tile 0 never went through it)
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) *reinterpret_cast<float4*>(my_row + k * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+      asm volatile("fence.proxy.async;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        for (int i = 1; i < nt; ++i)
+          for (int hf = 0; hf < 2; ++hf) tma_store_2d(&tmDQ, stg, hf * 32, s_row0 + i * 128);
+        tma_store_commit();
+      }
+    }
+    if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
+    if (lane == 0) tma_store_wait<0>();
   } else {
     // ------------------------------------------------------------ math warps
     const int quad = warp & 3, cb = warp >> 2;
@@ -533,154 +727,8 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float sl2 = a.scale * LOG2E;
     const float dscale = dropout_scale(a.thr16);
-    uint8_t* my_dq = sDQ + warp * 2048;
     bool ok = true;
 
-    // The dQ sums of the slice that this CTA works on live in a place of its own in dq_acc (nt tiles of 128
-    // rows of 64 columns) and nowhere else, so 148 slices stay in L2 instead of every slice passing through
-    // memory twice, and no pass converts or clears them: key tile 0 stores its contributions, later ones
-    // add, and the last one of a query tile (its diagonal pair) reads the sum back, adds its own part from
-    // TMEM and stores bf16 into dQKV.  The same warp does all of it for its rows and columns.
-    const int s_row0 = static_cast<int>(blockIdx.x) * nt * 128 + quad * 32, s_col = cb * 16;
-    // rows past the end of a sequence are the next one's: P and dS, and so dQ, dK and dV, are zeros there
-    auto whole_rows = [&](int row) { return !RAGGED || row + 32 <= a.T; };
-    // adds the column sums of a staged bf16 tile (32 rows of `cols` columns) to dst: a lane takes two
-    // columns of every (64 / cols)-th row, so each load of the warp reads 128 contiguous bytes
-    auto add_colsum = [&](const uint8_t* tile, int cols, float* dst) {
-      const int pairs = cols >> 1, cp = lane % pairs, rows = 32 / pairs;
-      uint64_t sum = 0ull;
-      for (int row = lane / pairs; row < 32; row += rows) {
-        const int sw = cols == 32 ? ((row >> 1) & 3) : ((row >> 2) & 1);
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + row * cols * 2 + (((cp >> 2) ^ sw) << 4) + (cp & 3) * 4);
-        sum = f2_add(sum, f2_pack(bf16_lo(w), bf16_hi(w)));
-      }
-      float s0, s1;
-      f2_unpack(sum, s0, s1);
-      for (int o = pairs; o < 32; o <<= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      }
-      if (lane < pairs)
-        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst + cp * 2), "f"(s0), "f"(s1) : "memory");
-    };
-
-    // drains the dQ tile of pair g (query tile own + it of head h of sequence b, this warp's 16 columns)
-    auto drain_dq = [&](int g, int b, int h, int own, int it) {
-      if (!mbar_wait(&dq_full[g & 1], (g >> 1) & 1, abort_flag)) return false;
-      tc_fence_after();
-      uint32_t v[16];
-      tmem_ld16(tDQ + (g & 1) * 64 + lane_addr + cb * 16, v);
-      const bool last = it == 0;
-      if (lane == 0) {
-        if (last && own > 0) {
-          tma_store_wait<0>();                   // this warp's earlier contributions are in memory
-          asm volatile("fence.proxy.async;" ::: "memory");
-        } else {
-          tma_store_wait_read<0>();
-        }
-      }
-      __syncwarp();
-      tmem_ld_wait();
-      tc_fence_before();
-      const int qrow = (own + it) * 128;
-      if (last) {
-        float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
-        if (own > 0) {
-          const float4* src = reinterpret_cast<const float4*>(
-              a.dq_acc + (static_cast<long long>(s_row0) + qrow + lane) * HD + s_col);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 t = __ldcg(src + c);
-            f[c * 4 + 0] += t.x; f[c * 4 + 1] += t.y; f[c * 4 + 2] += t.z; f[c * 4 + 3] += t.w;
-          }
-        }
-        // 16 bf16 columns = 32-byte rows, 32B swizzle
-        uint8_t* rowp = my_dq + lane * 32;
-        const int sw = (lane >> 2) & 1;
-        const bool rows_whole = whole_rows(qrow + quad * 32);          // warp-uniform
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const uint4 w = make_uint4(pack_bf16x2(f[c * 8 + 0], f[c * 8 + 1]), pack_bf16x2(f[c * 8 + 2], f[c * 8 + 3]),
-                                     pack_bf16x2(f[c * 8 + 4], f[c * 8 + 5]), pack_bf16x2(f[c * 8 + 6], f[c * 8 + 7]));
-          *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = w;
-          if (!rows_whole && qrow + r < a.T)
-            *reinterpret_cast<uint4*>(a.dqkv + (static_cast<long long>(b) * a.T + qrow + r) * (3 * d_model) + h * HD + cb * 16 + c * 8) = w;
-        }
-        asm volatile("fence.proxy.async;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&dq_empty[g & 1]);
-          if (rows_whole) {
-            tma_store_2d(&tmDQB, my_dq, h * HD + cb * 16, b * a.T + qrow + quad * 32);
-            tma_store_commit();
-          }
-        }
-        if (a.dbias) add_colsum(my_dq, 16, a.dbias + h * HD + cb * 16);
-        return true;
-      }
-      uint8_t* rowp = my_dq + lane * 64;       // 16 fp32 columns = 64-byte rows, 64B swizzle
-      const int sw = (lane >> 1) & 3;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<float4*>(rowp + ((c ^ sw) << 4)) =
-            make_float4(__uint_as_float(v[c * 4 + 0]), __uint_as_float(v[c * 4 + 1]),
-                        __uint_as_float(v[c * 4 + 2]), __uint_as_float(v[c * 4 + 3]));
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&dq_empty[g & 1]);
-        // (own == 1 adds to what own == 0 stored: those stores were waited for at its diagonal pair)
-        if (own == 0) tma_store_2d(&tmDQ, my_dq, s_col, s_row0 + qrow);
-        else          tma_reduce_add_2d(&tmDQ, my_dq, s_col, s_row0 + qrow);
-        tma_store_commit();
-      }
-      return true;
-    };
-    // reads the finished dV / dK of key tile w out of TMEM, frees them, and stores them
-    auto finish_tile = [&](int w, int b, int h, int own) {
-      if (!mbar_wait(acc_full, w & 1, abort_flag)) return false;
-      tc_fence_after();
-      // 4 chunks of 32 columns: dV chunks 0,1 then dK chunks 0,1; warp group cb takes chunk cb
-      const uint32_t tacc = (cb < 2 ? tDV : tDK) + (cb & 1) * 32;
-      uint32_t v[32];
-      tmem_ld32(tacc + lane_addr, v);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
-      // 32 rows x 32 bf16 columns per warp: staged with 64-byte swizzle, one TMA store.  (Plain
-      // stores of 64-byte row pieces 6 KB apart kept the load/store unit busy for thousands of
-      // cycles per key tile and delayed every other warp's shared-memory traffic with them.)
-      if (lane == 0) tma_store_wait_read<0>();
-      __syncwarp();
-      uint8_t* rowp = my_dq + lane * 64;
-      const int sw = (lane >> 1) & 3;
-      const bool rows_whole = whole_rows(own * 128 + quad * 32);       // warp-uniform
-      const int t_idx = own * 128 + r, col = (cb < 2 ? 2 * d_model : d_model) + h * HD + (cb & 1) * 32;
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        uint4 wv;
-        wv.x = pack_bf16x2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-        wv.y = pack_bf16x2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-        wv.z = pack_bf16x2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-        wv.w = pack_bf16x2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-        *reinterpret_cast<uint4*>(rowp + ((q4 ^ sw) << 4)) = wv;
-        if (!rows_whole && t_idx < a.T)
-          *reinterpret_cast<uint4*>(a.dqkv + (static_cast<long long>(b) * a.T + t_idx) * (3 * d_model) + col + q4 * 8) = wv;
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && rows_whole) {
-        tma_store_2d(&tmDKV, my_dq, col, b * a.T + own * 128 + quad * 32);
-        tma_store_commit();
-      }
-      if (a.dbias) add_colsum(my_dq, 32, a.dbias + col);
-      return true;
-    };
-
-    int prev_h = 0, prev_b = 0, prev_own = 0, prev_it = 0;       // pair g - 1 / its key tile
     // per-row inputs of a pair: log-sum-exp, delta and the 32 dropout keep bits of this thread's
     // columns.  They are fetched one pair ahead so their latency never sits in the pair's chain.
     // Addresses advance by fixed strides from one query tile to the next, so they are rebuilt from
@@ -717,12 +765,10 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       }
     };
     FbWalk p = start;
-    int b = 0, h = 0;
     float lse_raw = 0.f, dlt = 0.f;
     uint32_t keep32 = 0xffffffffu;
     if (p.valid()) fetch(p, lse_raw, dlt, keep32);
     for (; p.valid() && ok; p.next()) {
-      if (p.it == 0 && p.own == 0) { b = p.bh / a.H; h = p.bh - b * a.H; }
       const bool diag = p.it == 0;
       float n_lse = 0.f, n_dlt = 0.f;
       uint32_t n_keep = 0xffffffffu;
@@ -775,33 +821,9 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_full);
-      // work left over from the previous pair, done while the tensor core runs this one
-      if (p.g > 0) {
-        ok = drain_dq(p.g - 1, prev_b, prev_h, prev_own, prev_it);
-        if (ok && p.first()) ok = finish_tile(p.w - 1, prev_b, prev_h, prev_own);
-      }
-      prev_h = h; prev_b = b; prev_own = p.own; prev_it = p.it;
       lse_raw = n_lse; dlt = n_dlt; keep32 = n_keep;
     }
-    if (ok && p.g > 0) {
-      ok = drain_dq(p.g - 1, prev_b, prev_h, prev_own, prev_it);
-      if (ok) ok = finish_tile(p.w - 1, prev_b, prev_h, prev_own);
-      if (ok && nt > 1) {
-        // hand the accumulator back all zero (query tile 0 never went through it)
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(my_dq + lane * 64 + c * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          for (int i = 1; i < nt; ++i) tma_store_2d(&tmDQ, my_dq, s_col, s_row0 + i * 128);
-          tma_store_commit();
-        }
-      }
-    }
     if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
-    if (lane == 0) tma_store_wait<0>();
   }
   tc_fence_before();
   __syncthreads();
@@ -850,20 +872,19 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
   const int mode = attn_bwd_schedule_mode();
   const bool ragged = (a.T & 127) != 0;
   const int bh = a.B * a.H, ctas = bh < 148 ? bh : 148, nt = (a.T + 127) / 128;
-  // every CTA of the walk has a place for the sums of one slice in dq_acc
-  const bool fits = nt == 1 || static_cast<long long>(ctas) * nt * 128 <= rows * a.H;
-  // The walk hands whole slices to CTAs; few, long ones leave SMs idle, which the grid of key tiles does not.  In
-  // pairs of tiles: a slice is nt (nt + 1) / 2 of them; a key tile by itself costs two more (start and end), and the
-  // conversion, clearing and column sums behind the grid about four.  Dropout 0.1, grid and walk, us: 37 x 328
-  // x 12 heads 138 and 90, 16 x 512 x 16 118 and 84, 25 x 400 x 12 138 and 132, 8 x 256 x 4 32 and 22.
-  const long long slice = static_cast<long long>(nt) * (nt + 1) / 2;
-  const long long grid_pairs = std::max(nt + 2ll, bh * (slice + 2 * nt) / 148) + 4;
-  // A tenth in favour of the grid: 30 x 1000 x 10, level by this count, 360 and 387 (it also leaves 4 x 512 x 16 there,
-  // 48 and 45).  Under 32 slices the grid whatever the count says, which is wrong for three key tiles: 384 keys
-  // and 1 to 5 slices 28 and 31 us, level from 16 on.  For one and two tiles the walk would be the faster there, too,
-  // as above the line: 4 slices of 128 keys 24 and 12, of 256 keys 26 and 21.
-  const bool walk = bh >= 32 && 10 * ((bh + 147) / 148 * slice + 1) <= 9 * grid_pairs;
-  if (mode == 1 || !fits || (mode == 0 && !walk)) {
+  // The walk hands whole slices to CTAs (each has a place for the sums of one in dq_acc: nt - 1 tiles of 128 rows, fewer
+  // than T); few, long ones leave SMs idle, which the grid of key tiles does not.  us, from launches of 1 to 320 slices
+  // of 1 to 8 tiles: a slice of nt (nt + 1) / 2 pairs of tiles takes the walk 2.2 a pair and 5 in all; the grid
+  // 11.5 with the conversion, clearing and column sums behind it, and the longer of its longest CTA (2.1 a query
+  // tile) and of all its CTAs' work (5 a pair, two pairs' worth per key tile to start and end).  Grid and walk: 1 slice
+  // of 2 tiles 15.7 and 13.9, of 3 18.4 and 20.5; 32 of 4 36 and 30, of 6 51 and 52; 64 of 6 80 and 52; 148 of 4 104
+  // and 39; 200 of 1000 keys 367 and 213.  Up to 16 slices the grid whatever the count says (the test of a replayed
+  // step counts that many launches); of one or two tiles the walk would take 0.5 to 0.9 of its time there.
+  const double slice = 0.5 * nt * (nt + 1);
+  const double walk_us = 5.0 + 2.2 * ((bh + 147) / 148) * slice;
+  const double grid_us = 11.5 + std::max(2.1 * nt, 5.0 * bh * (slice + 2 * nt) / 148);
+  const bool walk = bh > 16 && walk_us <= grid_us;
+  if (mode == 1 || (mode == 0 && !walk)) {
     constexpr int SMEM = 6 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
     static PerDeviceOnce attr;
     if (attr.first_use_on_device()) {
@@ -876,7 +897,7 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
     launch_chained(attn_bwd_fused64_kernel, dim3(grid), dim3(FB_THREADS), SMEM, stream, tq, td, tdq, a);
     ++*launched;
   } else {
-    constexpr int SMEM = 8 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
+    constexpr int SMEM = 8 * FB_TILE + 2 * FB_P + FBP_DRAIN_WARPS * 8192 + 256;
     auto kern = ragged ? attn_bwd_fused64_persistent_kernel<true> : attn_bwd_fused64_persistent_kernel<false>;
     static PerDeviceOnce attr[2];
     if (attr[ragged].first_use_on_device()) {
@@ -884,16 +905,13 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
       if (e != cudaSuccess) return (int)e;
       attr[ragged].mark_device();
     }
-    CUtensorMap tdkv;     // the packed dQKV activation, boxes of 32 rows x 32 columns for dK / dV
-    rc = make_tmap_2d_sw(&tdkv, a.dqkv, rows, 3 * d, 3 * d, 32, 32, 2, 64);
+    CUtensorMap tout;     // the packed dQKV activation, boxes of 32 rows x 64 columns
+    rc = make_tmap_2d_sw(&tout, a.dqkv, rows, 3 * d, 3 * d, 32, 64, 2, 128);
     if (rc) return rc;
-    CUtensorMap tdqb;     // the same, boxes of 32 rows x 16 columns for dQ
-    rc = make_tmap_2d_sw(&tdqb, a.dqkv, rows, 3 * d, 3 * d, 32, 16, 2, 32);
+    CUtensorMap tplace;   // dq_acc as rows of 64 columns, boxes of 32 rows x 32 columns
+    rc = make_tmap_2d_sw(&tplace, a.dq_acc, rows * a.H, 64, 64, 32, 32, 4, 128);
     if (rc) return rc;
-    CUtensorMap tplace;   // dq_acc as rows of 64 columns, boxes of 32 rows x 16 columns
-    rc = make_tmap_2d_sw(&tplace, a.dq_acc, rows * a.H, 64, 64, 32, 16, 4, 64);
-    if (rc) return rc;
-    launch_chained(kern, dim3(ctas), dim3(FB_THREADS), SMEM, stream, tq, td, tplace, tdkv, tdqb, a);
+    launch_chained(kern, dim3(ctas), dim3(FBP_THREADS), SMEM, stream, tq, td, tplace, tout, a);
     ++*launched;
     return (int)cudaGetLastError();                  // dQ, its bias sums and the clearing are done
   }

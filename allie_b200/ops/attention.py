@@ -45,9 +45,8 @@ def attention_bwd(qkv, out, lse, dout, dqkv, delta, B: int, T: int, H: int, hd: 
 
 
 def set_backward_schedule(mode: int) -> None:
-    """Schedule of the single-kernel head_dim-64 backward: 0 = chosen from the problem shape (from 32
-    (batch, head) slices on by a count of tile pairs), 1 = one key tile per CTA, 2 = persistent walk over
-    (batch, head) slices, where ``dq_acc`` has room for a slice per CTA."""
+    """Schedule of the single-kernel head_dim-64 backward: 0 = chosen from the problem shape (by what a count of
+    tile pairs says the two take), 1 = one key tile per CTA, 2 = persistent walk over (batch, head) slices."""
     rc = _lib.cuda().ab_attn_bwd_schedule(c_int(mode))
     if rc != 0:
         raise ValueError(f"bad attention backward schedule {mode}")
