@@ -212,6 +212,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
     const float dscale = dropout_scale(a.thr16);
     const long long bh = static_cast<long long>(b) * a.H + h;
     uint8_t* my_dq = sDQ + warp * 2048;
+    const uint64_t seed = uniform64(a.thr16 ? salted(a.seed, a.salt) : 0);
     bool ok = true;
 
     // drains dQ tile `it` (rows of query tile own+it, this warp's 16 columns) into the global
@@ -256,10 +257,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
         if (a.drop_mask) {
           keep32 = q_ok && own * 128 + cb * 32 < a.T ? a.drop_mask[row_elem0 >> 5] : 0u;
         } else {
-          keep32 = 0;
-#pragma unroll
-          for (int g = 0; g < 4; ++g)
-            keep32 |= dropout_keep8(salted(a.seed, a.salt), a.stream_id, (row_elem0 >> 3) + g, a.thr16) << (8 * g);
+          keep32 = dropout_keep32(seed, a.stream_id, row_elem0 >> 3, a.thr16);
         }
       }
       if (!mbar_wait(sdp_full, it & 1, abort_flag)) { ok = false; break; }
@@ -349,8 +347,8 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
 // Four warps of their own, one per TMEM lane quarter, take the results out: the dQ tile of every pair, and dV / dK
 // where a key tile ends.  Done by the math warps between pairs this was 1100 of a pair's 5000 clocks, and these are
 // what a pair waits for (the tensor core is done early, nobody waits for it).  us with
-// dropout 0.1, before and now: 64 x 512 x 16 heads 258 and 191, 32 x 512 x 20 188 and 141, 37 x 328 x 12 90 and 71,
-// 16 x 1000 x 16 267 and 218.
+// dropout 0.1, before and now: 64 x 512 x 16 heads 258 and 191, 32 x 512 x 20 188 and 141, 37 x 328 x 12 90 and 68,
+// 16 x 1000 x 16 267 and 197 (these two draw the keep bits again).
 
 constexpr int FBP_DRAIN_WARPS = 4;
 constexpr int FBP_THREADS = FB_THREADS + FBP_DRAIN_WARPS * 32;
@@ -727,6 +725,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float sl2 = a.scale * LOG2E;
     const float dscale = dropout_scale(a.thr16);
+    const uint64_t seed = uniform64(a.thr16 ? salted(a.seed, a.salt) : 0);
     bool ok = true;
 
     // per-row inputs of a pair: log-sum-exp, delta and the 32 dropout keep bits of this thread's
@@ -757,10 +756,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
           if (q_ok && (!RAGGED || w.own * 128 + cb * 32 < a.T)) keep32 = a.drop_mask[keep_off];
         } else {
           const uint64_t row_elem0 = static_cast<uint64_t>(row_off) * a.T + w.own * 128 + cb * 32;
-          keep32 = 0;
-#pragma unroll
-          for (int g4 = 0; g4 < 4; ++g4)
-            keep32 |= dropout_keep8(salted(a.seed, a.salt), a.stream_id, (row_elem0 >> 3) + g4, a.thr16) << (8 * g4);
+          keep32 = dropout_keep32(seed, a.stream_id, row_elem0 >> 3, a.thr16);
         }
       }
     };

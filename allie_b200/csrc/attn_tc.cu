@@ -757,6 +757,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     const int cb = warp >> 2;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float sl2 = a.scale * LOG2E;
+    const uint64_t seed = uniform64(a.thr16 ? salted(a.seed, a.salt) : 0);
     const float dscale = dropout_scale(a.thr16);
     const long long bh = static_cast<long long>(b) * a.H + h;
     bool ok = true;
@@ -793,7 +794,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             // keys past the end of the sequence have no bits: their words are the next row's, or past the mask
             const uint32_t keep = a.drop_mask
                 ? (q_ok && kj * 128 + col0 < a.T ? (a.drop_mask[e0 >> 5] >> (e0 & 31)) & 0xffu : 0u)
-                : dropout_keep8(salted(a.seed, a.salt), a.stream_id, e0 >> 3, a.thr16);
+                : dropout_keep8(seed, a.stream_id, e0 >> 3, a.thr16);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const bool kp = (keep >> i) & 1u;
