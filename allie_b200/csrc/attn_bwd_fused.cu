@@ -347,7 +347,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
 // Four warps of their own, one per TMEM lane quarter, take the results out: the dQ tile of every pair, and dV / dK
 // where a key tile ends.  Done by the math warps between pairs this was 1100 of a pair's 5000 clocks, and these are
 // what a pair waits for (the tensor core is done early, nobody waits for it).  us with
-// dropout 0.1, before and now: 64 x 512 x 16 heads 258 and 191, 32 x 512 x 20 188 and 141, 37 x 328 x 12 90 and 68,
+// dropout 0.1, before and now: 64 x 512 x 16 heads 258 and 187, 32 x 512 x 20 188 and 137, 37 x 328 x 12 90 and 68,
 // 16 x 1000 x 16 267 and 197 (these two draw the keep bits again).
 
 constexpr int FBP_DRAIN_WARPS = 4;
@@ -567,11 +567,11 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     // the trip to L2 were 6000 of 7500 clocks.
     auto fetch_sum = [&](int own) {
       if (lane == 0) {
-        // They are in memory: the last was for the second pair of key tile own - 1, behind which came nt - own - 1
-        // pairs and the stores of that tile's dV / dK (a whole tile, so a group of its own).
+        // They are in memory: the last was for the second pair of key tile own - 1.  Behind it came nt - own - 1 pairs
+        // and, before the last of these, that tile's dV / dK, a bulk group each.
         if (nt - own >= 3) tma_store_wait<3>();
         else if (nt - own == 2) tma_store_wait<2>();
-        else tma_store_wait<1>();
+        else tma_store_wait<0>();
         tma_store_wait_read<0>();                // and the staging tiles are free
         asm volatile("fence.proxy.async;" ::: "memory");
       }
@@ -669,7 +669,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
         }
         if (m == 1) tc_fence_before();
         else if (lane == 0) tma_store_wait_read<0>();                  // the staging tiles are free
-        __syncwarp();
+        __syncwarp();                                                  // (and their column sums taken)
         if (m == 1 && lane == 0) mbar_arrive(acc_empty);
         const int col = (m ? d_model : 2 * d_model) + h * HD;
 #pragma unroll
@@ -698,8 +698,11 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     int b = 0, h = 0;
     for (FbWalk p = start; p.valid() && ok; p.next()) {
       if (p.it == 0 && p.own == 0) { b = p.bh / a.H; h = p.bh - b * a.H; }
-      ok = drain_dq(p.g, b, h, p.own, p.it);
+      // dV / dK first: the next key tile's products wait for their place, dQ has two.  (Slices of one tile are bound
+      // by these warps, which would only wait for dV / dK.)
+      if (nt == 1) ok = drain_dq(p.g, b, h, p.own, p.it);
       if (ok && p.last()) ok = finish_tile(p.w, b, h, p.own);
+      if (ok && nt > 1) ok = drain_dq(p.g, b, h, p.own, p.it);
       __syncwarp();                                // the staging tiles have been read by all lanes
     }
     if (ok && start.valid() && nt > 1) {
