@@ -262,7 +262,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       if (!a.take_over) break;
       // before the block leaves, too: the answer is written to its shared memory
       ok = __all_sync(0xffffffffu, mbar_wait_landed(grid_bar, asked & 1)) && ok;
-      if (!grid_taken_block(grid_next, block)) break;       // none left, and none may be asked for after that
+      if (!ok || !grid_taken_block(grid_next, block)) break;      // none left, and none may be asked for after that
       if (a.row0) rows = make_int2(__ldg(a.row0 + block.z), __ldg(a.row0 + block.z + 1));
       fence_proxy_async_smem();
       __syncwarp();

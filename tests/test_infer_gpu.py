@@ -150,3 +150,8 @@ def test_padding_token_inside_a_game():
     for i, j in enumerate(last.tolist()):
         assert torch.equal(got.logits[i], out["logits"][i, j].float().cpu())
         assert float(got.value[i]) == float(out["value_logits"][i, j])
+
+
+def test_many_short_games_in_dependent_launches():
+    """240 rows (programmatic launches) of 120 games: more attention items than CTAs fit the GPU."""
+    test_packed_last_positions_and_cache(4, 256, [2, 1, 3] * 40)
