@@ -904,7 +904,10 @@ static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int
   if (err != cudaSuccess) return (int)err;
   // Blocks that all fit at once start by themselves: taken over while the grid starts, an item would wait behind
   // another (8 x 256 x 4 heads with dropout, 64 items: 12.3 and 14.3 us).
-  a.take_over = static_cast<long long>(grid.x) * grid.y * grid.z > 2ll * sms;
+  // Never in programmatic chains: a run whose short games (few rows, many items) made such launches did not end, and
+  // what a grid whose blocks are taken over tells its dependents is not known.
+  const bool chain = dependent || g_pdl_chain;
+  a.take_over = !chain && static_cast<long long>(grid.x) * grid.y * grid.z > 2ll * sms;
   if (dependent) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
