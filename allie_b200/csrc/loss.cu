@@ -105,9 +105,11 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ la
   }
 }
 
-// One warp per row.  acc[1] += sum (v-y)^2 over valid value labels, acc[2] likewise for time.  A row's loads go out
-// 1024 columns at a time (128 at a time were as many trips to memory: 6.2 us for 4 rows of 1024 behind a cold cache,
-// 2.7 so).  `ahead`: a programmatic dependent that reads the heads' weights before it waits.
+// One warp per row.  acc[1] += sum (v-y)^2 over valid value labels, acc[2] likewise for time.  AHEAD: a programmatic
+// dependent of few rows that reads the heads' weights before it waits; its loads go out 1024 columns at a time (128 at a
+// time were as many trips to memory: 6.2 us for 4 rows of 1024 behind a cold cache, 2.7 so).  Otherwise 128 at a time:
+// with many rows the warps in flight count, which the wide loads' registers cost (7749 rows of 384: 7.2 and 10.8 us).
+template <bool AHEAD>
 __global__ void __launch_bounds__(256)
 heads_fwd_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ wv,
                  const float* __restrict__ bv, const float* __restrict__ wt,
@@ -115,8 +117,8 @@ heads_fwd_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ 
                  const float* __restrict__ time_labels, const int* __restrict__ counts,
                  float value_coef, float time_coef, float* __restrict__ value_out,
                  float* __restrict__ time_out, float* __restrict__ dv, float* __restrict__ dt,
-                 float* __restrict__ acc, int M, int d, int ahead) {
-  constexpr int U = 8;
+                 float* __restrict__ acc, int M, int d) {
+  constexpr int U = AHEAD ? 8 : 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n4 = d >> 2;
   const int row = blockIdx.x * 8 + warp;
   float4 a[U], b[U];
@@ -131,14 +133,14 @@ heads_fwd_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ 
       }
     }
   };
-  if (ahead) weights(lane);
+  if (AHEAD) weights(lane);
   griddep_enter();
   float lv = 0.f, lt = 0.f;
   if (row < M) {
     const uint2* hr = reinterpret_cast<const uint2*>(h + (long long)row * d);
     float sv = 0.f, st = 0.f;
     for (int c0 = lane; c0 < n4; c0 += 32 * U) {
-      if (!ahead || c0 != lane) weights(c0);
+      if (!AHEAD || c0 != lane) weights(c0);
       uint2 p[U];
 #pragma unroll
       for (int i = 0; i < U; ++i) p[i] = c0 + 32 * i < n4 ? hr[c0 + 32 * i] : make_uint2(0u, 0u);
@@ -264,9 +266,9 @@ int ab_heads_fwd(const void* h, const float* wv, const float* bv, const float* w
                  float value_coef, float time_coef, float* value_out, float* time_out, float* dv,
                  float* dt, float* acc, int M, int d, cudaStream_t stream) {
   if (d % 4) return -1;
-  ab::launch_chained(ab::heads_fwd_kernel, dim3((M + 7) / 8), dim3(256), 0, stream, 
+  ab::launch_chained(ab::heads_fwd_kernel<false>, dim3((M + 7) / 8), dim3(256), 0, stream, 
       (const __nv_bfloat16*)h, wv, bv, wt, bt, value_labels, time_labels, counts, value_coef,
-      time_coef, value_out, time_out, dv, dt, acc, M, d, 0);
+      time_coef, value_out, time_out, dv, dt, acc, M, d);
   return (int)cudaGetLastError();
 }
 
@@ -274,9 +276,9 @@ int ab_heads_fwd(const void* h, const float* wv, const float* bv, const float* w
 int ab_heads_fwd_ahead(const void* h, const float* wv, const float* bv, const float* wt, const float* bt,
                        float* value_out, float* time_out, int M, int d, cudaStream_t stream) {
   if (d % 4) return -1;
-  return (int)ab::launch_dependent(ab::heads_fwd_kernel, dim3((M + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)h,
+  return (int)ab::launch_dependent(ab::heads_fwd_kernel<true>, dim3((M + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)h,
                                    wv, bv, wt, bt, (const float*)nullptr, (const float*)nullptr, (const int*)nullptr, 0.f,
-                                   0.f, value_out, time_out, (float*)nullptr, (float*)nullptr, (float*)nullptr, M, d, 1);
+                                   0.f, value_out, time_out, (float*)nullptr, (float*)nullptr, (float*)nullptr, M, d);
 }
 
 int ab_heads_bwd_w(const void* h, const float* dv, const float* dt, float* dwv, float* dbv,
