@@ -356,10 +356,10 @@ constexpr int FBP_THREADS = FB_THREADS + FBP_DRAIN_WARPS * 32;
 struct FbWalk {
   int bh, own, it, nt, bh_end, step;
   int w, g;      // key tiles and pairs done so far by this CTA
-  __device__ __forceinline__ bool valid() const { return bh < bh_end; }
-  __device__ __forceinline__ bool first() const { return it == 0; }
-  __device__ __forceinline__ bool last() const { return it == nt - own - 1; }
-  __device__ __forceinline__ void next() {
+  __host__ __device__ __forceinline__ bool valid() const { return bh < bh_end; }
+  __host__ __device__ __forceinline__ bool first() const { return it == 0; }
+  __host__ __device__ __forceinline__ bool last() const { return it == nt - own - 1; }
+  __host__ __device__ __forceinline__ void next() {
     ++g;
     if (++it == nt - own) {
       it = 0; ++w;
@@ -367,6 +367,25 @@ struct FbWalk {
     }
   }
 };
+
+// A drain warp's bulk operations on a dQ place are ordered by waits only: groups of one thread may be performed in any
+// order, whatever they were issued in.  How many of its latest groups may be under way still
+// - when the sum of query tile `own` is read (the diagonal pair of key tile own > 0).  The last addition to it was for the
+//   second pair of key tile own - 1; behind that came nt - own - 1 pairs and, before the last of these, that tile's
+//   dV / dK, a group each.
+__host__ __device__ constexpr int fb_open_at_sum(int nt, int own) { return nt - own >= 3 ? 3 : nt - own == 2 ? 2 : 0; }
+// - when key tile own > 0 adds to a query tile (it > 0).  At its first addition everything up to the key tile before is
+//   complete: what that one stored (own == 1) or added there comes first, so the sums are always taken in the same order.
+//   All that came since is this key tile's diagonal pair (a pair's time ago) and, if this pair is its last, dV / dK.
+constexpr int FB_NO_WAIT = -1;
+__host__ __device__ constexpr int fb_open_at_add(int it) { return it == 1 ? 1 : FB_NO_WAIT; }
+
+__device__ __forceinline__ void fb_wait_groups(int open) {
+  if (open >= 3) tma_store_wait<3>();
+  else if (open == 2) tma_store_wait<2>();
+  else if (open == 1) tma_store_wait<1>();
+  else if (open == 0) tma_store_wait<0>();
+}
 
 // RAGGED: T is no multiple of 128; the last 32-row blocks of a sequence are stored row by row
 template <bool RAGGED>
@@ -567,12 +586,8 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     // the trip to L2 were 6000 of 7500 clocks.
     auto fetch_sum = [&](int own) {
       if (lane == 0) {
-        // They are in memory: the last was for the second pair of key tile own - 1.  Behind it came nt - own - 1 pairs
-        // and, before the last of these, that tile's dV / dK, a bulk group each.
-        if (nt - own >= 3) tma_store_wait<3>();
-        else if (nt - own == 2) tma_store_wait<2>();
-        else tma_store_wait<0>();
-        tma_store_wait_read<0>();                // and the staging tiles are free
+        fb_wait_groups(fb_open_at_sum(nt, own)); // the additions are complete,
+        tma_store_wait_read<0>();                // and the staging tiles free
         asm volatile("fence.proxy.async;" ::: "memory");
       }
       __syncwarp();
@@ -639,7 +654,8 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
         } else if (own == 0) {
           tma_store_2d(&tmDQ, stg, 0, s_row0 + qrow);
           tma_store_2d(&tmDQ, stg + 4096, 32, s_row0 + qrow);
-        } else {     // (own == 1 adds to what own == 0 stored: those stores were waited for at its diagonal pair)
+        } else {
+          fb_wait_groups(fb_open_at_add(it));
           tma_reduce_add_2d(&tmDQ, stg, 0, s_row0 + qrow);
           tma_reduce_add_2d(&tmDQ, stg + 4096, 32, s_row0 + qrow);
         }
@@ -934,6 +950,34 @@ extern "C" int ab_attn_bwd_schedule(int mode) {
   if (mode < 0 || mode > 2) return -1;
   ab::g_attn_bwd_schedule = mode;
   return 0;
+}
+
+// For tests: what a drain warp of the walk does to the dQ places over `slices` slices of nt tiles, in its order; four
+// numbers each: what (0 store, 1 add, 2 read, 3 dQ out, 4 dV / dK out; all but reads are a bulk group), slice, query tile (of
+// 3 and 4: 0), and how many of the groups before may be under way still (-1: any number).  Returns how many (no
+// more than `room` are written).
+extern "C" int ab_attn_bwd_walk_order(int nt, int slices, int* out, int room) {
+  using namespace ab;
+  int n = 0;
+  auto put = [&](int what, int slice, int tile, int open) {
+    if (n < room) { out[4 * n] = what; out[4 * n + 1] = slice; out[4 * n + 2] = tile; out[4 * n + 3] = open; }
+    ++n;
+  };
+  auto drain_dq = [&](const FbWalk& p) {
+    if (p.it == 0 && p.own > 0) put(2, p.bh, p.own, fb_open_at_sum(nt, p.own));
+    if (p.it == 0) put(3, p.bh, 0, FB_NO_WAIT);
+    else if (p.own == 0) put(0, p.bh, p.it, FB_NO_WAIT);
+    else put(1, p.bh, p.own + p.it, fb_open_at_add(p.it));
+  };
+  FbWalk p = {};
+  p.nt = nt; p.bh_end = slices; p.step = 1;
+  for (; p.valid(); p.next()) {
+    if (nt == 1) drain_dq(p);
+    if (p.last()) put(4, p.bh, 0, FB_NO_WAIT);
+    if (nt > 1) drain_dq(p);
+  }
+  for (int i = 1; i < nt; ++i) put(0, slices, i, FB_NO_WAIT);      // handed back all zero
+  return n;
 }
 
 // Stand-alone entry to the dQ conversion (bf16 copy into the packed dQKV activation, then clear).

@@ -1,0 +1,39 @@
+"""Order of the bulk operations on the dQ sums of the attention backward's walk (host replay, no GPU needed)."""
+import ctypes
+
+import pytest
+
+from allie_b200.ops import _lib
+
+pytestmark = pytest.mark.skipif(not _lib.have_cuda_lib(), reason="kernel library not built")
+
+STORE, ADD, READ, DQ_OUT, DKV_OUT = range(5)
+
+
+@pytest.mark.parametrize("nt", list(range(1, 13)) + [32])
+def test_every_sum_waits_for_what_it_builds_on(nt):
+    """Bulk groups of a thread complete in any order unless it waits: with as many of the latest under way as the
+    waits allow, whatever touches the sum of a query tile finds everything before it on that tile complete."""
+    room = 8192
+    buf, slices = (ctypes.c_int * (4 * room))(), 3
+    n = _lib.cuda().ab_attn_bwd_walk_order(nt, slices, buf, room)
+    assert 0 < n <= room
+    open_groups, content, adds = [], {}, 0          # tiles of the groups under way; contributions per tile
+    for i in range(n):
+        what, slice_, tile, may_be_open = buf[4 * i:4 * i + 4]
+        if may_be_open >= 0:
+            open_groups = open_groups[len(open_groups) - may_be_open:] if may_be_open else []
+        if what in (STORE, ADD, READ):
+            assert tile not in open_groups, (i, what, slice_, tile)
+        if what == STORE:
+            content[tile] = [slice_]
+        elif what == ADD:
+            assert content[tile] and set(content[tile]) == {slice_}
+            content[tile].append(slice_)
+            adds += 1
+        elif what == READ:                          # all key tiles before the query tile have contributed
+            assert content.pop(tile) == [slice_] * tile
+        if what != READ:
+            open_groups.append(tile if what in (STORE, ADD) else None)
+    assert adds == slices * (nt - 1) * (nt - 2) // 2
+    assert content == {tile: [slices] for tile in range(1, nt)}
