@@ -218,7 +218,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
     // drains dQ tile `it` (rows of query tile own+it, this warp's 16 columns) into the global
     // fp32 accumulator with one TMA reduce-add
     auto drain_dq = [&](int it) {
-      if (!mbar_wait(&dq_full[it & 1], (it >> 1) & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(&dq_full[it & 1], (it >> 1) & 1, abort_flag)) return false;
       tc_fence_after();
       uint32_t v[16];
       tmem_ld16(tDQ + (it & 1) * 64 + lane_addr + cb * 16, v);
@@ -260,7 +260,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
           keep32 = dropout_keep32(seed, a.stream_id, row_elem0 >> 3, a.thr16);
         }
       }
-      if (!mbar_wait(sdp_full, it & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(sdp_full, it & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
@@ -286,7 +286,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
           else      fb_math16<false, false>(sv, dv, pw, dw, r, col0, sl2, lse_l2, dlt * a.scale, a.scale, dscale, k16);
         }
         // the shared P / dS tiles feed the previous pair's products until pds_empty completes
-        if (hf == 0 && it > 0 && !mbar_wait(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
+        if (hf == 0 && it > 0 && !mbar_wait_warp(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
         const uint32_t poff = (col0 >> 6) * 16384;
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
@@ -305,7 +305,7 @@ attn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tmQKV,
       if (it > 0) ok = drain_dq(it - 1);
     }
     if (ok) ok = drain_dq(n_iter - 1);
-    if (ok && !mbar_wait(acc_full, 0, abort_flag)) ok = false;
+    if (ok && !mbar_wait_warp(acc_full, 0, abort_flag)) ok = false;
     if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
     if (ok) {
       tc_fence_after();
@@ -604,7 +604,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     auto drain_dq = [&](int g, int b, int h, int own, int it) {
       const bool last = it == 0, summed = last && own > 0;
       if (summed) fetch_sum(own);
-      const bool there = mbar_wait(&dq_full[g & 1], (g >> 1) & 1, abort_flag);
+      const bool there = mbar_wait_warp(&dq_full[g & 1], (g >> 1) & 1, abort_flag);
       asm volatile("cp.async.wait_all;" ::: "memory");
       if (!there) return false;
       tc_fence_after();
@@ -666,7 +666,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
     };
     // reads the finished dV / dK of key tile w out of TMEM, frees them, and stores them
     auto finish_tile = [&](int w, int b, int h, int own) {
-      if (!mbar_wait(acc_full, w & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(acc_full, w & 1, abort_flag)) return false;
       tc_fence_after();
       const bool rows_whole = whole_rows(own * 128 + quad * 32);       // warp-uniform
       const int t_idx = own * 128 + r;
@@ -792,7 +792,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
         q.next();
         if (q.valid()) fetch(q, n_lse, n_dlt, n_keep);
       }
-      if (!mbar_wait(sdp_full, p.g & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(sdp_full, p.g & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const float lse_l2 = lse_raw * LOG2E;          // +inf for rows outside the sequence
 #pragma unroll
@@ -821,7 +821,7 @@ attn_bwd_fused64_persistent_kernel(const __grid_constant__ CUtensorMap tmQKV,
         if (hf == 0) {
           // the shared P / dS tiles feed the previous pair's dV / dK / dQ products until
           // pds_empty completes; the first half of this pair's math has run under them
-          if (p.g > 0 && !mbar_wait(pds_empty, (p.g - 1) & 1, abort_flag)) { ok = false; break; }
+          if (p.g > 0 && !mbar_wait_warp(pds_empty, (p.g - 1) & 1, abort_flag)) { ok = false; break; }
         }
         const uint32_t poff = (col0 >> 6) * 16384;
 #pragma unroll

@@ -337,7 +337,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&xchg[quad]);
       met ^= 1;
-      return mbar_wait(&xchg[quad], met ^ 1, abort_flag);
+      return mbar_wait_warp(&xchg[quad], met ^ 1, abort_flag);
     };
     const float sl2 = a.scale * LOG2E;
     const uint64_t sl2_2 = f2_bcast(sl2);
@@ -371,7 +371,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             }
           }
         }
-        if (!(ok = mbar_wait(s_full, tile, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(s_full, tile, abort_flag))) break;
         tc_fence_after();
         uint32_t v[64];
 #pragma unroll
@@ -402,7 +402,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         if (j == 0) {
           m_ref = mx;
         } else if (__any_sync(0xffffffffu, mx > m_ref)) {
-          if (!(ok = mbar_wait(pv_full, tile ^ 1, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(pv_full, tile ^ 1, abort_flag))) break;
           tc_fence_after();
           const float m_new = fmaxf(m_ref, mx);
           grow = ex2_fast((m_ref - m_new) * sl2);
@@ -446,7 +446,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             for (int i = 0; i < 16; ++i) w[i] &= m[i];
           }
           // P of the tile before is read by its product until that completes
-          if (c == 0 && j > 0 && !(ok = mbar_wait(pv_full, tile ^ 1, abort_flag))) break;
+          if (c == 0 && j > 0 && !(ok = mbar_wait_warp(pv_full, tile ^ 1, abort_flag))) break;
           if (c == 0) tc_fence_after();
           tmem_st16(tP + lane_addr + hf * 32 + c * 16, w);
         }
@@ -467,7 +467,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       if (!ok) break;
       const int T = it->T, h = it->h, b = it->b, row = it->first + qt * AT_BM + quad * 32;    // this warp's first row
       item_done(n);
-      if (!(ok = mbar_wait(pv_full, tile ^ 1, abort_flag))) break;
+      if (!(ok = mbar_wait_warp(pv_full, tile ^ 1, abort_flag))) break;
       tc_fence_after();
       float* slot = s_row + met * 256;
       slot[hf * 128 + r] = l_run;
@@ -770,8 +770,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       const float dlt = q_ok ? a.delta[bh * a.T + q_idx] : 0.f;
       const bool diag = (qi == kj);
       const uint64_t row_elem0 = (static_cast<uint64_t>(bh) * a.T + q_idx) * a.T + kj * 128 + cb * 32;
-      if (!mbar_wait(sdp_full, it & 1, abort_flag)) { ok = false; break; }
-      if (it > 0 && !mbar_wait(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(sdp_full, it & 1, abort_flag)) { ok = false; break; }
+      if (it > 0 && !mbar_wait_warp(pds_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {      // two 16-column pieces keep the register count low
@@ -829,7 +829,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       __syncwarp();
       if (lane == 0) { mbar_arrive(sdp_empty); mbar_arrive(pds_full); }
     }
-    if (ok && !mbar_wait(acc_full, 0, abort_flag)) ok = false;
+    if (ok && !mbar_wait_warp(acc_full, 0, abort_flag)) ok = false;
     if (!ok) { *abort_flag = ST_TIMEOUT_TMEM_FULL; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
     if (ok) {
       tc_fence_after();

@@ -173,7 +173,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
     const int stage = hi * DA_RING + ch % DA_RING;
     const uint32_t parity = (ch / DA_RING) & 1;
     const int cnt = min(n, (ch + 1) * DA_CHUNK) - ch * DA_CHUNK;
-    if (!mbar_wait(&full[stage], parity, abort_flag)) {
+    if (!mbar_wait_warp(&full[stage], parity, abort_flag)) {
       *abort_flag = 1;
       atomicCAS(status, 0, ST_TIMEOUT_MISC);
       return;

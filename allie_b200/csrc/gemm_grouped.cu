@@ -340,7 +340,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const int mrow_w = mrow0 + rank * BM + quad * 32;        // first row of this warp, inside the group
       const int mrow = mrow_w + lane;
       const int nbase = ncol0 + part * COLS_PER_WARP;
-      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
+      if (!mbar_wait_warp(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         break;

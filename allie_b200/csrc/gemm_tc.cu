@@ -287,7 +287,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       const int ab = it & 1;
       const int m0w = (tile / n_tiles) * TM + quad * ROWS, m = m0w + lane;   // first row of this warp's block
       const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
-      if (!mbar_wait(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
+      if (!mbar_wait_warp(&tfull_bar[ab], (acc_phase >> ab) & 1, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         break;
@@ -552,7 +552,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         for (int c = 0; c < COLS_PER_WARP / 2; ++c) sum[c] = 0;
         for (; kb0 < kb1; kb0 += g.accum_steps) {
           const int ab = n_acc & 1;
-          if (!mbar_wait(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
+          if (!mbar_wait_warp(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
             *abort_flag = ST_TIMEOUT_TMEM_FULL;
             atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
             ok = false;
@@ -599,7 +599,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const int m = m0w + lane;
         const int nbase = (tile % n_tiles) * BN + part * COLS_PER_WARP;
         const bool staged = stage_aux && m0w < g.M && nbase < g.N;
-        if (!mbar_wait(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
+        if (!mbar_wait_warp(&tfull_bar[ab], (n_acc >> 1) & 1, abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_FULL;
           atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
           if (staged) mbar_wait_landed(&aux_bar[e], aux_phase);     // before the warp leaves
@@ -610,7 +610,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const uint32_t taddr =
             tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ab * BN + part * COLS_PER_WARP;
         auto wait_aux = [&]() {
-          if (!mbar_wait(&aux_bar[e], aux_phase, abort_flag)) {
+          if (!mbar_wait_warp(&aux_bar[e], aux_phase, abort_flag)) {
             *abort_flag = ST_TIMEOUT_FULL;
             atomicCAS(g.status, 0, ST_TIMEOUT_FULL);
             mbar_wait_landed(&aux_bar[e], aux_phase);

@@ -194,7 +194,7 @@ lmhead_ce_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           s_lab[part * BM + rloc] = rlab;
           __syncwarp();
           if (lane == 0) mbar_arrive(stat_bar);
-          if (!mbar_wait(stat_bar, unit_it & 1, abort_flag)) {     // bounded, and it sees another warp's abort
+          if (!mbar_wait_warp(stat_bar, unit_it & 1, abort_flag)) {     // bounded, and it sees another warp's abort
             *abort_flag = ST_TIMEOUT_MISC;
             atomicCAS(g.status, 0, ST_TIMEOUT_MISC);
             ok = false;
@@ -213,7 +213,7 @@ lmhead_ce_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           lse = M4 + logf(L4);
           if (part == 0 && label >= 0) loss_local += lse - lab;
         }
-        if (!mbar_wait(&tfull_bar[ab], acc_phase[ab], abort_flag)) {
+        if (!mbar_wait_warp(&tfull_bar[ab], acc_phase[ab], abort_flag)) {
           *abort_flag = ST_TIMEOUT_TMEM_FULL;
           atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
           ok = false;
@@ -427,7 +427,7 @@ lmhead_ce_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     float rm = -INFINITY, rl = 0.f, rlab = -INFINITY;
     bool ok = true;
     for (int t = 0; t < tiles && ok; ++t) {
-      if (!mbar_wait(&tfull_bar[t], 0, abort_flag)) {
+      if (!mbar_wait_warp(&tfull_bar[t], 0, abort_flag)) {
         *abort_flag = ST_TIMEOUT_TMEM_FULL;
         atomicCAS(g.status, 0, ST_TIMEOUT_TMEM_FULL);
         ok = false;
@@ -463,7 +463,7 @@ lmhead_ce_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     s_stat[(8 + part) * BM + rloc] = rlab;
     __syncwarp();
     if (lane == 0) mbar_arrive(stat_bar);
-    if (ok && !mbar_wait(stat_bar, 0, abort_flag)) {
+    if (ok && !mbar_wait_warp(stat_bar, 0, abort_flag)) {
       *abort_flag = ST_TIMEOUT_MISC;
       atomicCAS(g.status, 0, ST_TIMEOUT_MISC);
       ok = false;
@@ -497,7 +497,7 @@ lmhead_ce_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         for (int c = 0; c < C; ++c) mbar_arrive_cluster(mapa_shared(smem_u32(all_bar), c));
       }
     }
-    if (ok && !mbar_wait(all_bar, 0, abort_flag)) {
+    if (ok && !mbar_wait_warp(all_bar, 0, abort_flag)) {
       *abort_flag = ST_TIMEOUT_MISC;
       atomicCAS(g.status, 0, ST_TIMEOUT_MISC);
       ok = false;
