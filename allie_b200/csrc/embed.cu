@@ -65,10 +65,17 @@ __device__ __forceinline__ float elo_frac(int id, int vocab) {
   return static_cast<float>(e - 500) / 2500.f;
 }
 
-// A thread per four columns (two groups of them beyond 1024 columns): what counts for few rows is one trip to memory
-// for the ids and one for the embeddings.  (A warp per row, which made the second trip every 128 columns: 6.7 us for
-// 4 rows of 1024 from a cold cache, 3.0 so.)
+// FEW rows (up to EMBED_FEW): a thread per four columns (two groups of them beyond 1024 columns), because what counts there
+// is one trip to memory for the ids and one for the embeddings.  More rows: a warp per row, whose ids, addresses and
+// tests serve all its columns; with those for every four columns, and threads left over where 256 is no multiple of
+// d / 4, instruction issue is the bound.  us from a cold cache, warp per row and thread per four columns, 384 / 1024 /
+// 1280 columns: 4 rows 8.2 and 8.2 / 12.3 and 8.2 / 12.3 and 8.2; 1184 rows 10.3 and 8.2 / 13.3 and 10.3 / 14.4 and
+// 10.3; 2048 10.3 and 9.2 / 14.3 and 12.3 / 15.4 and 12.3; 4096 10.3 and 10.2 / 14.4 and 15.3 / 16.4 and 16.4;
+// 7749 10.3 and 12.3 / 16.4 and 20.5 / 18.5 and 22.5; 32768 20.5 and 28.7 / 38.0 and 59.4 / 45.2 and 67.6 (with
+// dropout 24.6 and 36.9 / 47.2 and 77.8 / 57.4 and 88.1).
+constexpr int EMBED_FEW = 3072;
 constexpr int EMBED_THREADS = 256;
+template <bool FEW>
 __global__ void __launch_bounds__(EMBED_THREADS)
 embed_fwd_kernel(const int* __restrict__ ids, const int* __restrict__ pos,
                  const float* __restrict__ wte, const float* __restrict__ wpe,
@@ -77,8 +84,9 @@ embed_fwd_kernel(const int* __restrict__ ids, const int* __restrict__ pos,
                  const unsigned long long* __restrict__ salt) {
   griddep_enter();
   seed = salted(seed, salt);
-  const int n4 = d >> 2, rows = n4 < EMBED_THREADS ? EMBED_THREADS / n4 : 1;        // of a block
-  const int r = n4 < EMBED_THREADS ? threadIdx.x / n4 : 0;
+  const int n4 = d >> 2, across = FEW ? EMBED_THREADS : 32;            // threads of a row, where it has that many columns
+  const int rows = !FEW ? EMBED_THREADS / 32 : n4 < EMBED_THREADS ? EMBED_THREADS / n4 : 1;      // of a block
+  const int r = !FEW ? threadIdx.x / 32 : n4 < EMBED_THREADS ? threadIdx.x / n4 : 0;
   const int row = blockIdx.x * rows + r;
   if (r >= rows || row >= M) return;
   const int id = ids[row];
@@ -92,7 +100,7 @@ embed_fwd_kernel(const int* __restrict__ ids, const int* __restrict__ pos,
   const float4* c1 = reinterpret_cast<const float4*>(ctrl + d);
   float4* xr = reinterpret_cast<float4*>(x + (long long)row * d);
   const float scale = dropout_scale(thr16);
-  for (int c4 = threadIdx.x - r * n4; c4 < n4; c4 += EMBED_THREADS) {
+  for (int c4 = threadIdx.x - r * (FEW ? n4 : 32); c4 < n4; c4 += across) {
     float4 v;
     if (is_elo) {
       const float4 a = __ldg(c0 + c4), b = __ldg(c1 + c4);
@@ -205,9 +213,11 @@ int ab_embed_fwd(const int* ids, const int* pos, const float* wte, const float* 
                  const float* ctrl, float* x, int M, int d, int vocab, unsigned long long seed,
                  unsigned int stream_id, unsigned int thr16, cudaStream_t stream) {
   if (d % 4) return -1;
-  const int rows = d / 4 < ab::EMBED_THREADS ? ab::EMBED_THREADS / (d / 4) : 1;
-  ab::launch_chained(ab::embed_fwd_kernel, dim3((M + rows - 1) / rows), dim3(ab::EMBED_THREADS), 0, stream, ids, pos, wte, wpe, ctrl, x, M, d, vocab,
-                                                        seed, stream_id, thr16, ab::seed_salt_ptr());
+  const bool few = M <= ab::EMBED_FEW && d >= 4;
+  const int rows = !few ? ab::EMBED_THREADS / 32 : d / 4 < ab::EMBED_THREADS ? ab::EMBED_THREADS / (d / 4) : 1;
+  ab::launch_chained(few ? ab::embed_fwd_kernel<true> : ab::embed_fwd_kernel<false>, dim3((M + rows - 1) / rows),
+                     dim3(ab::EMBED_THREADS), 0, stream, ids, pos, wte, wpe, ctrl, x, M, d, vocab, seed, stream_id, thr16,
+                     ab::seed_salt_ptr());
   return (int)cudaGetLastError();
 }
 

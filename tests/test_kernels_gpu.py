@@ -359,9 +359,11 @@ def test_dependent_layernorm_waits_for_its_weights(d):
     assert torch.equal(y, want)
 
 
-@pytest.mark.parametrize("M,d", [(1, 128), (5, 96), (7, 384), (3, 1024), (4, 1280), (300, 256), (9, 2048)])
+@pytest.mark.parametrize("M,d", [(1, 128), (5, 96), (7, 384), (3, 1024), (4, 1280), (300, 256), (9, 2048),
+                                 (3072, 100), (3073, 100), (3077, 384), (3079, 1280)])
 def test_embedding_rows_of_any_width(M, d):
-    """Several rows to a block, one, and a row in two rounds: control token, dropped and kept elements."""
+    """Several rows to a block, one, and a row in two rounds, beyond 3072 rows a warp each: control token, dropped and
+    kept elements."""
     from allie_b200.ops import _lib, kernels as K
 
     torch.manual_seed(11)
