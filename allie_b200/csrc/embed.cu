@@ -238,7 +238,7 @@ extern "C" int ab_dropout_mask_host(unsigned long long seed, unsigned int stream
                                     unsigned int thr16, unsigned char* out) {
   if (n & 7) return -1;
   for (long long g = 0; g < n / 8; ++g) {
-    const uint32_t keep = ab::dropout_keep8(seed, stream, static_cast<uint64_t>(g), thr16);
+    const uint32_t keep = thr16 ? ab::dropout_keep8(seed, stream, static_cast<uint64_t>(g), thr16) : 0xffu;   // 0: none dropped
     for (int j = 0; j < 8; ++j) out[g * 8 + j] = (keep >> j) & 1u;
   }
   return 0;
