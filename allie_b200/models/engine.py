@@ -37,6 +37,7 @@ from . import unwrap
 from .oracle import Conv1D, MoEMLP
 
 ALIGN = 64  # elements; keeps every parameter view 256-byte (fp32) / 128-byte (bf16) aligned
+INFER_ONE_PIECE = 10 << 20  # bytes that a pass of `infer_last` works in up to which they are one allocation
 
 
 def partition_parameter_names(model: nn.Module) -> tuple[list[str], list[str]]:
@@ -797,6 +798,8 @@ class B200Engine:
         # A request for one game waits for the host until its first kernel is on its way: one allocation for what
         # the pass works in (bytes, each part on a 256-byte boundary), one for its results, the model's part
         # of the arguments copied (13 allocations and 40 stores of attributes otherwise: 106 us before the launches, 98 so).
+        # Passes over many rows take their buffers one by one: in one piece, whose size differs from batch to batch, 200
+        # batches of 1 to 128 games (24 layers of 1024) kept 5.0 GB of the allocator's memory instead of 3.9.
         a = Infer()
         ctypes.memmove(ctypes.byref(a), ctypes.byref(self._infer_model), ctypes.sizeof(Infer))
         sizes = (4 * M * d, 2 * M * d, 6 * M * d, 2 * M * d, 2 * M * F, 4 * n * d, 2 * n * d, 2 * n * d)
@@ -804,9 +807,14 @@ class B200Engine:
         for size in sizes:
             offsets.append(total)
             total += -(-size // 256) * 256
-        scratch = torch.empty(total, dtype=torch.uint8, device=dev)
-        base = scratch.data_ptr()
-        a.x, a.ln, a.qkv, a.att, a.act, a.x_last, a.att_last, a.h = (base + o for o in offsets)
+        if total <= INFER_ONE_PIECE:
+            scratch = torch.empty(total, dtype=torch.uint8, device=dev)
+            base = scratch.data_ptr()
+            at = [base + o for o in offsets]
+        else:
+            scratch = [torch.empty(size, dtype=torch.uint8, device=dev) for size in sizes]
+            at = [t.data_ptr() for t in scratch]
+        a.x, a.ln, a.qkv, a.att, a.act, a.x_last, a.att_last, a.h = at
         logits = torch.empty(n, V, dtype=torch.bfloat16, device=dev)
         a.logits = logits.data_ptr()
         value = time = None

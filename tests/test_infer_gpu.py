@@ -155,3 +155,37 @@ def test_padding_token_inside_a_game():
 def test_many_short_games_in_dependent_launches():
     """240 rows (programmatic launches) of 120 games: more attention items than CTAs fit the GPU."""
     test_packed_last_positions_and_cache(4, 256, [2, 1, 3] * 40)
+
+
+def test_buffers_of_many_rows_are_not_one_piece(monkeypatch):
+    """One piece for a few rows only, and the same results either way."""
+    from allie_b200.data import UCITokenizer
+    from allie_b200.models import engine, initialize_model
+
+    torch.manual_seed(0)
+    tok = UCITokenizer(max_length=256, vocab_size_multiple_of=128)
+    model = initialize_model(tok, "gpt2", use_control_token=True, use_regression_head=True, n_layer=2, n_embd=256,
+                             n_head=4, n_positions=256)
+    eng = engine.B200Engine(model, "cuda")
+    rng = np.random.default_rng(2)
+    empty, asked = torch.empty, []
+
+    def counted(*shape, **kw):
+        t = empty(*shape, **kw)
+        if t.is_cuda:
+            asked.append(t.nbytes)
+        return t
+
+    def run(games):
+        asked.clear()
+        with monkeypatch.context() as m:
+            m.setattr(engine.torch, "empty", counted)
+            return eng.infer_last(games), list(asked)
+
+    few, many = ([rng.integers(0, 1968, size=n) for n in lens] for lens in ([90], [250] * 20))
+    assert len(run(few)[1]) == 3                                   # the pass, logits, value and time
+    want, sizes = run(many)
+    assert max(sizes) <= 5000 * 8 * 256                            # the widest buffer of a row: 4 * 256 bf16
+    monkeypatch.setattr(engine, "INFER_ONE_PIECE", 1 << 40)
+    got, sizes = run(many)
+    assert len(sizes) == 3 and all(torch.equal(a, b) for a, b in zip(want, got))
