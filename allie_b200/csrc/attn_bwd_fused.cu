@@ -877,6 +877,21 @@ static int attn_bwd_schedule_mode() {
   return g_attn_bwd_schedule;
 }
 
+// The walk hands whole slices to CTAs (each has a place for the sums of one in dq_acc: nt - 1 tiles of 128 rows, fewer
+// than T); few, long ones leave SMs idle, which the grid of key tiles does not.  us, from launches of 1 to 320 slices
+// of 1 to 8 tiles in a replayed graph: a slice of nt (nt + 1) / 2 pairs of tiles takes the walk 2.2 a pair and 8 in
+// all; the grid 12 with the conversion, clearing and column sums behind it, and the longer of its longest CTA (1.7 a
+// query tile) and of all its CTAs' work (4 a pair, one and a half pairs' worth per key tile to start and end).  Of the 190 sizes
+// measured none loses more than 3 % to the other form.  Grid and walk: 16 slices of 1 tile 14.8 and 7.7, of 2 17.6 and
+// 14.8, of 3 19.9 and 21.7, of 4 22.5 and 30; 32 of 4 26 and 30; 148 of 2 36 and 17, of 4 73 and 33; 200 of 1000 keys
+// 244 and 186.
+static bool fb_walks(int bh, int nt, int sms) {
+  const double slice = 0.5 * nt * (nt + 1);
+  const double walk_us = 8.0 + 2.2 * ((bh + sms - 1) / sms) * slice;
+  const double grid_us = 12.0 + std::max(1.7 * nt, 4.0 * bh * (slice + 1.5 * nt) / sms);
+  return walk_us <= grid_us;
+}
+
 int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const AttnBwdArgs& a,
                             int* launched, cudaStream_t stream) {
   CUtensorMap tdq;
@@ -886,20 +901,10 @@ int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const 
   if (rc) return rc;
   const int mode = attn_bwd_schedule_mode();
   const bool ragged = (a.T & 127) != 0;
-  const int bh = a.B * a.H, ctas = bh < 148 ? bh : 148, nt = (a.T + 127) / 128;
-  // The walk hands whole slices to CTAs (each has a place for the sums of one in dq_acc: nt - 1 tiles of 128 rows, fewer
-  // than T); few, long ones leave SMs idle, which the grid of key tiles does not.  us, from launches of 1 to 320 slices
-  // of 1 to 8 tiles: a slice of nt (nt + 1) / 2 pairs of tiles takes the walk 2.2 a pair and 5 in all; the grid
-  // 11.5 with the conversion, clearing and column sums behind it, and the longer of its longest CTA (2.1 a query
-  // tile) and of all its CTAs' work (5 a pair, two pairs' worth per key tile to start and end).  Grid and walk: 1 slice
-  // of 2 tiles 15.7 and 13.9, of 3 18.4 and 20.5; 32 of 4 36 and 30, of 6 51 and 52; 64 of 6 80 and 52; 148 of 4 104
-  // and 39; 200 of 1000 keys 367 and 213.  Up to 16 slices the grid whatever the count says (the test of a replayed
-  // step counts that many launches); of one or two tiles the walk would take 0.5 to 0.9 of its time there.
-  const double slice = 0.5 * nt * (nt + 1);
-  const double walk_us = 5.0 + 2.2 * ((bh + 147) / 148) * slice;
-  const double grid_us = 11.5 + std::max(2.1 * nt, 5.0 * bh * (slice + 2 * nt) / 148);
-  const bool walk = bh > 16 && walk_us <= grid_us;
-  if (mode == 1 || (mode == 0 && !walk)) {
+  int sms = 0;
+  if (const cudaError_t e = device_sms(&sms)) return (int)e;
+  const int bh = a.B * a.H, ctas = bh < sms ? bh : sms, nt = (a.T + 127) / 128;
+  if (mode == 1 || (mode == 0 && !fb_walks(bh, nt, sms))) {
     constexpr int SMEM = 6 * FB_TILE + 2 * FB_P + FB_MATH_WARPS * 2048 + 256;
     static PerDeviceOnce attr;
     if (attr.first_use_on_device()) {
@@ -951,6 +956,9 @@ extern "C" int ab_attn_bwd_schedule(int mode) {
   ab::g_attn_bwd_schedule = mode;
   return 0;
 }
+
+// For tests: whether schedule 0 walks `slices` (batch, head) slices of T keys on a GPU of `sms` SMs
+extern "C" int ab_attn_bwd_walks(int slices, int T, int sms) { return ab::fb_walks(slices, (T + 127) / 128, sms); }
 
 // For tests: what a drain warp of the walk does to the dQ places over `slices` slices of nt tiles, in its order; four
 // numbers each: what (0 store, 1 add, 2 read, 3 dQ out, 4 dV / dK out; all but reads are a bulk group), slice, query tile (of

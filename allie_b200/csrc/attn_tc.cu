@@ -898,10 +898,8 @@ static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int
     attr.mark_device();
   }
   dim3 grid((a.T + 127) / 128, a.H, a.B);
-  int dev = 0, sms = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (err != cudaSuccess) return (int)err;
+  int sms = 0;
+  if (const cudaError_t e = device_sms(&sms)) return (int)e;
   // Blocks that all fit at once start by themselves: taken over while the grid starts, an item would wait behind
   // another (8 x 256 x 4 heads with dropout, 64 items: 12.3 and 14.3 us).
   // Not in programmatic chains, as a precaution: when a grid whose blocks are taken over releases its dependents was

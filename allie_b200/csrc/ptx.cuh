@@ -28,6 +28,12 @@ struct PerDeviceOnce {
   void mark_device() { mask.fetch_or(bit(), std::memory_order_release); }
 };
 
+inline cudaError_t device_sms(int* n) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev);
+}
+
 // ---------------------------------------------------------------- status ---
 // Kernels report trouble through a device status word owned by the host
 // wrapper (never by trapping).  0 means success.

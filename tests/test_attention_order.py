@@ -1,4 +1,5 @@
-"""Order of the bulk operations on the dQ sums of the attention backward's walk (host replay, no GPU needed)."""
+"""The attention backward's walk: which launches take it, and the order of its bulk operations on the dQ sums (host
+rules and a replay, no GPU needed)."""
 import ctypes
 
 import pytest
@@ -37,3 +38,12 @@ def test_every_sum_waits_for_what_it_builds_on(nt):
             open_groups.append(tile if what in (STORE, ADD) else None)
     assert adds == slices * (nt - 1) * (nt - 2) // 2
     assert content == {tile: [slices] for tile in range(1, nt)}
+
+
+@pytest.mark.parametrize("slices,T,walks", [
+    (1, 128, 1), (4, 256, 1), (16, 128, 1), (16, 256, 1), (16, 384, 0), (20, 384, 0), (16, 512, 0), (32, 512, 0), (48, 512, 1),
+    (32, 640, 0), (48, 640, 1), (32, 1024, 0), (148, 1024, 1), (200, 1000, 1), (320, 128, 1), (1024, 512, 1),
+])
+def test_the_form_that_measured_faster(slices, T, walks):
+    """Sizes at which one form of the backward beats the other by more than 3 % on a GPU of 148 SMs."""
+    assert _lib.cuda().ab_attn_bwd_walks(slices, T, 148) == walks
