@@ -21,7 +21,6 @@ struct AttnArgs {
   // key / value cache [sequence][head][slots][hd] that a packed batch's keys and values also go to, or null
   __nv_bfloat16 *kc, *vc;
   int slots;
-  int take_over;            // forward: blocks take the place of those that have not started
   int* status;
 };
 

@@ -1,15 +1,16 @@
 // Causal flash attention on tcgen05 (forward; the backward kernels follow further down).
 //
-// An item is one 128-row query tile of one (batch, head).  Two CTAs share an SM and stay: a CTA that has asked for an
-// item's tiles takes the place of a block of the grid that has not started (`grid_take_block`) and goes on with
-// that one's item, so that loads run ahead of the items and blocks with short ones do more of them.  Per 128-row
-// key/value tile:
+// An item is one 128-row query tile of one (batch, head); two CTAs share an SM.  In launches of many items CTAs stay: one
+// that has asked for an item's tiles takes the place of a block of the grid that has not started
+// (`grid_take_block`) and goes on with that one's item, so that loads run ahead of the items and blocks with short
+// ones do more of them.  In launches of few, and in programmatic chains, a CTA does its own item and leaves (ONE;
+// `fwd_takes_over` has the rule).  Per 128-row key/value tile:
 //   warp 9              : S = Q K^T          -> TMEM (128 lanes = query rows, 128 fp32 columns)
 //   warps 0-7           : two threads per query row, 64 keys each: S in registers, maximum (exchanged
 //                         through shared memory), exponentials, dropout, P -> TMEM as packed bf16 (the A
 //                         operand of the second product)
 //   warp 9              : O += P V           -> TMEM
-//   warp 8              : items; TMA loads of Q and of K/V tiles through rings that go on from item to item
+//   warp 8              : items; TMA loads of Q and of K/V tiles (through rings that go on from item to item)
 // Q, K and V are read straight out of the packed [B*T, 3*d] QKV activation with 2-D TMA boxes
 // (64 columns x 128 rows), and O is written in the [B*T, d] layout the projection GEMM reads.
 // V is consumed MN-major (rows = keys), so no transposes exist anywhere.
@@ -29,6 +30,8 @@
 // 256 x 128 tokens 86 and 61, 64 x 512 x 16 117 and 97, with dropout (and with the generator's keys in uniform
 // registers and its bits by carry) 176 and 150, 37 x 328 x 12 with dropout 57 and 51; heads of 128, 256 prompts x 8
 // 121 and 90.  A tile takes 1650 clocks per SM, of which the exponential unit needs 1024.
+#include <algorithm>
+
 #include "attn_common.cuh"
 
 namespace ab {
@@ -82,7 +85,10 @@ struct KvMaps {
 template <>
 struct KvMaps<false> {};
 
-template <int HD, bool KV>
+// ONE: a block does its own item and leaves, without the ring of items, the hand-back of Q tiles and the end marker, which
+// cost a launch of few items half a microsecond (us so and with them: 64 items of 128 keys 5.6 and 6.1, 108 of three
+// key tiles 8.2 and 8.9).
+template <int HD, bool KV, bool ONE>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmO,
                 const __grid_constant__ KvMaps<KV> cache, const AttnArgs a) {
@@ -126,11 +132,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   const int warp = warp_number(), lane = threadIdx.x & 31;
   const int d_model = a.H * HD;
 
+  auto item_of = [&](uint3 block) {
+    FwdItem it;
+    it.qt = (a.T + AT_BM - 1) / AT_BM - 1 - static_cast<int>(block.x);       // heaviest tiles first
+    it.h = block.y; it.b = block.z;
+    // packed batch: sequence b owns rows [row0[b], row0[b + 1]) of the activation
+    it.first = a.row0 ? __ldg(a.row0 + it.b) : it.b * a.T;
+    it.T = a.row0 ? __ldg(a.row0 + it.b + 1) - it.first : a.T;
+    return it;
+  };
   // The set-up may run under the kernel before; the producer asks for the first item's rows as soon as that is done.
-  int2 first_rows = make_int2(0, 0);
+  FwdItem it = {};
   if (warp == FWD_TMA_WARP) {
     griddep_wait();
-    if (a.row0) first_rows = make_int2(__ldg(a.row0 + blockIdx.z), __ldg(a.row0 + blockIdx.z + 1));
+    it = item_of(make_uint3(blockIdx.x, blockIdx.y, blockIdx.z));
+    if (ONE && lane == 0) {
+      items[0] = it;
+      if (it.qt * AT_BM >= it.T) items[0].qt = -1;
+    }
   }
   if (warp == 0) {                           // a barrier per lane
     const uint64_t* bar = bars + lane;
@@ -157,9 +176,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 
   // n-th item of this CTA, for a whole warp (bounded; null when a wait ran out).  It stays until item_done.
   auto next_item = [&](int n) -> const volatile FwdItem* {
+    if (ONE) return &items[0];
     return mbar_wait_warp(&item_full[n % FWD_QUEUE], (n / FWD_QUEUE) & 1, abort_flag) ? &items[n % FWD_QUEUE] : nullptr;
   };
   auto item_done = [&](int n) {
+    if (ONE) return;
     __syncwarp();
     if (lane == 0) mbar_arrive(&item_empty[n % FWD_QUEUE]);
   };
@@ -203,29 +224,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       return true;
     };
     auto push = [&](const FwdItem& it) {
+      if (ONE) return true;
       const int s = n % FWD_QUEUE;
       if (!mbar_wait_warp(&item_empty[s], ((n / FWD_QUEUE) & 1) ^ 1, abort_flag)) return false;
       if (lead) { items[s] = it; mbar_arrive(&item_full[s]); }
       __syncwarp();
       return true;
     };
-    uint3 block = make_uint3(blockIdx.x, blockIdx.y, blockIdx.z);
-    int2 rows = first_rows;                      // of the block's sequence: first row, and the next one's
     for (int asked = 0; ok; ++asked) {
       // the place of a block that has not started yet; the answer is needed when this one's loads are out
-      if (a.take_over) {
+      if (!ONE) {
         mbar_expect_tx(grid_bar, 16, lead);
         grid_take_block(grid_next, grid_bar, lead);
       }
-      FwdItem it;
-      it.qt = (a.T + AT_BM - 1) / AT_BM - 1 - static_cast<int>(block.x);       // heaviest tiles first
-      it.h = block.y; it.b = block.z;
-      // packed batch: sequence b owns rows [row0[b], row0[b + 1]) of the activation
-      it.first = a.row0 ? rows.x : it.b * a.T;
-      it.T = a.row0 ? rows.y - rows.x : a.T;
       if (it.qt * AT_BM < it.T) {
         const int qs = n % STAGES;
-        if ((ok = mbar_wait_warp(&q_empty[qs], ((n / STAGES) & 1) ^ 1, abort_flag))) {
+        if (ONE || (ok = mbar_wait_warp(&q_empty[qs], ((n / STAGES) & 1) ^ 1, abort_flag))) {
           mbar_expect_tx(&q_full[qs], TILE_BYTES, lead);
 #pragma unroll
           for (int p = 0; p < PANELS; ++p)
@@ -259,15 +273,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           keep_slot = (static_cast<long long>(it.b) * a.H + it.h) * a.slots + it.qt * AT_BM;
         }
       }
-      if (!a.take_over) break;
+      if (ONE) break;
       // before the block leaves, too: the answer is written to its shared memory
       ok = __all_sync(0xffffffffu, mbar_wait_landed(grid_bar, asked & 1)) && ok;
+      uint3 block;
       if (!ok || !grid_taken_block(grid_next, block)) break;      // none left, and none may be asked for after that
-      if (a.row0) rows = make_int2(__ldg(a.row0 + block.z), __ldg(a.row0 + block.z + 1));
+      it = item_of(block);
       fence_proxy_async_smem();
       __syncwarp();
     }
-    if (ok) { FwdItem end = {-1, 0, 0, 0, 0}; ok = push(end); }
+    if (!ONE && ok) { FwdItem end = {-1, 0, 0, 0, 0}; ok = push(end); }
     if (KV && ok && keep >= 0) ok = store_kept();
     if (!ok) { *abort_flag = ST_TIMEOUT_EMPTY; if (lead) atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY); }
     // when a wait ran out, nobody has waited for these: they land before the block leaves
@@ -321,7 +336,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         umma_commit(pv_full, lead);
         if (C::P_IN_S && j + 1 < nkv && !(ok = issue_qk(t + 1))) break;
       }
-      if (!ok) break;
+      if (!ok || ONE) break;
       g += nkv;
     }
     if (!ok) { *abort_flag = ST_TIMEOUT_FULL; if (lead) atomicCAS(a.status, 0, ST_TIMEOUT_FULL); }
@@ -456,7 +471,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(p_full);                     // one arrival per warp
-          if (leaving) {                           // that has been read by now
+          if (!ONE && leaving) {                   // that has been read by now
             tma_store_wait_read<0>();
             mbar_arrive(&q_empty[qs ^ 1]);
           }
@@ -509,6 +524,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           tma_store_commit();
         }
       }
+      if (ONE) break;
       // The tile may be loaded again once the stores have read it: with two tiles that is said behind the first
       // keys of the next item, with one the next item's Q waits for it.
       if (STAGES == 1 || !leaving) {
@@ -871,8 +887,40 @@ namespace ab {
 int launch_attn_bwd_fused64(const CUtensorMap& tq, const CUtensorMap& td, const AttnBwdArgs& a,
                             int* launched, cudaStream_t stream);   // attn_bwd_fused.cu
 
+template <int HD, bool KV, bool ONE>
+static int launch_attn_fwd_kernel(const CUtensorMap& tm, const CUtensorMap& tmo, const KvMaps<KV>& cache, dim3 grid,
+                                  const AttnArgs& a, int dependent, cudaStream_t stream) {
+  constexpr int SMEM = FwdCfg<HD>::SMEM;
+  auto kern = attn_fwd_kernel<HD, KV, ONE>;
+  static PerDeviceOnce attr;
+  if (attr.first_use_on_device()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return (int)e;
+    // two CTAs per SM only fit when the SM is configured for its largest shared-memory carve-out
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return (int)e;
+    attr.mark_device();
+  }
+  if (dependent) return (int)launch_dependent(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, cache, a);
+  launch_chained(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, cache, a);
+  return (int)cudaGetLastError();
+}
+
+// Whether blocks are taken over.  An item is then tied to a CTA when that one starts on the item before, heaviest items
+// first, while the grid gives it to whoever is free; so it takes more rounds of the resident CTAs to pay the longer
+// the items are, and with heads of 128, whose one Q tile lets the next item's loads wait for the output, two at
+// least.  us, a block per item and taken over, from 150 sizes between 16 and 12000 items, heads of 64: 320 items of
+// 128 keys 10.0 and 8.7, 900 18.9 and 14.6; 320 of 512 keys 14.9 and 16.9, 600 21.5 and 21.8, 900 29.2 and 27.9,
+// 1500 46.6 and 40.5; 600 of 1000 keys 33.0 and 34.6, 900 44.0 and 44.0, 1500 68.4 and 63.2.  The rule's choice is
+// 0.5 % from the better of the two on average, 11 % at worst (450 items of two key tiles fill a wave and a
+// half).
+static bool fwd_takes_over(long long items, int tiles, int hd, int sms) {
+  return 2 * items > 2ll * sms * std::max(hd == 128 ? 4 : 2, tiles);
+}
+
 template <int HD, bool KV>
-static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int dependent,
+static int launch_attn_fwd(const CUtensorMap& tm, const AttnArgs& a, uint64_t rows, int dependent,
                            cudaStream_t stream) {
   // output map: boxes of 32 rows x 64 columns (half a math warp's rows at head_dim 128)
   CUtensorMap tmo;
@@ -885,42 +933,15 @@ static int launch_attn_fwd(const CUtensorMap& tm, AttnArgs a, uint64_t rows, int
     if ((rc = make_tmap_2d_sw(&cache.k, a.kc, slots, HD, HD, 32, 64, 2, 128)) != 0) return rc;
     if ((rc = make_tmap_2d_sw(&cache.v, a.vc, slots, HD, HD, 32, 64, 2, 128)) != 0) return rc;
   }
-  constexpr int SMEM = FwdCfg<HD>::SMEM;
-  auto kern = attn_fwd_kernel<HD, KV>;
-  static PerDeviceOnce attr;
-  if (attr.first_use_on_device()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    // two CTAs per SM only fit when the SM is configured for its largest shared-memory carve-out
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return (int)e;
-    attr.mark_device();
-  }
   dim3 grid((a.T + 127) / 128, a.H, a.B);
   int sms = 0;
   if (const cudaError_t e = device_sms(&sms)) return (int)e;
-  // Blocks that all fit at once start by themselves: taken over while the grid starts, an item would wait behind
-  // another (8 x 256 x 4 heads with dropout, 64 items: 12.3 and 14.3 us).
   // Not in programmatic chains, as a precaution: when a grid whose blocks are taken over releases its dependents was
   // not established, and a wait for it has no limit.  No fault was traced to it.
   const bool chain = dependent || g_pdl_chain;
-  a.take_over = !chain && static_cast<long long>(grid.x) * grid.y * grid.z > 2ll * sms;
-  if (dependent) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(FWD_THREADS);
-    cfg.dynamicSmemBytes = SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kern, tm, tmo, cache, a);
-  }
-  launch_chained(kern, grid, dim3(FWD_THREADS), SMEM, stream, tm, tmo, cache, a);
-  return (int)cudaGetLastError();
+  const bool take_over = !chain && fwd_takes_over(static_cast<long long>(grid.x) * grid.y * grid.z, grid.x, HD, sms);
+  return take_over ? launch_attn_fwd_kernel<HD, KV, false>(tm, tmo, cache, grid, a, dependent, stream)
+                   : launch_attn_fwd_kernel<HD, KV, true>(tm, tmo, cache, grid, a, dependent, stream);
 }
 
 template <int HD, int MODE>
@@ -974,6 +995,9 @@ int ab_attn_fwd(const void* qkv, void* out, float* lse, unsigned int* drop_mask,
   const uint64_t rows = (uint64_t)B * T;
   return hd == 64 ? launch_attn_fwd<64, false>(tm, a, rows, 0, stream) : launch_attn_fwd<128, false>(tm, a, rows, 0, stream);
 }
+
+// For tests: whether blocks are taken over in a launch of `items` items of up to `tiles` key tiles, outside chains
+int ab_attn_fwd_takes_over(int items, int tiles, int hd, int sms) { return ab::fwd_takes_over(items, tiles, hd, sms); }
 
 // The same over a packed batch without padding (inference: no dropout, no log-sum-exp): sequence b is
 // rows [row0[b], row0[b+1]) of qkv [rows, 3*H*hd]; T = longest sequence.  `dependent`: launched as a

@@ -363,7 +363,7 @@ def test_blocks_that_take_over_others(hd, H, lens):
         assert torch.allclose(alone.float(), ref, rtol=2e-2, atol=2e-2)
 
 
-@pytest.mark.parametrize("B,T,H,hd", [(24, 296, 8, 64), (40, 512, 4, 64), (24, 384, 5, 128)])
+@pytest.mark.parametrize("B,T,H,hd", [(24, 296, 8, 64), (40, 512, 4, 64), (24, 384, 5, 128), (64, 384, 5, 128)])
 def test_dropout_of_blocks_that_take_over_others(B, T, H, hd):
     """Keep bits of every item as the host draws them, and the outputs as fp32 gives them with these."""
     from allie_b200.ops import _lib

@@ -1,5 +1,5 @@
-"""The attention backward's walk: which launches take it, and the order of its bulk operations on the dQ sums (host
-rules and a replay, no GPU needed)."""
+"""The attention kernels' forms: which launches take which, and the order of the backward walk's bulk operations on the
+dQ sums (host rules and a replay, no GPU needed)."""
 import ctypes
 
 import pytest
@@ -47,3 +47,11 @@ def test_every_sum_waits_for_what_it_builds_on(nt):
 def test_the_form_that_measured_faster(slices, T, walks):
     """Sizes at which one form of the backward beats the other by more than 3 % on a GPU of 148 SMs."""
     assert _lib.cuda().ab_attn_bwd_walks(slices, T, 148) == walks
+
+
+@pytest.mark.parametrize("hd,tiles,least", [(64, 1, 297), (64, 2, 297), (64, 3, 445), (64, 4, 593), (64, 8, 1185),
+                                            (128, 1, 593), (128, 4, 593), (128, 8, 1185)])
+def test_launches_of_few_items_keep_a_block_per_item(hd, tiles, least):
+    rule = _lib.cuda().ab_attn_fwd_takes_over
+    assert rule(least, tiles, hd, 148) == 1
+    assert all(rule(n, tiles, hd, 148) == 0 for n in (1, 16, 296, least - 1))
