@@ -413,19 +413,24 @@ def test_gemm_asks_for_the_next_weights(M, nbytes):
     assert torch.equal(want, got)
 
 
-@pytest.mark.parametrize("M,N,K", [
-    (1280, 3840, 16384),            # 75 tiles: a round of whole ones and one cut into 32 parts
-    (1280, 1280, 16384),            # 25: two parts each, 24 pairs take what is left
-    (1280, 5120, 4104),             # 100: a round, 26 in two parts and the rest; a last step of 8
-    (1000, 1096, 8200), (2048, 1024, 12000), (520, 264, 40000), (1024, 4096, 8192),
+@pytest.mark.parametrize("M,N,K,shares", [
+    (1280, 3840, 16384, True),      # 75 tiles: a round of whole ones and one cut into 32 parts
+    (1280, 1280, 16384, True),      # 25: two parts each, 24 pairs take what is left
+    (1280, 5120, 4104, True),       # 100: a round, 26 in two parts and the rest; a last step of 8
+    (1000, 1096, 8200, False), (2048, 1024, 12000, True), (520, 264, 40000, True), (1024, 4096, 8192, False),
+    (1024, 4096, 32768, True),
 ])
-def test_weight_gradients_in_equal_shares(routes, M, N, K):
-    """Shares of the contraction that are no equal parts, edges of tiles, and sums handed over every few steps:
-    no accumulator sums up more than 32 steps of 64, of 16 products each addition, which are cut off at
+def test_weight_gradients_in_equal_shares(routes, M, N, K, shares):
+    """Shares of the contraction that are no equal parts, edges of tiles, and sums handed over every few steps.
+
+    Every element: no accumulator sums up more than 32 steps of 64, of 16 products each addition, which are cut off at
     2^-23 of a partial sum below 6 sqrt(2048); each of the K / 2048 parts adds one such error at most, the fp32
-    additions of the parts 2^-24 of 6 sqrt(K) each."""
+    additions of the parts 2^-24 of 6 sqrt(K) each.  That would hold for longer chains, too; their error in the
+    2-norm grows with the steps an accumulator sums up, 6.6e-8 each on the GPU (16 steps 9.9e-7, 32 2.1e-6, 64
+    4.4e-6, whole contractions here 1.2e-6 to 3.1e-5), so 1e-7 for each of the steps that there should be
+    tells a chain that was not cut, in all of these but the last but one, whose parts are shorter anyway."""
     from allie_b200.ops import _lib
-    from allie_b200.ops.gemm import gemm
+    from allie_b200.ops.gemm import gemm, num_sms, pick_k_splits
 
     torch.manual_seed(9)
     a, dy = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
@@ -434,9 +439,15 @@ def test_weight_gradients_in_equal_shares(routes, M, N, K):
     torch.cuda.synchronize()
     _lib.check_status()
     assert routes == [PAIR + ACCUM]
+    steps = -(-K // 64)
+    tiles = -(-M // 256) * -(-N // 256)
+    assert (_lib.cuda().ab_gemm_even_units(tiles, steps, num_sms() // 2, None, 0) > 0) == shares
+    want = a.double().t() @ dy.double()
+    off = dw.double() - 3.0 - want
     parts = K / 2048 + 1
     bound = parts * (128 * 2 ** -23 * 6 * 2048 ** 0.5 + 2 ** -24 * 6 * K ** 0.5) + 1e-5
-    assert ((dw.double() - 3.0 - a.double().t() @ dy.double()).abs() <= bound).all()
+    assert (off.abs() <= bound).all()
+    assert float(off.norm() / want.norm()) <= 1e-7 * min(32, -(-steps // pick_k_splits(M, N, K)))
 
 
 @pytest.mark.parametrize("M", [1, 20, 64, 65, 90, 128, 200])
