@@ -905,12 +905,19 @@ static GemmPlan gemm_plan(int a_mn, int b_mn, int M, int N, const AbGemmEpilogue
   else if (one_wave) p.kernel = tiles(64) <= max_ctas ? 64 : 128;
   else if (narrow)   p.kernel = 128;
   else               p.kernel = pair ? PLAN_PAIR : 256;
-  // 64 x 32 tiles where they fit a wave and 128 x 64 ones leave three quarters of the SMs idle: a step of the
-  // contraction takes 165 clocks (12 KB of operands) instead of 320 (24 KB, and MMAs of 128 rows that take 67 clocks
-  // whatever their columns).  Per launch of a chain, us, before and now: 90 x 1024 x 4096 14.7 and 10.7, 90 x 1024 x 1024
-  // with residual 6.5 and 5.4, 200 x 1024 x 4096 15.0 and 11.2.  With 64 x 64 tiles as well where 64 x 32 are too many
-  // (90 x 3072 x 1024 5.9 and 5.6) neighbouring launches of a pass no longer fit the SMs together, and their
-  // set-up waits: one game 1230 us as it was, 1250 so, 1180 without.
+  // 64 x 32 tiles wherever they fit a wave: a step of the contraction takes 165 clocks (12 KB of operands) instead of
+  // 320 (24 KB, and MMAs of 128 rows that take 67 clocks whatever their columns).  128 x 64 tiles leave three quarters of
+  // the SMs idle there with more than 64 rows, and half of them and more with up to 64.  Per launch of a chain, us, with
+  // 128 x 64 and with 64 x 32: 90 x 1024 x 4096 14.7 and 10.7, 90 x 1024 x 1024 with residual 6.5 and 5.4, 200 x 1024 x
+  // 4096 15.0 and 11.2; 1 row x 2048 x 1024 6.2 and 5.3, x 3072 6.8 and 6.2, x 4096 7.5 and 6.7, x 4608 7.9 and 7.1;
+  // 32 rows x 3072 x 1024 6.2 and 5.4, x 4096 7.0 and 6.0; 64 rows x 4096 x 1024 5.4 both, x 4608 5.6 both.  Whole
+  // passes of up to 64 rows, never, only where a quarter of the SMs would have 128 x 64 tiles, and as it is: one game
+  // of 20 tokens (24 layers of 1024) 1163, 1133 and 1058 us, of 768 columns 646, 656 and 638; 32 trees 6697, 6684 and
+  // 6310, of 1280 columns 4265, 4220 and 3868.
+  // Problems of one wave: 512 to 1100 rows x 256 to 576 columns x 64 to 4096, plain, GELU or residual, 0.72 to 0.98 of the time
+  // with 128 x 64 (512 x 256 x 1024 with residual and dropout 8.3 and 6.5).
+  // With 64 x 64 tiles as well where 64 x 32 are too many (90 x 3072 x 1024 5.9 and 5.6) neighbouring launches of a
+  // pass no longer fit the SMs together, and their set-up waits: one game 1230 us as it was, 1250 so, 1180 without.
   if (p.kernel == 64 && k_splits == 1 && !ep.m_limit && !ep.k_limit &&
       static_cast<long long>((M + 63) / 64) * ((N + 31) / 32) <= max_ctas)
     p.kernel = PLAN_64X32;
@@ -995,7 +1002,7 @@ extern "C" int ab_gemm_even_units(int tiles, int steps, int pairs, int* out, int
 }
 
 // What ab_gemm_bf16 would run for the same arguments, without running it: the columns of the single-CTA
-// kernel's tile (64 also where it takes half of that by half of the rows), or 512 + EpiKind on CTA pairs.  Passes beside the GEMM: see `passes`.
+// kernel's tile (32: of 64 rows, else of 128), or 512 + EpiKind on CTA pairs.  Passes beside the GEMM: see `passes`.
 extern "C" int ab_gemm_route(const void*, int a_mn, long long, const void*, int b_mn, long long, int M, int N, int,
                              const AbGemmEpilogue* ep, int k_splits, int max_ctas, int*, cudaStream_t) {
   using namespace ab;
@@ -1005,7 +1012,6 @@ extern "C" int ab_gemm_route(const void*, int a_mn, long long, const void*, int 
   GemmPlan plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas);
   if (plan.dot_pass) { e.act = 0; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
   if (plan.colsum_pass) { e.colsum = nullptr; plan = gemm_plan(a_mn, b_mn, M, N, e, k_splits, max_ctas); }
-  if (plan.kernel == PLAN_64X32) return 64;
   if (plan.kernel != PLAN_PAIR) return plan.kernel;
   GemmArgs g;
   g.ep = e;

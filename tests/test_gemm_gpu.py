@@ -11,7 +11,7 @@ ANY, BF16, GELU, GELU_GRAD, MUL, RESID, ACCUM, DOT = range(8)
 
 @pytest.fixture
 def routes(monkeypatch):
-    """What each GEMM of a test was dispatched to: 64, 128 or 256 (tile columns of the single-CTA kernel), or
+    """What each GEMM of a test was dispatched to: 32, 64, 128 or 256 (tile columns of the single-CTA kernel), or
     PAIR + kind."""
     from allie_b200.ops import _lib
 
@@ -215,7 +215,7 @@ def test_gemm_gelu_derivative_kept_in_aux():
 
 @pytest.mark.parametrize("drop_p", [0.0, 0.1])
 @pytest.mark.parametrize("M,N,K,route", [
-    (512, 256, 64, 64), (520, 264, 72, 64), (1100, 800, 256, 64),        # one wave of smaller tiles
+    (512, 256, 64, 32), (520, 264, 72, 32), (1100, 800, 256, 64),        # one wave of smaller tiles
     (2560, 1024, 64, PAIR + RESID),      # one tile per pair, both column groups of every warp
     (2440, 1032, 72, PAIR + RESID),      # rows past a tile, eight columns in the last tile
     (4744, 800, 256, PAIR + RESID),      # last column tile ends behind a warp's first group
@@ -370,7 +370,7 @@ def test_gemm_column_sums_and_head_products(routes, M, N, K):
         assert ((dot.double() - prod.sum(-1)).abs() <= 1e-6 + 64 * 2.0 ** -23 * prod.abs().sum(-1)).all()
 
 
-@pytest.mark.parametrize("M,N,K,route", [(4744, 808, 72, PAIR + RESID), (512, 256, 64, 64)])
+@pytest.mark.parametrize("M,N,K,route", [(4744, 808, 72, PAIR + RESID), (512, 256, 64, 32)])
 def test_gemm_residual_drops_non_finite_values(routes, M, N, K, route):
     """A dropped element adds nothing to the residual, whatever it was: Inf and NaN of one row of the product
     stay out of its dropped columns."""
@@ -451,14 +451,17 @@ def test_weight_gradients_in_equal_shares(routes, M, N, K, shares):
 
 
 @pytest.mark.parametrize("M", [1, 20, 64, 65, 90, 128, 200])
-@pytest.mark.parametrize("N,K", [(1024, 1024), (1024, 72), (264, 520), (40, 4096)])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (1024, 72), (264, 520), (40, 4096), (1048, 200), (4096, 136), (4736, 64),
+                                 (4744, 64)])
 @pytest.mark.parametrize("b_mn", [True, False])
-def test_gemm_small_tiles(M, N, K, b_mn):
-    """Tiles of 64 rows x 32 columns: edges, a contraction that ends inside a stage, all epilogues; and the same
-    bits as the tiles give that a larger batch of the same rows takes (contractions are not split)."""
+def test_gemm_small_tiles(routes, M, N, K, b_mn):
+    """Tiles of 64 rows x 32 columns, wherever they are at most as many as the SMs: edges, a contraction that ends inside
+    a stage, all epilogues; and the same bits as the tiles give that a larger batch of the same rows takes (contractions
+    are not split)."""
     from allie_b200.ops import _lib
-    from allie_b200.ops.gemm import gemm
+    from allie_b200.ops.gemm import gemm, num_sms
 
+    few = N >= 1024 and -(-M // 64) * -(-N // 32) <= num_sms()
     torch.manual_seed(10)
     a = torch.randn(M, K, device="cuda").bfloat16()
     w = (torch.randn(K, N, device="cuda") / K ** 0.5).bfloat16()
@@ -479,6 +482,7 @@ def test_gemm_small_tiles(M, N, K, b_mn):
     kept = dropped != resid
     assert M * N < 1000 or abs(kept.double().mean() - 0.75) < 0.03
     assert ((dropped - resid).double()[kept] - (ref / 0.75)[kept]).abs().max() < 1e-3
+    assert routes == [32 if few else 64 if N >= 1024 else 128] * 5
     more = torch.cat([a, torch.randn(3000, K, device="cuda").bfloat16()])
     assert torch.equal(gemm(more, b, b_mn=b_mn, bias=bias)[:M], plain)
     _lib.check_status()
