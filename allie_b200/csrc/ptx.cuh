@@ -201,8 +201,8 @@ __device__ __forceinline__ void griddep_enter() {
 
 // Host side: launches made through launch_chained carry the programmatic-stream-serialization
 // attribute while g_pdl_chain is set (only around the capture of a training micro-step; defined in
-// embed.cu).  Every kernel launched this way starts with griddep_enter() or, for the GEMMs, does
-// its set-up first and then waits.
+// embed.cu).  Every kernel launched this way starts with griddep_enter() or, as the GEMMs and the attention
+// forward, does its set-up first and then waits.
 extern int g_pdl_chain;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
